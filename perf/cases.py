@@ -295,3 +295,96 @@ def tolerance(case):
     if op == "decode_step":
         return {"rel": 3e-2}  # 0.4 to 1.3 % over one to four layers with a rounding to bf16 after every operator
     return {"rel": 1e-2}  # 1.7e-3 for one rounding to bf16, 2.3e-3 where the dequantised weights are rounded to bf16 too
+
+
+# ---------------------------------------------------------------------------
+# the same results in 64 bits, by torch alone
+# ---------------------------------------------------------------------------
+
+def _int4_weights(lin):
+    """(q - z) * s of one int4 linear: [K, N]."""
+    wq, z = lin["wq"], lin["z"]
+    q = torch.stack((wq & 15, wq >> 4), dim=1).reshape(-1, wq.shape[1]).double()
+    zero = torch.stack((z & 15, z >> 4), dim=2).reshape(z.shape[0], -1).double()
+    return (q - zero.repeat_interleave(128, 0)) * lin["s"].double().repeat_interleave(128, 0)
+
+
+_E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
+
+
+def _operator_dequantised(fmt, group, w):
+    """Weights of the operator API's formats: [N, K]."""
+    packed, n = w["packed"], w["packed"].shape[0]
+    if fmt == "affine4":
+        values = torch.stack([(packed >> (4 * j)) & 15 for j in range(8)], dim=2).reshape(n, -1).double()
+    elif fmt == "affine8":
+        values = packed.double()
+    elif fmt == "mxfp8":
+        values = packed.view(torch.float8_e4m3fn).float().double()
+    else:
+        table = torch.tensor(_E2M1 + tuple(-v for v in _E2M1), dtype=torch.float64, device=packed.device)
+        values = table[torch.stack((packed & 15, packed >> 4), dim=2).reshape(n, -1).long()]
+    if fmt.startswith("affine"):
+        scale = w["scales"].double()
+    elif fmt == "nvfp4":
+        scale = w["scales"].view(torch.float8_e4m3fn).float().double()
+    else:
+        scale = torch.exp2(w["scales"].double() - 127)
+    values = (values.reshape(n, -1, group) * scale[:, :, None]).reshape(n, -1)
+    return values + w["biases"].double().repeat_interleave(group, 1) if fmt.startswith("affine") else values
+
+
+def _exact_decode_step(state):
+    step = state["step"]
+    shape, model, b = step.shape, step.model, step.B
+    hq, hkv, hd = shape.n_heads, shape.n_kv_heads, shape.head_dim
+
+    def norm(h, w):
+        return h * torch.rsqrt(h.square().mean(-1, keepdim=True) + shape.eps) * w.double()
+
+    angle = step.pos.double()[:, None] * shape.rope_theta ** (-2.0 * torch.arange(hd // 2, device="cuda", dtype=torch.float64) / hd)
+    cos, sin = torch.cos(angle)[:, None], torch.sin(angle)[:, None]
+
+    def rope(t):
+        lo, hi = t[..., :hd // 2], t[..., hd // 2:]
+        return torch.cat((lo * cos - hi * sin, hi * cos + lo * sin), -1)
+
+    h = model["embed"][step.ids.long()].double()
+    keys, values = [], []
+    for layer, kc, vc in zip(model["layers"], state["kc"], state["vc"]):
+        n = norm(h, layer["attn_norm"])
+        q, k, v = ((n @ _int4_weights(layer[name])).reshape(b, -1, hd) for name in "qkv")
+        q, k = rope(q), rope(k)
+        keys.append(k.reshape(b, -1))
+        values.append(v.reshape(b, -1))
+        p = torch.softmax(q.reshape(b, hkv, hq // hkv, hd) @ torch.cat((kc.double(), k[:, :, None]), 2).mT / hd ** 0.5, -1)
+        h = h + (p @ torch.cat((vc.double(), v[:, :, None]), 2)).reshape(b, -1) @ _int4_weights(layer["o"])
+        n = norm(h, layer["mlp_norm"])
+        h = h + (torch.nn.functional.silu(n @ _int4_weights(layer["gate"])) * (n @ _int4_weights(layer["up"]))) @ _int4_weights(layer["down"])
+    return [norm(h, model["final_norm"]) @ model["lm_head"].double(), torch.stack(keys), torch.stack(values)]
+
+
+def exact(case, seed):
+    """What ``run`` returns for the inputs of ``prepare(case, seed)``, in 64 bits."""
+    if case["op"] == "program":  # its weights lie in the runtime's buffers: drawn again, in prepare's order
+        gen = _gen(seed)
+        x = {k: _normal((case["m"], k), gen, torch.bfloat16) for k in (case["d"], case["ffn"])}
+        outs = []
+        for k, n in linears(case):
+            w, s = _int8((k, n), gen), _uniform((n,), 0.005, 0.02, gen)
+            outs.append(((x[k].double() @ w.double()) * s.double()).cpu())
+        return outs
+    state = prepare(case, seed)
+    op = state["op"]
+    if op == "int8_f32":
+        return state["x"].double() @ state["w"].double() * state["s"].double()
+    if op == "int8_dot":
+        acc = state["a"].double() @ state["b"].double()
+        return acc if state["row"] is None else acc * state["row"].double()[:, None] * state["col"].double()
+    if op == "int8_layer":
+        return [x.double() @ w.double() * s.double() for x, w, s in state["lins"]]
+    if op == "int4_layer":
+        return [x.double() @ _int4_weights(lin) for x, lin in state["lins"]]
+    if op == "decode_step":
+        return _exact_decode_step(state)
+    return [x.double() @ _operator_dequantised(state["format"], state["group"], w).T for x, _, w in state["lins"]]
