@@ -17,6 +17,8 @@ int i8gemm_tcgen05(const void* a, const void* b, int32_t* acc, const float* row_
 int w8a16_tcgen05(const uint16_t* x, const int8_t* w, const float* scale, uint16_t* y, int64_t M,
                   int64_t N, int64_t K, int64_t ldy, uint32_t flags, uint32_t* signal, uint32_t* arrive,
                   cudaStream_t stream);
+int w8a16_decode(const uint16_t* x, const int8_t* w, const float* scale, uint16_t* y, int64_t M, int64_t N, int64_t K,
+                 int64_t ldy, uint32_t flags, cudaStream_t stream);
 
 namespace simple {
 
@@ -212,6 +214,9 @@ static int w8a16_entry(const char* name, const uint16_t* x, const int8_t* w, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool tma_ok = K > 0 && K % 8 == 0 && N % 16 == 0 && ldy % 2 == 0 && aligned(x, 16) &&
                       aligned(w, 16) && aligned(y, 4);
+  // few rows, results that stay on this GPU: the HBM-bound kernel
+  if (tma_ok && M <= 32 && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
+    return w8a16_decode(x, w, scale, y, M, N, K, ldy, flags, s);
   if (tma_ok && M * N >= 128 * 128 && !force_simple())
     return w8a16_tcgen05(x, w, scale, y, M, N, K, ldy, flags, signal, arrive, s);
   QMM_REQUIRE(!(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr, QMM_ERR_UNSUPPORTED,

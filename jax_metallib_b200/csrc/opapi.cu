@@ -14,7 +14,7 @@
 // These CUDA-core kernels take any M and f32 or f16 activations.  Decode-sized
 // f16 problems (M <= 16) go to the tensor-core kernels instead: the TMA-ring
 // kernels of opapi_tc.cu where the shape allows, else affine_tc_kernel below.
-#include "common.cuh"
+#include "opapi_decode.cuh"
 
 namespace qmm {
 
@@ -27,24 +27,15 @@ bool mx_ring_covers(int64_t M, int64_t N, int64_t K, int mode, int dtype, const 
 int mx_ring_launch(int mode, const void* x, const void* w, const void* scales, void* y, int64_t M, int64_t N, int64_t K,
                    void* stream);
 
+// the tcgen05 GEMM: any M, f16 or f32 activations
+bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, const void* x, const void* w, const void* y);
+int opgemm_launch(int fmt, const void* x, const void* w, const void* scales, const float* biases, void* y, int64_t M, int64_t N,
+                  int64_t K, int64_t gs, int f32, void* stream);
+
 namespace opapi {
 
 constexpr int kWarpsPerBlock = 4;
 constexpr int RM = 8;  // activation rows per pass
-
-__device__ __constant__ float kE2M1[16] = {0.0f,  0.5f,  1.0f,  1.5f,  2.0f,  3.0f,  4.0f,  6.0f,
-                                           -0.0f, -0.5f, -1.0f, -1.5f, -2.0f, -3.0f, -4.0f, -6.0f};
-
-__device__ __forceinline__ float decode_e4m3(uint32_t b) {
-  if ((b & 127u) == 127u) return __uint_as_float(0x7FC00000u);
-  const __half h = __ushort_as_half(static_cast<unsigned short>((b & 127u) << 7));
-  const float v = __half2float(h) * 256.0f;
-  return (b & 128u) ? -v : v;
-}
-__device__ __forceinline__ float decode_e8m0(uint32_t b) {
-  if (b == 0xFFu) return __uint_as_float(0x7FC00000u);
-  return __uint_as_float(b == 0 ? 0x00400000u : (b << 23));
-}
 
 template <typename T>
 __device__ __forceinline__ void load8(const T* p, float (&v)[8]);
@@ -68,55 +59,6 @@ __device__ __forceinline__ void load8<__half>(const __half* p, float (&v)[8]) {
 }
 __device__ __forceinline__ void store1(float* p, float v) { *p = v; }
 __device__ __forceinline__ void store1(__half* p, float v) { *p = __float2half_rn(v); }
-
-// Decoders: eight dequantised weights for column n, k = k8 .. k8+7.
-struct Affine4 {
-  const uint32_t* w; const float* s; const float* b; int K; int gs;
-  __device__ __forceinline__ void operator()(int n, int k8, float (&o)[8]) const {
-    const uint32_t word = __ldg(w + static_cast<size_t>(n) * (K / 8) + k8 / 8);
-    const int g = k8 / gs;
-    const float sc = __ldg(s + static_cast<size_t>(n) * (K / gs) + g);
-    const float bi = __ldg(b + static_cast<size_t>(n) * (K / gs) + g);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = fmaf(sc, static_cast<float>((word >> (4 * j)) & 0xFu), bi);
-  }
-};
-struct Affine8 {
-  const uint8_t* w; const float* s; const float* b; int K; int gs;
-  __device__ __forceinline__ void operator()(int n, int k8, float (&o)[8]) const {
-    const uint2 words = __ldg(reinterpret_cast<const uint2*>(w + static_cast<size_t>(n) * K + k8));
-    const int g = k8 / gs;
-    const float sc = __ldg(s + static_cast<size_t>(n) * (K / gs) + g);
-    const float bi = __ldg(b + static_cast<size_t>(n) * (K / gs) + g);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      o[j] = fmaf(sc, static_cast<float>((words.x >> (8 * j)) & 0xFFu), bi);
-      o[4 + j] = fmaf(sc, static_cast<float>((words.y >> (8 * j)) & 0xFFu), bi);
-    }
-  }
-};
-template <int MODE>  // 0 mxfp4 (group 32, e8m0), 1 mxfp8 (group 32, e8m0), 2 nvfp4 (group 16, e4m3)
-struct Mx {
-  const uint8_t* w; const uint8_t* s; int K;
-  __device__ __forceinline__ void operator()(int n, int k8, float (&o)[8]) const {
-    constexpr int gs = (MODE == 2) ? 16 : 32;
-    const uint32_t sb = __ldg(s + static_cast<size_t>(n) * (K / gs) + k8 / gs);
-    const float sc = (MODE == 2) ? decode_e4m3(sb) : decode_e8m0(sb);
-    if (MODE == 1) {
-      const uint2 words = __ldg(reinterpret_cast<const uint2*>(w + static_cast<size_t>(n) * K + k8));
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        o[j] = sc * decode_e4m3((words.x >> (8 * j)) & 0xFFu);
-        o[4 + j] = sc * decode_e4m3((words.y >> (8 * j)) & 0xFFu);
-      }
-    } else {
-      const uint32_t word =
-          __ldg(reinterpret_cast<const uint32_t*>(w + static_cast<size_t>(n) * (K / 2) + k8 / 2));
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = sc * kE2M1[(word >> (4 * j)) & 0xFu];
-    }
-  }
-};
 
 template <typename T, typename Dec>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
@@ -606,6 +548,8 @@ int qmm_affine_matmul(const void* x, const void* w_packed, const float* scales, 
     return affine_ring_launch(bits, x, w_packed, scales, biases, y, M, N, K, group_size, stream);
   if (tcq::covers(M, N, K, bits, group_size, dtype, x, w_packed))
     return tcq::launch(bits, x, w_packed, scales, biases, y, M, N, K, group_size, stream);
+  if (opgemm_covers(M, N, K, bits == 4 ? 0 : 1, group_size, x, w_packed, y))
+    return opgemm_launch(bits == 4 ? 0 : 1, x, w_packed, scales, biases, y, M, N, K, group_size, dtype == QMM_F32, stream);
   // rows of 16-byte words: the vectorised kernel
   if (aligned(w_packed, 16) && K % (bits == 4 ? 32 : 16) == 0) {
     if (bits == 4) {
@@ -648,6 +592,8 @@ int qmm_mx_matmul(const void* x, const uint8_t* w_packed, const uint8_t* scales,
   static_assert(QMM_MXFP4 == 0 && QMM_MXFP8 == 1 && QMM_NVFP4 == 2, "mode numbering shared with the tensor-core kernel");
   if (mx_ring_covers(M, N, K, mode, dtype, x, w_packed, scales))   // decode-sized f16 problems: the tensor-core kernel
     return mx_ring_launch(mode, x, w_packed, scales, y, M, N, K, stream);
+  if (opgemm_covers(M, N, K, 2 + mode, gs, x, w_packed, y))
+    return opgemm_launch(2 + mode, x, w_packed, scales, nullptr, y, M, N, K, gs, dtype == QMM_F32, stream);
   if (aligned(w_packed, 16) && K % 32 == 0) {  // rows of 16-byte words: the vectorised kernel
     if (mode == QMM_MXFP4) {
       VMx<0> d{w_packed, scales, k};

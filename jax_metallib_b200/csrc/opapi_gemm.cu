@@ -1,0 +1,751 @@
+// Operator-API matmuls (weights [N, K], K contiguous) on the 5th-generation tensor cores: any number of rows,
+// f16 or f32 activations, all five weight formats.
+//
+//   y[m,n] = sum over groups g of  s[n,g] * sum_{k in g} x[m,k] c[n,k]  (+ b[n,g] * sum_{k in g} x[m,k])
+//
+// The weights go to tcgen05.mma as their bare codes c (a centred integer, or the e2m1 / e4m3 element), which
+// both 16-bit types hold exactly: f16 against f16 activations, bf16 against f32 activations, which are cut into
+// three bf16 terms that add up to all 24 bits.  Every product is therefore exact.  The accumulator of one unit of
+// k (a scale group of up to 128 k) is read back from TMEM and multiplied by the group's f32 scale into f32
+// registers, so that scales and biases stay in 32 bits and the tensor core adds up no more than 128 k before a
+// correctly rounded f32 addition takes over.  nvfp4, whose groups of 16 would be too short for that, multiplies
+// its elements by their e4m3 scale first: 2 + 4 significant bits, exact as well.
+//
+// A CTA computes 128 columns (the MMA's 128 rows: a lane of the accumulator is a column, so a scale is one
+// register) x BM rows over a slice of K; the CTAs of a cluster share an output tile and add their slices over
+// distributed shared memory in a fixed order.  Warps: a TMA producer (raw weights in boxes of 128 rows x 128
+// bytes, activations), an MMA issuer, eight workers that turn raw codes into the swizzled operand (and f32
+// activations into their three terms, and sum the activations of a unit for the biases) and four or eight
+// promoters that drain the accumulators.
+//
+// What the split cannot represent takes an exact path: a unit whose activations are not finite (0 * inf of a
+// centred code is not what scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
+// the promoters from global memory with the arithmetic of the CUDA-core kernels.
+#include <cooperative_groups.h>
+
+#include "opapi_decode.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace qmm {
+namespace opg {
+
+enum { kAffine4 = 0, kAffine8 = 1, kMxfp4 = 2, kMxfp8 = 3, kNvfp4 = 4 };
+
+constexpr int BN = 128;               // output columns per CTA
+constexpr int BK = 64;                // k per operand stage: one 128-byte row of 16-bit values
+constexpr int kWorkerWarps = 8;
+constexpr int kRawBox = BN * 128;     // 16 KB of raw weights
+constexpr int kABytes = BN * BK * 2;  // 16 KB
+constexpr int kXSlots = 4;            // f16 activations: operand tiles straight from TMA
+constexpr int kAccBufs = 4;           // accumulators between the tensor core and the promoters
+constexpr int kInfo = 16;             // units whose activation sums and flags are kept
+constexpr int kConsumed = 12;         // a multiple of the operand ring (2 or 3) and of kXSlots
+constexpr int kMaxCluster = 8;
+
+template <int FMT, bool XF32, int BM>
+struct Cfg {
+  static constexpr int kBits = (FMT == kAffine8 || FMT == kMxfp8) ? 8 : 4;
+  static constexpr bool kBias = FMT == kAffine4 || FMT == kAffine8;
+  static constexpr bool kUnitInfo = kBias || XF32;          // sums and / or flags travel with a unit
+  static constexpr int kTerms = XF32 ? 3 : 1;
+  static constexpr int kBoxK = 128 * 8 / kBits;             // k per raw box
+  static constexpr int kStagesPerBox = kBoxK / BK;          // 4 or 2
+  static constexpr int kXTile = BM * BK * 2;                // one 16-bit operand tile of activations
+  static constexpr int kXRaw = BM * BK * 4;                 // raw f32 activations of a stage
+  static constexpr int kOps = BM == 32 ? 2 : 3;             // operand stages
+  static constexpr int kOpBytes = kABytes + (XF32 ? 3 * kXTile : 0);
+  static constexpr int kXRing = XF32 ? (BM == 32 ? 2 : 3) : kXSlots;
+  static constexpr int kXBytes = XF32 ? kXRaw : kXTile;
+  static constexpr int kRawBoxes = BM == 32 ? (XF32 ? 2 : 3) : 3;
+  static constexpr int kOffX = kOps * kOpBytes;
+  static constexpr int kOffRaw = kOffX + kXRing * kXBytes;
+  static constexpr int kOffInfo = kOffRaw + kRawBoxes * kRawBox;
+  static constexpr int kOffFlags = kOffInfo + kInfo * BM * 4;
+  static constexpr int kOffBar = kOffFlags + kInfo * 8;
+  static constexpr int kSmem = kOffBar + 512 + 1024;
+  static constexpr int kPromoters = BM == 32 ? 4 : 8;
+  static constexpr int kThreads = (2 + kWorkerWarps + kPromoters) * 32;
+  static constexpr int kMinBlocks = BM == 32 ? 2 : 1;
+  static constexpr int kCols = BM * 4 / kPromoters;         // accumulator columns per promoter: 32, 32 or 64
+  static_assert(BM * BN * 4 <= kOffInfo, "the result tile reuses the rings");
+  static_assert(kSmem * kMinBlocks <= 227 * 1024, "shared memory");
+};
+
+struct Args {
+  const void* x;
+  const uint8_t* w;
+  const void* scales;
+  const float* biases;
+  void* y;
+  int M, N, K, gs, pu;        // pu: k per unit (32, 64 or 128)
+  int blocks, block_k;        // K in blocks of the slice granularity
+  uint32_t idesc;
+  int* status;
+};
+
+__device__ __forceinline__ uint32_t lop_and_or(uint32_t a, uint32_t m, uint32_t o) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(m), "r"(o));
+  return r;
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if (BF16) asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if (BF16) asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ void e2m1_to_f16(uint32_t w, uint32_t (&r)[4]) {
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\tmov.b32 {b0, b1, b2, b3}, %4;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %0, b0;\n\tcvt.rn.f16x2.e2m1x2 %1, b1;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %2, b2;\n\tcvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+      : "r"(w));
+}
+__device__ __forceinline__ void e4m3_to_f16(uint32_t w, uint32_t& p01, uint32_t& p23) {
+  asm("{\n\t.reg .b16 h0, h1;\n\tmov.b32 {h0, h1}, %2;\n\t"
+      "cvt.rn.f16x2.e4m3x2 %0, h0;\n\tcvt.rn.f16x2.e4m3x2 %1, h1;\n\t}"
+      : "=r"(p01), "=r"(p23)
+      : "r"(w));
+}
+__device__ __forceinline__ uint32_t f16x2_to_bf16x2(uint32_t h) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+  return dev::pack_bf16x2(f.x, f.y);
+}
+
+// Eight codes of k .. k+7 -> eight 16-bit operand values in k order.  For 4-bit formats `lo` holds all eight.
+//   integers:  128 + q or 1024 + q by OR-ing the code into a constant's mantissa, minus 128 + 8 (4-bit) etc.:
+//              the centred q - 8 or q - 128, exact
+//   e2m1:      cvt to f16; for bf16 the code's exponent and mantissa are moved into place (worth 2^-126 of the
+//              element) and multiplied by 2^126
+//   e4m3:      cvt to f16, then to bf16 (4 significant bits: exact)
+template <int FMT, bool BF16>
+__device__ __forceinline__ uint4 convert8(uint32_t lo, uint32_t hi, uint32_t scale2) {
+  uint32_t r[4];
+  if (FMT == kAffine8) {
+    if (BF16) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t t = __byte_perm(i < 2 ? lo : hi, 0u, (i & 1) ? 0x4342 : 0x4140);
+        // 128 + (q & 127), plus -128 (q >= 128) or -256
+        const uint32_t a = lop_and_or(t, 0x007F007Fu, 0x43004300u);
+        const uint32_t c = lop_and_or(~t, 0x00800080u, 0xC300C300u);
+        asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r[i]) : "r"(a), "r"(c));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t t = __byte_perm(i < 2 ? lo : hi, 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
+        r[i] = sub2<false>(t, 0x64806480u);  // 1024 + q - 1152
+      }
+    }
+  } else if (FMT == kMxfp8) {
+    e4m3_to_f16(lo, r[0], r[1]);
+    e4m3_to_f16(hi, r[2], r[3]);
+    if (BF16) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = f16x2_to_bf16x2(r[i]);
+    }
+  } else if (!BF16 && (FMT == kMxfp4 || FMT == kNvfp4)) {
+    e2m1_to_f16(lo, r);
+  } else {
+    const uint32_t e = lo & 0x0F0F0F0Fu, o = (lo >> 4) & 0x0F0F0F0Fu;  // even and odd k
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      // byte 0 = e[i], byte 2 = o[i]; bytes 1 and 3 are e[0] and are masked off
+      const uint32_t p = __byte_perm(e, o, static_cast<uint32_t>(i) | (4u + i) << 8);
+      if (FMT == kAffine4) {
+        const uint32_t t = lop_and_or(p, 0x000F000Fu, BF16 ? 0x43004300u : 0x64006400u);
+        r[i] = sub2<BF16>(t, BF16 ? 0x43084308u : 0x64086408u);          // 128 + q - 136 or 1024 + q - 1032
+      } else {
+        const uint32_t mag = (p & 0x00070007u) << 6, sgn = (p & 0x00080008u) << 12;
+        r[i] = mul2<true>(mag | sgn, 0x7E807E80u);                       // times 2^126
+      }
+    }
+  }
+  if (FMT == kNvfp4) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = mul2<BF16>(r[i], scale2);
+  }
+  return make_uint4(r[0], r[1], r[2], r[3]);
+}
+
+// e4m3 scale byte -> (s, s) in f16 or bf16
+template <bool BF16>
+__device__ __forceinline__ uint32_t e4m3_pair(uint32_t b) {
+  uint32_t p, unused;
+  e4m3_to_f16(b | (b << 8), p, unused);
+  return BF16 ? f16x2_to_bf16x2(p) : p;
+}
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// sum_{k in [k0, k1)} x[m,k] * weight[n,k], as the CUDA-core kernels compute it
+template <int FMT, bool XF32>
+__device__ __noinline__ float exact_unit(const Args& a, int m, int n, int k0, int k1) {
+  float acc = 0.f;
+  for (int k = k0; k < k1; k += 8) {
+    float wv[8];
+    if constexpr (FMT == kAffine4) {
+      opapi::Affine4 d{reinterpret_cast<const uint32_t*>(a.w), static_cast<const float*>(a.scales), a.biases, a.K, a.gs};
+      d(n, k, wv);
+    } else if constexpr (FMT == kAffine8) {
+      opapi::Affine8 d{a.w, static_cast<const float*>(a.scales), a.biases, a.K, a.gs};
+      d(n, k, wv);
+    } else {
+      opapi::Mx<FMT - kMxfp4> d{a.w, static_cast<const uint8_t*>(a.scales), a.K};
+      d(n, k, wv);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const size_t i = static_cast<size_t>(m) * a.K + k + j;
+      const float xv = XF32 ? __ldg(static_cast<const float*>(a.x) + i) : __half2float(static_cast<const __half*>(a.x)[i]);
+      acc = fmaf(xv, wv[j], acc);
+    }
+  }
+  return acc;
+}
+
+template <int FMT, bool XF32, int BM>
+__global__ void __launch_bounds__(Cfg<FMT, XF32, BM>::kThreads, Cfg<FMT, XF32, BM>::kMinBlocks)
+opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ Args a) {
+  using C = Cfg<FMT, XF32, BM>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  float* xsum = reinterpret_cast<float*>(smem + C::kOffInfo);        // [kInfo][BM]
+  uint8_t* flags = smem + C::kOffFlags;                              // [kInfo][8], one byte per worker warp
+  uint64_t* wfull = reinterpret_cast<uint64_t*>(smem + C::kOffBar);  // raw weights landed
+  uint64_t* wempty = wfull + C::kRawBoxes;                           // raw weights read
+  uint64_t* xfull = wempty + C::kRawBoxes;                           // activations landed
+  uint64_t* xempty = xfull + C::kXRing;                              // raw f32 activations read (f32 only)
+  uint64_t* full = xempty + C::kXRing;                               // operand stage written
+  uint64_t* consumed = full + C::kOps;                               // the MMAs of a stage retired
+  uint64_t* tfull = consumed + kConsumed;                            // a unit's accumulator complete
+  uint64_t* tempty = tfull + kAccBufs;                               // and drained
+  uint64_t* ifull = tempty + kAccBufs;                               // sums and flags of a unit written
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ifull + kInfo);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int KS = gridDim.x, rank = blockIdx.x;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.z * BN;
+  const int k_begin = static_cast<int>(static_cast<long long>(a.blocks) * rank / KS) * a.block_k;
+  const int k_end = min(a.K, static_cast<int>(static_cast<long long>(a.blocks) * (rank + 1) / KS) * a.block_k);
+  const int stages = (k_end - k_begin + BK - 1) / BK;
+  const int units = (k_end - k_begin + a.pu - 1) / a.pu;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::kRawBoxes; ++i) { dev::mbar_init(&wfull[i], 1); dev::mbar_init(&wempty[i], kWorkerWarps); }
+    for (int i = 0; i < C::kXRing; ++i) { dev::mbar_init(&xfull[i], 1); dev::mbar_init(&xempty[i], kWorkerWarps); }
+    for (int i = 0; i < C::kOps; ++i) dev::mbar_init(&full[i], kWorkerWarps);
+    for (int i = 0; i < kConsumed; ++i) dev::mbar_init(&consumed[i], 1);
+    for (int i = 0; i < kAccBufs; ++i) { dev::mbar_init(&tfull[i], 1); dev::mbar_init(&tempty[i], C::kPromoters); }
+    for (int i = 0; i < kInfo; ++i) dev::mbar_init(&ifull[i], kWorkerWarps);
+    dev::fence_mbar_init();
+  }
+  if (warp == 1) {
+    dev::tmem_alloc(tmem_slot, kAccBufs * BM);
+    dev::tmem_relinquish();
+  }
+  dev::tc_fence_before();
+  __syncthreads();
+  dev::tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+  dev::pdl_wait();
+  dev::pdl_launch_dependents();
+
+  constexpr int kFirstPromoter = 2 + kWorkerWarps;
+  float* tile = reinterpret_cast<float*>(smem);   // [BM][BN] f32 partial results, once the rings are idle
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer ---------------------------
+    if (lane == 0) {
+      dev::tma_prefetch_desc(&wmap);
+      dev::tma_prefetch_desc(&xmap);
+      const int boxes = (stages + C::kStagesPerBox - 1) / C::kStagesPerBox;
+      int wi = 0, xi = 0;
+      // weights run ahead of the activations as far as their ring allows
+      while (wi < boxes || xi < stages) {
+        if (wi < boxes && wi < xi / C::kStagesPerBox + C::kRawBoxes) {
+          const int s = wi % C::kRawBoxes;
+          if (!dev::mbar_wait_relaxed(&wempty[s], ((wi / C::kRawBoxes) & 1) ^ 1, a.status, 90)) break;
+          dev::mbar_expect_tx(&wfull[s], kRawBox);
+          dev::tma_load_2d(smem + C::kOffRaw + s * kRawBox, &wmap, &wfull[s], k_begin * C::kBits / 8 + wi * 128, n0);
+          ++wi;
+          continue;
+        }
+        const int s = xi % C::kXRing;
+        if (XF32) {
+          if (!dev::mbar_wait_relaxed(&xempty[s], ((xi / C::kXRing) & 1) ^ 1, a.status, 91)) break;
+        } else if (xi >= C::kXRing) {
+          const int prev = xi - C::kXRing;
+          if (!dev::mbar_wait_relaxed(&consumed[prev % kConsumed], (prev / kConsumed) & 1, a.status, 91)) break;
+        }
+        dev::mbar_expect_tx(&xfull[s], C::kXBytes);
+        dev::tma_load_2d(smem + C::kOffX + s * C::kXBytes, &xmap, &xfull[s], k_begin + xi * BK, m0);
+        ++xi;
+      }
+      // every copy has landed before this CTA's shared memory is reused, whatever the other warps did
+      for (int i = wi > C::kRawBoxes ? wi - C::kRawBoxes : 0; i < wi; ++i)
+        if (!dev::mbar_wait_relaxed(&wfull[i % C::kRawBoxes], (i / C::kRawBoxes) & 1, a.status, 92)) break;
+      for (int i = xi > C::kXRing ? xi - C::kXRing : 0; i < xi; ++i)
+        if (!dev::mbar_wait_relaxed(&xfull[i % C::kXRing], (i / C::kXRing) & 1, a.status, 93)) break;
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer -----------------------------
+    if (lane == 0) {
+      constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // SBO, version, 128-byte swizzle
+      const uint32_t op_lo = ((dev::smem_u32(smem) >> 4) & 0x3FFF) | ((16u >> 4) << 16);
+      const uint32_t x_lo = ((dev::smem_u32(smem + C::kOffX) >> 4) & 0x3FFF) | ((16u >> 4) << 16);
+      const int steps_per_unit = a.pu / 16;
+      const int per = steps_per_unit < 4 ? steps_per_unit : 4;   // k-steps of a stage that belong to one unit
+      int u = 0, in_unit = 0;
+      bool ok = true;
+      for (int st = 0; ok && st < stages; ++st) {
+        const int s = st % C::kOps;
+        if (!dev::mbar_wait(&full[s], (st / C::kOps) & 1, a.status, 94)) break;
+        dev::tc_fence_after();
+        const uint32_t a_lo = op_lo + s * (C::kOpBytes >> 4);
+        const uint32_t b_lo = XF32 ? a_lo + (kABytes >> 4) : x_lo + (st % C::kXRing) * (C::kXTile >> 4);
+        for (int j0 = 0; j0 < 4 && u < units; j0 += per) {         // (the zero half of a last stage is skipped)
+          const int buf = u % kAccBufs;
+          if (in_unit == 0) {
+            if (!dev::mbar_wait(&tempty[buf], ((u / kAccBufs) & 1) ^ 1, a.status, 95)) { ok = false; break; }
+            dev::tc_fence_after();
+          }
+          const uint32_t d = tmem_base + buf * BM;
+          // the smallest terms first: the accumulator is still small when they are added
+#pragma unroll
+          for (int t = C::kTerms - 1; t >= 0; --t)
+            for (int j = j0; j < j0 + per; ++j)
+              dev::umma_f16_lh(d, a_lo + j * 2, kDescHi, b_lo + t * (C::kXTile >> 4) + j * 2, kDescHi, a.idesc,
+                               (in_unit != 0 || t != C::kTerms - 1 || j != j0) ? 1u : 0u);
+          in_unit += per;
+          if (in_unit == steps_per_unit || st == stages - 1) {
+            dev::tc_commit(&tfull[buf]);
+            in_unit = 0;
+            ++u;
+          }
+        }
+        if (ok) dev::tc_commit(&consumed[st % kConsumed]);
+      }
+    }
+    __syncwarp();
+  } else if (warp < kFirstPromoter) {
+    // ------------------------------ workers --------------------------------
+    const int ww = warp - 2, wt = threadIdx.x - 64;   // 0 .. 255
+    const int stages_per_unit = a.pu > BK ? a.pu / BK : 1;
+    const int units_per_stage = a.pu < BK ? BK / a.pu : 1;
+    uint32_t flag_carry = 0;
+    for (int st = 0; st < stages; ++st) {
+      const int op = st % C::kOps;
+      uint8_t* opA = smem + op * C::kOpBytes;
+      const int box = st / C::kStagesPerBox, sub = st % C::kStagesPerBox, rs = box % C::kRawBoxes;
+      const uint8_t* raw = smem + C::kOffRaw + rs * kRawBox;
+      // nvfp4: the two scales of this thread's 32 k, fetched before the wait for the weights
+      uint32_t nsc[2] = {0u, 0u};
+      if (FMT == kNvfp4) {
+        const int n = n0 + (wt >> 1), k = k_begin + st * BK + (wt & 1) * 32;
+        if (n < a.N && k < a.K) {
+          const uint8_t* sp = static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(n) * (a.K / 16) + k / 16;
+          nsc[0] = __ldg(sp);
+          nsc[1] = __ldg(sp + 1);
+        }
+      }
+      if (sub == 0 && !dev::mbar_wait_warp(&wfull[rs], (box / C::kRawBoxes) & 1, a.status, 96)) break;
+      uint4 v[2];
+      if (C::kBits == 4) {
+        const int row = wt >> 1, c = sub * 2 + (wt & 1);
+        v[0] = *reinterpret_cast<const uint4*>(raw + row * 128 + ((c ^ (row & 7)) << 4));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int row = (wt >> 2) + i * 64, c = sub * 4 + (wt & 3);
+          v[i] = *reinterpret_cast<const uint4*>(raw + row * 128 + ((c ^ (row & 7)) << 4));
+        }
+      }
+      if (sub == C::kStagesPerBox - 1 || st == stages - 1) {
+        __syncwarp();
+        if (lane == 0) dev::mbar_arrive(&wempty[rs]);
+      }
+      uint4 o[4];
+      if (C::kBits == 4) {
+        uint32_t sc[2] = {0u, 0u};
+        if (FMT == kNvfp4) { sc[0] = e4m3_pair<XF32>(nsc[0]); sc[1] = e4m3_pair<XF32>(nsc[1]); }
+        o[0] = convert8<FMT, XF32>(v[0].x, 0u, sc[0]);
+        o[1] = convert8<FMT, XF32>(v[0].y, 0u, sc[0]);
+        o[2] = convert8<FMT, XF32>(v[0].z, 0u, sc[1]);
+        o[3] = convert8<FMT, XF32>(v[0].w, 0u, sc[1]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          o[2 * i] = convert8<FMT, XF32>(v[i].x, v[i].y, 0u);
+          o[2 * i + 1] = convert8<FMT, XF32>(v[i].z, v[i].w, 0u);
+        }
+      }
+      if (st >= C::kOps) {   // the MMAs that read this operand stage before have retired
+        const int prev = st - C::kOps;
+        if (!dev::mbar_wait_warp(&consumed[prev % kConsumed], (prev / kConsumed) & 1, a.status, 97)) break;
+      }
+      if (C::kBits == 4) {
+        const int row = wt >> 1;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(opA + row * 128 + ((((wt & 1) * 4 + i) ^ (row & 7)) << 4)) = o[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = (wt >> 2) + (i >> 1) * 64;
+          *reinterpret_cast<uint4*>(opA + row * 128 + ((((wt & 3) * 2 + (i & 1)) ^ (row & 7)) << 4)) = o[i];
+        }
+      }
+      // ---- activations: eight lanes per row, eight k each
+      const int xs = st % C::kXRing;
+      if (!dev::mbar_wait_warp(&xfull[xs], (st / C::kXRing) & 1, a.status, 98)) break;
+      const int slot = (units_per_stage == 2 ? 2 * st : st / stages_per_unit) % kInfo;   // first unit of this stage
+      const bool first = st % stages_per_unit == 0;
+      const bool last = st % stages_per_unit == stages_per_unit - 1 || st == stages - 1;
+      if (C::kUnitInfo) {
+        const uint8_t* xt = smem + C::kOffX + xs * C::kXBytes;
+        uint32_t bad = 0;   // bit 0: first half of the stage, bit 1: second half
+#pragma unroll
+        for (int i = 0; i < BM / 32; ++i) {
+          const int row = (wt >> 3) + i * 32, j = wt & 7;
+          float f[8];
+          bool odd = false;
+          if (XF32) {
+            const float4 p = *reinterpret_cast<const float4*>(xt + row * 256 + j * 32);
+            const float4 q = *reinterpret_cast<const float4*>(xt + row * 256 + j * 32 + 16);
+            f[0] = p.x; f[1] = p.y; f[2] = p.z; f[3] = p.w;
+            f[4] = q.x; f[5] = q.y; f[6] = q.z; f[7] = q.w;
+            // x = hi + mid + lo: the top 8 bits, the next 8, the rest
+            uint32_t mi[8], lo[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const uint32_t b = __float_as_uint(f[e]);
+              const uint32_t mag = b & 0x7FFFFFFFu;
+              odd |= mag != 0u && mag - (27u << 23) >= (200u << 23);
+              const float r = f[e] - __uint_as_float(b & 0xFFFF0000u);
+              mi[e] = __float_as_uint(r);
+              lo[e] = __float_as_uint(r - __uint_as_float(mi[e] & 0xFFFF0000u));
+            }
+            uint8_t* xo = opA + kABytes + row * 128 + ((j ^ (row & 7)) << 4);
+            uint32_t h[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) h[e] = __byte_perm(__float_as_uint(f[2 * e]), __float_as_uint(f[2 * e + 1]), 0x7632);
+            *reinterpret_cast<uint4*>(xo) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(xo + C::kXTile) =
+                make_uint4(__byte_perm(mi[0], mi[1], 0x7632), __byte_perm(mi[2], mi[3], 0x7632),
+                           __byte_perm(mi[4], mi[5], 0x7632), __byte_perm(mi[6], mi[7], 0x7632));
+            *reinterpret_cast<uint4*>(xo + 2 * C::kXTile) =
+                make_uint4(__byte_perm(lo[0], lo[1], 0x7632), __byte_perm(lo[2], lo[3], 0x7632),
+                           __byte_perm(lo[4], lo[5], 0x7632), __byte_perm(lo[6], lo[7], 0x7632));
+          } else {
+            const uint4 p = *reinterpret_cast<const uint4*>(xt + row * 128 + ((j ^ (row & 7)) << 4));
+            const uint32_t h[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 q = __half22float2(*reinterpret_cast<const __half2*>(&h[e]));
+              f[2 * e] = q.x;
+              f[2 * e + 1] = q.y;
+            }
+          }
+          if (C::kBias) {
+            float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+            if (units_per_stage == 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 4);
+            if (!XF32) odd = !(fabsf(sum) < INFINITY);   // f16 sums cannot overflow: inf or NaN was among the values
+            if (units_per_stage == 2) {
+              if ((j & 3) == 0) xsum[((slot + (j >> 2)) % kInfo) * BM + row] = sum;
+            } else if (j == 0) {
+              float* d = xsum + slot * BM + row;
+              *d = first ? sum : *d + sum;
+            }
+          }
+          const uint32_t b = __ballot_sync(0xFFFFFFFFu, odd);
+          bad |= (b & 0x0F0F0F0Fu ? 1u : 0u) | (b & 0xF0F0F0F0u ? 2u : 0u);
+        }
+        if (units_per_stage == 2) {
+          if (lane < 2) flags[((slot + lane) % kInfo) * 8 + ww] = (bad >> lane) & 1;
+        } else {
+          flag_carry = first ? bad : (flag_carry | bad);
+          if (lane == 0) flags[slot * 8 + ww] = flag_carry != 0;
+        }
+        if (XF32) {
+          __syncwarp();
+          if (lane == 0) dev::mbar_arrive(&xempty[xs]);
+        }
+      }
+      dev::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) {
+        dev::mbar_arrive(&full[op]);
+        if (C::kUnitInfo) {
+          if (units_per_stage == 2) {
+            dev::mbar_arrive(&ifull[slot]);
+            dev::mbar_arrive(&ifull[(slot + 1) % kInfo]);
+          } else if (last) {
+            dev::mbar_arrive(&ifull[slot]);
+          }
+        }
+      }
+    }
+  } else {
+    // ------------------------------ promoters ------------------------------
+    const int q = warp & 3, half = (warp - kFirstPromoter) >> 2;
+    const int n = n0 + q * 32 + lane;
+    const int nc = min(n, a.N - 1);
+    const int c0 = half * C::kCols;
+    const int units_per_group = (FMT == kNvfp4) ? 1 : a.gs / a.pu;
+    const int u_base = k_begin / a.pu;
+    const int G = (FMT == kNvfp4) ? 1 : a.K / a.gs;
+    const int total_units = (a.K + a.pu - 1) / a.pu;
+    uint64_t acc[C::kCols / 2];
+#pragma unroll
+    for (int i = 0; i < C::kCols / 2; ++i) acc[i] = 0ull;
+    auto load_scale = [&](int u, float& s, float& b) {
+      s = 1.f;
+      b = 0.f;
+      const int uu = min(u_base + u, total_units - 1);
+      if (C::kBias) {
+        const size_t i = static_cast<size_t>(nc) * G + uu / units_per_group;
+        s = __ldg(static_cast<const float*>(a.scales) + i);
+        b = __ldg(a.biases + i);
+      } else if (FMT != kNvfp4) {
+        s = opapi::decode_e8m0(__ldg(static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(nc) * G + uu));
+      }
+    };
+    constexpr int kAhead = 4;   // scales are requested four units early
+    float sv[kAhead], bv[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) load_scale(i, sv[i], bv[i]);
+    bool ok = true;
+    for (int ub = 0; ok && ub < units; ub += kAhead) {
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int u = ub + i;
+        if (!ok || u >= units) break;
+        const int buf = u % kAccBufs, slot = u % kInfo;
+        const float s = sv[i];
+        // the code went in centred: scale * q + bias = scale * (q - 8) + (bias + 8 scale)
+        const float b = C::kBias ? fmaf(FMT == kAffine4 ? 8.f : 128.f, s, bv[i]) : 0.f;
+        load_scale(u + kAhead, sv[i], bv[i]);
+        bool exact = false;
+        if (C::kUnitInfo) {
+          if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) { ok = false; break; }
+          const uint2 fl = *reinterpret_cast<const uint2*>(flags + slot * 8);
+          exact = (fl.x | fl.y) != 0u;
+        }
+        if (!dev::mbar_wait_relaxed_warp(&tfull[buf], (u / kAccBufs) & 1, a.status, 100)) { ok = false; break; }
+        dev::tc_fence_after();
+        if (C::kUnitInfo && exact) {
+          const int k0 = k_begin + u * a.pu, k1 = min(a.K, k0 + a.pu);
+#pragma unroll 1
+          for (int c = 0; c < C::kCols; ++c) {
+            if (m0 + c0 + c >= a.M) break;
+            const float v = exact_unit<FMT, XF32>(a, m0 + c0 + c, nc, k0, k1);
+#pragma unroll
+            for (int e = 0; e < C::kCols / 2; ++e) {   // registers cannot be indexed
+              float v0, v1;
+              unpack2(acc[e], v0, v1);
+              if (c == 2 * e) v0 += v;
+              if (c == 2 * e + 1) v1 += v;
+              acc[e] = pack2(v0, v1);
+            }
+          }
+        } else {
+          const uint64_t s2 = pack2(s, s), b2 = pack2(b, b);
+#pragma unroll
+          for (int c = 0; c < C::kCols; c += 16) {   // 16 at a time: 64 accumulators leave no room for more
+            uint32_t r[16];
+            dev::tmem_ld_32x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0 + c, r);
+            dev::tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
+            if (C::kBias) {
+              const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(xsum + slot * BM + c0 + c);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const ulonglong2 t = xp[e];
+                fma2(acc[c / 2 + 2 * e], b2, t.x);
+                fma2(acc[c / 2 + 2 * e + 1], b2, t.y);
+              }
+            }
+          }
+        }
+        dev::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) dev::mbar_arrive(&tempty[buf]);
+      }
+    }
+    // ---- this slice's results, [row][column], into the idle rings (after every warp is done with them)
+    dev::tc_fence_before();
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < C::kCols; c += 2) {
+      float v0, v1;
+      unpack2(acc[c / 2], v0, v1);
+      tile[(c0 + c) * BN + q * 32 + lane] = v0;
+      tile[(c0 + c + 1) * BN + q * 32 + lane] = v1;
+    }
+  }
+  if (warp < kFirstPromoter) {
+    dev::tc_fence_before();
+    __syncthreads();
+  }
+  // TMEM goes back before this CTA waits for its cluster: a CTA never holds it while it depends on another one
+  if (warp == 1) {
+    dev::tc_fence_after();
+    dev::tmem_dealloc(tmem_base, kAccBufs * BM);
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  if (KS > 1) cluster.sync();
+  else __syncthreads();
+  const int rows = min(BM, a.M - m0);
+  const bool pairs = (a.N & 1) == 0;
+  for (int e = rank * C::kThreads + threadIdx.x; e < rows * (BN / 2); e += KS * C::kThreads) {
+    const int m = e / (BN / 2), c = (e % (BN / 2)) * 2, n = n0 + c;
+    if (n >= a.N) continue;
+    float2 v = make_float2(0.f, 0.f);
+    for (int r = 0; r < KS; ++r) {
+      const float2 p = *reinterpret_cast<const float2*>((KS > 1 ? cluster.map_shared_rank(tile, r) : tile) + m * BN + c);
+      v.x += p.x;
+      v.y += p.y;
+    }
+    const size_t i = static_cast<size_t>(m0 + m) * a.N + n;
+    if (XF32) {
+      float* y = static_cast<float*>(a.y) + i;
+      if (pairs) *reinterpret_cast<float2*>(y) = v;
+      else { y[0] = v.x; if (n + 1 < a.N) y[1] = v.y; }
+    } else {
+      __half* y = static_cast<__half*>(a.y) + i;
+      if (pairs) *reinterpret_cast<__half2*>(y) = __floats2half2_rn(v.x, v.y);
+      else { y[0] = __float2half_rn(v.x); if (n + 1 < a.N) y[1] = __float2half_rn(v.y); }
+    }
+  }
+  if (KS > 1) cluster.sync();   // peers keep their shared memory alive until it has been read
+}
+
+// CTAs that share an output tile: the fewest rounds of resident CTAs, a round costing its stages and about twelve
+// more for the prologue and the hand-over.
+static int cluster_size(int tiles, int blocks, int stages, int per_sm) {
+  const int slots = num_sms() * per_sm;
+  int best = 1;
+  long long best_cost = -1;
+  for (int ks = 1; ks <= kMaxCluster && ks <= blocks; ++ks) {
+    const long long waves = (static_cast<long long>(tiles) * ks + slots - 1) / slots;
+    const long long cost = waves * ((stages + ks - 1) / ks + 12);
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = ks; }
+  }
+  return best;
+}
+
+template <int FMT, bool XF32, int BM>
+static int launch(Args a, cudaStream_t stream) {
+  using C = Cfg<FMT, XF32, BM>;
+  CUtensorMap wmap, xmap;
+  const uint64_t row_bytes = static_cast<uint64_t>(a.K) * C::kBits / 8;
+  if (int rc = make_tensor_map_2d(&wmap, a.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)a.N, row_bytes, row_bytes, BN, 128,
+                                  CU_TENSOR_MAP_SWIZZLE_128B))
+    return rc;
+  if (int rc = make_tensor_map_2d(&xmap, a.x, XF32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                                  XF32 ? 4 : 2, (uint64_t)a.M, (uint64_t)a.K, (uint64_t)a.K * (XF32 ? 4 : 2), BM, BK,
+                                  XF32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B))
+    return rc;
+  static std::atomic<uint64_t> configured{0};
+  auto kern = opgemm_kernel<FMT, XF32, BM>;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), C::kSmem, configured)) return rc;
+  // a unit is a scale group or a part of one; slices of K begin on a raw box and on a unit
+  a.pu = FMT == kNvfp4 ? 128 : (a.gs % 128 == 0 ? 128 : (a.gs % 64 == 0 ? 64 : 32));
+  a.block_k = C::kBoxK;
+  a.blocks = (a.K + a.block_k - 1) / a.block_k;
+  a.idesc = dev::make_idesc(/*c=f32*/ 1, XF32 ? 1 : 0, XF32 ? 1 : 0, /*both K-major*/ 0, 0, BN, BM);
+  a.status = device_status_word();
+  const int nt = (a.N + BN - 1) / BN, mt = (a.M + BM - 1) / BM;
+  const int ks = cluster_size(nt * mt, a.blocks, (a.K + BK - 1) / BK, C::kMinBlocks);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ks, mt, nt);
+  cfg.blockDim = dim3(C::kThreads);
+  cfg.dynamicSmemBytes = C::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ks;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ks > 1 ? 2 : 1;
+  QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, a));
+  return QMM_OK;
+}
+
+template <int FMT>
+static int launch_fmt(const Args& a, int f32, cudaStream_t stream) {
+  if (f32) {
+    // a stage of 128 rows would need 64 KB for the three terms of the activations alone
+    return a.M <= 32 ? launch<FMT, true, 32>(a, stream) : launch<FMT, true, 64>(a, stream);
+  }
+  return a.M <= 32 ? launch<FMT, false, 32>(a, stream)
+                   : (a.M <= 64 ? launch<FMT, false, 64>(a, stream) : launch<FMT, false, 128>(a, stream));
+}
+
+}  // namespace opg
+
+// fmt: 0 affine 4-bit, 1 affine 8-bit, 2 mxfp4, 3 mxfp8, 4 nvfp4.  K and the group a multiple of 32 (nvfp4: K), weights
+// and activations 16-byte aligned, results aligned for pairs.
+bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, const void* x, const void* w, const void* y) {
+  using namespace opg;
+  if (K % 32 != 0 || (fmt <= kAffine8 && gs % 32 != 0)) return false;
+  if (!aligned(x, 16) || !aligned(w, 16) || !aligned(y, 8)) return false;
+  return (M + 31) / 32 <= 65535 && (N + BN - 1) / BN <= 65535;
+}
+
+int opgemm_launch(int fmt, const void* x, const void* w, const void* scales, const float* biases, void* y, int64_t M, int64_t N,
+                  int64_t K, int64_t gs, int f32, void* stream) {
+  using namespace opg;
+  if (int st = read_device_status())
+    return set_error(QMM_ERR_TIMEOUT, "quantized matmul: an earlier kernel gave up a wait (status 0x%x); "
+                     "call qmm_clear_device_status() after handling it", st);
+  Args a = {};
+  a.x = x;
+  a.w = static_cast<const uint8_t*>(w);
+  a.scales = scales;
+  a.biases = biases;
+  a.y = y;
+  a.M = static_cast<int>(M);
+  a.N = static_cast<int>(N);
+  a.K = static_cast<int>(K);
+  a.gs = static_cast<int>(gs);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (fmt) {
+    case kAffine4: return launch_fmt<kAffine4>(a, f32, st);
+    case kAffine8: return launch_fmt<kAffine8>(a, f32, st);
+    case kMxfp4: return launch_fmt<kMxfp4>(a, f32, st);
+    case kMxfp8: return launch_fmt<kMxfp8>(a, f32, st);
+    default: return launch_fmt<kNvfp4>(a, f32, st);
+  }
+}
+
+}  // namespace qmm

@@ -1,0 +1,343 @@
+// int8 per-channel weight-only matmul at few rows (sm_100a).
+//
+//   y[M,N] = bf16( (x[M,K] @ float(w[K,N])) * scale[N] )        x bf16, w int8 row-major, scale f32
+//
+// Bound by HBM: the weights (K*N bytes) are read once.  A cluster of KS CTAs owns blocks of 128
+// columns and splits K between its CTAs; every CTA runs a ring of TMA stages (64 k x 128 columns of
+// weights, 128-byte swizzle, and the same 64 k of the activations), fed by one warp and drained by
+// eight; the ring runs on over the cluster's column blocks, so that the loads of a block overlap the
+// hand-over of the one before.  A consumer warp owns 32 columns and half of a stage's k:
+// ldmatrix.trans hands it registers with two k of two neighbouring columns, which become two bf16
+// pairs by two logic operations and one exact add each, and mma.sync.m16n8k16 (f32 accumulate) takes
+// the weights as its 16-row operand and the activations as its 8-column operand, so that M = 1
+// wastes tensor work, which is free here, and not memory traffic.  tcgen05 has nothing to add at
+// these sizes: its operand would have to pass through shared memory a second time after the
+// conversion.
+//
+// The partial tiles of a cluster (KS CTAs x two k halves) meet in distributed shared memory, each
+// CTA adds its share of the elements in a fixed order: deterministic, no workspace, no atomics.
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace qmm {
+namespace w8d {
+
+constexpr int kCols = 128;           // columns per tile
+constexpr int kBK = 64;              // k per stage
+constexpr int kConsumerWarps = 8;    // 4 column groups of 32 x 2 halves of a stage's k
+constexpr int kThreads = (kConsumerWarps + 1) * 32;
+constexpr int kWBytes = kBK * kCols;
+constexpr int kMaxCluster = 8;
+
+template <int MT>
+struct Smem {
+  static constexpr int kX = MT * 8 * kBK * 2;              // activations of a stage: [MT * 8 rows][128 bytes]
+  static constexpr int kStage = kWBytes + kX;
+  static constexpr int kStages = MT == 1 ? 9 : (MT == 2 ? 7 : 6);
+  static constexpr int kPartBufs = MT <= 2 ? 2 : 1;        // tiles whose partial results may be in flight
+  static constexpr int kPart = MT * 8 * kCols * 4;         // partial tile of one k half
+  static constexpr int kOffPart = kStages * kStage;
+  static constexpr int kOffBar = kOffPart + kPartBufs * 2 * kPart;
+  static constexpr int kTotal = kOffBar + (2 * kStages + 2 * kPartBufs) * 8 + 1024;  // + alignment slack
+  static_assert(2 * kTotal <= 226 * 1024, "two CTAs per SM");
+};
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                               uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// The int8 values in bytes 0 and 2 of a register -> two bf16, exactly: 128 + (b & 127) plus -128 (b >= 0) or -256.
+__device__ __forceinline__ uint32_t bytes02_to_bf16x2(uint32_t t) {
+  uint32_t a, c, r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(a) : "r"(t), "r"(0x007F007Fu), "r"(0x43004300u));  // (t & m) | k
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(c) : "r"(t), "r"(0x00800080u), "r"(0xC300C300u));
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(c));
+  return r;
+}
+
+// Arrives (release, cluster scope) on the barrier at the same place of CTA `rank`'s shared memory.
+__device__ __forceinline__ void arrive_remote(uint64_t* bar, int rank) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(dev::smem_u32(bar)), "r"(rank)
+      : "memory");
+}
+__device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(dev::smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded, all lanes leave with the same answer.
+__device__ __forceinline__ bool wait_cluster_warp(uint64_t* bar, uint32_t parity, int* status, int tag) {
+  bool ok = try_wait_cluster(bar, parity);
+  if (!ok) {
+    const uint64_t t0 = dev::globaltimer_ns();
+    while (!(ok = try_wait_cluster(bar, parity)))
+      if (dev::globaltimer_ns() - t0 > dev::kWaitLimitNs) break;
+    if (!ok && status) atomicExch(status, (tag << 16) | QMM_ERR_TIMEOUT);
+  }
+  return __all_sync(0xFFFFFFFFu, ok);
+}
+
+template <int MT>
+__global__ void __launch_bounds__(kThreads, 2)
+w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+                    const float* __restrict__ scale, uint16_t* __restrict__ y, int M, int N, long long ldy, int stages_total,
+                    int independent, int* status) {
+  using L = Smem<MT>;
+  constexpr int S = L::kStages, PB = L::kPartBufs;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
+  uint64_t* empty = full + S;
+  uint64_t* ready = empty + S;       // every CTA of the cluster has written its partial tile
+  uint64_t* vacant = ready + PB;     // every CTA of the cluster has read this CTA's partial tile
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int KS = gridDim.x, rank = blockIdx.x;      // the cluster is the grid's x extent
+  const int blocks = (N + kCols - 1) / kCols;
+  const int it_begin = (stages_total * rank) / KS, it_end = (stages_total * (rank + 1)) / KS;
+  cg::cluster_group cluster = cg::this_cluster();
+
+  if (independent) dev::pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    dev::tma_prefetch_desc(&wmap);
+    dev::tma_prefetch_desc(&xmap);
+    for (int s = 0; s < S; ++s) {
+      dev::mbar_init(&full[s], 1);
+      dev::mbar_init(&empty[s], kConsumerWarps);
+    }
+    for (int b = 0; b < PB; ++b) {
+      dev::mbar_init(&ready[b], KS * kConsumerWarps);
+      dev::mbar_init(&vacant[b], KS * kConsumerWarps);
+    }
+    dev::fence_mbar_init();
+  }
+  cluster.sync();   // barriers of every CTA are initialised before a peer arrives on them
+  if (!independent) {
+    dev::pdl_wait();
+    dev::pdl_launch_dependents();
+  }
+
+  if (warp == kConsumerWarps) {
+    // ------------------------------ producer ------------------------------
+    if (lane == 0) {
+      const uint64_t policy = dev::policy_evict_first();
+      int n = 0;   // stages issued
+      bool ok = true;
+      for (int cb = blockIdx.y; ok && cb < blocks; cb += gridDim.y)
+        for (int it = it_begin; it < it_end; ++it, ++n) {
+          const int s = n % S;
+          if (!dev::mbar_wait_relaxed(&empty[s], ((n / S) & 1) ^ 1, status, 80)) { ok = false; break; }
+          uint8_t* st = smem + s * L::kStage;
+          dev::mbar_expect_tx(&full[s], L::kStage);   // rows and columns past the ends arrive as zeros
+          dev::tma_load_2d_hint(st, &wmap, &full[s], cb * kCols, it * kBK, policy);
+          dev::tma_load_2d(st + kWBytes, &xmap, &full[s], it * kBK, 0);
+        }
+      // no copy may still be on its way into this CTA's shared memory when it leaves, whatever the consumers did
+      for (int i = n > S ? n - S : 0; i < n; ++i)
+        if (!dev::mbar_wait_relaxed(&full[i % S], (i / S) & 1, status, 81)) break;
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------ consumers -----------------------------
+    const int cgrp = warp & 3, kh = warp >> 2;
+    const int g8 = lane >> 2, t4 = lane & 3;
+    // weights: lane l addresses k row 32 kh + l, 16-byte chunks 2 cgrp and 2 cgrp + 1 (XOR-swizzled by the row)
+    const uint32_t w_row = (kh * 32 + lane) * 128;
+    const uint32_t w_off0 = w_row + (((2 * cgrp) ^ (lane & 7)) << 4);
+    const uint32_t w_off1 = w_row + (((2 * cgrp + 1) ^ (lane & 7)) << 4);
+    // activations: lane l addresses row l & 7 of the 8-k chunk 4 kh + (l >> 3)
+    const uint32_t x_off = kWBytes + (lane & 7) * 128 + (((4 * kh + (lane >> 3)) ^ (lane & 7)) << 4);
+    const uint32_t ring = dev::smem_u32(smem);
+    int s = 0;
+    uint32_t ph = 0;
+    int tile = 0;
+    bool ok = true;
+    for (int cb = blockIdx.y; cb < blocks; cb += gridDim.y, ++tile) {
+      float acc[2][MT][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[j][mt][i] = 0.f;
+      for (int it = it_begin; it < it_end; ++it) {
+        if (!dev::mbar_wait_relaxed_warp(&full[s], ph, status, 82)) { ok = false; break; }
+        const uint32_t st = ring + s * L::kStage;
+        uint32_t wr[2][4], xr[MT][4];
+        ldmatrix_x4_trans(st + w_off0, wr[0]);
+        ldmatrix_x4_trans(st + w_off1, wr[1]);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) ldmatrix_x4(st + x_off + mt * 1024, xr[mt]);
+        __syncwarp();
+        if (lane == 0) dev::mbar_arrive(&empty[s]);   // the stage is in registers
+#pragma unroll
+        for (int q = 0; q < 2; ++q)   // 16 k each
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t a0 = bytes02_to_bf16x2(wr[j][2 * q]), a1 = bytes02_to_bf16x2(wr[j][2 * q] >> 8);
+            const uint32_t a2 = bytes02_to_bf16x2(wr[j][2 * q + 1]), a3 = bytes02_to_bf16x2(wr[j][2 * q + 1] >> 8);
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(acc[j][mt], a0, a1, a2, a3, xr[mt][2 * q], xr[mt][2 * q + 1]);
+          }
+        if (++s == S) { s = 0; ph ^= 1; }
+      }
+      if (!ok) break;
+      // ---- hand the partial tile over; CTA `rank` adds every KS-th run of column pairs, in CTA order
+      const int b = tile % PB;
+      if (tile >= PB && !wait_cluster_warp(&vacant[b], ((tile / PB) & 1) ^ 1, status, 83)) break;
+      float* part = reinterpret_cast<float*>(smem + L::kOffPart + b * 2 * L::kPart);
+      float* mine = part + kh * (L::kPart / 4);
+      // rows 2 t4, 2 t4 + 1 of columns 2 g8, 2 g8 + 1 of each 16-column block
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+            *reinterpret_cast<float2*>(mine + (mt * 8 + 2 * t4 + r) * kCols + cgrp * 32 + j * 16 + 2 * g8) =
+                make_float2(acc[j][mt][r], acc[j][mt][2 + r]);
+      __syncwarp();
+      if (lane < KS) arrive_remote(&ready[b], lane);
+      if (!wait_cluster_warp(&ready[b], (tile / PB) & 1, status, 84)) break;
+      const int col0 = cb * kCols;
+      for (int e = rank * (kConsumerWarps * 32) + threadIdx.x; e < M * (kCols / 2); e += KS * (kConsumerWarps * 32)) {
+        const int m = e / (kCols / 2), c = (e % (kCols / 2)) * 2;
+        if (col0 + c >= N) continue;
+        float2 v = make_float2(0.f, 0.f);
+        for (int r = 0; r < KS; ++r) {
+          const float* p = cluster.map_shared_rank(part, r) + m * kCols + c;
+          const float2 lo = *reinterpret_cast<const float2*>(p);
+          const float2 hi = *reinterpret_cast<const float2*>(p + L::kPart / 4);
+          v.x += lo.x + hi.x;
+          v.y += lo.y + hi.y;
+        }
+        const float2 sc = make_float2(__ldg(scale + col0 + c), __ldg(scale + col0 + c + 1));
+        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(m) * ldy + col0 + c) = dev::pack_bf16x2(v.x * sc.x, v.y * sc.y);
+      }
+      __syncwarp();
+      if (lane < KS) arrive_remote(&vacant[b], lane);
+    }
+  }
+  cluster.sync();   // peers keep their shared memory alive until it has been read
+}
+
+struct Grid {
+  int ks, clusters;
+};
+
+static void set_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int ks) {
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ks;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+}
+
+// Clusters of `ks` CTAs that the current device holds at once (asked once per device and size).
+template <int MT>
+static int resident_clusters(int ks) {
+  static std::atomic<int> cache[kMaxDevices][kMaxCluster + 1];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 2 * num_sms() / ks;
+  int n = cache[dev][ks].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(ks, 1024);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Smem<MT>::kTotal;
+  set_attrs(cfg, attr, ks);
+  if (cudaOccupancyMaxActiveClusters(&n, w8a16_decode_kernel<MT>, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = 2 * num_sms() / ks;
+  }
+  cache[dev][ks].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// Resident clusters walk the column blocks, so the launch takes as many rounds as the busiest cluster has blocks; a
+// round costs its stages and the hand-over of the partial tiles.
+template <int MT>
+static Grid choose_grid(int blocks, int stages_total) {
+  Grid best = {1, 1};
+  long long best_cost = -1;
+  for (int ks = 1; ks <= kMaxCluster && ks <= stages_total; ++ks) {
+    const int c = resident_clusters<MT>(ks);
+    const int rounds = (blocks + c - 1) / c;
+    const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + 2);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best.ks = ks;
+      best.clusters = blocks < c ? blocks : c;
+    }
+  }
+  return best;
+}
+
+template <int MT>
+static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const float* scale, uint16_t* y, int M, int N, long long ldy,
+                  int stages_total, int independent, cudaStream_t stream) {
+  using L = Smem<MT>;
+  static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
+  auto kern = w8a16_decode_kernel<MT>;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
+  const Grid g = choose_grid<MT>((N + kCols - 1) / kCols, stages_total);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(g.ks, g.clusters);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.stream = stream;
+  set_attrs(cfg, attr, g.ks);
+  QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, scale, y, M, N, ldy, stages_total, independent, device_status_word()));
+  return QMM_OK;
+}
+
+}  // namespace w8d
+
+// M <= 32; K % 8 == 0, N % 16 == 0, x and w 16-byte, y 4-byte aligned, ldy even (checked by the caller).
+int w8a16_decode(const uint16_t* x, const int8_t* w, const float* scale, uint16_t* y, int64_t M, int64_t N, int64_t K, int64_t ldy,
+                 uint32_t flags, cudaStream_t stream) {
+  using namespace w8d;
+  const int mt = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
+  CUtensorMap wmap, xmap;
+  if (int rc = make_tensor_map_2d(&wmap, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)N, kBK, kCols,
+                                  CU_TENSOR_MAP_SWIZZLE_128B))
+    return rc;
+  if (int rc = make_tensor_map_2d(&xmap, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)K * 2, mt * 8,
+                                  kBK, CU_TENSOR_MAP_SWIZZLE_128B))
+    return rc;
+  const int stages_total = static_cast<int>((K + kBK - 1) / kBK);
+  const int ind = (flags & QMM_GEMM_INDEPENDENT) ? 1 : 0;
+  const int m = static_cast<int>(M), n = static_cast<int>(N);
+  if (mt == 1) return launch<1>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
+  if (mt == 2) return launch<2>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
+  return launch<4>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
+}
+
+}  // namespace qmm
