@@ -382,10 +382,6 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
           v[i] = *reinterpret_cast<const uint4*>(raw + row * 128 + ((c ^ (row & 7)) << 4));
         }
       }
-      if (sub == C::kStagesPerBox - 1 || st == stages - 1) {
-        __syncwarp();
-        if (lane == 0) dev::mbar_arrive(&wempty[rs]);
-      }
       uint4 o[4];
       if (C::kBits == 4) {
         uint32_t sc[2] = {0u, 0u};
@@ -490,14 +486,14 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
           flag_carry = first ? bad : (flag_carry | bad);
           if (lane == 0) flags[slot * 8 + ww] = flag_carry != 0;
         }
-        if (XF32) {
-          __syncwarp();
-          if (lane == 0) dev::mbar_arrive(&xempty[xs]);
-        }
       }
       dev::fence_proxy_async();
       __syncwarp();
       if (lane == 0) {
+        // raw weights and activations go back after the fence that completed the stores made from them: an arrival
+        // right behind the loads let a refill overtake them
+        if (sub == C::kStagesPerBox - 1 || st == stages - 1) dev::mbar_arrive(&wempty[rs]);
+        if (XF32) dev::mbar_arrive(&xempty[xs]);
         dev::mbar_arrive(&full[op]);
         if (C::kUnitInfo) {
           if (units_per_stage == 2) {

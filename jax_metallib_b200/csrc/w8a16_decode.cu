@@ -8,14 +8,15 @@
 // eight; the ring runs on over the cluster's column blocks, so that the loads of a block overlap the
 // hand-over of the one before.  A consumer warp owns 32 columns and half of a stage's k:
 // ldmatrix.trans hands it registers with two k of two neighbouring columns, which become two bf16
-// pairs by two logic operations and one exact add each, and mma.sync.m16n8k16 (f32 accumulate) takes
+// pairs by a logic operation and an exact multiply-add each, and mma.sync.m16n8k16 (f32 accumulate) takes
 // the weights as its 16-row operand and the activations as its 8-column operand, so that M = 1
 // wastes tensor work, which is free here, and not memory traffic.  tcgen05 has nothing to add at
 // these sizes: its operand would have to pass through shared memory a second time after the
 // conversion.
 //
-// The partial tiles of a cluster (KS CTAs x two k halves) meet in distributed shared memory, each
-// CTA adds its share of the elements in a fixed order: deterministic, no workspace, no atomics.
+// The partial tiles of a cluster (KS CTAs x two k halves) meet in distributed shared memory; warps
+// of their own add each CTA's share of the elements in a fixed order while the consumers go on with
+// the next block: deterministic, no workspace, no atomics.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -28,7 +29,7 @@ namespace w8d {
 constexpr int kCols = 128;           // columns per tile
 constexpr int kBK = 64;              // k per stage
 constexpr int kConsumerWarps = 8;    // 4 column groups of 32 x 2 halves of a stage's k
-constexpr int kThreads = (kConsumerWarps + 1) * 32;
+constexpr int kFirstReducer = kConsumerWarps + 1;
 constexpr int kWBytes = kBK * kCols;
 constexpr int kMaxCluster = 8;
 
@@ -36,13 +37,17 @@ template <int MT>
 struct Smem {
   static constexpr int kX = MT * 8 * kBK * 2;              // activations of a stage: [MT * 8 rows][128 bytes]
   static constexpr int kStage = kWBytes + kX;
+  // resident CTAs: a warp's chain ldmatrix -> convert -> MMA is latency-bound, so as many as registers allow
+  static constexpr int kPerSm = 2;
+  static constexpr int kReducers = MT <= 2 ? 3 : 4;                     // warps that add the partial tiles
+  static constexpr int kThreads = (kFirstReducer + kReducers) * 32;
   static constexpr int kStages = MT == 1 ? 9 : (MT == 2 ? 7 : 6);
   static constexpr int kPartBufs = MT <= 2 ? 2 : 1;        // tiles whose partial results may be in flight
   static constexpr int kPart = MT * 8 * kCols * 4;         // partial tile of one k half
   static constexpr int kOffPart = kStages * kStage;
   static constexpr int kOffBar = kOffPart + kPartBufs * 2 * kPart;
   static constexpr int kTotal = kOffBar + (2 * kStages + 2 * kPartBufs) * 8 + 1024;  // + alignment slack
-  static_assert(2 * kTotal <= 226 * 1024, "two CTAs per SM");
+  static_assert(kPerSm * (kTotal + 1024) <= 228 * 1024, "resident CTAs");
 };
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
@@ -61,12 +66,13 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// The int8 values in bytes 0 and 2 of a register -> two bf16, exactly: 128 + (b & 127) plus -128 (b >= 0) or -256.
+// The int8 values v in bytes 0 and 2 of a register -> two bf16 v / 64, exactly, in two instructions: v + 128 in the
+// low byte of a bf16 reads as (v + 128) * 2^-133 (a subnormal up to 127, the first binade above), and one fused
+// multiply-add brings it to (v + 128) / 64 - 2.  The factor 64 goes back in with the channel's scale.
 __device__ __forceinline__ uint32_t bytes02_to_bf16x2(uint32_t t) {
-  uint32_t a, c, r;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(a) : "r"(t), "r"(0x007F007Fu), "r"(0x43004300u));  // (t & m) | k
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(c) : "r"(t), "r"(0x00800080u), "r"(0xC300C300u));
-  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(c));
+  uint32_t u, r;
+  asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(u) : "r"(t), "r"(0x00FF00FFu), "r"(0x00800080u));  // (t & m) ^ k
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(u), "r"(0x7F007F00u), "r"(0xC000C000u));   // * 2^127 - 2
   return r;
 }
 
@@ -101,7 +107,7 @@ __device__ __forceinline__ bool wait_cluster_warp(uint64_t* bar, uint32_t parity
 }
 
 template <int MT>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(Smem<MT>::kThreads, Smem<MT>::kPerSm)
 w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                     const float* __restrict__ scale, uint16_t* __restrict__ y, int M, int N, long long ldy, int stages_total,
                     int independent, int* status) {
@@ -129,7 +135,7 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     }
     for (int b = 0; b < PB; ++b) {
       dev::mbar_init(&ready[b], KS * kConsumerWarps);
-      dev::mbar_init(&vacant[b], KS * kConsumerWarps);
+      dev::mbar_init(&vacant[b], KS * L::kReducers);
     }
     dev::fence_mbar_init();
   }
@@ -159,7 +165,7 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         if (!dev::mbar_wait_relaxed(&full[i % S], (i / S) & 1, status, 81)) break;
     }
     __syncwarp();
-  } else {
+  } else if (warp < kConsumerWarps) {
     // ------------------------------ consumers -----------------------------
     const int cgrp = warp & 3, kh = warp >> 2;
     const int g8 = lane >> 2, t4 = lane & 3;
@@ -174,6 +180,7 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     uint32_t ph = 0;
     int tile = 0;
     bool ok = true;
+    const int never = stages_total < 0;   // false, but not to the compiler
     for (int cb = blockIdx.y; cb < blocks; cb += gridDim.y, ++tile) {
       float acc[2][MT][4];
 #pragma unroll
@@ -190,8 +197,6 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         ldmatrix_x4_trans(st + w_off1, wr[1]);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) ldmatrix_x4(st + x_off + mt * 1024, xr[mt]);
-        __syncwarp();
-        if (lane == 0) dev::mbar_arrive(&empty[s]);   // the stage is in registers
 #pragma unroll
         for (int q = 0; q < 2; ++q)   // 16 k each
 #pragma unroll
@@ -201,10 +206,18 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(acc[j][mt], a0, a1, a2, a3, xr[mt][2 * q], xr[mt][2 * q + 1]);
           }
+        // The slot goes back only when its bytes are in registers: an arrival that merely follows the loads in program
+        // order let the refill overtake the last of them (seen with remote shared-memory traffic on the same SM), so
+        // its address is made to depend on what they returned.
+        uint32_t dep = wr[0][3] ^ wr[1][3];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) dep ^= xr[mt][3];
+        // (lane 0's copy stands for the warp's: ldmatrix completes for all lanes at once)
+        if (lane == 0) dev::mbar_arrive(&empty[s] + ((dep == 0x7FC1FFC1u) & never));
         if (++s == S) { s = 0; ph ^= 1; }
       }
       if (!ok) break;
-      // ---- hand the partial tile over; CTA `rank` adds every KS-th run of column pairs, in CTA order
+      // ---- hand the partial tile over to the reducers of the cluster
       const int b = tile % PB;
       if (tile >= PB && !wait_cluster_warp(&vacant[b], ((tile / PB) & 1) ^ 1, status, 83)) break;
       float* part = reinterpret_cast<float*>(smem + L::kOffPart + b * 2 * L::kPart);
@@ -220,21 +233,39 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 make_float2(acc[j][mt][r], acc[j][mt][2 + r]);
       __syncwarp();
       if (lane < KS) arrive_remote(&ready[b], lane);
+    }
+  } else {
+    // ------------------------------ reducers ------------------------------
+    // CTA `rank` adds every KS-th run of column pairs, in CTA order
+    constexpr int kR = L::kReducers * 32;
+    const int tid = threadIdx.x - kFirstReducer * 32;
+    int tile = 0;
+    for (int cb = blockIdx.y; cb < blocks; cb += gridDim.y, ++tile) {
+      const int b = tile % PB;
+      const float* part = reinterpret_cast<const float*>(smem + L::kOffPart + b * 2 * L::kPart);
       if (!wait_cluster_warp(&ready[b], (tile / PB) & 1, status, 84)) break;
       const int col0 = cb * kCols;
-      for (int e = rank * (kConsumerWarps * 32) + threadIdx.x; e < M * (kCols / 2); e += KS * (kConsumerWarps * 32)) {
+      for (int e = rank * kR + tid; e < M * (kCols / 2); e += KS * kR) {
         const int m = e / (kCols / 2), c = (e % (kCols / 2)) * 2;
         if (col0 + c >= N) continue;
+        float2 lo[kMaxCluster], hi[kMaxCluster];
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r)
+          if (r < KS) {
+            const float* p = cluster.map_shared_rank(part, r) + m * kCols + c;
+            lo[r] = *reinterpret_cast<const float2*>(p);
+            hi[r] = *reinterpret_cast<const float2*>(p + L::kPart / 4);
+          }
         float2 v = make_float2(0.f, 0.f);
-        for (int r = 0; r < KS; ++r) {
-          const float* p = cluster.map_shared_rank(part, r) + m * kCols + c;
-          const float2 lo = *reinterpret_cast<const float2*>(p);
-          const float2 hi = *reinterpret_cast<const float2*>(p + L::kPart / 4);
-          v.x += lo.x + hi.x;
-          v.y += lo.y + hi.y;
-        }
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r)
+          if (r < KS) {
+            v.x += lo[r].x + hi[r].x;
+            v.y += lo[r].y + hi[r].y;
+          }
         const float2 sc = make_float2(__ldg(scale + col0 + c), __ldg(scale + col0 + c + 1));
-        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(m) * ldy + col0 + c) = dev::pack_bf16x2(v.x * sc.x, v.y * sc.y);
+        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(m) * ldy + col0 + c) =
+            dev::pack_bf16x2(v.x * 64.f * sc.x, v.y * 64.f * sc.y);
       }
       __syncwarp();
       if (lane < KS) arrive_remote(&vacant[b], lane);
@@ -263,23 +294,24 @@ template <int MT>
 static int resident_clusters(int ks) {
   static std::atomic<int> cache[kMaxDevices][kMaxCluster + 1];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 2 * num_sms() / ks;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return Smem<MT>::kPerSm * num_sms() / ks;
   int n = cache[dev][ks].load(std::memory_order_relaxed);
   if (n > 0) return n;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(ks, 1024);
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(Smem<MT>::kThreads);
   cfg.dynamicSmemBytes = Smem<MT>::kTotal;
   set_attrs(cfg, attr, ks);
   if (cudaOccupancyMaxActiveClusters(&n, w8a16_decode_kernel<MT>, &cfg) != cudaSuccess || n < 1) {
     (void)cudaGetLastError();
-    n = 2 * num_sms() / ks;
+    n = Smem<MT>::kPerSm * num_sms() / ks;
   }
   cache[dev][ks].store(n, std::memory_order_relaxed);
   return n;
 }
 
+constexpr int kRoundCost = 6;
 // Resident clusters walk the column blocks, so the launch takes as many rounds as the busiest cluster has blocks; a
 // round costs its stages and the hand-over of the partial tiles.
 template <int MT>
@@ -289,7 +321,7 @@ static Grid choose_grid(int blocks, int stages_total) {
   for (int ks = 1; ks <= kMaxCluster && ks <= stages_total; ++ks) {
     const int c = resident_clusters<MT>(ks);
     const int rounds = (blocks + c - 1) / c;
-    const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + 2);
+    const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + kRoundCost);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best.ks = ks;
@@ -310,7 +342,7 @@ static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const float*
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(g.ks, g.clusters);
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(Smem<MT>::kThreads);
   cfg.dynamicSmemBytes = L::kTotal;
   cfg.stream = stream;
   set_attrs(cfg, attr, g.ks);
