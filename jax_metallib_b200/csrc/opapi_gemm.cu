@@ -3,7 +3,7 @@
 //
 //   y[m,n] = sum over groups g of  s[n,g] * sum_{k in g} x[m,k] c[n,k]  (+ b[n,g] * sum_{k in g} x[m,k])
 //
-// The weights go to tcgen05.mma as their bare codes c (a centred integer, or the e2m1 / e4m3 element), which
+// The weights go to tcgen05.mma as their bare codes c (an integer, or the e2m1 / e4m3 element), which
 // both 16-bit types hold exactly: f16 against f16 activations, bf16 against f32 activations, which are cut into
 // three bf16 terms that add up to all 24 bits.  Every product is therefore exact.  The accumulator of one unit of
 // k (a scale group of up to 128 k) is read back from TMEM and multiplied by the group's f32 scale into f32
@@ -18,8 +18,8 @@
 // activations into their three terms, and sum the activations of a unit for the biases) and four or eight
 // promoters that drain the accumulators.
 //
-// What the split cannot represent takes an exact path: a unit whose activations are not finite (0 * inf of a
-// centred code is not what scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
+// What the split cannot represent takes an exact path: a unit whose activations are not finite (inf times
+// code plus inf times bias is not what inf times scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
 // the promoters from global memory with the arithmetic of the CUDA-core kernels.
 #include <cooperative_groups.h>
 
@@ -122,8 +122,10 @@ __device__ __forceinline__ uint32_t f16x2_to_bf16x2(uint32_t h) {
 }
 
 // Eight codes of k .. k+7 -> eight 16-bit operand values in k order.  For 4-bit formats `lo` holds all eight.
-//   integers:  128 + q or 1024 + q by OR-ing the code into a constant's mantissa, minus 128 + 8 (4-bit) etc.:
-//              the centred q - 8 or q - 128, exact
+//   integers:  128 + q or 1024 + q by OR-ing the code into a constant's mantissa, minus that constant.  An 8-bit code
+//              in bf16 reads as q * 2^-133 where it stands (a subnormal up to 127, the first binade above) and is
+//              multiplied by 2^127: q / 64, the group's scale makes up for it.  Codes are not centred: a flat group
+//              has scale 1, code 0 and its value as bias, which a centred code would cancel away.
 //   e2m1:      cvt to f16; for bf16 the code's exponent and mantissa are moved into place (worth 2^-126 of the
 //              element) and multiplied by 2^126
 //   e4m3:      cvt to f16, then to bf16 (4 significant bits: exact)
@@ -131,21 +133,11 @@ template <int FMT, bool BF16>
 __device__ __forceinline__ uint4 convert8(uint32_t lo, uint32_t hi, uint32_t scale2) {
   uint32_t r[4];
   if (FMT == kAffine8) {
-    if (BF16) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t t = __byte_perm(i < 2 ? lo : hi, 0u, (i & 1) ? 0x4342 : 0x4140);
-        // 128 + (q & 127), plus -128 (q >= 128) or -256
-        const uint32_t a = lop_and_or(t, 0x007F007Fu, 0x43004300u);
-        const uint32_t c = lop_and_or(~t, 0x00800080u, 0xC300C300u);
-        asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r[i]) : "r"(a), "r"(c));
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t t = __byte_perm(i < 2 ? lo : hi, 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
-        r[i] = sub2<false>(t, 0x64806480u);  // 1024 + q - 1152
-      }
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t sel = (i & 1) ? 0x4342 : 0x4140;
+      if (BF16) r[i] = mul2<true>(__byte_perm(i < 2 ? lo : hi, 0u, sel), 0x7F007F00u);   // q * 2^-133 * 2^127
+      else r[i] = sub2<false>(__byte_perm(i < 2 ? lo : hi, 0x64646464u, sel), 0x64006400u);
     }
   } else if (FMT == kMxfp8) {
     e4m3_to_f16(lo, r[0], r[1]);
@@ -164,7 +156,7 @@ __device__ __forceinline__ uint4 convert8(uint32_t lo, uint32_t hi, uint32_t sca
       const uint32_t p = __byte_perm(e, o, static_cast<uint32_t>(i) | (4u + i) << 8);
       if (FMT == kAffine4) {
         const uint32_t t = lop_and_or(p, 0x000F000Fu, BF16 ? 0x43004300u : 0x64006400u);
-        r[i] = sub2<BF16>(t, BF16 ? 0x43084308u : 0x64086408u);          // 128 + q - 136 or 1024 + q - 1032
+        r[i] = sub2<BF16>(t, BF16 ? 0x43004300u : 0x64006400u);
       } else {
         const uint32_t mag = (p & 0x00070007u) << 6, sgn = (p & 0x00080008u) << 12;
         r[i] = mul2<true>(mag | sgn, 0x7E807E80u);                       // times 2^126
@@ -197,6 +189,13 @@ __device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
 __device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
+
+__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ void add2(uint64_t& acc, uint64_t a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
 
 // sum_{k in [k0, k1)} x[m,k] * weight[n,k], as the CUDA-core kernels compute it
 template <int FMT, bool XF32>
@@ -541,9 +540,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         const int u = ub + i;
         if (!ok || u >= units) break;
         const int buf = u % kAccBufs, slot = u % kInfo;
-        const float s = sv[i];
-        // the code went in centred: scale * q + bias = scale * (q - 8) + (bias + 8 scale)
-        const float b = C::kBias ? fmaf(FMT == kAffine4 ? 8.f : 128.f, s, bv[i]) : 0.f;
+        const float s = (FMT == kAffine8 && XF32) ? sv[i] * 64.f : sv[i], b = bv[i];
         load_scale(u + kAhead, sv[i], bv[i]);
         bool exact = false;
         if (C::kUnitInfo) {
@@ -575,17 +572,22 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             uint32_t r[16];
             dev::tmem_ld_32x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0 + c, r);
             dev::tc_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
             if (C::kBias) {
+              // scale and bias terms cancel in part: they meet before they are added to the running sum
               const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(xsum + slot * BM + c0 + c);
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const ulonglong2 t = xp[e];
-                fma2(acc[c / 2 + 2 * e], b2, t.x);
-                fma2(acc[c / 2 + 2 * e + 1], b2, t.y);
+                uint64_t v0 = fmul2(b2, t.x), v1 = fmul2(b2, t.y);
+                fma2(v0, s2, pack2(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1])));
+                fma2(v1, s2, pack2(__uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3])));
+                add2(acc[c / 2 + 2 * e], v0);
+                add2(acc[c / 2 + 2 * e + 1], v1);
               }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
             }
           }
         }
@@ -672,7 +674,10 @@ static int launch(Args a, cudaStream_t stream) {
   auto kern = opgemm_kernel<FMT, XF32, BM>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), C::kSmem, configured)) return rc;
   // a unit is a scale group or a part of one; slices of K begin on a raw box and on a unit
-  a.pu = FMT == kNvfp4 ? 128 : (a.gs % 128 == 0 ? 128 : (a.gs % 64 == 0 ? 64 : 32));
+  a.pu = FMT == kNvfp4 || a.gs % 128 == 0 ? 128 : (a.gs % 64 == 0 ? 64 : 32);
+  // the tensor core's own additions are truncated: against f32 results (128 k: 2.5e-7 of the result, 64 k: 1e-7) they
+  // are cut short, against f16 results they do not show
+  if (XF32 && a.pu > 64) a.pu = 64;
   a.block_k = C::kBoxK;
   a.blocks = (a.K + a.block_k - 1) / a.block_k;
   a.idesc = dev::make_idesc(/*c=f32*/ 1, XF32 ? 1 : 0, XF32 ? 1 : 0, /*both K-major*/ 0, 0, BN, BM);

@@ -151,6 +151,7 @@ struct qmm_rt_device {
   std::mutex stream_mu;
   bool streams_ready = false;
   cudaStream_t exec = nullptr, d2h = nullptr;
+  cudaMemPool_t pool = nullptr;  // of this client alone; null: the device's default pool
   std::string kind, debug, text;
   std::unique_ptr<qmm_rt_memory> memory;
   std::atomic<int64_t> bytes_in_use{0};
@@ -241,6 +242,8 @@ int after_stream(qmm_rt_client* c, cudaStream_t stream, std::function<void()> fn
   return QMM_OK;
 }
 
+constexpr uint64_t kPoolKeepBytes = 256ull << 20;
+
 int device_ready(qmm_rt_device* d) {
   QMM_REQUIRE(d != nullptr, QMM_ERR_INVALID_ARGUMENT, "null device");
   std::lock_guard<std::mutex> lock(d->stream_mu);
@@ -248,6 +251,20 @@ int device_ready(qmm_rt_device* d) {
   QMM_CUDA_TRY(cudaSetDevice(d->ordinal));
   QMM_CUDA_TRY(cudaStreamCreateWithFlags(&d->exec, cudaStreamNonBlocking));
   QMM_CUDA_TRY(cudaStreamCreateWithFlags(&d->d2h, cudaStreamNonBlocking));
+  // A pool of the client's own that keeps up to kPoolKeepBytes of freed memory: the default pool hands everything
+  // back to the driver whenever the host waits, so that each execution mapped its results afresh (a program of four
+  // linears at eight rows, host to host: 1.3-2.1 ms a pass).  It goes with the client.
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = d->ordinal;
+  if (cudaMemPoolCreate(&d->pool, &props) == cudaSuccess) {
+    uint64_t keep = kPoolKeepBytes;
+    cudaMemPoolSetAttribute(d->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  } else {
+    d->pool = nullptr;
+    (void)cudaGetLastError();
+  }
   d->streams_ready = true;
   return QMM_OK;
 }
@@ -292,7 +309,8 @@ int new_buffer(qmm_rt_client* c, qmm_rt_device* dev, int dtype, const int64_t* d
   // a zero-element shape still gets an address of its own (a placeholder allocation)
   const size_t alloc = bytes ? bytes : 256;
   void* p = nullptr;
-  QMM_CUDA_TRY(cudaMallocAsync(&p, alloc, dev->exec));
+  if (dev->pool) QMM_CUDA_TRY(cudaMallocFromPoolAsync(&p, alloc, dev->pool, dev->exec));
+  else QMM_CUDA_TRY(cudaMallocAsync(&p, alloc, dev->exec));
   auto* b = new qmm_rt_buffer();
   b->client = c;
   b->device = dev;
@@ -470,6 +488,7 @@ int qmm_rt_client_destroy(qmm_rt_client* c) {
     cudaSetDevice(d->ordinal);
     cudaStreamDestroy(d->exec);
     cudaStreamDestroy(d->d2h);
+    if (d->pool) cudaMemPoolDestroy(d->pool);  // buffers that are still out keep their memory until they are freed
   }
   delete c;
   return QMM_OK;
@@ -816,6 +835,16 @@ static int read_to_host(qmm_rt_buffer* b, void* dst, int64_t offset, int64_t siz
                         dev->d2h);
   if (e != cudaSuccess) return fail(QMM_ERR_CUDA, cudaGetErrorString(e));
   EventRef producer = b->ready;
+  // A copy into pageable memory is complete when the call returns.  Then the event completes here: the host function
+  // and the completion thread cost two thread wake-ups, 0.2-0.3 ms per result.
+  if (cudaStreamQuery(dev->d2h) == cudaSuccess) {
+    // the producer is done too, but its own completion job may not have run yet: ask what that job would ask
+    if (producer && producer->ready.load() && producer->status != QMM_OK) st->finish(producer->status, producer->message);
+    else if (qmm_device_status() != 0) st->finish(QMM_ERR_TIMEOUT, "a kernel of this launch (or an earlier one) gave up waiting");
+    else st->finish(QMM_OK, "");
+    return QMM_OK;
+  }
+  (void)cudaGetLastError();  // "not ready" is no error
   if (after_stream(b->client, dev->d2h, [st, producer] {
         // a producer that failed (a kernel wait that gave up) taints what was read
         if (producer && producer->ready.load() && producer->status != QMM_OK) st->finish(producer->status, producer->message);

@@ -33,15 +33,16 @@ constexpr int kFirstReducer = kConsumerWarps + 1;
 constexpr int kWBytes = kBK * kCols;
 constexpr int kMaxCluster = 8;
 
-template <int MT>
+template <int MT, bool XF32>
 struct Smem {
-  static constexpr int kX = MT * 8 * kBK * 2;              // activations of a stage: [MT * 8 rows][128 bytes]
+  static constexpr int kXBox = MT * 8 * 128;               // [MT * 8 rows][128 bytes]: 64 k of bf16 or 32 k of f32
+  static constexpr int kX = XF32 ? 2 * kXBox : kXBox;      // activations of a stage
   static constexpr int kStage = kWBytes + kX;
   // resident CTAs: a warp's chain ldmatrix -> convert -> MMA is latency-bound, so as many as registers allow
   static constexpr int kPerSm = 2;
   static constexpr int kReducers = MT <= 2 ? 3 : 4;                     // warps that add the partial tiles
   static constexpr int kThreads = (kFirstReducer + kReducers) * 32;
-  static constexpr int kStages = MT == 1 ? 9 : (MT == 2 ? 7 : 6);
+  static constexpr int kStages = MT == 1 ? 8 : 6;
   static constexpr int kPartBufs = MT <= 2 ? 2 : 1;        // tiles whose partial results may be in flight
   static constexpr int kPart = MT * 8 * kCols * 4;         // partial tile of one k half
   static constexpr int kOffPart = kStages * kStage;
@@ -76,6 +77,32 @@ __device__ __forceinline__ uint32_t bytes02_to_bf16x2(uint32_t t) {
   return r;
 }
 
+// Four f32 -> their bf16 terms, as pairs of k: the top 8 significant bits, the next 8, the rest.  Infinities and NaN
+// have no second and third term, and a NaN stays one when it is cut.
+__device__ __forceinline__ void split4(uint32_t (&v)[4], uint32_t (&hi)[2], uint32_t (&mid)[2], uint32_t (&lo)[2]) {
+  uint32_t m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = __float_as_uint(__uint_as_float(v[i]) - __uint_as_float(v[i] & 0xFFFF0000u));
+    l[i] = __float_as_uint(__uint_as_float(m[i]) - __uint_as_float(m[i] & 0xFFFF0000u));
+  }
+  const uint32_t top = max(max(v[0] & 0x7FFFFFFFu, v[1] & 0x7FFFFFFFu), max(v[2] & 0x7FFFFFFFu, v[3] & 0x7FFFFFFFu));
+  if (top >= 0x7F800000u) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if ((v[i] & 0x7FFFFFFFu) >= 0x7F800000u) {
+        if ((v[i] & 0x7FFFFFFFu) > 0x7F800000u) v[i] |= 0x00400000u;
+        m[i] = l[i] = 0u;
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    hi[i] = __byte_perm(v[2 * i], v[2 * i + 1], 0x7632);
+    mid[i] = __byte_perm(m[2 * i], m[2 * i + 1], 0x7632);
+    lo[i] = __byte_perm(l[2 * i], l[2 * i + 1], 0x7632);
+  }
+}
+
 // Arrives (release, cluster scope) on the barrier at the same place of CTA `rank`'s shared memory.
 __device__ __forceinline__ void arrive_remote(uint64_t* bar, int rank) {
   asm volatile(
@@ -106,12 +133,12 @@ __device__ __forceinline__ bool wait_cluster_warp(uint64_t* bar, uint32_t parity
   return __all_sync(0xFFFFFFFFu, ok);
 }
 
-template <int MT>
-__global__ void __launch_bounds__(Smem<MT>::kThreads, Smem<MT>::kPerSm)
-w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
-                    const float* __restrict__ scale, uint16_t* __restrict__ y, int M, int N, long long ldy, int stages_total,
-                    int independent, int* status) {
-  using L = Smem<MT>;
+template <int MT, bool XF32>
+__global__ void __launch_bounds__(Smem<MT, XF32>::kThreads, Smem<MT, XF32>::kPerSm)
+w8_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+                 const float* __restrict__ scale, void* __restrict__ y, int M, int N, long long ldy, int stages_total,
+                 int independent, int* status) {
+  using L = Smem<MT, XF32>;
   constexpr int S = L::kStages, PB = L::kPartBufs;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -121,7 +148,9 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
   uint64_t* vacant = ready + PB;     // every CTA of the cluster has read this CTA's partial tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KS = gridDim.x, rank = blockIdx.x;      // the cluster is the grid's x extent
-  const int blocks = (N + kCols - 1) / kCols;
+  // tile t: rows (t % row_tiles) * MT * 8 .. of column block t / row_tiles
+  const int row_tiles = (M + MT * 8 - 1) / (MT * 8);
+  const int tiles = ((N + kCols - 1) / kCols) * row_tiles;
   const int it_begin = (stages_total * rank) / KS, it_end = (stages_total * (rank + 1)) / KS;
   cg::cluster_group cluster = cg::this_cluster();
 
@@ -151,15 +180,19 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
       const uint64_t policy = dev::policy_evict_first();
       int n = 0;   // stages issued
       bool ok = true;
-      for (int cb = blockIdx.y; ok && cb < blocks; cb += gridDim.y)
+      for (int t = blockIdx.y; ok && t < tiles; t += gridDim.y) {
+        const int col0 = (t / row_tiles) * kCols, row0 = (t % row_tiles) * MT * 8;
         for (int it = it_begin; it < it_end; ++it, ++n) {
           const int s = n % S;
           if (!dev::mbar_wait_relaxed(&empty[s], ((n / S) & 1) ^ 1, status, 80)) { ok = false; break; }
           uint8_t* st = smem + s * L::kStage;
           dev::mbar_expect_tx(&full[s], L::kStage);   // rows and columns past the ends arrive as zeros
-          dev::tma_load_2d_hint(st, &wmap, &full[s], cb * kCols, it * kBK, policy);
-          dev::tma_load_2d(st + kWBytes, &xmap, &full[s], it * kBK, 0);
+          if (row_tiles == 1) dev::tma_load_2d_hint(st, &wmap, &full[s], col0, it * kBK, policy);
+          else dev::tma_load_2d(st, &wmap, &full[s], col0, it * kBK);   // the next row tile reads them again
+          dev::tma_load_2d(st + kWBytes, &xmap, &full[s], it * kBK, row0);
+          if (XF32) dev::tma_load_2d(st + kWBytes + L::kXBox, &xmap, &full[s], it * kBK + 32, row0);
         }
+      }
       // no copy may still be on its way into this CTA's shared memory when it leaves, whatever the consumers did
       for (int i = n > S ? n - S : 0; i < n; ++i)
         if (!dev::mbar_wait_relaxed(&full[i % S], (i / S) & 1, status, 81)) break;
@@ -169,19 +202,24 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     // ------------------------------ consumers -----------------------------
     const int cgrp = warp & 3, kh = warp >> 2;
     const int g8 = lane >> 2, t4 = lane & 3;
-    // weights: lane l addresses k row 32 kh + l, 16-byte chunks 2 cgrp and 2 cgrp + 1 (XOR-swizzled by the row)
-    const uint32_t w_row = (kh * 32 + lane) * 128;
-    const uint32_t w_off0 = w_row + (((2 * cgrp) ^ (lane & 7)) << 4);
-    const uint32_t w_off1 = w_row + (((2 * cgrp + 1) ^ (lane & 7)) << 4);
-    // activations: lane l addresses row l & 7 of the 8-k chunk 4 kh + (l >> 3)
-    const uint32_t x_off = kWBytes + (lane & 7) * 128 + (((4 * kh + (lane >> 3)) ^ (lane & 7)) << 4);
+    // weights: lane l addresses one k row, 16-byte chunks 2 cgrp and 2 cgrp + 1 (XOR-swizzled by the row).  bf16
+    // activations: row 32 kh + l.  f32 activations: a thread reads four neighbouring k of a row (16 bytes) per 16-k
+    // step, so slots 2t, 2t + 1, 2t + 8, 2t + 9 of a step stand for its k 4t .. 4t + 3 and the rows are dealt likewise.
+    const int w_k = kh * 32 + (XF32 ? (lane >> 4) * 16 + ((lane & 7) >> 1) * 4 + (lane & 1) + ((lane >> 3) & 1) * 2 : lane);
+    const uint32_t w_off0 = w_k * 128 + (((2 * cgrp) ^ (w_k & 7)) << 4);
+    const uint32_t w_off1 = w_k * 128 + (((2 * cgrp + 1) ^ (w_k & 7)) << 4);
+    // activations: bf16: lane l addresses row l & 7 of the 8-k chunk 4 kh + (l >> 3); f32: row x_row, chunk t4 of the
+    // step (rows r and r + 4 share a quarter-warp: no bank conflict)
+    const int x_row = XF32 ? ((g8 >> 1) | ((g8 & 1) << 2)) : (lane & 7);
+    const uint32_t x_off = kWBytes + (XF32 ? kh * L::kXBox : 0) + x_row * 128 +
+                           (XF32 ? 0 : (((4 * kh + (lane >> 3)) ^ x_row) << 4));
     const uint32_t ring = dev::smem_u32(smem);
     int s = 0;
     uint32_t ph = 0;
     int tile = 0;
     bool ok = true;
     const int never = stages_total < 0;   // false, but not to the compiler
-    for (int cb = blockIdx.y; cb < blocks; cb += gridDim.y, ++tile) {
+    for (int t = blockIdx.y; t < tiles; t += gridDim.y, ++tile) {
       float acc[2][MT][4];
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -192,27 +230,76 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
       for (int it = it_begin; it < it_end; ++it) {
         if (!dev::mbar_wait_relaxed_warp(&full[s], ph, status, 82)) { ok = false; break; }
         const uint32_t st = ring + s * L::kStage;
-        uint32_t wr[2][4], xr[MT][4];
+        uint32_t wr[2][4];
         ldmatrix_x4_trans(st + w_off0, wr[0]);
         ldmatrix_x4_trans(st + w_off1, wr[1]);
+        uint32_t dep = wr[0][3] ^ wr[1][3];
+        if constexpr (!XF32) {
+          uint32_t xr[MT][4];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) ldmatrix_x4(st + x_off + mt * 1024, xr[mt]);
+          for (int mt = 0; mt < MT; ++mt) ldmatrix_x4(st + x_off + mt * 1024, xr[mt]);
 #pragma unroll
-        for (int q = 0; q < 2; ++q)   // 16 k each
+          for (int q = 0; q < 2; ++q)   // 16 k each
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const uint32_t a0 = bytes02_to_bf16x2(wr[j][2 * q]), a1 = bytes02_to_bf16x2(wr[j][2 * q] >> 8);
+              const uint32_t a2 = bytes02_to_bf16x2(wr[j][2 * q + 1]), a3 = bytes02_to_bf16x2(wr[j][2 * q + 1] >> 8);
+#pragma unroll
+              for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(acc[j][mt], a0, a1, a2, a3, xr[mt][2 * q], xr[mt][2 * q + 1]);
+            }
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) dep ^= xr[mt][3];
+        } else {
+          // x = hi + mid + lo, bf16 each and exact together; the smallest terms are added first, into an accumulator
+          // that starts at zero every stage: a correctly rounded f32 addition takes over after 32 k
+          float d[2][MT][4];
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) d[j][mt][i] = 0.f;
+          uint32_t term[3][2][MT][2];   // [hi, mid, lo][16-k step][row tile][k pair]
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+              uint32_t v[4];
+              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                           : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                           : "r"(st + x_off + mt * 1024 + (((q * 4 + t4) ^ x_row) << 4)));
+              dep ^= v[3];
+              split4(v, term[0][q][mt], term[1][q][mt], term[2][q][mt]);
+            }
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            const uint32_t a0 = bytes02_to_bf16x2(wr[j][2 * q]), a1 = bytes02_to_bf16x2(wr[j][2 * q] >> 8);
-            const uint32_t a2 = bytes02_to_bf16x2(wr[j][2 * q + 1]), a3 = bytes02_to_bf16x2(wr[j][2 * q + 1] >> 8);
+            uint32_t a[2][4];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(acc[j][mt], a0, a1, a2, a3, xr[mt][2 * q], xr[mt][2 * q + 1]);
+            for (int q = 0; q < 2; ++q) {
+              a[q][0] = bytes02_to_bf16x2(wr[j][2 * q]);
+              a[q][1] = bytes02_to_bf16x2(wr[j][2 * q] >> 8);
+              a[q][2] = bytes02_to_bf16x2(wr[j][2 * q + 1]);
+              a[q][3] = bytes02_to_bf16x2(wr[j][2 * q + 1] >> 8);
+            }
+#pragma unroll
+            for (int e = 2; e >= 0; --e)
+#pragma unroll
+              for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+                  mma_bf16_16816(d[j][mt], a[q][0], a[q][1], a[q][2], a[q][3], term[e][q][mt][0], term[e][q][mt][1]);
           }
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) acc[j][mt][i] += d[j][mt][i];
+        }
         // The slot goes back only when its bytes are in registers: an arrival that merely follows the loads in program
         // order let the refill overtake the last of them (seen with remote shared-memory traffic on the same SM), so
         // its address is made to depend on what they returned.
-        uint32_t dep = wr[0][3] ^ wr[1][3];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) dep ^= xr[mt][3];
-        // (lane 0's copy stands for the warp's: ldmatrix completes for all lanes at once)
+        // Lane 0's copy stands for the warp's: a shared load completes for all lanes at once.
         if (lane == 0) dev::mbar_arrive(&empty[s] + ((dep == 0x7FC1FFC1u) & never));
         if (++s == S) { s = 0; ph ^= 1; }
       }
@@ -222,14 +309,14 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
       if (tile >= PB && !wait_cluster_warp(&vacant[b], ((tile / PB) & 1) ^ 1, status, 83)) break;
       float* part = reinterpret_cast<float*>(smem + L::kOffPart + b * 2 * L::kPart);
       float* mine = part + kh * (L::kPart / 4);
-      // rows 2 t4, 2 t4 + 1 of columns 2 g8, 2 g8 + 1 of each 16-column block
+      // rows 2 t4, 2 t4 + 1 (f32: t4, t4 + 4) of columns 2 g8, 2 g8 + 1 of each 16-column block
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
           for (int r = 0; r < 2; ++r)
-            *reinterpret_cast<float2*>(mine + (mt * 8 + 2 * t4 + r) * kCols + cgrp * 32 + j * 16 + 2 * g8) =
+            *reinterpret_cast<float2*>(mine + (mt * 8 + (XF32 ? t4 + 4 * r : 2 * t4 + r)) * kCols + cgrp * 32 + j * 16 + 2 * g8) =
                 make_float2(acc[j][mt][r], acc[j][mt][2 + r]);
       __syncwarp();
       if (lane < KS) arrive_remote(&ready[b], lane);
@@ -240,12 +327,13 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     constexpr int kR = L::kReducers * 32;
     const int tid = threadIdx.x - kFirstReducer * 32;
     int tile = 0;
-    for (int cb = blockIdx.y; cb < blocks; cb += gridDim.y, ++tile) {
+    for (int t = blockIdx.y; t < tiles; t += gridDim.y, ++tile) {
       const int b = tile % PB;
       const float* part = reinterpret_cast<const float*>(smem + L::kOffPart + b * 2 * L::kPart);
       if (!wait_cluster_warp(&ready[b], (tile / PB) & 1, status, 84)) break;
-      const int col0 = cb * kCols;
-      for (int e = rank * kR + tid; e < M * (kCols / 2); e += KS * kR) {
+      const int col0 = (t / row_tiles) * kCols, row0 = (t % row_tiles) * MT * 8;
+      const int rows = min(MT * 8, M - row0);
+      for (int e = rank * kR + tid; e < rows * (kCols / 2); e += KS * kR) {
         const int m = e / (kCols / 2), c = (e % (kCols / 2)) * 2;
         if (col0 + c >= N) continue;
         float2 lo[kMaxCluster], hi[kMaxCluster];
@@ -264,8 +352,11 @@ w8a16_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             v.y += lo[r].y + hi[r].y;
           }
         const float2 sc = make_float2(__ldg(scale + col0 + c), __ldg(scale + col0 + c + 1));
-        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(m) * ldy + col0 + c) =
-            dev::pack_bf16x2(v.x * 64.f * sc.x, v.y * 64.f * sc.y);
+        const size_t i = static_cast<size_t>(row0 + m) * ldy + col0 + c;
+        v.x = v.x * 64.f * sc.x;
+        v.y = v.y * 64.f * sc.y;
+        if (XF32) *reinterpret_cast<float2*>(static_cast<float*>(y) + i) = v;
+        else *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(y) + i) = dev::pack_bf16x2(v.x, v.y);
       }
       __syncwarp();
       if (lane < KS) arrive_remote(&vacant[b], lane);
@@ -290,59 +381,59 @@ static void set_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], i
 }
 
 // Clusters of `ks` CTAs that the current device holds at once (asked once per device and size).
-template <int MT>
+template <int MT, bool XF32>
 static int resident_clusters(int ks) {
   static std::atomic<int> cache[kMaxDevices][kMaxCluster + 1];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return Smem<MT>::kPerSm * num_sms() / ks;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return Smem<MT, XF32>::kPerSm * num_sms() / ks;
   int n = cache[dev][ks].load(std::memory_order_relaxed);
   if (n > 0) return n;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(ks, 1024);
-  cfg.blockDim = dim3(Smem<MT>::kThreads);
-  cfg.dynamicSmemBytes = Smem<MT>::kTotal;
+  cfg.blockDim = dim3(Smem<MT, XF32>::kThreads);
+  cfg.dynamicSmemBytes = Smem<MT, XF32>::kTotal;
   set_attrs(cfg, attr, ks);
-  if (cudaOccupancyMaxActiveClusters(&n, w8a16_decode_kernel<MT>, &cfg) != cudaSuccess || n < 1) {
+  if (cudaOccupancyMaxActiveClusters(&n, w8_decode_kernel<MT, XF32>, &cfg) != cudaSuccess || n < 1) {
     (void)cudaGetLastError();
-    n = Smem<MT>::kPerSm * num_sms() / ks;
+    n = Smem<MT, XF32>::kPerSm * num_sms() / ks;
   }
   cache[dev][ks].store(n, std::memory_order_relaxed);
   return n;
 }
 
 constexpr int kRoundCost = 6;
-// Resident clusters walk the column blocks, so the launch takes as many rounds as the busiest cluster has blocks; a
+// Resident clusters walk the tiles, so the launch takes as many rounds as the busiest cluster has tiles; a
 // round costs its stages and the hand-over of the partial tiles.
-template <int MT>
-static Grid choose_grid(int blocks, int stages_total) {
+template <int MT, bool XF32>
+static Grid choose_grid(int tiles, int stages_total) {
   Grid best = {1, 1};
   long long best_cost = -1;
   for (int ks = 1; ks <= kMaxCluster && ks <= stages_total; ++ks) {
-    const int c = resident_clusters<MT>(ks);
-    const int rounds = (blocks + c - 1) / c;
+    const int c = resident_clusters<MT, XF32>(ks);
+    const int rounds = (tiles + c - 1) / c;
     const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + kRoundCost);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best.ks = ks;
-      best.clusters = blocks < c ? blocks : c;
+      best.clusters = tiles < c ? tiles : c;
     }
   }
   return best;
 }
 
-template <int MT>
-static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const float* scale, uint16_t* y, int M, int N, long long ldy,
+template <int MT, bool XF32>
+static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const float* scale, void* y, int M, int N, long long ldy,
                   int stages_total, int independent, cudaStream_t stream) {
-  using L = Smem<MT>;
+  using L = Smem<MT, XF32>;
   static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
-  auto kern = w8a16_decode_kernel<MT>;
+  auto kern = w8_decode_kernel<MT, XF32>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
-  const Grid g = choose_grid<MT>((N + kCols - 1) / kCols, stages_total);
+  const Grid g = choose_grid<MT, XF32>(((N + kCols - 1) / kCols) * ((M + MT * 8 - 1) / (MT * 8)), stages_total);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(g.ks, g.clusters);
-  cfg.blockDim = dim3(Smem<MT>::kThreads);
+  cfg.blockDim = dim3(Smem<MT, XF32>::kThreads);
   cfg.dynamicSmemBytes = L::kTotal;
   cfg.stream = stream;
   set_attrs(cfg, attr, g.ks);
@@ -367,9 +458,27 @@ int w8a16_decode(const uint16_t* x, const int8_t* w, const float* scale, uint16_
   const int stages_total = static_cast<int>((K + kBK - 1) / kBK);
   const int ind = (flags & QMM_GEMM_INDEPENDENT) ? 1 : 0;
   const int m = static_cast<int>(M), n = static_cast<int>(N);
-  if (mt == 1) return launch<1>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
-  if (mt == 2) return launch<2>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
-  return launch<4>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
+  if (mt == 1) return launch<1, false>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
+  if (mt == 2) return launch<2, false>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
+  return launch<4, false>(wmap, xmap, scale, y, m, n, ldy, stages_total, ind, stream);
+}
+
+// Any M; K % 4 == 0, N % 16 == 0, x and w 16-byte, y 8-byte aligned (checked by the caller).  Row tiles of 8 or 16: the
+// three terms of the activations and two sets of accumulators fill the registers.
+int w8a32_tc(const float* x, const int8_t* w, const float* scale, float* y, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
+  using namespace w8d;
+  const int mt = M <= 8 ? 1 : 2;
+  CUtensorMap wmap, xmap;
+  if (int rc = make_tensor_map_2d(&wmap, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)N, kBK, kCols,
+                                  CU_TENSOR_MAP_SWIZZLE_128B))
+    return rc;
+  if (int rc = make_tensor_map_2d(&xmap, x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)M, (uint64_t)K, (uint64_t)K * 4, mt * 8,
+                                  32, CU_TENSOR_MAP_SWIZZLE_128B))
+    return rc;
+  const int stages_total = static_cast<int>((K + kBK - 1) / kBK);
+  const int m = static_cast<int>(M), n = static_cast<int>(N);
+  return mt == 1 ? launch<1, true>(wmap, xmap, scale, y, m, n, n, stages_total, 0, stream)
+                 : launch<2, true>(wmap, xmap, scale, y, m, n, n, stages_total, 0, stream);
 }
 
 }  // namespace qmm

@@ -17,6 +17,9 @@
 namespace cg = cooperative_groups;
 
 namespace qmm {
+
+int w8a32_tc(const float* x, const int8_t* w, const float* scale, float* y, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+
 namespace w8a32 {
 
 constexpr int TM = 32, TN = 32;
@@ -120,6 +123,13 @@ extern "C" int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float
               QMM_ERR_INVALID_ARGUMENT, "qmm_w8a32_perchannel: bad shape");
   if (M == 0 || N == 0) return QMM_OK;  // empty result: nothing to launch, pointers may be null
   QMM_REQUIRE(x && w && scale && y, QMM_ERR_INVALID_ARGUMENT, "qmm_w8a32_perchannel: null pointer");
+  // rows that TMA can describe: the tensor-core kernel
+  if (K > 0 && K % 4 == 0 && N % 16 == 0 && aligned(x, 16) && aligned(w, 16) && aligned(y, 8) && M < (1 << 24) &&
+      N * ((M + 7) / 8) < (1ll << 36)) {
+    if (int st = read_device_status())
+      return set_error(QMM_ERR_TIMEOUT, "a previous kernel gave up waiting (status word 0x%x)", st);
+    return w8a32_tc(x, w, scale, y, M, N, K, static_cast<cudaStream_t>(stream));
+  }
   const unsigned gx = static_cast<unsigned>((N + TN - 1) / TN);
   const unsigned gy = static_cast<unsigned>((M + TM - 1) / TM);
   QMM_REQUIRE(gy <= 65535, QMM_ERR_UNSUPPORTED, "qmm_w8a32_perchannel: M too large");

@@ -273,6 +273,8 @@ def affine_dequantize(packed, scales, biases, *, bits: int = 4, group_size: int 
 
 def _to_device(a, torch, device, dtype=None):
     if _is_torch(a):
+        if a.device == device and (dtype is None or a.dtype == dtype) and a.is_contiguous():
+            return a
         t = a.to(device)
     else:
         t = torch.from_numpy(np.ascontiguousarray(a)).to(device)
@@ -285,10 +287,10 @@ def _launch_matmul(x, call, N, K, out_dtype):
     """Shared driver: flatten batch dims, run the kernel in x's dtype, cast, restore dims."""
     import torch
 
-    if not torch.cuda.is_available():
+    is_t = _is_torch(x)
+    if not (is_t and x.is_cuda) and not torch.cuda.is_available():
         raise RuntimeError("quantized matmul needs a CUDA device: this build has no CPU fallback")
     _lib.load()
-    is_t = _is_torch(x)
     device = x.device if (is_t and x.is_cuda) else torch.device("cuda", torch.cuda.current_device())
     xt = _to_device(x, torch, device)
     if xt.dtype == torch.float32:
@@ -326,7 +328,7 @@ def quantized_matmul(x, w_packed, scales, *, mode: str = "mxfp4", K: int, out_dt
         if wp.shape != (N, K // pack) or sc.shape != (N, K // cfg["group_size"]):
             raise ValueError(f"packed weights {tuple(wp.shape)} / scales {tuple(sc.shape)} do not match N={N}, K={K}")
         _lib.check(_lib.load().qmm_mx_matmul(x2.data_ptr(), wp.data_ptr(), sc.data_ptr(), y.data_ptr(), M, N, K,
-                                             _lib.MX_MODE_IDS[mode], tag, torch.cuda.current_stream().cuda_stream))
+                                             _lib.MX_MODE_IDS[mode], tag, torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())))
 
     return _launch_matmul(x, call, N, K, out_dtype)
 
@@ -356,6 +358,6 @@ def affine_quantized_matmul(x, w_packed, scales, biases, *, bits: int = 4, group
             raise ValueError(f"packed weights {tuple(wp.shape)} / scales {tuple(sc.shape)} do not match N={N}, K={K}")
         _lib.check(_lib.load().qmm_affine_matmul(x2.data_ptr(), wp.data_ptr(), sc.data_ptr(), bi.data_ptr(),
                                                  y.data_ptr(), M, N, K, bits, group_size, tag,
-                                                 torch.cuda.current_stream().cuda_stream))
+                                                 torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())))
 
     return _launch_matmul(x, call, N, K, out_dtype)
