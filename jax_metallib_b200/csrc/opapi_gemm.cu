@@ -124,20 +124,22 @@ __device__ __forceinline__ uint32_t f16x2_to_bf16x2(uint32_t h) {
 // Eight codes of k .. k+7 -> eight 16-bit operand values in k order.  For 4-bit formats `lo` holds all eight.
 //   integers:  128 + q or 1024 + q by OR-ing the code into a constant's mantissa, minus that constant.  An 8-bit code
 //              in bf16 reads as q * 2^-133 where it stands (a subnormal up to 127, the first binade above) and is
-//              multiplied by 2^127: q / 64, the group's scale makes up for it.  Codes are not centred: a flat group
-//              has scale 1, code 0 and its value as bias, which a centred code would cancel away.
+//              multiplied by 2^127: q / 64, the group's scale makes up for it.  Against f32 results a code may go in
+//              centred (centred(): q - 8 or q - 128).
 //   e2m1:      cvt to f16; for bf16 the code's exponent and mantissa are moved into place (worth 2^-126 of the
 //              element) and multiplied by 2^126
 //   e4m3:      cvt to f16, then to bf16 (4 significant bits: exact)
 template <int FMT, bool BF16>
-__device__ __forceinline__ uint4 convert8(uint32_t lo, uint32_t hi, uint32_t scale2) {
+__device__ __forceinline__ uint4 convert8(uint32_t lo, uint32_t hi, uint32_t scale2, bool centre) {
   uint32_t r[4];
   if (FMT == kAffine8) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint32_t sel = (i & 1) ? 0x4342 : 0x4140;
-      if (BF16) r[i] = mul2<true>(__byte_perm(i < 2 ? lo : hi, 0u, sel), 0x7F007F00u);   // q * 2^-133 * 2^127
-      else r[i] = sub2<false>(__byte_perm(i < 2 ? lo : hi, 0x64646464u, sel), 0x64006400u);
+      if (BF16) {   // q * 2^-133 * 2^127, minus 2 for a centred code
+        const uint32_t c = centre ? 0xC000C000u : 0u;
+        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r[i]) : "r"(__byte_perm(i < 2 ? lo : hi, 0u, sel)), "r"(0x7F007F00u), "r"(c));
+      } else r[i] = sub2<false>(__byte_perm(i < 2 ? lo : hi, 0x64646464u, sel), 0x64006400u);
     }
   } else if (FMT == kMxfp8) {
     e4m3_to_f16(lo, r[0], r[1]);
@@ -156,7 +158,7 @@ __device__ __forceinline__ uint4 convert8(uint32_t lo, uint32_t hi, uint32_t sca
       const uint32_t p = __byte_perm(e, o, static_cast<uint32_t>(i) | (4u + i) << 8);
       if (FMT == kAffine4) {
         const uint32_t t = lop_and_or(p, 0x000F000Fu, BF16 ? 0x43004300u : 0x64006400u);
-        r[i] = sub2<BF16>(t, BF16 ? 0x43004300u : 0x64006400u);
+        r[i] = sub2<BF16>(t, BF16 ? (centre ? 0x43084308u : 0x43004300u) : 0x64006400u);
       } else {
         const uint32_t mag = (p & 0x00070007u) << 6, sgn = (p & 0x00080008u) << 12;
         r[i] = mul2<true>(mag | sgn, 0x7E807E80u);                       // times 2^126
@@ -168,6 +170,15 @@ __device__ __forceinline__ uint4 convert8(uint32_t lo, uint32_t hi, uint32_t sca
     for (int i = 0; i < 4; ++i) r[i] = mul2<BF16>(r[i], scale2);
   }
   return make_uint4(r[0], r[1], r[2], r[3]);
+}
+
+// Whether a group's integer codes go in centred (f32 results).  scale * q + bias = scale * (q - c) + (bias + c * scale):
+// the usual group spans zero, its bias is about -c * scale, and the two parts of its sum would cancel to half their
+// size.  A flat group has scale 1, code 0 and its value as bias: centring it would make the parts large instead.
+template <int FMT>
+__device__ __forceinline__ bool centred(float s, float b, float& shifted) {
+  shifted = fmaf(FMT == kAffine4 ? 8.f : 128.f, s, b);
+  return fabsf(shifted) < fabsf(b);
 }
 
 // e4m3 scale byte -> (s, s) in f16 or bf16
@@ -354,7 +365,33 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     const int stages_per_unit = a.pu > BK ? a.pu / BK : 1;
     const int units_per_stage = a.pu < BK ? BK / a.pu : 1;
     uint32_t flag_carry = 0;
+    // f32 results: scale and bias of this thread's rows in the next stage, for the decision to centre their codes
+    constexpr bool kCentre = C::kBias && XF32;
+    constexpr int kRows = C::kBits == 4 ? 1 : 2;
+    float csc[kRows], cbi[kRows];
+    auto load_centre = [&](int st) {
+      if (kCentre) {
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+          const int n = min(n0 + (C::kBits == 4 ? (wt >> 1) : (wt >> 2) + i * 64), a.N - 1);
+          const int k = min(k_begin + st * BK + (C::kBits == 4 ? (wt & 1) * 32 : (wt & 3) * 16), a.K - 1);
+          const size_t g = static_cast<size_t>(n) * (a.K / a.gs) + k / a.gs;
+          csc[i] = __ldg(static_cast<const float*>(a.scales) + g);
+          cbi[i] = __ldg(a.biases + g);
+        }
+      }
+    };
+    load_centre(0);
     for (int st = 0; st < stages; ++st) {
+      bool centre[2] = {false, false};
+      if (kCentre) {
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+          float shifted;
+          centre[i] = centred<FMT>(csc[i], cbi[i], shifted);
+        }
+        if (st + 1 < stages) load_centre(st + 1);
+      }
       const int op = st % C::kOps;
       uint8_t* opA = smem + op * C::kOpBytes;
       const int box = st / C::kStagesPerBox, sub = st % C::kStagesPerBox, rs = box % C::kRawBoxes;
@@ -385,15 +422,15 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       if (C::kBits == 4) {
         uint32_t sc[2] = {0u, 0u};
         if (FMT == kNvfp4) { sc[0] = e4m3_pair<XF32>(nsc[0]); sc[1] = e4m3_pair<XF32>(nsc[1]); }
-        o[0] = convert8<FMT, XF32>(v[0].x, 0u, sc[0]);
-        o[1] = convert8<FMT, XF32>(v[0].y, 0u, sc[0]);
-        o[2] = convert8<FMT, XF32>(v[0].z, 0u, sc[1]);
-        o[3] = convert8<FMT, XF32>(v[0].w, 0u, sc[1]);
+        o[0] = convert8<FMT, XF32>(v[0].x, 0u, sc[0], centre[0]);
+        o[1] = convert8<FMT, XF32>(v[0].y, 0u, sc[0], centre[0]);
+        o[2] = convert8<FMT, XF32>(v[0].z, 0u, sc[1], centre[0]);
+        o[3] = convert8<FMT, XF32>(v[0].w, 0u, sc[1], centre[0]);
       } else {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          o[2 * i] = convert8<FMT, XF32>(v[i].x, v[i].y, 0u);
-          o[2 * i + 1] = convert8<FMT, XF32>(v[i].z, v[i].w, 0u);
+          o[2 * i] = convert8<FMT, XF32>(v[i].x, v[i].y, 0u, centre[i]);
+          o[2 * i + 1] = convert8<FMT, XF32>(v[i].z, v[i].w, 0u, centre[i]);
         }
       }
       if (st >= C::kOps) {   // the MMAs that read this operand stage before have retired
@@ -540,7 +577,12 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         const int u = ub + i;
         if (!ok || u >= units) break;
         const int buf = u % kAccBufs, slot = u % kInfo;
-        const float s = (FMT == kAffine8 && XF32) ? sv[i] * 64.f : sv[i], b = bv[i];
+        const float s = (FMT == kAffine8 && XF32) ? sv[i] * 64.f : sv[i];
+        float b = bv[i];
+        if (C::kBias && XF32) {
+          float shifted;
+          if (centred<FMT>(sv[i], bv[i], shifted)) b = shifted;
+        }
         load_scale(u + kAhead, sv[i], bv[i]);
         bool exact = false;
         if (C::kUnitInfo) {
