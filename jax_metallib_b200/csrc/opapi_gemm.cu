@@ -6,17 +6,17 @@
 // The weights go to tcgen05.mma as their bare codes c (an integer, or the e2m1 / e4m3 element), which
 // both 16-bit types hold exactly: f16 against f16 activations, bf16 against f32 activations, which are cut into
 // three bf16 terms that add up to all 24 bits.  Every product is therefore exact.  The accumulator of one unit of
-// k (a scale group of up to 128 k) is read back from TMEM and multiplied by the group's f32 scale into f32
-// registers, so that scales and biases stay in 32 bits and the tensor core adds up no more than 128 k before a
+// k (a scale group or a part of one, up to 64 k) is read back from TMEM and multiplied by the group's f32 scale into f32
+// registers, so that scales and biases stay in 32 bits and the tensor core adds up no more than 64 k before a
 // correctly rounded f32 addition takes over.  nvfp4, whose groups of 16 would be too short for that, multiplies
 // its elements by their e4m3 scale first: 2 + 4 significant bits, exact as well.
 //
 // A CTA computes 128 columns (the MMA's 128 rows: a lane of the accumulator is a column, so a scale is one
 // register) x BM rows over a slice of K; the CTAs of a cluster share an output tile and add their slices over
-// distributed shared memory in a fixed order.  Warps: a TMA producer (raw weights in boxes of 128 rows x 128
-// bytes, activations), an MMA issuer, eight workers that turn raw codes into the swizzled operand (and f32
-// activations into their three terms, and sum the activations of a unit for the biases) and four or eight
-// promoters that drain the accumulators.
+// distributed shared memory in a fixed order.  Warps: two TMA producers (raw weights in boxes of 128 rows x 128
+// bytes with their scales; activations), groups of one MMA issuer and four workers that turn raw codes into the swizzled operand (and f32
+// activations into their three terms, and sum the activations of a unit for the biases) and four to
+// sixteen promoters that drain the accumulators.
 //
 // What the split cannot represent takes an exact path: a unit whose activations are not finite (inf times
 // code plus inf times bias is not what inf times scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
@@ -34,14 +34,15 @@ enum { kAffine4 = 0, kAffine8 = 1, kMxfp4 = 2, kMxfp8 = 3, kNvfp4 = 4 };
 
 constexpr int BN = 128;               // output columns per CTA
 constexpr int BK = 64;                // k per operand stage: one 128-byte row of 16-bit values
-constexpr int kWorkerWarps = 8;
+constexpr int kGroupWarps = 4;        // warps that convert one stage; the groups take the stages in turn
 constexpr int kRawBox = BN * 128;     // 16 KB of raw weights
 constexpr int kABytes = BN * BK * 2;  // 16 KB
-constexpr int kXSlots = 4;            // f16 activations: operand tiles straight from TMA
 constexpr int kAccBufs = 4;           // accumulators between the tensor core and the promoters
 constexpr int kInfo = 16;             // units whose activation sums and flags are kept
-constexpr int kConsumed = 12;         // a multiple of the operand ring (2 or 3) and of kXSlots
+constexpr int kConsumed = 12;         // a multiple of the operand ring (3 or 4) and of the activation ring
 constexpr int kMaxCluster = 8;
+constexpr int kSBoxes = 3;            // boxes of scales (and biases) on their way to the promoters
+constexpr int kSBoxBytes = 2 * BN * 16;
 
 template <int FMT, bool XF32, int BM>
 struct Cfg {
@@ -53,23 +54,32 @@ struct Cfg {
   static constexpr int kStagesPerBox = kBoxK / BK;          // 4 or 2
   static constexpr int kXTile = BM * BK * 2;                // one 16-bit operand tile of activations
   static constexpr int kXRaw = BM * BK * 4;                 // raw f32 activations of a stage
-  static constexpr int kOps = BM == 32 ? 2 : 3;             // operand stages
+  // A stage passes through a worker in ~0.6 us of dependent waits, loads and stores, whatever its share of the work:
+  // throughput comes from stages converted side by side.  (One group of eight warps: 1.2 us per stage for mxfp8,
+  // 2.5 us with activation sums, 3.3 us with f32 activations.)
+  static constexpr int kGroups = BM == 32 ? 4 : (BM == 64 ? 3 : 2);
+  static constexpr int kWorkerWarps = kGroups * kGroupWarps;
+  static constexpr int kOps = XF32 && BM == 64 ? 3 : 4;         // operand stages
   static constexpr int kOpBytes = kABytes + (XF32 ? 3 * kXTile : 0);
-  static constexpr int kXRing = XF32 ? (BM == 32 ? 2 : 3) : kXSlots;
+  static constexpr int kXRing = XF32 && BM == 64 ? 3 : 4;
   static constexpr int kXBytes = XF32 ? kXRaw : kXTile;
-  static constexpr int kRawBoxes = BM == 32 ? (XF32 ? 2 : 3) : 3;
+  static constexpr int kRawBoxes = XF32 && BM == 64 ? 2 : 3;
   static constexpr int kOffX = kOps * kOpBytes;
   static constexpr int kOffRaw = kOffX + kXRing * kXBytes;
   static constexpr int kOffInfo = kOffRaw + kRawBoxes * kRawBox;
-  static constexpr int kOffFlags = kOffInfo + kInfo * BM * 4;
-  static constexpr int kOffBar = kOffFlags + kInfo * 8;
+  static constexpr int kOffS = kOffInfo + kInfo * BM * 4;
+  static constexpr int kOffFlags = kOffS + (FMT == kNvfp4 ? 0 : kSBoxes * kSBoxBytes);
+  static constexpr int kOffBar = kOffFlags + kInfo * kGroupWarps;
   static constexpr int kSmem = kOffBar + 512 + 1024;
-  static constexpr int kPromoters = BM == 32 ? 4 : 8;
-  static constexpr int kThreads = (2 + kWorkerWarps + kPromoters) * 32;
-  static constexpr int kMinBlocks = BM == 32 ? 2 : 1;
-  static constexpr int kCols = BM * 4 / kPromoters;         // accumulator columns per promoter: 32, 32 or 64
+  static constexpr int kPromoters = BM / 8;               // four lane quarters x 32 columns each
+  static constexpr int kFirstIssuer = 2;
+  static constexpr int kFirstWorker = kFirstIssuer + kGroups;   // one issuing warp per group
+  static constexpr int kFirstPromoter = kFirstWorker + kWorkerWarps;
+  static constexpr int kThreads = (kFirstPromoter + kPromoters) * 32;
+  static constexpr int kCols = 32;                        // accumulator columns per promoter
+  static_assert(kOps <= kAccBufs, "one unit per stage: an accumulator's previous unit is issued before the next is full");
   static_assert(BM * BN * 4 <= kOffInfo, "the result tile reuses the rings");
-  static_assert(kSmem * kMinBlocks <= 227 * 1024, "shared memory");
+  static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 
 struct Args {
@@ -78,8 +88,9 @@ struct Args {
   const void* scales;
   const float* biases;
   void* y;
-  int M, N, K, gs, pu;        // pu: k per unit (32, 64 or 128)
+  int M, N, K, gs, pu;        // pu: k per unit (32 or 64)
   int blocks, block_k;        // K in blocks of the slice granularity
+  int sbox_k;                 // k per box of scales; 0: their rows are not made of 16-byte pieces, promoters read them
   uint32_t idesc;
   int* status;
 };
@@ -235,13 +246,14 @@ __device__ __noinline__ float exact_unit(const Args& a, int m, int n, int k0, in
 }
 
 template <int FMT, bool XF32, int BM>
-__global__ void __launch_bounds__(Cfg<FMT, XF32, BM>::kThreads, Cfg<FMT, XF32, BM>::kMinBlocks)
-opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ Args a) {
+__global__ void __launch_bounds__(Cfg<FMT, XF32, BM>::kThreads, 1)
+opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+              const __grid_constant__ CUtensorMap smap, const __grid_constant__ CUtensorMap bmap, const __grid_constant__ Args a) {
   using C = Cfg<FMT, XF32, BM>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   float* xsum = reinterpret_cast<float*>(smem + C::kOffInfo);        // [kInfo][BM]
-  uint8_t* flags = smem + C::kOffFlags;                              // [kInfo][8], one byte per worker warp
+  uint8_t* flags = smem + C::kOffFlags;                              // [kInfo][4], one byte per warp of a group
   uint64_t* wfull = reinterpret_cast<uint64_t*>(smem + C::kOffBar);  // raw weights landed
   uint64_t* wempty = wfull + C::kRawBoxes;                           // raw weights read
   uint64_t* xfull = wempty + C::kRawBoxes;                           // activations landed
@@ -251,7 +263,9 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
   uint64_t* tfull = consumed + kConsumed;                            // a unit's accumulator complete
   uint64_t* tempty = tfull + kAccBufs;                               // and drained
   uint64_t* ifull = tempty + kAccBufs;                               // sums and flags of a unit written
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ifull + kInfo);
+  uint64_t* sfull = ifull + kInfo;                                   // a box of scales landed
+  uint64_t* sempty = sfull + kSBoxes;                                // and read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sempty + kSBoxes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KS = gridDim.x, rank = blockIdx.x;
@@ -261,14 +275,20 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
   const int stages = (k_end - k_begin + BK - 1) / BK;
   const int units = (k_end - k_begin + a.pu - 1) / a.pu;
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < C::kRawBoxes; ++i) { dev::mbar_init(&wfull[i], 1); dev::mbar_init(&wempty[i], kWorkerWarps); }
-    for (int i = 0; i < C::kXRing; ++i) { dev::mbar_init(&xfull[i], 1); dev::mbar_init(&xempty[i], kWorkerWarps); }
-    for (int i = 0; i < C::kOps; ++i) dev::mbar_init(&full[i], kWorkerWarps);
-    for (int i = 0; i < kConsumed; ++i) dev::mbar_init(&consumed[i], 1);
-    for (int i = 0; i < kAccBufs; ++i) { dev::mbar_init(&tfull[i], 1); dev::mbar_init(&tempty[i], C::kPromoters); }
-    for (int i = 0; i < kInfo; ++i) dev::mbar_init(&ifull[i], kWorkerWarps);
+  if (warp == 0) {   // one barrier of each kind per lane
+    if (lane < C::kRawBoxes) { dev::mbar_init(&wfull[lane], 1); dev::mbar_init(&wempty[lane], C::kStagesPerBox * kGroupWarps); }
+    if (lane < C::kXRing) { dev::mbar_init(&xfull[lane], 1); dev::mbar_init(&xempty[lane], kGroupWarps); }
+    if (lane < C::kOps) dev::mbar_init(&full[lane], kGroupWarps);
+    if (lane < kConsumed) dev::mbar_init(&consumed[lane], 1);
+    if (lane < kAccBufs) { dev::mbar_init(&tfull[lane], 1); dev::mbar_init(&tempty[lane], C::kPromoters); }
+    if (lane < kInfo) dev::mbar_init(&ifull[lane], kGroupWarps);
+    if (lane < kSBoxes) { dev::mbar_init(&sfull[lane], 1); dev::mbar_init(&sempty[lane], C::kPromoters); }
     dev::fence_mbar_init();
+  } else if (warp == 2 && lane == 0) {
+    dev::tma_prefetch_desc(&wmap);
+    dev::tma_prefetch_desc(&xmap);
+    dev::tma_prefetch_desc(&smap);
+    dev::tma_prefetch_desc(&bmap);
   }
   if (warp == 1) {
     dev::tmem_alloc(tmem_slot, kAccBufs * BM);
@@ -281,26 +301,14 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
   dev::pdl_wait();
   dev::pdl_launch_dependents();
 
-  constexpr int kFirstPromoter = 2 + kWorkerWarps;
+  constexpr int kFirstPromoter = C::kFirstPromoter;
   float* tile = reinterpret_cast<float*>(smem);   // [BM][BN] f32 partial results, once the rings are idle
 
   if (warp == 0) {
-    // ------------------------------ TMA producer ---------------------------
+    // ------------------------ TMA producer: activations --------------------
     if (lane == 0) {
-      dev::tma_prefetch_desc(&wmap);
-      dev::tma_prefetch_desc(&xmap);
-      const int boxes = (stages + C::kStagesPerBox - 1) / C::kStagesPerBox;
-      int wi = 0, xi = 0;
-      // weights run ahead of the activations as far as their ring allows
-      while (wi < boxes || xi < stages) {
-        if (wi < boxes && wi < xi / C::kStagesPerBox + C::kRawBoxes) {
-          const int s = wi % C::kRawBoxes;
-          if (!dev::mbar_wait_relaxed(&wempty[s], ((wi / C::kRawBoxes) & 1) ^ 1, a.status, 90)) break;
-          dev::mbar_expect_tx(&wfull[s], kRawBox);
-          dev::tma_load_2d(smem + C::kOffRaw + s * kRawBox, &wmap, &wfull[s], k_begin * C::kBits / 8 + wi * 128, n0);
-          ++wi;
-          continue;
-        }
+      int xi = 0;
+      for (; xi < stages; ++xi) {
         const int s = xi % C::kXRing;
         if (XF32) {
           if (!dev::mbar_wait_relaxed(&xempty[s], ((xi / C::kXRing) & 1) ^ 1, a.status, 91)) break;
@@ -310,50 +318,90 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         }
         dev::mbar_expect_tx(&xfull[s], C::kXBytes);
         dev::tma_load_2d(smem + C::kOffX + s * C::kXBytes, &xmap, &xfull[s], k_begin + xi * BK, m0);
-        ++xi;
       }
       // every copy has landed before this CTA's shared memory is reused, whatever the other warps did
-      for (int i = wi > C::kRawBoxes ? wi - C::kRawBoxes : 0; i < wi; ++i)
-        if (!dev::mbar_wait_relaxed(&wfull[i % C::kRawBoxes], (i / C::kRawBoxes) & 1, a.status, 92)) break;
       for (int i = xi > C::kXRing ? xi - C::kXRing : 0; i < xi; ++i)
         if (!dev::mbar_wait_relaxed(&xfull[i % C::kXRing], (i / C::kXRing) & 1, a.status, 93)) break;
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer -----------------------------
+    // ------------------- TMA producer: raw weights and scales --------------
+    // A box of scales goes out just before the weights of its first stage.
+    if (lane == 0) {
+      const int boxes = (stages + C::kStagesPerBox - 1) / C::kStagesPerBox;
+      const bool boxed = FMT != kNvfp4 && a.sbox_k != 0;
+      const int sstages = boxed ? a.sbox_k / BK : 1;   // stages per box of scales
+      const int sboxes = boxed ? (stages + sstages - 1) / sstages : 0;
+      int wi = 0, si = 0;
+      while (wi < boxes) {
+        while (si < sboxes && si * sstages < (wi + 1) * C::kStagesPerBox) {
+          const int s = si % kSBoxes;
+          if (!dev::mbar_wait_relaxed(&sempty[s], ((si / kSBoxes) & 1) ^ 1, a.status, 89)) goto drained;
+          uint8_t* dst = smem + C::kOffS + s * kSBoxBytes;
+          dev::mbar_expect_tx(&sfull[s], C::kBias ? kSBoxBytes : BN * 16);
+          const int c = (k_begin + si * a.sbox_k) / a.gs;   // first group of the box
+          dev::tma_load_2d(dst, &smap, &sfull[s], c, n0);
+          if (C::kBias) dev::tma_load_2d(dst + BN * 16, &bmap, &sfull[s], c, n0);
+          ++si;
+        }
+        const int s = wi % C::kRawBoxes;
+        if (!dev::mbar_wait_relaxed(&wempty[s], ((wi / C::kRawBoxes) & 1) ^ 1, a.status, 90)) break;
+        dev::mbar_expect_tx(&wfull[s], kRawBox);
+        dev::tma_load_2d(smem + C::kOffRaw + s * kRawBox, &wmap, &wfull[s], k_begin * C::kBits / 8 + wi * 128, n0);
+        ++wi;
+      }
+    drained:
+      for (int i = wi > C::kRawBoxes ? wi - C::kRawBoxes : 0; i < wi; ++i)
+        if (!dev::mbar_wait_relaxed(&wfull[i % C::kRawBoxes], (i / C::kRawBoxes) & 1, a.status, 92)) break;
+      for (int i = si > kSBoxes ? si - kSBoxes : 0; i < si; ++i)
+        if (!dev::mbar_wait_relaxed(&sfull[i % kSBoxes], (i / kSBoxes) & 1, a.status, 88)) break;
+    }
+    __syncwarp();
+  } else if (warp < C::kFirstWorker) {
+    // ------------------------------ MMA issuers ----------------------------
+    // One per worker group: an MMA costs its issuing thread some 140 clocks, which with twelve of them per stage (f32)
+    // would bound everything; the units of different stages are independent.
     if (lane == 0) {
       constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // SBO, version, 128-byte swizzle
       const uint32_t op_lo = ((dev::smem_u32(smem) >> 4) & 0x3FFF) | ((16u >> 4) << 16);
       const uint32_t x_lo = ((dev::smem_u32(smem + C::kOffX) >> 4) & 0x3FFF) | ((16u >> 4) << 16);
-      const int steps_per_unit = a.pu / 16;
-      const int per = steps_per_unit < 4 ? steps_per_unit : 4;   // k-steps of a stage that belong to one unit
-      int u = 0, in_unit = 0;
+      const int units_per_stage = a.pu < BK ? BK / a.pu : 1;
       bool ok = true;
-      for (int st = 0; ok && st < stages; ++st) {
+      for (int st = warp - C::kFirstIssuer; ok && st < stages; st += C::kGroups) {
         const int s = st % C::kOps;
         if (!dev::mbar_wait(&full[s], (st / C::kOps) & 1, a.status, 94)) break;
+        // Two units per stage: a stage may be full while the one four units back, which shares its accumulators, has not
+        // been issued; its parity would read as drained.  With one unit per stage the operand ring keeps that apart.
+        if (units_per_stage == 2 && st >= 2 &&
+            !dev::mbar_wait(&consumed[(st - 2) % kConsumed], ((st - 2) / kConsumed) & 1, a.status, 102))
+          break;
         dev::tc_fence_after();
         const uint32_t a_lo = op_lo + s * (C::kOpBytes >> 4);
         const uint32_t b_lo = XF32 ? a_lo + (kABytes >> 4) : x_lo + (st % C::kXRing) * (C::kXTile >> 4);
-        for (int j0 = 0; j0 < 4 && u < units; j0 += per) {         // (the zero half of a last stage is skipped)
+        for (int h = 0; h < units_per_stage; ++h) {
+          const int u = st * units_per_stage + h;
+          if (u >= units) break;                                   // the zero half of a last stage
           const int buf = u % kAccBufs;
-          if (in_unit == 0) {
-            if (!dev::mbar_wait(&tempty[buf], ((u / kAccBufs) & 1) ^ 1, a.status, 95)) { ok = false; break; }
-            dev::tc_fence_after();
-          }
+          if (!dev::mbar_wait(&tempty[buf], ((u / kAccBufs) & 1) ^ 1, a.status, 95)) { ok = false; break; }
+          dev::tc_fence_after();
           const uint32_t d = tmem_base + buf * BM;
           // the smallest terms first: the accumulator is still small when they are added
+          if (units_per_stage == 1) {
 #pragma unroll
-          for (int t = C::kTerms - 1; t >= 0; --t)
-            for (int j = j0; j < j0 + per; ++j)
-              dev::umma_f16_lh(d, a_lo + j * 2, kDescHi, b_lo + t * (C::kXTile >> 4) + j * 2, kDescHi, a.idesc,
-                               (in_unit != 0 || t != C::kTerms - 1 || j != j0) ? 1u : 0u);
-          in_unit += per;
-          if (in_unit == steps_per_unit || st == stages - 1) {
-            dev::tc_commit(&tfull[buf]);
-            in_unit = 0;
-            ++u;
+            for (int t = C::kTerms - 1; t >= 0; --t)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                dev::umma_f16_lh(d, a_lo + j * 2, kDescHi, b_lo + t * (C::kXTile >> 4) + j * 2, kDescHi, a.idesc,
+                                 (t != C::kTerms - 1 || j != 0) ? 1u : 0u);
+          } else {
+#pragma unroll
+            for (int t = C::kTerms - 1; t >= 0; --t)
+#pragma unroll
+              for (int j = 0; j < 2; ++j)
+                dev::umma_f16_lh(d, a_lo + h * 4 + j * 2, kDescHi, b_lo + t * (C::kXTile >> 4) + h * 4 + j * 2, kDescHi, a.idesc,
+                                 (t != C::kTerms - 1 || j != 0) ? 1u : 0u);
           }
+          dev::tc_commit(&tfull[buf]);
         }
         if (ok) dev::tc_commit(&consumed[st % kConsumed]);
       }
@@ -361,106 +409,93 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     __syncwarp();
   } else if (warp < kFirstPromoter) {
     // ------------------------------ workers --------------------------------
-    const int ww = warp - 2, wt = threadIdx.x - 64;   // 0 .. 255
-    const int stages_per_unit = a.pu > BK ? a.pu / BK : 1;
+    const int grp = (warp - C::kFirstWorker) / kGroupWarps, ww = (warp - C::kFirstWorker) % kGroupWarps;
+    const int wt = ww * 32 + lane;                    // 0 .. 127
     const int units_per_stage = a.pu < BK ? BK / a.pu : 1;
-    uint32_t flag_carry = 0;
-    // f32 results: scale and bias of this thread's rows in the next stage, for the decision to centre their codes
+    constexpr int kW = C::kBits == 4 ? 2 : 4;         // 16-byte pieces of weights per thread: row wrow(i), piece wpiece of the stage
+    const int wpiece = C::kBits == 4 ? (wt & 1) : (wt & 3);
+    auto wrow = [&](int i) { return C::kBits == 4 ? (wt >> 1) + i * 64 : (wt >> 2) + i * 32; };
+    constexpr int kPieceK = C::kBits == 4 ? 32 : 16;  // k of a piece
+    // f32 results: scale and bias of this thread's rows in its next stage, for the decision to centre their codes
     constexpr bool kCentre = C::kBias && XF32;
-    constexpr int kRows = C::kBits == 4 ? 1 : 2;
-    float csc[kRows], cbi[kRows];
+    float csc[kW], cbi[kW];
     auto load_centre = [&](int st) {
       if (kCentre) {
 #pragma unroll
-        for (int i = 0; i < kRows; ++i) {
-          const int n = min(n0 + (C::kBits == 4 ? (wt >> 1) : (wt >> 2) + i * 64), a.N - 1);
-          const int k = min(k_begin + st * BK + (C::kBits == 4 ? (wt & 1) * 32 : (wt & 3) * 16), a.K - 1);
+        for (int i = 0; i < kW; ++i) {
+          const int n = min(n0 + wrow(i), a.N - 1), k = min(k_begin + st * BK + wpiece * kPieceK, a.K - 1);
           const size_t g = static_cast<size_t>(n) * (a.K / a.gs) + k / a.gs;
           csc[i] = __ldg(static_cast<const float*>(a.scales) + g);
           cbi[i] = __ldg(a.biases + g);
         }
       }
     };
-    load_centre(0);
-    for (int st = 0; st < stages; ++st) {
-      bool centre[2] = {false, false};
-      if (kCentre) {
-#pragma unroll
-        for (int i = 0; i < kRows; ++i) {
-          float shifted;
-          centre[i] = centred<FMT>(csc[i], cbi[i], shifted);
-        }
-        if (st + 1 < stages) load_centre(st + 1);
-      }
+    load_centre(grp);
+    for (int st = grp; st < stages; st += C::kGroups) {
       const int op = st % C::kOps;
       uint8_t* opA = smem + op * C::kOpBytes;
       const int box = st / C::kStagesPerBox, sub = st % C::kStagesPerBox, rs = box % C::kRawBoxes;
       const uint8_t* raw = smem + C::kOffRaw + rs * kRawBox;
-      // nvfp4: the two scales of this thread's 32 k, fetched before the wait for the weights
-      uint32_t nsc[2] = {0u, 0u};
+      bool centre[kW];
+#pragma unroll
+      for (int i = 0; i < kW; ++i) {
+        float shifted;
+        centre[i] = kCentre && centred<FMT>(csc[i], cbi[i], shifted);
+      }
+      if (st + C::kGroups < stages) load_centre(st + C::kGroups);
+      // nvfp4: the two scales of each piece's 32 k, fetched before the wait for the weights
+      uint32_t nsc[kW][2];
       if (FMT == kNvfp4) {
-        const int n = n0 + (wt >> 1), k = k_begin + st * BK + (wt & 1) * 32;
-        if (n < a.N && k < a.K) {
-          const uint8_t* sp = static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(n) * (a.K / 16) + k / 16;
-          nsc[0] = __ldg(sp);
-          nsc[1] = __ldg(sp + 1);
+#pragma unroll
+        for (int i = 0; i < kW; ++i) {
+          const int n = n0 + wrow(i), k = k_begin + st * BK + wpiece * 32;
+          nsc[i][0] = nsc[i][1] = 0u;
+          if (n < a.N && k < a.K) {
+            const uint8_t* sp = static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(n) * (a.K / 16) + k / 16;
+            nsc[i][0] = __ldg(sp);
+            nsc[i][1] = __ldg(sp + 1);
+          }
         }
       }
-      if (sub == 0 && !dev::mbar_wait_warp(&wfull[rs], (box / C::kRawBoxes) & 1, a.status, 96)) break;
-      uint4 v[2];
-      if (C::kBits == 4) {
-        const int row = wt >> 1, c = sub * 2 + (wt & 1);
-        v[0] = *reinterpret_cast<const uint4*>(raw + row * 128 + ((c ^ (row & 7)) << 4));
-      } else {
+      if (!dev::mbar_wait_relaxed_warp(&wfull[rs], (box / C::kRawBoxes) & 1, a.status, 96)) break;
+      uint4 v[kW];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int row = (wt >> 2) + i * 64, c = sub * 4 + (wt & 3);
-          v[i] = *reinterpret_cast<const uint4*>(raw + row * 128 + ((c ^ (row & 7)) << 4));
-        }
-      }
-      uint4 o[4];
-      if (C::kBits == 4) {
-        uint32_t sc[2] = {0u, 0u};
-        if (FMT == kNvfp4) { sc[0] = e4m3_pair<XF32>(nsc[0]); sc[1] = e4m3_pair<XF32>(nsc[1]); }
-        o[0] = convert8<FMT, XF32>(v[0].x, 0u, sc[0], centre[0]);
-        o[1] = convert8<FMT, XF32>(v[0].y, 0u, sc[0], centre[0]);
-        o[2] = convert8<FMT, XF32>(v[0].z, 0u, sc[1], centre[0]);
-        o[3] = convert8<FMT, XF32>(v[0].w, 0u, sc[1], centre[0]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          o[2 * i] = convert8<FMT, XF32>(v[i].x, v[i].y, 0u, centre[i]);
-          o[2 * i + 1] = convert8<FMT, XF32>(v[i].z, v[i].w, 0u, centre[i]);
-        }
+      for (int i = 0; i < kW; ++i) {
+        const int row = wrow(i), c = sub * (C::kBits == 4 ? 2 : 4) + wpiece;
+        v[i] = *reinterpret_cast<const uint4*>(raw + row * 128 + ((c ^ (row & 7)) << 4));
       }
       if (st >= C::kOps) {   // the MMAs that read this operand stage before have retired
         const int prev = st - C::kOps;
-        if (!dev::mbar_wait_warp(&consumed[prev % kConsumed], (prev / kConsumed) & 1, a.status, 97)) break;
+        if (!dev::mbar_wait_relaxed_warp(&consumed[prev % kConsumed], (prev / kConsumed) & 1, a.status, 97)) break;
       }
-      if (C::kBits == 4) {
-        const int row = wt >> 1;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(opA + row * 128 + ((((wt & 1) * 4 + i) ^ (row & 7)) << 4)) = o[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = (wt >> 2) + (i >> 1) * 64;
-          *reinterpret_cast<uint4*>(opA + row * 128 + ((((wt & 3) * 2 + (i & 1)) ^ (row & 7)) << 4)) = o[i];
+      for (int i = 0; i < kW; ++i) {
+        const int row = wrow(i);
+        auto put = [&](int chunk, const uint4& o) {
+          *reinterpret_cast<uint4*>(opA + row * 128 + ((chunk ^ (row & 7)) << 4)) = o;
+        };
+        if (C::kBits == 4) {
+          uint32_t sc[2] = {0u, 0u};
+          if (FMT == kNvfp4) { sc[0] = e4m3_pair<XF32>(nsc[i][0]); sc[1] = e4m3_pair<XF32>(nsc[i][1]); }
+          put(wpiece * 4, convert8<FMT, XF32>(v[i].x, 0u, sc[0], centre[i]));
+          put(wpiece * 4 + 1, convert8<FMT, XF32>(v[i].y, 0u, sc[0], centre[i]));
+          put(wpiece * 4 + 2, convert8<FMT, XF32>(v[i].z, 0u, sc[1], centre[i]));
+          put(wpiece * 4 + 3, convert8<FMT, XF32>(v[i].w, 0u, sc[1], centre[i]));
+        } else {
+          put(wpiece * 2, convert8<FMT, XF32>(v[i].x, v[i].y, 0u, centre[i]));
+          put(wpiece * 2 + 1, convert8<FMT, XF32>(v[i].z, v[i].w, 0u, centre[i]));
         }
       }
       // ---- activations: eight lanes per row, eight k each
       const int xs = st % C::kXRing;
-      if (!dev::mbar_wait_warp(&xfull[xs], (st / C::kXRing) & 1, a.status, 98)) break;
-      const int slot = (units_per_stage == 2 ? 2 * st : st / stages_per_unit) % kInfo;   // first unit of this stage
-      const bool first = st % stages_per_unit == 0;
-      const bool last = st % stages_per_unit == stages_per_unit - 1 || st == stages - 1;
+      if (!dev::mbar_wait_relaxed_warp(&xfull[xs], (st / C::kXRing) & 1, a.status, 98)) break;
+      const int slot = (units_per_stage * st) % kInfo;   // first unit of this stage (a unit with sums is at most a stage)
       if (C::kUnitInfo) {
         const uint8_t* xt = smem + C::kOffX + xs * C::kXBytes;
         uint32_t bad = 0;   // bit 0: first half of the stage, bit 1: second half
-#pragma unroll
-        for (int i = 0; i < BM / 32; ++i) {
-          const int row = (wt >> 3) + i * 32, j = wt & 7;
+#pragma unroll (XF32 ? 2 : 4)
+        for (int i = 0; i < BM / 16; ++i) {
+          const int row = (wt >> 3) + i * 16, j = wt & 7;
           float f[8];
           bool odd = false;
           if (XF32) {
@@ -509,18 +544,16 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             if (units_per_stage == 2) {
               if ((j & 3) == 0) xsum[((slot + (j >> 2)) % kInfo) * BM + row] = sum;
             } else if (j == 0) {
-              float* d = xsum + slot * BM + row;
-              *d = first ? sum : *d + sum;
+              xsum[slot * BM + row] = sum;
             }
           }
           const uint32_t b = __ballot_sync(0xFFFFFFFFu, odd);
           bad |= (b & 0x0F0F0F0Fu ? 1u : 0u) | (b & 0xF0F0F0F0u ? 2u : 0u);
         }
         if (units_per_stage == 2) {
-          if (lane < 2) flags[((slot + lane) % kInfo) * 8 + ww] = (bad >> lane) & 1;
-        } else {
-          flag_carry = first ? bad : (flag_carry | bad);
-          if (lane == 0) flags[slot * 8 + ww] = flag_carry != 0;
+          if (lane < 2) flags[((slot + lane) % kInfo) * kGroupWarps + ww] = (bad >> lane) & 1;
+        } else if (lane == 0) {
+          flags[slot * kGroupWarps + ww] = bad != 0;
         }
       }
       dev::fence_proxy_async();
@@ -528,16 +561,12 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       if (lane == 0) {
         // raw weights and activations go back after the fence that completed the stores made from them: an arrival
         // right behind the loads let a refill overtake them
-        if (sub == C::kStagesPerBox - 1 || st == stages - 1) dev::mbar_arrive(&wempty[rs]);
+        dev::mbar_arrive(&wempty[rs]);
         if (XF32) dev::mbar_arrive(&xempty[xs]);
         dev::mbar_arrive(&full[op]);
         if (C::kUnitInfo) {
-          if (units_per_stage == 2) {
-            dev::mbar_arrive(&ifull[slot]);
-            dev::mbar_arrive(&ifull[(slot + 1) % kInfo]);
-          } else if (last) {
-            dev::mbar_arrive(&ifull[slot]);
-          }
+          dev::mbar_arrive(&ifull[slot]);
+          if (units_per_stage == 2) dev::mbar_arrive(&ifull[(slot + 1) % kInfo]);
         }
       }
     }
@@ -555,8 +584,6 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
 #pragma unroll
     for (int i = 0; i < C::kCols / 2; ++i) acc[i] = 0ull;
     auto load_scale = [&](int u, float& s, float& b) {
-      s = 1.f;
-      b = 0.f;
       const int uu = min(u_base + u, total_units - 1);
       if (C::kBias) {
         const size_t i = static_cast<size_t>(nc) * G + uu / units_per_group;
@@ -566,76 +593,83 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         s = opapi::decode_e8m0(__ldg(static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(nc) * G + uu));
       }
     };
-    constexpr int kAhead = 4;   // scales are requested four units early
-    float sv[kAhead], bv[kAhead];
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i) load_scale(i, sv[i], bv[i]);
-    bool ok = true;
-    for (int ub = 0; ok && ub < units; ub += kAhead) {
-#pragma unroll
-      for (int i = 0; i < kAhead; ++i) {
-        const int u = ub + i;
-        if (!ok || u >= units) break;
-        const int buf = u % kAccBufs, slot = u % kInfo;
-        const float s = (FMT == kAffine8 && XF32) ? sv[i] * 64.f : sv[i];
-        float b = bv[i];
-        if (C::kBias && XF32) {
-          float shifted;
-          if (centred<FMT>(sv[i], bv[i], shifted)) b = shifted;
+    // Scales come in boxes (one TMA copy for all promoters), else each promoter reads its lanes' values a unit ahead.
+    const int units_per_box = FMT != kNvfp4 && a.sbox_k ? a.sbox_k / a.pu : 0;
+    float s_next = 1.f, b_next = 0.f;
+    if (units_per_box == 0) load_scale(0, s_next, b_next);
+    int box = 0, in_box = 0;
+    for (int u = 0; u < units; ++u) {
+      const int buf = u % kAccBufs, slot = u % kInfo;
+      float s = s_next, b = b_next;
+      if (units_per_box) {
+        const int sb = box % kSBoxes;
+        if (in_box == 0 && !dev::mbar_wait_relaxed_warp(&sfull[sb], (box / kSBoxes) & 1, a.status, 101)) break;
+        const uint8_t* row = smem + C::kOffS + sb * kSBoxBytes + (q * 32 + lane) * 16;
+        if (C::kBias) {
+          const int c = in_box / units_per_group;
+          s = reinterpret_cast<const float*>(row)[c];
+          b = reinterpret_cast<const float*>(row + BN * 16)[c];
+        } else {
+          s = opapi::decode_e8m0(row[in_box]);
         }
-        load_scale(u + kAhead, sv[i], bv[i]);
-        bool exact = false;
-        if (C::kUnitInfo) {
-          if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) { ok = false; break; }
-          const uint2 fl = *reinterpret_cast<const uint2*>(flags + slot * 8);
-          exact = (fl.x | fl.y) != 0u;
-        }
-        if (!dev::mbar_wait_relaxed_warp(&tfull[buf], (u / kAccBufs) & 1, a.status, 100)) { ok = false; break; }
-        dev::tc_fence_after();
-        if (C::kUnitInfo && exact) {
-          const int k0 = k_begin + u * a.pu, k1 = min(a.K, k0 + a.pu);
+      } else {
+        load_scale(u + 1, s_next, b_next);
+      }
+      if (C::kBias && XF32) {
+        float shifted;
+        if (centred<FMT>(s, b, shifted)) b = shifted;
+      }
+      if (FMT == kAffine8 && XF32) s *= 64.f;
+      bool exact = false;
+      if (C::kUnitInfo) {
+        if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) break;
+        exact = *reinterpret_cast<const uint32_t*>(flags + slot * kGroupWarps) != 0u;
+      }
+      if (!dev::mbar_wait_relaxed_warp(&tfull[buf], (u / kAccBufs) & 1, a.status, 100)) break;
+      dev::tc_fence_after();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
+      if (C::kUnitInfo && exact) {
+        // the unit's exact sums take the accumulator's place (registers cannot be indexed)
+        const int k0 = k_begin + u * a.pu, k1 = min(a.K, k0 + a.pu);
 #pragma unroll 1
-          for (int c = 0; c < C::kCols; ++c) {
-            if (m0 + c0 + c >= a.M) break;
-            const float v = exact_unit<FMT, XF32>(a, m0 + c0 + c, nc, k0, k1);
+        for (int c = 0; c < C::kCols; ++c)
+          dev::tmem_st_32x1(taddr + c, m0 + c0 + c < a.M ? __float_as_uint(exact_unit<FMT, XF32>(a, m0 + c0 + c, nc, k0, k1)) : 0u);
+        dev::tc_wait_st();
+        s = 1.f;
+      }
+      const uint64_t s2 = pack2(s, s), b2 = pack2(b, b);
+      const bool with_bias = C::kBias && !exact;
 #pragma unroll
-            for (int e = 0; e < C::kCols / 2; ++e) {   // registers cannot be indexed
-              float v0, v1;
-              unpack2(acc[e], v0, v1);
-              if (c == 2 * e) v0 += v;
-              if (c == 2 * e + 1) v1 += v;
-              acc[e] = pack2(v0, v1);
-            }
+      for (int c = 0; c < C::kCols; c += 16) {
+        uint32_t r[16];
+        dev::tmem_ld_32x16(taddr + c, r);
+        dev::tc_wait_ld();
+        if (with_bias) {
+          // scale and bias terms cancel in part: they meet before they are added to the running sum
+          const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(xsum + slot * BM + c0 + c);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const ulonglong2 t = xp[e];
+            uint64_t v0 = fmul2(b2, t.x), v1 = fmul2(b2, t.y);
+            fma2(v0, s2, pack2(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1])));
+            fma2(v1, s2, pack2(__uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3])));
+            add2(acc[c / 2 + 2 * e], v0);
+            add2(acc[c / 2 + 2 * e + 1], v1);
           }
         } else {
-          const uint64_t s2 = pack2(s, s), b2 = pack2(b, b);
 #pragma unroll
-          for (int c = 0; c < C::kCols; c += 16) {   // 16 at a time: 64 accumulators leave no room for more
-            uint32_t r[16];
-            dev::tmem_ld_32x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0 + c, r);
-            dev::tc_wait_ld();
-            if (C::kBias) {
-              // scale and bias terms cancel in part: they meet before they are added to the running sum
-              const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(xsum + slot * BM + c0 + c);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const ulonglong2 t = xp[e];
-                uint64_t v0 = fmul2(b2, t.x), v1 = fmul2(b2, t.y);
-                fma2(v0, s2, pack2(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1])));
-                fma2(v1, s2, pack2(__uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3])));
-                add2(acc[c / 2 + 2 * e], v0);
-                add2(acc[c / 2 + 2 * e + 1], v1);
-              }
-            } else {
-#pragma unroll
-              for (int e = 0; e < 8; ++e)
-                fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
-            }
-          }
+          for (int e = 0; e < 8; ++e)
+            fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
         }
-        dev::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) dev::mbar_arrive(&tempty[buf]);
+      }
+      dev::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) dev::mbar_arrive(&tempty[buf]);
+      if (units_per_box && ++in_box == units_per_box) {
+        // the arrival's address depends on the value read last: it cannot overtake the load
+        if (lane == 0) dev::mbar_arrive(&sempty[box % kSBoxes] + (__float_as_uint(s + b) == 0x7FC1FFC1u && a.M < 0));
+        in_box = 0;
+        ++box;
       }
     }
     // ---- this slice's results, [row][column], into the idle rings (after every warp is done with them)
@@ -688,8 +722,8 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
 
 // CTAs that share an output tile: the fewest rounds of resident CTAs, a round costing its stages and about twelve
 // more for the prologue and the hand-over.
-static int cluster_size(int tiles, int blocks, int stages, int per_sm) {
-  const int slots = num_sms() * per_sm;
+static int cluster_size(int tiles, int blocks, int stages) {
+  const int slots = num_sms();
   int best = 1;
   long long best_cost = -1;
   for (int ks = 1; ks <= kMaxCluster && ks <= blocks; ++ks) {
@@ -715,17 +749,31 @@ static int launch(Args a, cudaStream_t stream) {
   static std::atomic<uint64_t> configured{0};
   auto kern = opgemm_kernel<FMT, XF32, BM>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), C::kSmem, configured)) return rc;
-  // a unit is a scale group or a part of one; slices of K begin on a raw box and on a unit
-  a.pu = FMT == kNvfp4 || a.gs % 128 == 0 ? 128 : (a.gs % 64 == 0 ? 64 : 32);
-  // the tensor core's own additions are truncated: against f32 results (128 k: 2.5e-7 of the result, 64 k: 1e-7) they
-  // are cut short, against f16 results they do not show
-  if (XF32 && a.pu > 64) a.pu = 64;
-  a.block_k = C::kBoxK;
+  // A unit is a scale group or a part of one, and no more than a stage: its MMAs come from one thread, and the tensor
+  // core's own, truncated additions have to be cut short against f32 results (128 k: 2.5e-7 of the result, 64 k: 1e-7).
+  // Slices of K begin on a box of raw weights and on a box of scales.
+  a.pu = FMT == kNvfp4 || a.gs % 64 == 0 ? 64 : 32;
+  const bool boxed = FMT == kNvfp4 ? false
+                     : C::kBias    ? a.gs <= 128 && (a.K / a.gs) % 4 == 0 && 128 % a.gs == 0 && aligned(a.scales, 16) && aligned(a.biases, 16)
+                                   : a.K % 512 == 0 && aligned(a.scales, 16);
+  a.sbox_k = !boxed ? 0 : (C::kBias ? 4 * a.gs : 512);
+  a.block_k = a.sbox_k > C::kBoxK ? a.sbox_k : C::kBoxK;
+  CUtensorMap smap = wmap, bmap = wmap;   // placeholders where they are not used
+  if (boxed) {
+    const uint64_t G = static_cast<uint64_t>(a.K / a.gs);
+    const auto type = C::kBias ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    const int esz = C::kBias ? 4 : 1;
+    if (int rc = make_tensor_map_2d(&smap, a.scales, type, esz, (uint64_t)a.N, G, G * esz, BN, 16 / esz, CU_TENSOR_MAP_SWIZZLE_NONE))
+      return rc;
+    if (C::kBias)
+      if (int rc = make_tensor_map_2d(&bmap, a.biases, type, esz, (uint64_t)a.N, G, G * esz, BN, 16 / esz, CU_TENSOR_MAP_SWIZZLE_NONE))
+        return rc;
+  }
   a.blocks = (a.K + a.block_k - 1) / a.block_k;
   a.idesc = dev::make_idesc(/*c=f32*/ 1, XF32 ? 1 : 0, XF32 ? 1 : 0, /*both K-major*/ 0, 0, BN, BM);
   a.status = device_status_word();
   const int nt = (a.N + BN - 1) / BN, mt = (a.M + BM - 1) / BM;
-  const int ks = cluster_size(nt * mt, a.blocks, (a.K + BK - 1) / BK, C::kMinBlocks);
+  const int ks = cluster_size(nt * mt, a.blocks, (a.K + BK - 1) / BK);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ks, mt, nt);
   cfg.blockDim = dim3(C::kThreads);
@@ -740,7 +788,7 @@ static int launch(Args a, cudaStream_t stream) {
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ks > 1 ? 2 : 1;
-  QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, a));
+  QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, smap, bmap, a));
   return QMM_OK;
 }
 
