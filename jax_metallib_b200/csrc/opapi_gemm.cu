@@ -38,7 +38,7 @@ constexpr int kGroupWarps = 4;        // warps that convert one stage; the group
 constexpr int kRawBox = BN * 128;     // 16 KB of raw weights
 constexpr int kABytes = BN * BK * 2;  // 16 KB
 constexpr int kAccBufs = 4;           // accumulators between the tensor core and the promoters
-constexpr int kInfo = 16;             // units whose activation sums and flags are kept
+constexpr int kInfo = 32;             // units whose activation sums and flags are kept (power of two)
 constexpr int kConsumed = 12;         // a multiple of the operand ring (3 or 4) and of the activation ring
 constexpr int kMaxCluster = 8;
 constexpr int kSBoxes = 3;            // boxes of scales (and biases) on their way to the promoters
@@ -70,7 +70,7 @@ struct Cfg {
   static constexpr int kOffS = kOffInfo + kInfo * BM * 4;
   static constexpr int kOffFlags = kOffS + (FMT == kNvfp4 ? 0 : kSBoxes * kSBoxBytes);
   static constexpr int kOffBar = kOffFlags + kInfo * kGroupWarps;
-  static constexpr int kSmem = kOffBar + 512 + 1024;
+  static constexpr int kSmem = kOffBar + 640 + 1024;
   static constexpr int kPromoters = BM / 8;               // four lane quarters x 32 columns each
   static constexpr int kFirstIssuer = 2;
   static constexpr int kFirstWorker = kFirstIssuer + kGroups;   // one issuing warp per group
@@ -79,6 +79,7 @@ struct Cfg {
   static constexpr int kCols = 32;                        // accumulator columns per promoter
   static_assert(kOps <= kAccBufs, "one unit per stage: an accumulator's previous unit is issued before the next is full");
   static_assert(BM * BN * 4 <= kOffInfo, "the result tile reuses the rings");
+  static_assert((kAccBufs & (kAccBufs - 1)) == 0 && (kInfo & (kInfo - 1)) == 0 && kInfo <= 32, "ring sizes");
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 
@@ -597,18 +598,17 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     const int units_per_box = FMT != kNvfp4 && a.sbox_k ? a.sbox_k / a.pu : 0;
     float s_next = 1.f, b_next = 0.f;
     if (units_per_box == 0) load_scale(0, s_next, b_next);
-    int box = 0, in_box = 0;
+    int in_box = 0, in_group = 0, comp = 0;   // unit of the box, unit of the group, group of the box
+    uint32_t sb = 0, sb_phase = 0, phase = 0;  // ring slot and parity of the box; parity of the accumulators' round
     for (int u = 0; u < units; ++u) {
-      const int buf = u % kAccBufs, slot = u % kInfo;
+      const int buf = u & (kAccBufs - 1), slot = u & (kInfo - 1);
       float s = s_next, b = b_next;
       if (units_per_box) {
-        const int sb = box % kSBoxes;
-        if (in_box == 0 && !dev::mbar_wait_relaxed_warp(&sfull[sb], (box / kSBoxes) & 1, a.status, 101)) break;
+        if (in_box == 0 && !dev::mbar_wait_relaxed_warp(&sfull[sb], sb_phase, a.status, 101)) break;
         const uint8_t* row = smem + C::kOffS + sb * kSBoxBytes + (q * 32 + lane) * 16;
         if (C::kBias) {
-          const int c = in_box / units_per_group;
-          s = reinterpret_cast<const float*>(row)[c];
-          b = reinterpret_cast<const float*>(row + BN * 16)[c];
+          s = reinterpret_cast<const float*>(row)[comp];
+          b = reinterpret_cast<const float*>(row + BN * 16)[comp];
         } else {
           s = opapi::decode_e8m0(row[in_box]);
         }
@@ -625,7 +625,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) break;
         exact = *reinterpret_cast<const uint32_t*>(flags + slot * kGroupWarps) != 0u;
       }
-      if (!dev::mbar_wait_relaxed_warp(&tfull[buf], (u / kAccBufs) & 1, a.status, 100)) break;
+      if (!dev::mbar_wait_relaxed_warp(&tfull[buf], phase, a.status, 100)) break;
       dev::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
       if (C::kUnitInfo && exact) {
@@ -640,10 +640,15 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       const uint64_t s2 = pack2(s, s), b2 = pack2(b, b);
       const bool with_bias = C::kBias && !exact;
 #pragma unroll
-      for (int c = 0; c < C::kCols; c += 16) {
+      for (int c = 0; c < C::kCols; c += 16) {   // 16 at a time: registers
         uint32_t r[16];
         dev::tmem_ld_32x16(taddr + c, r);
         dev::tc_wait_ld();
+        if (c + 16 == C::kCols) {                // the last values are in registers: the buffer goes back
+          dev::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) dev::mbar_arrive(&tempty[buf]);
+        }
         if (with_bias) {
           // scale and bias terms cancel in part: they meet before they are added to the running sum
           const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(xsum + slot * BM + c0 + c);
@@ -662,14 +667,13 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
         }
       }
-      dev::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) dev::mbar_arrive(&tempty[buf]);
+      if (buf == kAccBufs - 1) phase ^= 1;
+      if (++in_group == units_per_group) { in_group = 0; ++comp; }
       if (units_per_box && ++in_box == units_per_box) {
         // the arrival's address depends on the value read last: it cannot overtake the load
-        if (lane == 0) dev::mbar_arrive(&sempty[box % kSBoxes] + (__float_as_uint(s + b) == 0x7FC1FFC1u && a.M < 0));
-        in_box = 0;
-        ++box;
+        if (lane == 0) dev::mbar_arrive(&sempty[sb] + (__float_as_uint(s + b) == 0x7FC1FFC1u && a.M < 0));
+        in_box = comp = 0;
+        if (++sb == kSBoxes) { sb = 0; sb_phase ^= 1; }
       }
     }
     // ---- this slice's results, [row][column], into the idle rings (after every warp is done with them)
@@ -720,15 +724,50 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
   if (KS > 1) cluster.sync();   // peers keep their shared memory alive until it has been read
 }
 
-// CTAs that share an output tile: the fewest rounds of resident CTAs, a round costing its stages and about twelve
-// more for the prologue and the hand-over.
+static void set_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int ks) {
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ks;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+}
+
+// Clusters of `ks` CTAs that the current device holds at once (asked once per device and size).
+template <int FMT, bool XF32, int BM>
+static int resident_clusters(int ks) {
+  static std::atomic<int> cache[kMaxDevices][kMaxCluster + 1];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return num_sms() / ks;
+  int n = cache[dev][ks].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(ks, 1, 1024);
+  cfg.blockDim = dim3(Cfg<FMT, XF32, BM>::kThreads);
+  cfg.dynamicSmemBytes = Cfg<FMT, XF32, BM>::kSmem;
+  set_attrs(cfg, attr, ks);
+  if (cudaOccupancyMaxActiveClusters(&n, opgemm_kernel<FMT, XF32, BM>, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = num_sms() / ks > 0 ? num_sms() / ks : 1;
+  }
+  cache[dev][ks].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// CTAs that share an output tile: the fewest rounds of resident clusters (six CTAs to a cluster, for one, leave SMs of
+// every GPC idle), a round costing its stages and, for the prologue and the hand-over, about as much as kRoundCost more.
+constexpr int kRoundCost = 16;
+template <int FMT, bool XF32, int BM>
 static int cluster_size(int tiles, int blocks, int stages) {
-  const int slots = num_sms();
   int best = 1;
   long long best_cost = -1;
   for (int ks = 1; ks <= kMaxCluster && ks <= blocks; ++ks) {
-    const long long waves = (static_cast<long long>(tiles) * ks + slots - 1) / slots;
-    const long long cost = waves * ((stages + ks - 1) / ks + 12);
+    const int c = resident_clusters<FMT, XF32, BM>(ks);
+    const int slice = (blocks + ks - 1) / ks;   // the longest slice, in blocks
+    const long long cost = static_cast<long long>((tiles + c - 1) / c) * (slice * ((stages + blocks - 1) / blocks) + kRoundCost);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = ks; }
   }
   return best;
@@ -773,21 +812,14 @@ static int launch(Args a, cudaStream_t stream) {
   a.idesc = dev::make_idesc(/*c=f32*/ 1, XF32 ? 1 : 0, XF32 ? 1 : 0, /*both K-major*/ 0, 0, BN, BM);
   a.status = device_status_word();
   const int nt = (a.N + BN - 1) / BN, mt = (a.M + BM - 1) / BM;
-  const int ks = cluster_size(nt * mt, a.blocks, (a.K + BK - 1) / BK);
+  const int ks = cluster_size<FMT, XF32, BM>(nt * mt, a.blocks, (a.K + BK - 1) / BK);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ks, mt, nt);
   cfg.blockDim = dim3(C::kThreads);
   cfg.dynamicSmemBytes = C::kSmem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = ks;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = ks > 1 ? 2 : 1;
+  set_attrs(cfg, attr, ks);
   QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, smap, bmap, a));
   return QMM_OK;
 }
