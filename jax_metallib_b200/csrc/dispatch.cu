@@ -17,6 +17,8 @@ int i8gemm_tcgen05(const void* a, const void* b, int32_t* acc, const float* row_
 int w8a16_tcgen05(const uint16_t* x, const int8_t* w, const float* scale, uint16_t* y, int64_t M,
                   int64_t N, int64_t K, int64_t ldy, uint32_t flags, uint32_t* signal, uint32_t* arrive,
                   cudaStream_t stream);
+int i8_skinny(const void* a, const void* b, int32_t* acc, const float* row_scale, const float* col_scale, float* out, int64_t M,
+              int64_t N, int64_t K, int a_unsigned, int b_unsigned, bool aligned_rows, cudaStream_t stream);
 int w8a16_decode(const uint16_t* x, const int8_t* w, const float* scale, uint16_t* y, int64_t M, int64_t N, int64_t K,
                  int64_t ldy, uint32_t flags, cudaStream_t stream);
 
@@ -141,6 +143,16 @@ static int force_simple() {
   return env_int_once("QMM_FORCE_SIMPLE", 0, cache);
 }
 
+// Which int8 dots take the kernel for few rows or rows that TMA cannot describe, instead of the GEMM.
+static bool i8_skinny_covers(int64_t M, int64_t N, int64_t K, bool tma_ok) {
+  if (N > (1 << 28) || M > (1 << 22) || (N + 127) / 128 * ((M + 7) / 8) > (1ll << 30)) return false;
+  // The GEMM's tiles of 256 columns leave most SMs idle when there are few of them; this kernel splits K but reads b once
+  // per 64 rows.  Measured (this kernel, the GEMM): 64 x 4096 x 4096 14.0, 21.3 us; 128 x 4096 x 4096 20.0, 22.2 us;
+  // 256 x 4096 x 4096 30.8, 22.2 us; 64 x 8192 x 8192 30.5, 37.3 us; 128 x 8192 x 8192 50.4, 38.4 us;
+  // 256 x 1024 x 1024 9.8, 10.4 us.
+  return !tma_ok || M <= 32 || (M + 63) / 64 * N <= 8192;
+}
+
 }  // namespace qmm
 
 extern "C" {
@@ -161,6 +173,8 @@ int qmm_i8i8_i32(const void* a, const void* b, int32_t* acc, const float* row_sc
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool tma_ok = K > 0 && K % 16 == 0 && N % 16 == 0 && aligned(a, 16) && aligned(b, 16) &&
                       (!acc || aligned(acc, 16)) && (!out || (aligned(out, 16) && aligned(col_scale, 16)));
+  if (K > 0 && !force_simple() && i8_skinny_covers(M, N, K, tma_ok))
+    return i8_skinny(a, b, acc, row_scale, col_scale, out, M, N, K, a_unsigned, b_unsigned, tma_ok, s);
   if (tma_ok && M * N >= 128 * 128 && !force_simple())
     return i8gemm_tcgen05(a, b, acc, row_scale, col_scale, out, M, N, K, a_unsigned, b_unsigned, s);
   QMM_REQUIRE(M <= 65535, QMM_ERR_UNSUPPORTED, "qmm_i8i8_i32: unaligned shape with M > 65535");
@@ -214,8 +228,10 @@ static int w8a16_entry(const char* name, const uint16_t* x, const int8_t* w, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool tma_ok = K > 0 && K % 8 == 0 && N % 16 == 0 && ldy % 2 == 0 && aligned(x, 16) &&
                       aligned(w, 16) && aligned(y, 4);
-  // few rows, results that stay on this GPU: the HBM-bound kernel
-  if (tma_ok && M <= 32 && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
+  // Few rows, results that stay on this GPU: the HBM-bound kernel.  It reads the weights once per 32 rows; the GEMM reads
+  // them once but does not split K, so that a narrow N leaves SMs idle: measured at M = 64, 4096 x 4096: 16 against 39 us,
+  // 14336 x 4096: 39 against 121 us, 4096 x 28672: 85 against 62 us; at M = 128, 8192 x 8192: 81 against 74 us.
+  if (tma_ok && (M <= 32 || (M + 31) / 32 * N <= 23000) && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
     return w8a16_decode(x, w, scale, y, M, N, K, ldy, flags, s);
   if (tma_ok && M * N >= 128 * 128 && !force_simple())
     return w8a16_tcgen05(x, w, scale, y, M, N, K, ldy, flags, signal, arrive, s);
