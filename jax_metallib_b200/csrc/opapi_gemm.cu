@@ -57,7 +57,7 @@ struct Cfg {
   // A stage passes through a worker in ~0.6 us of dependent waits, loads and stores, whatever its share of the work:
   // throughput comes from stages converted side by side.  (One group of eight warps: 1.2 us per stage for mxfp8,
   // 2.5 us with activation sums, 3.3 us with f32 activations.)
-  static constexpr int kGroups = BM == 32 ? 4 : (BM == 64 ? 3 : 2);
+  static constexpr int kGroups = 2;
   static constexpr int kWorkerWarps = kGroups * kGroupWarps;
   static constexpr int kOps = XF32 && BM == 64 ? 3 : 4;         // operand stages
   static constexpr int kOpBytes = kABytes + (XF32 ? 3 * kXTile : 0);
