@@ -37,9 +37,8 @@ constexpr int BK = 64;                // k per operand stage: one 128-byte row o
 constexpr int kGroupWarps = 4;        // warps that convert one stage; the groups take the stages in turn
 constexpr int kRawBox = BN * 128;     // 16 KB of raw weights
 constexpr int kABytes = BN * BK * 2;  // 16 KB
-constexpr int kAccBufs = 4;           // accumulators between the tensor core and the promoters
 constexpr int kInfo = 32;             // units whose activation sums and flags are kept (power of two)
-constexpr int kConsumed = 12;         // a multiple of the operand ring (3 or 4) and of the activation ring
+constexpr int kConsumed = 24;         // stages whose retirement can be asked for (more than twice the deepest ring)
 constexpr int kMaxCluster = 8;
 constexpr int kSBoxes = 3;            // boxes of scales (and biases) on their way to the promoters
 constexpr int kSBoxBytes = 2 * BN * 16;
@@ -59,27 +58,32 @@ struct Cfg {
   // 2.5 us with activation sums, 3.3 us with f32 activations.)
   static constexpr int kGroups = 2;
   static constexpr int kWorkerWarps = kGroups * kGroupWarps;
-  static constexpr int kOps = XF32 && BM == 64 ? 3 : 4;         // operand stages
+  // A stage takes 2-4 us from raw codes to retired MMAs and an accumulator about 1.5 us from one unit to the next,
+  // nearly all of it latency: the rings are as deep as shared memory and TMEM allow.
+  static constexpr int kOps = XF32 ? (BM == 32 ? 5 : 3) : (BM == 32 ? 8 : (BM == 64 ? 6 : 4));   // operand stages
+  static constexpr int kAccBufs = BM == 128 ? 4 : 8;        // accumulators between the tensor core and the promoters
   static constexpr int kOpBytes = kABytes + (XF32 ? 3 * kXTile : 0);
-  static constexpr int kXRing = XF32 && BM == 64 ? 3 : 4;
+  static constexpr int kXRing = XF32 ? (BM == 32 ? 4 : 3) : kOps;
   static constexpr int kXBytes = XF32 ? kXRaw : kXTile;
-  static constexpr int kRawBoxes = XF32 && BM == 64 ? 2 : 3;
+  static constexpr int kRawBoxes = XF32 ? 2 : 3;
   static constexpr int kOffX = kOps * kOpBytes;
   static constexpr int kOffRaw = kOffX + kXRing * kXBytes;
   static constexpr int kOffInfo = kOffRaw + kRawBoxes * kRawBox;
   static constexpr int kOffS = kOffInfo + kInfo * BM * 4;
   static constexpr int kOffFlags = kOffS + (FMT == kNvfp4 ? 0 : kSBoxes * kSBoxBytes);
   static constexpr int kOffBar = kOffFlags + kInfo * kGroupWarps;
-  static constexpr int kSmem = kOffBar + 640 + 1024;
+  static constexpr int kSmem = kOffBar + 1024 + 1024;
   static constexpr int kPromoters = BM / 8;               // four lane quarters x 32 columns each
   static constexpr int kFirstIssuer = 2;
   static constexpr int kFirstWorker = kFirstIssuer + kGroups;   // one issuing warp per group
   static constexpr int kFirstPromoter = kFirstWorker + kWorkerWarps;
   static constexpr int kThreads = (kFirstPromoter + kPromoters) * 32;
   static constexpr int kCols = 32;                        // accumulator columns per promoter
-  static_assert(kOps <= kAccBufs, "one unit per stage: an accumulator's previous unit is issued before the next is full");
+  // One thread issues all units of one accumulator, in order: its wait for the previous unit to be drained can then not
+  // take the drain of the unit before that for it (the parities are the same).
+  static_assert(kAccBufs % (2 * kGroups) == 0, "two units per stage, one issuer per group");
   static_assert(BM * BN * 4 <= kOffInfo, "the result tile reuses the rings");
-  static_assert((kAccBufs & (kAccBufs - 1)) == 0 && (kInfo & (kInfo - 1)) == 0 && kInfo <= 32, "ring sizes");
+  static_assert((kAccBufs & (kAccBufs - 1)) == 0 && (kInfo & (kInfo - 1)) == 0 && 2 * kOps + kAccBufs + 1 <= kInfo && kInfo <= 32 && 2 * kOps < kConsumed && kConsumed <= 32, "ring sizes");
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 
@@ -262,8 +266,8 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
   uint64_t* full = xempty + C::kXRing;                               // operand stage written
   uint64_t* consumed = full + C::kOps;                               // the MMAs of a stage retired
   uint64_t* tfull = consumed + kConsumed;                            // a unit's accumulator complete
-  uint64_t* tempty = tfull + kAccBufs;                               // and drained
-  uint64_t* ifull = tempty + kAccBufs;                               // sums and flags of a unit written
+  uint64_t* tempty = tfull + C::kAccBufs;                               // and drained
+  uint64_t* ifull = tempty + C::kAccBufs;                               // sums and flags of a unit written
   uint64_t* sfull = ifull + kInfo;                                   // a box of scales landed
   uint64_t* sempty = sfull + kSBoxes;                                // and read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sempty + kSBoxes);
@@ -281,7 +285,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     if (lane < C::kXRing) { dev::mbar_init(&xfull[lane], 1); dev::mbar_init(&xempty[lane], kGroupWarps); }
     if (lane < C::kOps) dev::mbar_init(&full[lane], kGroupWarps);
     if (lane < kConsumed) dev::mbar_init(&consumed[lane], 1);
-    if (lane < kAccBufs) { dev::mbar_init(&tfull[lane], 1); dev::mbar_init(&tempty[lane], C::kPromoters); }
+    if (lane < C::kAccBufs) { dev::mbar_init(&tfull[lane], 1); dev::mbar_init(&tempty[lane], C::kPromoters); }
     if (lane < kInfo) dev::mbar_init(&ifull[lane], kGroupWarps);
     if (lane < kSBoxes) { dev::mbar_init(&sfull[lane], 1); dev::mbar_init(&sempty[lane], C::kPromoters); }
     dev::fence_mbar_init();
@@ -292,7 +296,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     dev::tma_prefetch_desc(&bmap);
   }
   if (warp == 1) {
-    dev::tmem_alloc(tmem_slot, kAccBufs * BM);
+    dev::tmem_alloc(tmem_slot, C::kAccBufs * BM);
     dev::tmem_relinquish();
   }
   dev::tc_fence_before();
@@ -371,19 +375,14 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       for (int st = warp - C::kFirstIssuer; ok && st < stages; st += C::kGroups) {
         const int s = st % C::kOps;
         if (!dev::mbar_wait(&full[s], (st / C::kOps) & 1, a.status, 94)) break;
-        // Two units per stage: a stage may be full while the one four units back, which shares its accumulators, has not
-        // been issued; its parity would read as drained.  With one unit per stage the operand ring keeps that apart.
-        if (units_per_stage == 2 && st >= 2 &&
-            !dev::mbar_wait(&consumed[(st - 2) % kConsumed], ((st - 2) / kConsumed) & 1, a.status, 102))
-          break;
         dev::tc_fence_after();
         const uint32_t a_lo = op_lo + s * (C::kOpBytes >> 4);
         const uint32_t b_lo = XF32 ? a_lo + (kABytes >> 4) : x_lo + (st % C::kXRing) * (C::kXTile >> 4);
         for (int h = 0; h < units_per_stage; ++h) {
           const int u = st * units_per_stage + h;
           if (u >= units) break;                                   // the zero half of a last stage
-          const int buf = u % kAccBufs;
-          if (!dev::mbar_wait(&tempty[buf], ((u / kAccBufs) & 1) ^ 1, a.status, 95)) { ok = false; break; }
+          const int buf = u % C::kAccBufs;
+          if (!dev::mbar_wait(&tempty[buf], ((u / C::kAccBufs) & 1) ^ 1, a.status, 95)) { ok = false; break; }
           dev::tc_fence_after();
           const uint32_t d = tmem_base + buf * BM;
           // the smallest terms first: the accumulator is still small when they are added
@@ -402,7 +401,8 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 dev::umma_f16_lh(d, a_lo + h * 4 + j * 2, kDescHi, b_lo + t * (C::kXTile >> 4) + h * 4 + j * 2, kDescHi, a.idesc,
                                  (t != C::kTerms - 1 || j != 0) ? 1u : 0u);
           }
-          dev::tc_commit(&tfull[buf]);
+          // (a commit costs the thread as much as an MMA: one for the units of a stage)
+          if (h == units_per_stage - 1 || u == units - 1) dev::tc_commit(&tfull[buf]);
         }
         if (ok) dev::tc_commit(&consumed[st % kConsumed]);
       }
@@ -578,6 +578,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     const int nc = min(n, a.N - 1);
     const int c0 = half * C::kCols;
     const int units_per_group = (FMT == kNvfp4) ? 1 : a.gs / a.pu;
+    const int units_per_stage = a.pu < BK ? BK / a.pu : 1;
     const int u_base = k_begin / a.pu;
     const int G = (FMT == kNvfp4) ? 1 : a.K / a.gs;
     const int total_units = (a.K + a.pu - 1) / a.pu;
@@ -601,7 +602,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     int in_box = 0, in_group = 0, comp = 0;   // unit of the box, unit of the group, group of the box
     uint32_t sb = 0, sb_phase = 0, phase = 0;  // ring slot and parity of the box; parity of the accumulators' round
     for (int u = 0; u < units; ++u) {
-      const int buf = u & (kAccBufs - 1), slot = u & (kInfo - 1);
+      const int buf = u & (C::kAccBufs - 1), slot = u & (kInfo - 1);
       float s = s_next, b = b_next;
       if (units_per_box) {
         if (in_box == 0 && !dev::mbar_wait_relaxed_warp(&sfull[sb], sb_phase, a.status, 101)) break;
@@ -625,7 +626,9 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) break;
         exact = *reinterpret_cast<const uint32_t*>(flags + slot * kGroupWarps) != 0u;
       }
-      if (!dev::mbar_wait_relaxed_warp(&tfull[buf], phase, a.status, 100)) break;
+      // the units of a stage complete together, on the barrier of the last
+      const int last = units_per_stage == 2 ? min(u | 1, units - 1) & (C::kAccBufs - 1) : buf;
+      if (!dev::mbar_wait_relaxed_warp(&tfull[last], phase, a.status, 100)) break;
       dev::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
       if (C::kUnitInfo && exact) {
@@ -667,7 +670,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
         }
       }
-      if (buf == kAccBufs - 1) phase ^= 1;
+      if (buf == C::kAccBufs - 1) phase ^= 1;
       if (++in_group == units_per_group) { in_group = 0; ++comp; }
       if (units_per_box && ++in_box == units_per_box) {
         // the arrival's address depends on the value read last: it cannot overtake the load
@@ -694,7 +697,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
   // TMEM goes back before this CTA waits for its cluster: a CTA never holds it while it depends on another one
   if (warp == 1) {
     dev::tc_fence_after();
-    dev::tmem_dealloc(tmem_base, kAccBufs * BM);
+    dev::tmem_dealloc(tmem_base, C::kAccBufs * BM);
   }
   cg::cluster_group cluster = cg::this_cluster();
   if (KS > 1) cluster.sync();
@@ -836,11 +839,14 @@ static int launch_fmt(const Args& a, int f32, cudaStream_t stream) {
 
 }  // namespace opg
 
+// Which calls come here.  Up to three rows the CUDA-core kernels, which read x from cache and split every column over a
+// warp, have less to set up (affine4, f32, 4096 x 8192: 30 us at one row, 62 at four, here 32 for any of them;
+// 4096 x 12288: 32, 63, here 58).
 // fmt: 0 affine 4-bit, 1 affine 8-bit, 2 mxfp4, 3 mxfp8, 4 nvfp4.  K and the group a multiple of 32 (nvfp4: K), weights
 // and activations 16-byte aligned, results aligned for pairs.
 bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, const void* x, const void* w, const void* y) {
   using namespace opg;
-  if (K % 32 != 0 || (fmt <= kAffine8 && gs % 32 != 0)) return false;
+  if (M < 4 || K % 32 != 0 || (fmt <= kAffine8 && gs % 32 != 0)) return false;
   if (!aligned(x, 16) || !aligned(w, 16) || !aligned(y, 8)) return false;
   return (M + 31) / 32 <= 65535 && (N + BN - 1) / BN <= 65535;
 }
