@@ -797,7 +797,7 @@ static int launch(Args a, cudaStream_t stream) {
   a.pu = FMT == kNvfp4 || a.gs % 64 == 0 ? 64 : 32;
   const bool boxed = FMT == kNvfp4 ? false
                      : C::kBias    ? a.gs <= 128 && (a.K / a.gs) % 4 == 0 && 128 % a.gs == 0 && aligned(a.scales, 16) && aligned(a.biases, 16)
-                                   : a.K % 512 == 0 && aligned(a.scales, 16);
+                                   : a.K % 512 == 0 && a.K >= 2048 && aligned(a.scales, 16);   // (slices of a short K stay fine)
   a.sbox_k = !boxed ? 0 : (C::kBias ? 4 * a.gs : 512);
   a.block_k = a.sbox_k > C::kBoxK ? a.sbox_k : C::kBoxK;
   CUtensorMap smap = wmap, bmap = wmap;   // placeholders where they are not used

@@ -1,0 +1,161 @@
+"""The kernels that split K over a cluster, at the edges of their tiles, rings and routes, against 64-bit torch.
+
+Tolerances: results are one rounding of a sum in f32.  A product is exact, so what is left beside that rounding is the sum's own
+error, bounded by the number of additions on one element's path (truncated ones count twice) times 2^-24 of sum |x| |w|.
+"""
+
+import pytest
+import torch
+
+from jax_metallib_b200 import ops, quantized
+
+pytestmark = pytest.mark.gpu
+
+
+def _gen(seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return g
+
+
+def _sum_error(k, steps):
+    """Additions: ``steps`` truncated ones in a stage of 64 k, one per stage after that, and sixteen partial tiles."""
+    return (2 * steps + k / 64 + 16) * 2.0 ** -24
+
+
+def _check(y, x, w, scale, rounding, steps):
+    xd, wd = x.double(), w.double()
+    ref, size = (xd @ wd) * scale, (xd.abs() @ wd.abs()) * scale.abs()
+    bound = rounding * ref.abs() + _sum_error(x.shape[1], steps) * size * (1 + rounding)
+    assert bool(((y.double() - ref).abs() <= bound).all()), ((y.double() - ref).abs() / bound.clamp_min(1e-300)).max().item()
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 8, 16), (1, 4096, 4096), (8, 72, 144), (9, 1032, 1040), (16, 4096, 28672), (17, 64, 128),
+                                   (32, 4096, 28672), (33, 520, 272), (64, 14336, 256), (97, 1000, 5632)])
+def test_int8_weights_bf16_rows(cuda, m, k, n):
+    g = _gen(m + k + n)
+    x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    w = torch.randint(-128, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
+    s = torch.rand(n, device="cuda", generator=g) * 0.01 + 0.005
+    # one accumulator runs over a CTA's slice of K
+    _check(ops.w8a16_perchannel(x, w, s), x, w, s.double(), 2.0 ** -8, k // 16 + 1)
+    wide = torch.zeros(m, n + 32, dtype=torch.bfloat16, device="cuda")
+    ops.w8a16_perchannel(x, w, s, out=wide, out_col_offset=16)
+    assert torch.equal(wide[:, 16:16 + n], ops.w8a16_perchannel(x, w, s))
+    assert not wide[:, :16].any() and not wide[:, 16 + n:].any()
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 4, 16), (8, 100, 48), (9, 64, 128), (17, 1024, 1024), (33, 4, 16), (100, 2052, 400),
+                                   (256, 512, 144)])
+def test_int8_weights_f32_rows(cuda, m, k, n):
+    g = _gen(m + k + n)
+    x = torch.randn(m, k, device="cuda", generator=g) * torch.exp2(torch.randint(-20, 20, (m, 1), device="cuda", generator=g))
+    w = torch.randint(-128, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
+    s = torch.rand(n, device="cuda", generator=g) * 0.01 + 0.005
+    _check(ops.w8a32_perchannel(x, w, s), x, w, s.double(), 2.0 ** -22, 6)
+
+
+def test_int8_weights_f32_special_values(cuda):
+    x = torch.randn(5, 256, device="cuda", generator=_gen(1))
+    x[0, 3], x[1, 7], x[2, 5], x[2, 9], x[3, 200] = float("inf"), float("nan"), -float("inf"), float("inf"), 1e36
+    w = torch.randint(-128, 128, (256, 64), dtype=torch.int8, device="cuda", generator=_gen(2))
+    y, ref = ops.w8a32_perchannel(x, w, torch.full((64,), 1e-3, device="cuda")), (x.double() @ w.double()) * 1e-3
+    assert torch.equal(torch.isnan(y), torch.isnan(ref))
+    assert torch.equal(torch.nan_to_num(y[0], nan=0.0), torch.nan_to_num(ref[0].float(), nan=0.0))
+    _check(y[3:4], x[3:4], w, torch.tensor(1e-3, dtype=torch.float64, device="cuda"), 2.0 ** -22, 6)
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 17, 33, 65])
+@pytest.mark.parametrize("k,n", [(1, 1), (16, 17), (63, 65), (64, 128), (1000, 48), (331, 257), (2048, 1000)])
+@pytest.mark.parametrize("ta,tb,offset", [(torch.int8, torch.int8, 0), (torch.uint8, torch.int8, 1), (torch.int8, torch.uint8, 3),
+                                          (torch.uint8, torch.uint8, 2)])
+def test_int8_dot_any_rows(cuda, m, k, n, ta, tb, offset):
+    g = _gen(m * k + n)
+
+    def ints(rows, cols, t):  # a view that begins `offset` bytes into its allocation
+        lo = -128 if t == torch.int8 else 0
+        flat = torch.randint(lo, lo + 256, (rows * cols + offset,), dtype=torch.int16, device="cuda", generator=g).to(t)
+        return flat[offset:].view(rows, cols)
+
+    a, b = ints(m, k, ta), ints(k, n, tb)
+    rs, cs = torch.rand(m, device="cuda", generator=g), torch.rand(n, device="cuda", generator=g)
+    acc, out = ops.i8_dot(a, b, rs, cs)
+    ref = (a.double() @ b.double()).to(torch.int64)
+    assert torch.equal(acc.long(), ref)
+    assert torch.equal(out, ref.to(torch.int32).float() * rs[:, None] * cs)
+
+
+def _operator_weights(fmt, group, n, k, g):
+    """Packed weights, call arguments and the dequantised weights [N, K] in 64 bits."""
+    groups = (n, k // group)
+    if fmt.startswith("affine"):
+        bits = int(fmt[6:])
+        q = torch.randint(0, 1 << bits, (n, k), device="cuda", generator=g)
+        s = torch.rand(groups, device="cuda", generator=g) * 0.01 + 0.002
+        b = -s * (1 << bits) / 2 * (0.9 + 0.2 * torch.rand(groups, device="cuda", generator=g))
+        s[0], b[0], q[0] = 1.0, 0.04, 0    # a flat group
+        packed = q.to(torch.uint8)
+        if bits == 4:
+            v = (q.view(n, k // 8, 8) << (4 * torch.arange(8, device="cuda"))).sum(-1)
+            packed = torch.where(v >= 2 ** 31, v - 2 ** 32, v).to(torch.int32)
+        w = s.double().repeat_interleave(group, 1) * q.double() + b.double().repeat_interleave(group, 1)
+        size = s.double().repeat_interleave(group, 1) * q.double() + b.double().abs().repeat_interleave(group, 1)
+        return lambda x: quantized.affine_quantized_matmul(x, packed, s, b, bits=bits, group_size=group, K=k), w, size
+    if fmt == "mxfp8":
+        packed = (torch.randn(n, k, device="cuda", generator=g) * 100).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+        values = packed.view(torch.float8_e4m3fn).double()
+    else:
+        codes = torch.randint(0, 16, (n, k), dtype=torch.uint8, device="cuda", generator=g)
+        packed = codes[:, 0::2] | (codes[:, 1::2] << 4)
+        table = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6], device="cuda", dtype=torch.float64)
+        values = torch.cat((table, -table))[codes.long()]
+    if fmt == "nvfp4":
+        sb = (torch.rand(groups, device="cuda", generator=g) * 0.03 + 0.004).to(torch.float8_e4m3fn).view(torch.uint8)
+        scale = sb.view(torch.float8_e4m3fn).double()
+    else:
+        sb = torch.randint(100, 123, groups, dtype=torch.uint8, device="cuda", generator=g)
+        scale = torch.exp2(sb.double() - 127)
+    w = values * scale.repeat_interleave(group, 1)
+    return lambda x: quantized.quantized_matmul(x, packed, sb, mode=fmt, K=k), w, w.abs()
+
+
+FORMATS = [("affine4", 32), ("affine4", 64), ("affine4", 96), ("affine4", 128), ("affine8", 32), ("affine8", 128), ("mxfp4", 32),
+           ("mxfp8", 32), ("nvfp4", 16)]
+# rows at the edges of the tiles of 32, 64 and 128; K of half a stage, of several boxes and of none; ragged columns
+SHAPES = [(4, 384, 17), (17, 1152, 128), (33, 384, 200), (64, 2304, 130), (65, 1920, 333), (130, 5376, 260), (300, 1152, 96)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("m,k,n", SHAPES)
+@pytest.mark.parametrize("fmt,group", FORMATS)
+def test_operator_matmul(cuda, fmt, group, m, k, n, dtype):
+    k = (k + group - 1) // group * group
+    g = _gen(m + k + n)
+    run, w, size = _operator_weights(fmt, group, n, k, g)
+    x = torch.randn(m, k, device="cuda", generator=g).to(dtype)
+    y, ref = run(x).double(), x.double() @ w.T
+    # a unit of 64 k is twelve truncated additions (three terms), scaled, joined with its bias term and added in f32
+    bound = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -24) * ref.abs() + _sum_error(k, 16) * (x.double().abs() @ size.T)
+    if dtype == torch.float16:
+        bound += 2.0 ** -24   # results below the smallest normal number
+    assert bool(((y - ref).abs() <= bound).all()), ((y - ref).abs() / bound).max().item()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("fmt,group", [("affine4", 64), ("affine8", 32), ("mxfp4", 32), ("mxfp8", 32), ("nvfp4", 16)])
+@pytest.mark.parametrize("m", [20, 70])
+def test_operator_matmul_special_values(cuda, fmt, group, m, dtype):
+    g = _gen(m)
+    run, w, _ = _operator_weights(fmt, group, 160, 512, g)
+    x = torch.randn(m, 512, device="cuda", generator=g)
+    x[0, 5], x[1, 70], x[2, 100], x[2, 101], x[3, 400] = float("inf"), float("nan"), -float("inf"), float("inf"), -float("inf")
+    x[4] = 1e-38 if dtype == torch.float32 else 6e-8
+    x[5, 9] = 1e36 if dtype == torch.float32 else 6e4
+    x = x.to(dtype)
+    y, ref = run(x), x.double() @ w.T
+    assert torch.equal(torch.isnan(y), torch.isnan(ref))
+    assert torch.equal(torch.isinf(y[:4]), torch.isinf(ref[:4])) and torch.equal(torch.sign(y[0]), torch.sign(ref[0]).to(dtype))
+    if dtype == torch.float32:
+        size = x[5].double().abs() @ w.abs().T
+        assert bool(((y[5].double() - ref[5]).abs() <= 2.0 ** -24 * ref[5].abs() + _sum_error(512, 64) * size).all())
+        assert torch.allclose(y[4].double(), ref[4], rtol=1e-4, atol=512 * 2.0 ** -149)
