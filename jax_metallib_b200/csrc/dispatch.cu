@@ -1,7 +1,7 @@
-// Entry points whose work is routed between the tcgen05 GEMMs and plain
-// CUDA-core kernels.  The tensor-core kernels take every shape TMA can
-// describe (16-byte row pitches); anything else (the few-element shapes of the
-// reference's integer-dot tests, odd strides) runs on the simple kernels below.
+// Entry points whose work is routed between the tcgen05 GEMMs, the mma.sync
+// kernels that split K (few rows; int8 dots of any alignment) and plain
+// CUDA-core kernels, which are left for weight-only shapes that TMA cannot
+// describe (16-byte row pitches) and for K = 0.
 // Both routes are GPU code; there is no host fallback.
 #include <stddef.h>
 #include <stdlib.h>

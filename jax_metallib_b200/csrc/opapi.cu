@@ -11,9 +11,10 @@
 // weight = scale * q + bias (affine) or scale * element (MX) in f32, product
 // and accumulation in f32, one final cast; NaN codes propagate.
 //
-// These CUDA-core kernels take any M and f32 or f16 activations.  Decode-sized
-// f16 problems (M <= 16) go to the tensor-core kernels instead: the TMA-ring
-// kernels of opapi_tc.cu where the shape allows, else affine_tc_kernel below.
+// These CUDA-core kernels take any M and f32 or f16 activations, and run where nothing else does: up to three rows, K or
+// groups that are no multiple of 32, unaligned operands.  Decode-sized f16 problems (M <= 16) go to the TMA-ring
+// tensor-core kernels of opapi_tc.cu where the shape allows, then to affine_tc_kernel below; the rest goes to the
+// tcgen05 GEMM of opapi_gemm.cu.
 #include "opapi_decode.cuh"
 
 namespace qmm {

@@ -18,6 +18,11 @@
 // activations into their three terms, and sum the activations of a unit for the biases) and four to
 // sixteen promoters that drain the accumulators.
 //
+// Measured (four linears of a layer, before: one warp per four columns on CUDA cores): mxfp8, f16, M = 512, 4096 / 14336
+// wide 15.2 -> 0.88 ms; affine 4-bit, f32, M = 48, 2048 / 5632 wide 597 -> 103 us.  Bound by latency, not by a unit: a
+// stage takes 0.35-0.5 us per scale group through issuer, tensor core and promoter (two MMAs of a 32-k group are too
+// little work to hide a commit and a TMEM read), 0.25 of the bf16 rate at best.
+//
 // What the split cannot represent takes an exact path: a unit whose activations are not finite (inf times
 // code plus inf times bias is not what inf times scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
 // the promoters from global memory with the arithmetic of the CUDA-core kernels.
@@ -53,9 +58,9 @@ struct Cfg {
   static constexpr int kStagesPerBox = kBoxK / BK;          // 4 or 2
   static constexpr int kXTile = BM * BK * 2;                // one 16-bit operand tile of activations
   static constexpr int kXRaw = BM * BK * 4;                 // raw f32 activations of a stage
-  // A stage passes through a worker in ~0.6 us of dependent waits, loads and stores, whatever its share of the work:
-  // throughput comes from stages converted side by side.  (One group of eight warps: 1.2 us per stage for mxfp8,
-  // 2.5 us with activation sums, 3.3 us with f32 activations.)
+  // Groups of four workers and an issuer take the stages in turn.  With one group of eight warps a stage took 1.2 us
+  // (mxfp8) to 3.3 us (f32 activations); with three or four groups the registers per thread fall to 72 and the workers
+  // and promoters spill, which cost more than the groups gave (affine4, f32, M = 1, 4096 x 8192: 54 us against 33 us).
   static constexpr int kGroups = 2;
   static constexpr int kWorkerWarps = kGroups * kGroupWarps;
   // A stage takes 2-4 us from raw codes to retired MMAs and an accumulator about 1.5 us from one unit to the next,

@@ -2,6 +2,10 @@
 //
 //   y[M,N] = bf16( (x[M,K] @ float(w[K,N])) * scale[N] )        x bf16, w int8 row-major, scale f32
 //
+// and the same with f32 activations and results (any M; three bf16 terms per activation, see split4).
+// Measured at M = 1: 4096 x 28672 25 us (4.7 TB/s), 4096 x 6144 8.0 us, 14336 x 4096 14.0 us, the four linears of a layer
+// 57 us (one thread per column before: 1905 us); f32, 32 x 1024 x 1024 10.1 -> 6.7 us, 256 x 4096 x 4096 528 -> 149 us.
+//
 // Bound by HBM: the weights (K*N bytes) are read once.  A cluster of KS CTAs owns blocks of 128
 // columns and splits K between its CTAs; every CTA runs a ring of TMA stages (64 k x 128 columns of
 // weights, 128-byte swizzle, and the same 64 k of the activations), fed by one warp and drained by
@@ -12,7 +16,8 @@
 // the weights as its 16-row operand and the activations as its 8-column operand, so that M = 1
 // wastes tensor work, which is free here, and not memory traffic.  tcgen05 has nothing to add at
 // these sizes: its operand would have to pass through shared memory a second time after the
-// conversion.
+// conversion.  What is left above the weights' own time is the fill of the ring, the hand-over at the
+// end of a tile and, at M = 32, the MMAs.
 //
 // The partial tiles of a cluster (KS CTAs x two k halves) meet in distributed shared memory; warps
 // of their own add each CTA's share of the elements in a fixed order while the consumers go on with

@@ -2,6 +2,9 @@
 //
 //   y[M,N] = (x[M,K] @ float(w[K,N])) * scale[N]
 //
+// Rows that TMA can describe go to the tensor-core kernel of w8a16_decode.cu (three bf16 terms per activation); this
+// one takes the others (K no multiple of 4, N no multiple of 16, unaligned operands).
+//
 // Exact f32 FMA arithmetic (int8 -> f32 is exact; the scale is applied once
 // per output element instead of once per weight, which differs from the
 // un-fused order only by f32 rounding of the product).  At the sizes this is
