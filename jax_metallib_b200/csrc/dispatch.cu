@@ -145,7 +145,7 @@ static int force_simple() {
 
 // Which int8 dots take the kernel for few rows or rows that TMA cannot describe, instead of the GEMM.
 static bool i8_skinny_covers(int64_t M, int64_t N, int64_t K, bool tma_ok) {
-  if (N > (1 << 28) || M > (1 << 22) || (N + 127) / 128 * ((M + 7) / 8) > (1ll << 30)) return false;
+  if (M > 65535 || (N + 127) / 128 * ((M + 7) / 8) > (1ll << 30)) return false;
   // The GEMM's tiles of 256 columns leave most SMs idle when there are few of them; this kernel splits K but reads b once
   // per 64 rows.  Measured (this kernel, the GEMM): 64 x 4096 x 4096 14.0, 21.3 us; 128 x 4096 x 4096 20.0, 22.2 us;
   // 256 x 4096 x 4096 30.8, 22.2 us; 64 x 8192 x 8192 30.5, 37.3 us; 128 x 8192 x 8192 50.4, 38.4 us;

@@ -14,19 +14,20 @@
 // the instructions of the MMAs they feed at 64 rows, nothing against the one thread per result that ran before.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "split_k.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace qmm {
 namespace i8s {
 
+using namespace split;
+
 constexpr int kCols = 128;           // columns per tile
 constexpr int kBK = 64;              // k per stage
 constexpr int kConsumerWarps = 8;    // 4 column groups of 32 x 2 halves of a stage's k
 constexpr int kLoaderWarps = 4;      // rows without a tensor map
 constexpr int kWBytes = kBK * kCols;
-constexpr int kMaxCluster = 8;
 
 template <int MT, bool TMA>
 struct Smem {
@@ -46,11 +47,6 @@ struct Smem {
   static_assert(kPerSm * (kTotal + 1024) <= 228 * 1024, "resident CTAs");
 };
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
 template <bool AU, bool BU>
 __device__ __forceinline__ void mma_i8(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t x0, uint32_t x1) {
 #define QMM_MMA_I8(TB, TA)                                                                                              \
@@ -75,36 +71,6 @@ __device__ __forceinline__ uint4 load16_any(const uint8_t* p, const uint8_t* end
   const uint32_t sh = off * 8;
   return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh),
                     __funnelshift_r(w[3], w[4], sh));
-}
-
-// Arrives (release, cluster scope) on the barrier at the same place of CTA `rank`'s shared memory.
-__device__ __forceinline__ void arrive_remote(uint64_t* bar, int rank) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(dev::smem_u32(bar)), "r"(rank)
-      : "memory");
-}
-__device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(dev::smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded, all lanes leave with the same answer.
-__device__ __forceinline__ bool wait_cluster_warp(uint64_t* bar, uint32_t parity, int* status, int tag) {
-  bool ok = try_wait_cluster(bar, parity);
-  if (!ok) {
-    const uint64_t t0 = dev::globaltimer_ns();
-    while (!(ok = try_wait_cluster(bar, parity)))
-      if (dev::globaltimer_ns() - t0 > dev::kWaitLimitNs) break;
-    if (!ok && status) atomicExch(status, (tag << 16) | QMM_ERR_TIMEOUT);
-  }
-  return __all_sync(0xFFFFFFFFu, ok);
 }
 
 template <int MT, bool AU, bool BU, bool TMA>
@@ -340,63 +306,6 @@ i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   cluster.sync();   // peers keep their shared memory alive until it has been read
 }
 
-struct Grid {
-  int ks, clusters;
-};
-
-static void set_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int ks) {
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = ks;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-}
-
-// Clusters of `ks` CTAs that the current device holds at once (asked once per device and size).
-template <int MT, bool AU, bool BU, bool TMA>
-static int resident_clusters(int ks) {
-  static std::atomic<int> cache[kMaxDevices][kMaxCluster + 1];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return Smem<MT, TMA>::kPerSm * num_sms() / ks;
-  int n = cache[dev][ks].load(std::memory_order_relaxed);
-  if (n > 0) return n;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  cfg.gridDim = dim3(ks, 1024);
-  cfg.blockDim = dim3(Smem<MT, TMA>::kThreads);
-  cfg.dynamicSmemBytes = Smem<MT, TMA>::kTotal;
-  set_attrs(cfg, attr, ks);
-  if (cudaOccupancyMaxActiveClusters(&n, i8_skinny_kernel<MT, AU, BU, TMA>, &cfg) != cudaSuccess || n < 1) {
-    (void)cudaGetLastError();
-    n = Smem<MT, TMA>::kPerSm * num_sms() / ks;
-  }
-  cache[dev][ks].store(n, std::memory_order_relaxed);
-  return n;
-}
-
-constexpr int kRoundCost = 6;
-// Resident clusters walk the tiles, so the launch takes as many rounds as the busiest cluster has tiles; a
-// round costs its stages and the hand-over of the partial tiles.
-template <int MT, bool AU, bool BU, bool TMA>
-static Grid choose_grid(int tiles, int stages_total) {
-  Grid best = {1, 1};
-  long long best_cost = -1;
-  for (int ks = 1; ks <= kMaxCluster && ks <= stages_total; ++ks) {
-    const int c = resident_clusters<MT, AU, BU, TMA>(ks);
-    const int rounds = (tiles + c - 1) / c;
-    const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + kRoundCost);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best.ks = ks;
-      best.clusters = tiles < c ? tiles : c;
-    }
-  }
-  return best;
-}
-
 struct Args {
   const uint8_t *a, *b;
   int32_t* acc;
@@ -418,10 +327,13 @@ static int launch(const Args& p, cudaStream_t stream) {
       return rc;
   }
   static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
+  static std::atomic<int> resident[kMaxDevices][kMaxCluster + 1];
   auto kern = i8_skinny_kernel<MT, AU, BU, TMA>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
   const int stages_total = (p.K + kBK - 1) / kBK;
-  const Grid g = choose_grid<MT, AU, BU, TMA>(((p.N + kCols - 1) / kCols) * ((p.M + MT * 8 - 1) / (MT * 8)), stages_total);
+  const Grid g = choose_grid(((p.N + kCols - 1) / kCols) * ((p.M + MT * 8 - 1) / (MT * 8)), stages_total, [&](int ks) {
+    return resident_clusters(kern, L::kThreads, L::kTotal, L::kPerSm, ks, resident);
+  });
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(g.ks, g.clusters);

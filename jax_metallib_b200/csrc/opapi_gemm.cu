@@ -853,7 +853,7 @@ bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, const v
   using namespace opg;
   if (M < 4 || K % 32 != 0 || (fmt <= kAffine8 && gs % 32 != 0)) return false;
   if (!aligned(x, 16) || !aligned(w, 16) || !aligned(y, 8)) return false;
-  return (M + 31) / 32 <= 65535 && (N + BN - 1) / BN <= 65535;
+  return (M + 7) / 8 <= 65535 && (N + BN - 1) / BN <= 65535;
 }
 
 int opgemm_launch(int fmt, const void* x, const void* w, const void* scales, const float* biases, void* y, int64_t M, int64_t N,

@@ -1,0 +1,110 @@
+// Helpers of the kernels that split K over a thread-block cluster and add the partial tiles over distributed shared memory.
+#pragma once
+
+#include "common.cuh"
+
+namespace qmm {
+namespace split {
+
+constexpr int kMaxCluster = 8;
+
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                               uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Arrives (release, cluster scope) on the barrier at the same place of CTA `rank`'s shared memory.
+__device__ __forceinline__ void arrive_remote(uint64_t* bar, int rank) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(dev::smem_u32(bar)), "r"(rank)
+      : "memory");
+}
+__device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(dev::smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded, all lanes leave with the same answer.
+__device__ __forceinline__ bool wait_cluster_warp(uint64_t* bar, uint32_t parity, int* status, int tag) {
+  bool ok = try_wait_cluster(bar, parity);
+  if (!ok) {
+    const uint64_t t0 = dev::globaltimer_ns();
+    while (!(ok = try_wait_cluster(bar, parity)))
+      if (dev::globaltimer_ns() - t0 > dev::kWaitLimitNs) break;
+    if (!ok && status) atomicExch(status, (tag << 16) | QMM_ERR_TIMEOUT);
+  }
+  return __all_sync(0xFFFFFFFFu, ok);
+}
+
+struct Grid {
+  int ks, clusters;
+};
+
+inline void set_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int ks) {
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ks;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+}
+
+// Resident clusters walk the tiles, so a launch takes as many rounds as the busiest cluster has tiles; a round costs its
+// stages and the hand-over of the partial tiles (about six stages).  resident(ks): clusters of ks CTAs held at once.
+constexpr int kRoundCost = 6;
+template <typename Fn>
+inline Grid choose_grid(int tiles, int stages_total, Fn resident) {
+  Grid best = {1, 1};
+  long long best_cost = -1;
+  for (int ks = 1; ks <= kMaxCluster && ks <= stages_total; ++ks) {
+    const int c = resident(ks);
+    const int rounds = (tiles + c - 1) / c;
+    const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + kRoundCost);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best.ks = ks;
+      best.clusters = tiles < c ? tiles : c;
+    }
+  }
+  return best;
+}
+
+// Clusters of `ks` CTAs of a kernel that the current device holds at once; `cache` belongs to the kernel.
+template <typename Kern>
+inline int resident_clusters(Kern kern, int threads, int smem, int per_sm, int ks, std::atomic<int> (&cache)[kMaxDevices][kMaxCluster + 1]) {
+  const int guess = per_sm * num_sms() / ks > 0 ? per_sm * num_sms() / ks : 1;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return guess;
+  int n = cache[dev][ks].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(ks, 1024);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  set_attrs(cfg, attr, ks);
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = guess;
+  }
+  cache[dev][ks].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+}  // namespace split
+}  // namespace qmm

@@ -24,19 +24,20 @@
 // the next block: deterministic, no workspace, no atomics.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "split_k.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace qmm {
 namespace w8d {
 
+using namespace split;
+
 constexpr int kCols = 128;           // columns per tile
 constexpr int kBK = 64;              // k per stage
 constexpr int kConsumerWarps = 8;    // 4 column groups of 32 x 2 halves of a stage's k
 constexpr int kFirstReducer = kConsumerWarps + 1;
 constexpr int kWBytes = kBK * kCols;
-constexpr int kMaxCluster = 8;
 
 template <int MT, bool XF32>
 struct Smem {
@@ -60,17 +61,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
-__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                               uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // The int8 values v in bytes 0 and 2 of a register -> two bf16 v / 64, exactly, in two instructions: v + 128 in the
 // low byte of a bf16 reads as (v + 128) * 2^-133 (a subnormal up to 127, the first binade above), and one fused
@@ -106,36 +96,6 @@ __device__ __forceinline__ void split4(uint32_t (&v)[4], uint32_t (&hi)[2], uint
     mid[i] = __byte_perm(m[2 * i], m[2 * i + 1], 0x7632);
     lo[i] = __byte_perm(l[2 * i], l[2 * i + 1], 0x7632);
   }
-}
-
-// Arrives (release, cluster scope) on the barrier at the same place of CTA `rank`'s shared memory.
-__device__ __forceinline__ void arrive_remote(uint64_t* bar, int rank) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(dev::smem_u32(bar)), "r"(rank)
-      : "memory");
-}
-__device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(dev::smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded, all lanes leave with the same answer.
-__device__ __forceinline__ bool wait_cluster_warp(uint64_t* bar, uint32_t parity, int* status, int tag) {
-  bool ok = try_wait_cluster(bar, parity);
-  if (!ok) {
-    const uint64_t t0 = dev::globaltimer_ns();
-    while (!(ok = try_wait_cluster(bar, parity)))
-      if (dev::globaltimer_ns() - t0 > dev::kWaitLimitNs) break;
-    if (!ok && status) atomicExch(status, (tag << 16) | QMM_ERR_TIMEOUT);
-  }
-  return __all_sync(0xFFFFFFFFu, ok);
 }
 
 template <int MT, bool XF32>
@@ -370,71 +330,17 @@ w8_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   cluster.sync();   // peers keep their shared memory alive until it has been read
 }
 
-struct Grid {
-  int ks, clusters;
-};
-
-static void set_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int ks) {
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = ks;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-}
-
-// Clusters of `ks` CTAs that the current device holds at once (asked once per device and size).
-template <int MT, bool XF32>
-static int resident_clusters(int ks) {
-  static std::atomic<int> cache[kMaxDevices][kMaxCluster + 1];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return Smem<MT, XF32>::kPerSm * num_sms() / ks;
-  int n = cache[dev][ks].load(std::memory_order_relaxed);
-  if (n > 0) return n;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  cfg.gridDim = dim3(ks, 1024);
-  cfg.blockDim = dim3(Smem<MT, XF32>::kThreads);
-  cfg.dynamicSmemBytes = Smem<MT, XF32>::kTotal;
-  set_attrs(cfg, attr, ks);
-  if (cudaOccupancyMaxActiveClusters(&n, w8_decode_kernel<MT, XF32>, &cfg) != cudaSuccess || n < 1) {
-    (void)cudaGetLastError();
-    n = Smem<MT, XF32>::kPerSm * num_sms() / ks;
-  }
-  cache[dev][ks].store(n, std::memory_order_relaxed);
-  return n;
-}
-
-constexpr int kRoundCost = 6;
-// Resident clusters walk the tiles, so the launch takes as many rounds as the busiest cluster has tiles; a
-// round costs its stages and the hand-over of the partial tiles.
-template <int MT, bool XF32>
-static Grid choose_grid(int tiles, int stages_total) {
-  Grid best = {1, 1};
-  long long best_cost = -1;
-  for (int ks = 1; ks <= kMaxCluster && ks <= stages_total; ++ks) {
-    const int c = resident_clusters<MT, XF32>(ks);
-    const int rounds = (tiles + c - 1) / c;
-    const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + kRoundCost);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best.ks = ks;
-      best.clusters = tiles < c ? tiles : c;
-    }
-  }
-  return best;
-}
-
 template <int MT, bool XF32>
 static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const float* scale, void* y, int M, int N, long long ldy,
                   int stages_total, int independent, cudaStream_t stream) {
   using L = Smem<MT, XF32>;
   static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
+  static std::atomic<int> resident[kMaxDevices][kMaxCluster + 1];
   auto kern = w8_decode_kernel<MT, XF32>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
-  const Grid g = choose_grid<MT, XF32>(((N + kCols - 1) / kCols) * ((M + MT * 8 - 1) / (MT * 8)), stages_total);
+  const Grid g = choose_grid(((N + kCols - 1) / kCols) * ((M + MT * 8 - 1) / (MT * 8)), stages_total, [&](int ks) {
+    return resident_clusters(kern, L::kThreads, L::kTotal, L::kPerSm, ks, resident);
+  });
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(g.ks, g.clusters);

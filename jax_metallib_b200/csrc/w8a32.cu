@@ -127,7 +127,7 @@ extern "C" int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float
   if (M == 0 || N == 0) return QMM_OK;  // empty result: nothing to launch, pointers may be null
   QMM_REQUIRE(x && w && scale && y, QMM_ERR_INVALID_ARGUMENT, "qmm_w8a32_perchannel: null pointer");
   // rows that TMA can describe: the tensor-core kernel
-  if (K > 0 && K % 4 == 0 && N % 16 == 0 && aligned(x, 16) && aligned(w, 16) && aligned(y, 8) && M < (1 << 24) &&
+  if (K > 0 && K % 4 == 0 && N % 16 == 0 && aligned(x, 16) && aligned(w, 16) && aligned(y, 8) && (M + TM - 1) / TM <= 65535 &&
       N * ((M + 7) / 8) < (1ll << 36)) {
     if (int st = read_device_status())
       return set_error(QMM_ERR_TIMEOUT, "a previous kernel gave up waiting (status word 0x%x)", st);

@@ -45,6 +45,23 @@ def test_int8_weights_bf16_rows(cuda, m, k, n):
     assert not wide[:, :16].any() and not wide[:, 16 + n:].any()
 
 
+@pytest.mark.parametrize("packed", [True, False])
+@pytest.mark.parametrize("m,k,n", [(1, 128, 128), (8, 4096, 384), (9, 1280, 1536), (16, 14336, 256), (16, 384, 16384)])
+def test_int4_weights(cuda, m, k, n, packed):
+    g = _gen(m + k + n)
+    x = (torch.randn(m, k, device="cuda", generator=g) * 3 + 1).bfloat16()
+    x[0, 5] = 2e38   # one product of the largest activations does not overflow
+    wq = torch.randint(0, 256, (k // 2, n), dtype=torch.uint8, device="cuda", generator=g)
+    s = (torch.rand(k // 128, n, device="cuda", generator=g) * 0.008 + 0.002).bfloat16()
+    z = torch.randint(0, 16, (k // 128, n), dtype=torch.uint8, device="cuda", generator=g)
+    zp = z[:, 0::2] | (z[:, 1::2] << 4) if packed else z
+    y = ops.w4a16_g128(x, wq, s, zp, zeros_packed=packed)
+    q = torch.stack((wq & 15, wq >> 4), 1).reshape(k, n).double()
+    zr, sr = (v.double().repeat_interleave(128, 0) for v in (z, s))
+    ref, size = x.double() @ ((q - zr) * sr), x.double().abs() @ ((32 + q + zr) * sr)   # 16 + q and 16 + z are what is added up
+    assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + _sum_error(k, 4) * size * 1.01).all())
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 4, 16), (8, 100, 48), (9, 64, 128), (17, 1024, 1024), (33, 4, 16), (100, 2052, 400),
                                    (256, 512, 144)])
 def test_int8_weights_f32_rows(cuda, m, k, n):
