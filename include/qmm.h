@@ -101,7 +101,10 @@ QMM_API int qmm_set_cta_limit(int max_ctas);
  * HandleMultiply -> HandleDotGeneral
  * (src/pjrt_plugin/ops/shape_ops.mm:793-829, :93-153;
  *  src/pjrt_plugin/ops/binary_ops.mm:165-193, :1006-1019).
- * Exact f32 FMA arithmetic; the scale is applied once per output element. */
+ * The scale is applied once per output element.  With K % 4 == 0, N % 16 == 0,
+ * 16-byte aligned x and w and 8-byte aligned y the activations go to the tensor
+ * cores as three bf16 terms that hold all 24 bits (exact products, f32 sums);
+ * any other shape runs in f32 FMA arithmetic on CUDA cores. */
 QMM_API int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float* scale, float* y,
                                  int64_t M, int64_t N, int64_t K, void* stream);
 
@@ -115,7 +118,8 @@ QMM_API int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float* s
  * tcgen05 (kind::f16) GEMM with the int8->bf16 conversion done in shared
  * memory.  The tensor-core route needs K % 8 == 0, N % 16 == 0, an even ldy
  * and 16-byte aligned x and w (what TMA can address); any other shape runs on
- * a plain CUDA-core kernel. */
+ * a plain CUDA-core kernel.  On that route few rows (M <= 32, or ceil(M / 32) * N
+ * <= 23000) run a kernel that splits K over thread-block clusters. */
 QMM_API int qmm_w8a16_perchannel(const uint16_t* x_bf16, const int8_t* w, const float* scale,
                                  uint16_t* y_bf16, int64_t M, int64_t N, int64_t K, int64_t ldy,
                                  void* stream);
@@ -225,8 +229,9 @@ QMM_API int qmm_i8i8_i32(const void* a, const void* b, int32_t* acc, const float
  *  ops/binary_ops.mm:66-193, :644-1245).
  * Zero points are 4-bit values (0..15) in either form.
  * Requires group == 128, K % 128 == 0, N % 128 == 0, M >= 1.
- * M <= 32 runs the HBM-bound decode kernel (weights read once, split-K over
- * all SMs); larger M runs a tcgen05 GEMM whose converter warps dequantise the
+ * M <= 32 runs an HBM-bound decode kernel (weights read once; K split over
+ * thread-block clusters for M <= 16 and N <= 16384, else over all SMs with the
+ * partial sums in the workspace); larger M runs a tcgen05 GEMM whose converter warps dequantise the
  * nibbles in shared memory: bf16((q - z) * s) per weight, which is what the
  * StableHLO chain computes in bf16, f32 accumulation, one rounding of the
  * result.  That route needs no workspace (qmm_w4a16_g128_workspace_bytes
@@ -303,8 +308,9 @@ QMM_API int qmm_w4a16_g128_static_scratch(const uint16_t* x_bf16, const uint8_t*
  * scales (and biases) are 16-byte aligned, N is a multiple of 16 and, affine:
  * group_size is 64 / 128 / 256 (4-bit) or 32 / 64 / 128 (8-bit) with a multiple
  * of 4 groups per row; MX: K is a multiple of 512 (mxfp4, mxfp8) or 256
- * (nvfp4).  Other shapes, M > 16 and f32 activations run on CUDA-core kernels
- * with the same arithmetic (scale * q + bias or scale * element in f32, f32
+ * (nvfp4).  Everything else with M >= 4, 16-byte aligned x and w_packed, K (and,
+ * affine, group_size) a multiple of 32 runs a tcgen05 GEMM; what is left runs on
+ * CUDA-core kernels (scale * q + bias or scale * element in f32, f32
  * accumulation, one cast).  The tensor-core kernels apply the scale per group
  * instead of per weight: same result up to f32 rounding of the sums. */
 QMM_API int qmm_affine_matmul(const void* x, const void* w_packed, const float* scales,

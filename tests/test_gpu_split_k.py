@@ -176,3 +176,20 @@ def test_operator_matmul_special_values(cuda, fmt, group, m, dtype):
         size = x[5].double().abs() @ w.abs().T
         assert bool(((y[5].double() - ref[5]).abs() <= 2.0 ** -24 * ref[5].abs() + _sum_error(512, 64) * size).all())
         assert torch.allclose(y[4].double(), ref[4], rtol=1e-4, atol=512 * 2.0 ** -149)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("fmt,group", [("mxfp4", 32), ("mxfp8", 32), ("nvfp4", 16)])
+def test_operator_matmul_nan_codes(cuda, fmt, group, dtype):
+    g = _gen(5)
+    n, k = 40, 512
+    x = torch.randn(20, k, device="cuda", generator=g).to(dtype)
+    packed = torch.full((n, k if fmt == "mxfp8" else k // 2), 0x38 if fmt == "mxfp8" else 0x22, dtype=torch.uint8, device="cuda")
+    scales = torch.full((n, k // group), 0x38 if fmt == "nvfp4" else 127, dtype=torch.uint8, device="cuda")
+    scales[7, 3] = 0x7F if fmt == "nvfp4" else 0xFF
+    if fmt == "mxfp8":
+        packed[11, 200] = 0x7F
+    y = quantized.quantized_matmul(x, packed, scales, mode=fmt, K=k)
+    rows = torch.zeros(n, dtype=torch.bool, device="cuda")
+    rows[[7, 11] if fmt == "mxfp8" else [7]] = True
+    assert torch.equal(torch.isnan(y), rows.expand_as(y))
