@@ -28,7 +28,13 @@ static int* g_status_dev = nullptr;
 
 static void init_status_word() {
   void* h = nullptr;
-  if (cudaHostAlloc(&h, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+  // The first call may come while a stream is being captured, where an allocation would invalidate the capture unless
+  // this thread says that it does not belong to it.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  const bool exchanged = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+  const cudaError_t e = cudaHostAlloc(&h, 64, cudaHostAllocMapped | cudaHostAllocPortable);
+  if (exchanged) cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
     cudaGetLastError();
     return;
   }

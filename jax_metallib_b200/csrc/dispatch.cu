@@ -150,7 +150,7 @@ static bool i8_skinny_covers(int64_t M, int64_t N, int64_t K, bool tma_ok) {
   // per 64 rows.  Measured (this kernel, the GEMM): 64 x 4096 x 4096 14.0, 21.3 us; 128 x 4096 x 4096 20.0, 22.2 us;
   // 256 x 4096 x 4096 30.8, 22.2 us; 64 x 8192 x 8192 30.5, 37.3 us; 128 x 8192 x 8192 50.4, 38.4 us;
   // 256 x 1024 x 1024 9.8, 10.4 us.
-  return !tma_ok || M <= 32 || (M + 63) / 64 * N <= 8192;
+  return !tma_ok || (gemm_ctas() == num_sms() && (M <= 32 || (M + 63) / 64 * N <= 8192));
 }
 
 }  // namespace qmm
@@ -231,7 +231,8 @@ static int w8a16_entry(const char* name, const uint16_t* x, const int8_t* w, con
   // Few rows, results that stay on this GPU: the HBM-bound kernel.  It reads the weights once per 32 rows; the GEMM reads
   // them once but does not split K, so that a narrow N leaves SMs idle: measured at M = 64, 4096 x 4096: 16 against 39 us,
   // 14336 x 4096: 39 against 121 us, 4096 x 28672: 85 against 62 us; at M = 128, 8192 x 8192: 81 against 74 us.
-  if (tma_ok && (M <= 32 || (M + 31) / 32 * N <= 23000) && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
+  // (A caller that limits the GEMM's CTAs keeps the GEMM: the kernel for few rows fills the device.)
+  if (tma_ok && (M <= 32 || (M + 31) / 32 * N <= 23000) && gemm_ctas() == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
     return w8a16_decode(x, w, scale, y, M, N, K, ldy, flags, s);
   if (tma_ok && M * N >= 128 * 128 && !force_simple())
     return w8a16_tcgen05(x, w, scale, y, M, N, K, ldy, flags, signal, arrive, s);

@@ -4,6 +4,10 @@ Tolerances: results are one rounding of a sum in f32.  A product is exact, so wh
 error, bounded by the number of additions on one element's path (truncated ones count twice) times 2^-24 of sum |x| |w|.
 """
 
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -193,3 +197,29 @@ def test_operator_matmul_nan_codes(cuda, fmt, group, dtype):
     rows = torch.zeros(n, dtype=torch.bool, device="cuda")
     rows[[7, 11] if fmt == "mxfp8" else [7]] = True
     assert torch.equal(torch.isnan(y), rows.expand_as(y))
+
+
+@pytest.mark.parametrize("call", [
+    "ops.w8a16_perchannel(x.bfloat16(), w, s)", "ops.w8a32_perchannel(x, w, s)", "ops.i8_dot(w[:8], w.view(-1)[:1024 * 511].view(1024, 511))[0]",
+    "quantized.affine_quantized_matmul(x, p, g, g, bits=4, group_size=64, K=1024)"])
+def test_first_call_of_a_process_under_capture(cuda, call):
+    """Nothing that a first call sets up (status word, attributes, occupancy) may break a capture that is under way."""
+    program = f"""
+import torch
+from jax_metallib_b200 import _lib, ops, quantized
+_lib.load()
+x = torch.randn(8, 1024, device="cuda")
+w = torch.randint(-127, 128, (1024, 1024), dtype=torch.int8, device="cuda")
+s = torch.rand(1024, device="cuda")
+p = torch.randint(-2**31, 2**31 - 1, (1024, 128), dtype=torch.int32, device="cuda")
+g = torch.rand(1024, 16, device="cuda")
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    y = {call}
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(y, {call})
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", program], check=True, cwd=root, timeout=120)
