@@ -600,8 +600,67 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         s = opapi::decode_e8m0(__ldg(static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(nc) * G + uu));
       }
     };
-    // Scales come in boxes (one TMA copy for all promoters), else each promoter reads its lanes' values a unit ahead.
+    // Scales come in boxes (one TMA copy for all promoters), else each promoter reads its lanes' values ahead.
     const int units_per_box = FMT != kNvfp4 && a.sbox_k ? a.sbox_k / a.pu : 0;
+    if constexpr ((FMT == kMxfp4 || FMT == kMxfp8) && !XF32) {
+      // Two units a stage and nothing but a scale to each: one wait, one look at the scales and one hand-back for both.
+      float nx[2] = {1.f, 1.f}, unused;
+      if (units_per_box == 0) {
+        load_scale(0, nx[0], unused);
+        load_scale(1, nx[1], unused);
+      }
+      int in_box = 0;
+      uint32_t sb = 0, sb_phase = 0, phase = 0;
+      for (int u = 0; u < units; u += 2) {
+        const int buf = u & (C::kAccBufs - 1);
+        const bool both = u + 1 < units;
+        float s0 = nx[0], s1 = nx[1];
+        if (units_per_box) {
+          if (in_box == 0 && !dev::mbar_wait_relaxed_warp(&sfull[sb], sb_phase, a.status, 101)) break;
+          const uint32_t two = *reinterpret_cast<const uint16_t*>(smem + C::kOffS + sb * kSBoxBytes + (q * 32 + lane) * 16 + in_box);
+          s0 = opapi::decode_e8m0(two & 0xFFu);
+          s1 = opapi::decode_e8m0(two >> 8);
+        } else {
+          load_scale(u + 2, nx[0], unused);
+          load_scale(u + 3, nx[1], unused);
+        }
+        if (!dev::mbar_wait_relaxed_warp(&tfull[buf + (both ? 1 : 0)], phase, a.status, 100)) break;
+        dev::tc_fence_after();
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
+        const uint64_t s02 = pack2(s0, s0), s12 = pack2(s1, s1);
+#pragma unroll
+        for (int c = 0; c < C::kCols; c += 16) {
+          uint32_t r[16];
+          dev::tmem_ld_32x16(taddr + c, r);
+          dev::tc_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            fma2(acc[c / 2 + e], s02, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
+          if (both) {
+            dev::tmem_ld_32x16(taddr + BM + c, r);
+            dev::tc_wait_ld();
+          }
+          if (c + 16 == C::kCols) {
+            dev::tc_fence_before();
+            __syncwarp();
+            if (lane < 2) dev::mbar_arrive(&tempty[buf + lane]);
+          }
+          if (both) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              fma2(acc[c / 2 + e], s12, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
+          }
+        }
+        if (buf == C::kAccBufs - 2) phase ^= 1;
+        in_box += 2;
+        if (units_per_box && in_box == units_per_box) {
+          // the arrival's address depends on the values read last: it cannot overtake the load
+          if (lane == 0) dev::mbar_arrive(&sempty[sb] + (__float_as_uint(s0 + s1) == 0x7FC1FFC1u && a.M < 0));
+          in_box = 0;
+          if (++sb == kSBoxes) { sb = 0; sb_phase ^= 1; }
+        }
+      }
+    } else {
     float s_next = 1.f, b_next = 0.f;
     if (units_per_box == 0) load_scale(0, s_next, b_next);
     int in_box = 0, in_group = 0, comp = 0;   // unit of the box, unit of the group, group of the box
@@ -683,6 +742,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         in_box = comp = 0;
         if (++sb == kSBoxes) { sb = 0; sb_phase ^= 1; }
       }
+    }
     }
     // ---- this slice's results, [row][column], into the idle rings (after every warp is done with them)
     dev::tc_fence_before();
