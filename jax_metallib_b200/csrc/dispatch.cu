@@ -231,8 +231,13 @@ static int w8a16_entry(const char* name, const uint16_t* x, const int8_t* w, con
   // Few rows, results that stay on this GPU: the HBM-bound kernel.  It reads the weights once per 32 rows; the GEMM reads
   // them once but does not split K, so that a narrow N leaves SMs idle: measured at M = 64, 4096 x 4096: 16 against 39 us,
   // 14336 x 4096: 39 against 121 us, 4096 x 28672: 85 against 62 us; at M = 128, 8192 x 8192: 81 against 74 us.
+  // Its blocks are 32 rows x 128 columns.  Where K is short, a second one per CTA is what the GEMM does not have: K = 1024,
+  // 18432 columns (96 x 6144) 12.1 against 15.0 us, 20480 (320 x 2048) 16.9 against 14.5; K = 2048, 20480: 21.8 against 23.1.
+  // Shorter still, the rows it reads again count: K = 128, 8192 columns (128 x 2048) 6.0 against 7.3 us, 16384 (512 x 1024)
+  // 7.7 against 7.3.
   // (A caller that limits the GEMM's CTAs keeps the GEMM: the kernel for few rows fills the device.)
-  if (tma_ok && (M <= 32 || (M + 31) / 32 * N <= 23000) && gemm_ctas() == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
+  const int64_t few = K < 256 ? 8192 : K < 2048 ? 148 * 128 : 23000;
+  if (tma_ok && (M <= 32 || (M + 31) / 32 * N <= few) && gemm_ctas() == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
     return w8a16_decode(x, w, scale, y, M, N, K, ldy, flags, s);
   if (tma_ok && M * N >= 128 * 128 && !force_simple())
     return w8a16_tcgen05(x, w, scale, y, M, N, K, ldy, flags, signal, arrive, s);

@@ -35,7 +35,8 @@ def _check(y, x, w, scale, rounding, steps):
 
 
 @pytest.mark.parametrize("m,k,n", [(1, 8, 16), (1, 4096, 4096), (8, 72, 144), (9, 1032, 1040), (16, 4096, 28672), (17, 64, 128),
-                                   (32, 4096, 28672), (33, 520, 272), (64, 14336, 256), (97, 1000, 5632)])
+                                   (32, 4096, 28672), (33, 520, 272), (64, 14336, 256), (97, 1000, 5632),
+                                   (97, 1000, 4736), (97, 2048, 5744), (1024, 248, 256)])
 def test_int8_weights_bf16_rows(cuda, m, k, n):
     g = _gen(m + k + n)
     x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
