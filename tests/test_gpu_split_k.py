@@ -51,7 +51,8 @@ def test_int8_weights_bf16_rows(cuda, m, k, n):
 
 
 @pytest.mark.parametrize("packed", [True, False])
-@pytest.mark.parametrize("m,k,n", [(1, 128, 128), (8, 4096, 384), (9, 1280, 1536), (16, 14336, 256), (16, 384, 16384)])
+@pytest.mark.parametrize("m,k,n", [(1, 128, 128), (8, 4096, 384), (9, 1280, 1536), (16, 14336, 256), (16, 384, 16384),
+                                   (4, 4864, 12416), (5, 4864, 12416)])
 def test_int4_weights(cuda, m, k, n, packed):
     g = _gen(m + k + n)
     x = (torch.randn(m, k, device="cuda", generator=g) * 3 + 1).bfloat16()
