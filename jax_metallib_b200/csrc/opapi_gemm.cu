@@ -406,8 +406,10 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 dev::umma_f16_lh(d, a_lo + h * 4 + j * 2, kDescHi, b_lo + t * (C::kXTile >> 4) + h * 4 + j * 2, kDescHi, a.idesc,
                                  (t != C::kTerms - 1 || j != 0) ? 1u : 0u);
           }
-          // (a commit costs the thread as much as an MMA: one for the units of a stage)
-          if (h == units_per_stage - 1 || u == units - 1) dev::tc_commit(&tfull[buf]);
+          // A commit costs the thread as much as an MMA: one for the units of a stage, on the barrier of the stage's last
+          // buffer even if its last unit does not exist.  That barrier completes once in every round of the buffers, as
+          // the parity that the promoters wait for takes for granted; the one of a stage's first buffer never completes.
+          if (h == units_per_stage - 1 || u == units - 1) dev::tc_commit(&tfull[buf | (units_per_stage - 1)]);
         }
         if (ok) dev::tc_commit(&consumed[st % kConsumed]);
       }
@@ -624,7 +626,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
           load_scale(u + 2, nx[0], unused);
           load_scale(u + 3, nx[1], unused);
         }
-        if (!dev::mbar_wait_relaxed_warp(&tfull[buf + (both ? 1 : 0)], phase, a.status, 100)) break;
+        if (!dev::mbar_wait_relaxed_warp(&tfull[buf + 1], phase, a.status, 100)) break;   // the stage's barrier, also for one unit
         dev::tc_fence_after();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
         const uint64_t s02 = pack2(s0, s0), s12 = pack2(s1, s1);
@@ -690,9 +692,12 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) break;
         exact = *reinterpret_cast<const uint32_t*>(flags + slot * kGroupWarps) != 0u;
       }
-      // the units of a stage complete together, on the barrier of the last
-      const int last = units_per_stage == 2 ? min(u | 1, units - 1) & (C::kAccBufs - 1) : buf;
-      if (!dev::mbar_wait_relaxed_warp(&tfull[last], phase, a.status, 100)) break;
+      // The units of a stage complete together, on the barrier of its last buffer.  It is waited for before the first of
+      // them is handed back: a last stage of one unit asks for that buffer alone, and its commit would otherwise complete
+      // the next round of a barrier that some promoter has still to see complete this one.
+      if ((u & (units_per_stage - 1)) == 0 &&
+          !dev::mbar_wait_relaxed_warp(&tfull[buf | (units_per_stage - 1)], phase, a.status, 100))
+        break;
       dev::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
       if (C::kUnitInfo && exact) {

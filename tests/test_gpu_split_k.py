@@ -144,15 +144,11 @@ def _operator_weights(fmt, group, n, k, g):
 
 FORMATS = [("affine4", 32), ("affine4", 64), ("affine4", 96), ("affine4", 128), ("affine8", 32), ("affine8", 128), ("mxfp4", 32),
            ("mxfp8", 32), ("nvfp4", 16)]
-# rows at the edges of the tiles of 32, 64 and 128; K of half a stage, of several boxes and of none; ragged columns
+# rows at the edges of the tiles of 32, 64 and 128; K of several boxes and of none; ragged columns
 SHAPES = [(4, 384, 17), (17, 1152, 128), (33, 384, 200), (64, 2304, 130), (65, 1920, 333), (130, 5376, 260), (300, 1152, 96)]
 
 
-@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
-@pytest.mark.parametrize("m,k,n", SHAPES)
-@pytest.mark.parametrize("fmt,group", FORMATS)
-def test_operator_matmul(cuda, fmt, group, m, k, n, dtype):
-    k = (k + group - 1) // group * group
+def _check_operator(fmt, group, m, k, n, dtype):
     g = _gen(m + k + n)
     run, w, size = _operator_weights(fmt, group, n, k, g)
     x = torch.randn(m, k, device="cuda", generator=g).to(dtype)
@@ -161,7 +157,30 @@ def test_operator_matmul(cuda, fmt, group, m, k, n, dtype):
     bound = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -24) * ref.abs() + _sum_error(k, 16) * (x.double().abs() @ size.T)
     if dtype == torch.float16:
         bound += 2.0 ** -24   # results below the smallest normal number
-    assert bool(((y - ref).abs() <= bound).all()), ((y - ref).abs() / bound).max().item()
+    assert bool(((y - ref).abs() <= bound).all()), (k, ((y - ref).abs() / bound).max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("m,k,n", SHAPES)
+@pytest.mark.parametrize("fmt,group", FORMATS)
+def test_operator_matmul(cuda, fmt, group, m, k, n, dtype):
+    _check_operator(fmt, group, m, (k + group - 1) // group * group, n, dtype)
+
+
+# Units of 32 k, an odd number of them: the last stage is half filled.  16384 columns leave one CTA to a tile, whose slice is all
+# of K (1, 3, .. units, the last of them in every round of four or eight accumulators); 130 columns split K, and the last slice is odd.
+HALF_STAGES = {16384: (32, 96, 160, 224, 288, 352, 416, 480, 544, 672, 800, 864), 130: (288, 1056, 1440, 2080, 2400)}
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("n", sorted(HALF_STAGES))
+@pytest.mark.parametrize("m", [4, 48, 300])
+@pytest.mark.parametrize("fmt,group", [("affine4", 32), ("affine4", 96), ("affine8", 32), ("affine8", 160), ("mxfp4", 32), ("mxfp8", 32)])
+def test_operator_matmul_half_stage(cuda, fmt, group, m, n, dtype):
+    widths = [k for k in HALF_STAGES[n] if k % group == 0 and k % 64 == 32]
+    assert widths
+    for k in widths:
+        _check_operator(fmt, group, m, k, n, dtype)
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
