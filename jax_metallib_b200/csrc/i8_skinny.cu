@@ -253,11 +253,7 @@ i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) mma_i8<AU, BU>(acc[j][mt], w0, w1, w2, w3, xr[mt][0], xr[mt][1]);
         }
-        // The slot goes back only when its bytes are in registers: an arrival that merely follows the loads in program
-        // order let the refill overtake the last of them (seen with remote shared-memory traffic on the same SM), so
-        // its address is made to depend on what they returned.
-        // Lane 0's copy stands for the warp's: a shared load completes for all lanes at once.
-        if (lane == 0) dev::mbar_arrive(&empty[s] + ((dep == 0x7FC1FFC1u) & never));
+        release_slot(&empty[s], dep, never, lane);
         if (++s == S) { s = 0; ph ^= 1; }
       }
       if (!ok) break;

@@ -29,6 +29,7 @@
 #include <cooperative_groups.h>
 
 #include "opapi_decode.cuh"
+#include "split_k.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -656,8 +657,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         if (buf == C::kAccBufs - 2) phase ^= 1;
         in_box += 2;
         if (units_per_box && in_box == units_per_box) {
-          // the arrival's address depends on the values read last: it cannot overtake the load
-          if (lane == 0) dev::mbar_arrive(&sempty[sb] + (__float_as_uint(s0 + s1) == 0x7FC1FFC1u && a.M < 0));
+          split::release_slot(&sempty[sb], __float_as_uint(s0) ^ __float_as_uint(s1), a.M < 0, lane);
           in_box = 0;
           if (++sb == kSBoxes) { sb = 0; sb_phase ^= 1; }
         }
@@ -682,6 +682,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       } else {
         load_scale(u + 1, s_next, b_next);
       }
+      const uint32_t scale_dep = __float_as_uint(s) ^ __float_as_uint(b);
       if (C::kBias && XF32) {
         float shifted;
         if (centred<FMT>(s, b, shifted)) b = shifted;
@@ -742,8 +743,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       if (buf == C::kAccBufs - 1) phase ^= 1;
       if (++in_group == units_per_group) { in_group = 0; ++comp; }
       if (units_per_box && ++in_box == units_per_box) {
-        // the arrival's address depends on the value read last: it cannot overtake the load
-        if (lane == 0) dev::mbar_arrive(&sempty[sb] + (__float_as_uint(s + b) == 0x7FC1FFC1u && a.M < 0));
+        split::release_slot(&sempty[sb], scale_dep, a.M < 0, lane);
         in_box = comp = 0;
         if (++sb == kSBoxes) { sb = 0; sb_phase ^= 1; }
       }

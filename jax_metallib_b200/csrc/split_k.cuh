@@ -19,6 +19,15 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// Hands a slot of a ring back (one arrival per warp) once what every lane loaded from it is in registers: an arrival that
+// merely follows the loads in program order let the refill overtake the last of them (seen with remote shared-memory
+// traffic on the same SM).  `dep` combines what all of a lane's loads returned; the vote cannot be taken before the last
+// lane has it, and the arrival's address depends on the vote.  `never` is 0, but not to the compiler.
+__device__ __forceinline__ void release_slot(uint64_t* empty, uint32_t dep, int never, int lane) {
+  const int hit = __any_sync(0xFFFFFFFFu, dep == 0x7FC1FFC1u);
+  __syncwarp();
+  if (lane == 0) dev::mbar_arrive(empty + (hit & never));
+}
 // Arrives (release, cluster scope) on the barrier at the same place of CTA `rank`'s shared memory.
 __device__ __forceinline__ void arrive_remote(uint64_t* bar, int rank) {
   asm volatile(

@@ -192,13 +192,16 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
           const uint32_t s2 = *reinterpret_cast<const uint32_t*>(stp + L::kOffS + (lc + 16 * j) * 2);
           sc[j][0] = __uint_as_float(s2 << 16) * 16777216.f;
           sc[j][1] = __uint_as_float(s2 & 0xFFFF0000u) * 16777216.f;
+          dep ^= s2;
           uint32_t z0, z1;
           if (ZP) {
             const uint32_t zb = stp[L::kOffZ + (lc + 16 * j) / 2];
+            dep ^= zb;
             z0 = zb & 0xFu;
             z1 = zb >> 4;
           } else {
             const uint32_t zb = *reinterpret_cast<const uint16_t*>(stp + L::kOffZ + lc + 16 * j);
+            dep ^= zb;
             z0 = zb & 0xFFu;
             z1 = zb >> 8;
           }
@@ -235,10 +238,7 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             for (int i = 0; i < 4; ++i)
               acc[j][mt][i] = fmaf(sc[j][i >> 1], fmaf(-zf[j][i >> 1], xs[mt][i & 1], d[mt][i]), acc[j][mt][i]);
         }
-        // The slot goes back only when its bytes are in registers: an arrival that merely follows the loads in program
-        // order let the refill overtake the last of them, so its address is made to depend on what they returned.
-        dep ^= __float_as_uint(sc[1][1]) ^ __float_as_uint(zf[1][1]);
-        if (lane == 0) dev::mbar_arrive(&empty[s] + ((dep == 0x7FC1FFC1u) & never));
+        release_slot(&empty[s], dep, never, lane);
         if (++s == S) { s = 0; ph ^= 1; }
       }
       if (!ok) break;

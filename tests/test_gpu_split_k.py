@@ -108,6 +108,38 @@ def test_int8_dot_any_rows(cuda, m, k, n, ta, tb, offset):
     assert torch.equal(out, ref.to(torch.int32).float() * rs[:, None] * cs)
 
 
+# Three tiles and more to a cluster (296 CTAs are resident, 148 of the int8 dots' 64-row tiles): partial tiles change hands through
+# buffers that come back, the rings run on over the tiles.
+@pytest.mark.parametrize("m,k,n", [(3, 320, 124000), (16, 192, 124016), (32, 320, 124000), (31, 64, 115200)])
+def test_tiles_change_hands_bf16_rows(cuda, m, k, n):
+    g = _gen(m + k + n)
+    w = torch.randint(-128, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
+    s = torch.rand(n, device="cuda", generator=g) * 0.01 + 0.005
+    for _ in range(4):
+        x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+        _check(ops.w8a16_perchannel(x, w, s), x, w, s.double(), 2.0 ** -8, k // 16 + 1)
+
+
+@pytest.mark.parametrize("m,k,n", [(5, 320, 124000), (1000, 196, 2000)])
+def test_tiles_change_hands_f32_rows(cuda, m, k, n):
+    g = _gen(m + k + n)
+    w = torch.randint(-128, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
+    s = torch.rand(n, device="cuda", generator=g) * 0.01 + 0.005
+    for _ in range(4):
+        x = torch.randn(m, k, device="cuda", generator=g)
+        _check(ops.w8a32_perchannel(x, w, s), x, w, s.double(), 2.0 ** -22, 6)
+
+
+@pytest.mark.parametrize("m,k,n", [(8, 320, 124000), (16, 320, 124000), (32, 320, 124000), (1, 331, 124001), (17, 321, 124001),
+                                   (1000, 331, 5001)])
+def test_tiles_change_hands_int8_dot(cuda, m, k, n):
+    g = _gen(m + k + n)
+    b = torch.randint(-128, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
+    for _ in range(4):
+        a = torch.randint(-128, 128, (m, k), dtype=torch.int8, device="cuda", generator=g)
+        assert torch.equal(ops.i8_dot(a, b)[0].double(), a.double() @ b.double())
+
+
 def _operator_weights(fmt, group, n, k, g):
     """Packed weights, call arguments and the dequantised weights [N, K] in 64 bits."""
     groups = (n, k // group)
