@@ -4,7 +4,7 @@
 //
 // and the same with f32 activations and results (any M; three bf16 terms per activation, see split4).
 // Measured at M = 1: 4096 x 28672 25 us (4.7 TB/s), 4096 x 6144 8.0 us, 14336 x 4096 14.0 us, the four linears of a layer
-// 57 us (one thread per column before: 1905 us); f32, 32 x 1024 x 1024 10.1 -> 6.7 us, 256 x 4096 x 4096 528 -> 149 us.
+// 57 us (one thread per column before: 1905 us); f32, 32 x 1024 x 1024 10.1 -> 6.7 us, 256 x 4096 x 4096 528 -> 140 us.
 //
 // Bound by HBM: the weights (K*N bytes) are read once.  A cluster of KS CTAs owns blocks of 128
 // columns and splits K between its CTAs; every CTA runs a ring of TMA stages (64 k x 128 columns of
@@ -72,23 +72,18 @@ __device__ __forceinline__ uint32_t bytes02_to_bf16x2(uint32_t t) {
   return r;
 }
 
-// Four f32 -> their bf16 terms, as pairs of k: the top 8 significant bits, the next 8, the rest.  Infinities and NaN
-// have no second and third term, and a NaN stays one when it is cut.
-__device__ __forceinline__ void split4(uint32_t (&v)[4], uint32_t (&hi)[2], uint32_t (&mid)[2], uint32_t (&lo)[2]) {
+// Four f32 -> their bf16 terms, as pairs of k: the top 8 significant bits, the next 8, the rest.  Where the three do not
+// hold a value, its third term has bits below them: 16 low bits of `rest` are not all zero.  That is an infinity or NaN
+// (whose difference to itself is the NaN 0x7FFFFFFF), or a value whose last bits lie below bf16's smallest (2^-133, so
+// |x| < 2^-110).
+__device__ __forceinline__ void split4(const uint32_t (&v)[4], uint32_t (&hi)[2], uint32_t (&mid)[2], uint32_t (&lo)[2],
+                                       uint32_t& rest) {
   uint32_t m[4], l[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     m[i] = __float_as_uint(__uint_as_float(v[i]) - __uint_as_float(v[i] & 0xFFFF0000u));
     l[i] = __float_as_uint(__uint_as_float(m[i]) - __uint_as_float(m[i] & 0xFFFF0000u));
-  }
-  const uint32_t top = max(max(v[0] & 0x7FFFFFFFu, v[1] & 0x7FFFFFFFu), max(v[2] & 0x7FFFFFFFu, v[3] & 0x7FFFFFFFu));
-  if (top >= 0x7F800000u) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if ((v[i] & 0x7FFFFFFFu) >= 0x7F800000u) {
-        if ((v[i] & 0x7FFFFFFFu) > 0x7F800000u) v[i] |= 0x00400000u;
-        m[i] = l[i] = 0u;
-      }
+    rest |= l[i];
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
@@ -96,6 +91,54 @@ __device__ __forceinline__ void split4(uint32_t (&v)[4], uint32_t (&hi)[2], uint
     mid[i] = __byte_perm(m[2 * i], m[2 * i + 1], 0x7632);
     lo[i] = __byte_perm(l[2 * i], l[2 * i + 1], 0x7632);
   }
+}
+// Two registers of ldmatrix -> the MMA's weight operand for 16 k.
+__device__ __forceinline__ void weights4(uint32_t w0, uint32_t w1, uint32_t (&a)[4]) {
+  a[0] = bytes02_to_bf16x2(w0);
+  a[1] = bytes02_to_bf16x2(w0 >> 8);
+  a[2] = bytes02_to_bf16x2(w1);
+  a[3] = bytes02_to_bf16x2(w1 >> 8);
+}
+__device__ __forceinline__ void lds_v4(uint32_t addr, uint32_t (&v)[4]) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
+}
+// The sums over a stage's 32 k, 16 columns x 8 rows, where split4 does not hold every value: what it does not hold goes
+// into a second sum, times 2^64 (an infinity or NaN as it is).  A call, so that its registers do not count elsewhere.
+__device__ __noinline__ float4 awkward_tile(uint32_t w_addr, uint32_t x_addr, int t4, int x_row) {
+  uint32_t wr[4];
+  ldmatrix_x4_trans(w_addr, wr);
+  float d[2][4] = {};
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    uint32_t v[2][4], a[4];
+    lds_v4(x_addr + (((q * 4 + t4) ^ x_row) << 4), v[0]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float x = __uint_as_float(v[0][i]), m = x - __uint_as_float(v[0][i] & 0xFFFF0000u);
+      const float l = m - __uint_as_float(__float_as_uint(m) & 0xFFFF0000u);
+      const bool held = (__float_as_uint(l) & 0xFFFFu) == 0u;
+      v[1][i] = held ? 0u : __float_as_uint(x * 18446744073709551616.f);
+      if (!held) v[0][i] = 0u;
+      if ((v[1][i] & 0x7FFFFFFFu) > 0x7F800000u) v[1][i] |= 0x00400000u;   // stays a NaN when it is cut
+    }
+    weights4(wr[2 * q], wr[2 * q + 1], a);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      uint32_t hi[2], mid[2], lo[2], unused = 0;
+      split4(v[s], hi, mid, lo, unused);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {   // an infinity or NaN is its first term alone
+        if ((hi[i] & 0x7F80u) == 0x7F80u) mid[i] &= 0xFFFF0000u, lo[i] &= 0xFFFF0000u;
+        if ((hi[i] & 0x7F800000u) == 0x7F800000u) mid[i] &= 0xFFFFu, lo[i] &= 0xFFFFu;
+      }
+      mma_bf16_16816(d[s], a[0], a[1], a[2], a[3], lo[0], lo[1]);
+      mma_bf16_16816(d[s], a[0], a[1], a[2], a[3], mid[0], mid[1]);
+      mma_bf16_16816(d[s], a[0], a[1], a[2], a[3], hi[0], hi[1]);
+    }
+  }
+  constexpr float kSmall = 3.469446951953614e-18f;   // 2^-64, and 64 of the weights
+  return make_float4(fmaf(d[1][0], kSmall, d[0][0] * 64.f), fmaf(d[1][1], kSmall, d[0][1] * 64.f),
+                     fmaf(d[1][2], kSmall, d[0][2] * 64.f), fmaf(d[1][3], kSmall, d[0][3] * 64.f));
 }
 
 template <int MT, bool XF32>
@@ -195,71 +238,82 @@ w8_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       for (int it = it_begin; it < it_end; ++it) {
         if (!dev::mbar_wait_relaxed_warp(&full[s], ph, status, 82)) { ok = false; break; }
         const uint32_t st = ring + s * L::kStage;
-        uint32_t wr[2][4];
-        ldmatrix_x4_trans(st + w_off0, wr[0]);
-        ldmatrix_x4_trans(st + w_off1, wr[1]);
-        uint32_t dep = wr[0][3] ^ wr[1][3];
+        uint32_t dep;
         if constexpr (!XF32) {
-          uint32_t xr[MT][4];
+          uint32_t wr[2][4], xr[MT][4];
+          ldmatrix_x4_trans(st + w_off0, wr[0]);
+          ldmatrix_x4_trans(st + w_off1, wr[1]);
+          dep = wr[0][3] ^ wr[1][3];
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) ldmatrix_x4(st + x_off + mt * 1024, xr[mt]);
 #pragma unroll
           for (int q = 0; q < 2; ++q)   // 16 k each
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-              const uint32_t a0 = bytes02_to_bf16x2(wr[j][2 * q]), a1 = bytes02_to_bf16x2(wr[j][2 * q] >> 8);
-              const uint32_t a2 = bytes02_to_bf16x2(wr[j][2 * q + 1]), a3 = bytes02_to_bf16x2(wr[j][2 * q + 1] >> 8);
+              uint32_t a[4];
+              weights4(wr[j][2 * q], wr[j][2 * q + 1], a);
 #pragma unroll
-              for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(acc[j][mt], a0, a1, a2, a3, xr[mt][2 * q], xr[mt][2 * q + 1]);
+              for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(acc[j][mt], a[0], a[1], a[2], a[3], xr[mt][2 * q], xr[mt][2 * q + 1]);
             }
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) dep ^= xr[mt][3];
         } else {
           // x = hi + mid + lo, bf16 each and exact together; the smallest terms are added first, into an accumulator
           // that starts at zero every stage: a correctly rounded f32 addition takes over after 32 k
-          float d[2][MT][4];
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) d[j][mt][i] = 0.f;
-          uint32_t term[3][2][MT][2];   // [hi, mid, lo][16-k step][row tile][k pair]
+          uint32_t wr[2][4];
+          ldmatrix_x4_trans(st + w_off0, wr[0]);
+          ldmatrix_x4_trans(st + w_off1, wr[1]);
+          dep = wr[0][3] ^ wr[1][3];
+          uint32_t term[3][2][MT][2], rest = 0;   // [hi, mid, lo][16-k step][row tile][k pair]
 #pragma unroll
           for (int q = 0; q < 2; ++q)
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
               uint32_t v[4];
-              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-                           : "r"(st + x_off + mt * 1024 + (((q * 4 + t4) ^ x_row) << 4)));
+              lds_v4(st + x_off + mt * 1024 + (((q * 4 + t4) ^ x_row) << 4), v);
               dep ^= v[3];
-              split4(v, term[0][q][mt], term[1][q][mt], term[2][q][mt]);
+              split4(v, term[0][q][mt], term[1][q][mt], term[2][q][mt], rest);
+            }
+          if (!__any_sync(0xFFFFFFFFu, rest & 0xFFFFu)) {
+            float d[2][MT][4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) d[j][mt][i] = 0.f;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              uint32_t a[2][4];
+#pragma unroll
+              for (int q = 0; q < 2; ++q) weights4(wr[j][2 * q], wr[j][2 * q + 1], a[q]);
+#pragma unroll
+              for (int e = 2; e >= 0; --e)
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+#pragma unroll
+                  for (int mt = 0; mt < MT; ++mt)
+                    mma_bf16_16816(d[j][mt], a[q][0], a[q][1], a[q][2], a[q][3], term[e][q][mt][0], term[e][q][mt][1]);
             }
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            uint32_t a[2][4];
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              a[q][0] = bytes02_to_bf16x2(wr[j][2 * q]);
-              a[q][1] = bytes02_to_bf16x2(wr[j][2 * q] >> 8);
-              a[q][2] = bytes02_to_bf16x2(wr[j][2 * q + 1]);
-              a[q][3] = bytes02_to_bf16x2(wr[j][2 * q + 1] >> 8);
-            }
+              for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int e = 2; e >= 0; --e)
+                for (int i = 0; i < 4; ++i) acc[j][mt][i] = fmaf(d[j][mt][i], 64.f, acc[j][mt][i]);
+          } else {
 #pragma unroll
-              for (int q = 0; q < 2; ++q)
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-                  mma_bf16_16816(d[j][mt], a[q][0], a[q][1], a[q][2], a[q][3], term[e][q][mt][0], term[e][q][mt][1]);
+              for (int mt = 0; mt < MT; ++mt) {
+                const float4 e = awkward_tile(st + (j ? w_off1 : w_off0), st + x_off + mt * 1024, t4, x_row);
+                acc[j][mt][0] += e.x;
+                acc[j][mt][1] += e.y;
+                acc[j][mt][2] += e.z;
+                acc[j][mt][3] += e.w;
+                dep ^= __float_as_uint(e.x);
+              }
           }
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) acc[j][mt][i] += d[j][mt][i];
         }
         release_slot(&empty[s], dep, never, lane);
         if (++s == S) { s = 0; ph ^= 1; }
@@ -314,8 +368,8 @@ w8_decode_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
           }
         const float2 sc = make_float2(__ldg(scale + col0 + c), __ldg(scale + col0 + c + 1));
         const size_t i = static_cast<size_t>(row0 + m) * ldy + col0 + c;
-        v.x = v.x * 64.f * sc.x;
-        v.y = v.y * 64.f * sc.y;
+        v.x = XF32 ? v.x * sc.x : v.x * 64.f * sc.x;
+        v.y = XF32 ? v.y * sc.y : v.y * 64.f * sc.y;
         if (XF32) *reinterpret_cast<float2*>(static_cast<float*>(y) + i) = v;
         else *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(y) + i) = dev::pack_bf16x2(v.x, v.y);
       }

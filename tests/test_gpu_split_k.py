@@ -78,6 +78,24 @@ def test_int8_weights_f32_rows(cuda, m, k, n):
     _check(ops.w8a32_perchannel(x, w, s), x, w, s.double(), 2.0 ** -22, 6)
 
 
+@pytest.mark.parametrize("m,k,n", [(4, 96, 32), (8, 1024, 1024), (13, 260, 144), (40, 2048, 256)])
+def test_int8_weights_f32_small_rows(cuda, m, k, n):
+    """Activations down to the smallest f32, whole rows of them and among larger ones: no bit of them is lost."""
+    g = _gen(m + k + n)
+    w = torch.randint(-128, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
+    scale = (torch.rand(n, device="cuda", generator=g) + 0.5) * 2.0 ** 100
+    bits = torch.randn(m, k, device="cuda", generator=g).double()
+    wd = w.double()
+    for e in (-100, -109, -110, -111, -112, -118, -126, -133, -140, -148):
+        mixed = torch.where(torch.rand(m, k, device="cuda", generator=g) < 0.1, e, -100)
+        for x in ((bits * 2.0 ** e).float(), torch.ldexp(bits, mixed).float()):
+            xd = x.double()
+            y, ref, size = ops.w8a32_perchannel(x, w, scale).double(), (xd @ wd) * scale, (xd.abs() @ wd.abs()) * scale
+            # beside the sum's own error, additions below 2^-126 round to 2^-149: one per stage of 32 k, and the partial tiles
+            bound = 2.0 ** -22 * ref.abs() + _sum_error(k, 6) * size + (k / 32 + 20) * 2.0 ** -149 * scale
+            assert bool(((y - ref).abs() <= bound).all()), (e, ((y - ref).abs() / bound).max().item())
+
+
 def test_int8_weights_f32_special_values(cuda):
     x = torch.randn(5, 256, device="cuda", generator=_gen(1))
     x[0, 3], x[1, 7], x[2, 5], x[2, 9], x[3, 200] = float("inf"), float("nan"), -float("inf"), float("inf"), 1e36
