@@ -85,8 +85,8 @@ QMM_API int qmm_device_status(void);
 QMM_API int qmm_selftest_host(void);
 QMM_API void qmm_clear_device_status(void);
 
-/* Upper bound on the CTAs of the persistent tcgen05 GEMMs (qmm_w8a16_perchannel,
- * qmm_i8i8_i32); 0 = one per SM (the default).  Those kernels keep one CTA per
+/* Upper bound on the CTAs of the persistent kernels of qmm_w8a16_perchannel and
+ * qmm_i8i8_i32; 0 = what the device holds (the default).  Those kernels keep one CTA per
  * SM resident for the whole launch, so a communication kernel that should run
  * next to them (an NCCL all-gather of the previous output on a second stream)
  * finds no SM unless some are left free; a tensor-parallel caller sets the

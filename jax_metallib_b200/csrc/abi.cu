@@ -8,7 +8,7 @@
 
 #include <atomic>
 
-#include "common.cuh"
+#include "split_k.cuh"
 
 namespace qmm {
 
@@ -207,6 +207,14 @@ int qmm_selftest_host(void) {
   if (!qmm::mark_device_once(other, -1) || !qmm::mark_device_once(other, qmm::kMaxDevices)) return 4;
   std::atomic<int> cache{INT32_MIN};
   if (qmm::env_int_once("QMM_SELFTEST_UNSET_VARIABLE", 7, cache) != 7 || cache.load() != 7) return 5;
+  // a launch that splits K keeps to what the device holds and to the caller's limit, whatever the shape
+  for (int limit : {1, 3, 100, 147, INT_MAX})
+    for (int tiles : {1, 7, 148, 5000})
+      for (int stages : {1, 2, 65}) {
+        const qmm::split::Grid g = qmm::split::choose_grid(tiles, stages, [](int ks) { return 296 / ks; }, limit);
+        if (g.ks < 1 || g.clusters < 1 || g.ks > stages || g.clusters > tiles) return 6;
+        if (g.ks * g.clusters > 296 || g.ks * g.clusters > limit) return 7;
+      }
   return 0;
 }
 

@@ -356,9 +356,11 @@ static int launch(const Args& p, cudaStream_t stream) {
   auto kern = i8_skinny_kernel<MT, AU, BU, TMA>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
   const int stages_total = (p.K + kBK - 1) / kBK;
+  // a limit leaves SMs to a collective: one CTA to each of the others
+  const int limit = gemm_ctas() < num_sms() ? gemm_ctas() : INT_MAX;
   const Grid g = choose_grid(((p.N + kCols - 1) / kCols) * ((p.M + MT * 8 - 1) / (MT * 8)), stages_total, [&](int ks) {
     return resident_clusters(kern, L::kThreads, L::kTotal, L::kPerSm, ks, resident);
-  });
+  }, limit);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(g.ks, g.clusters);

@@ -1,6 +1,8 @@
 // Helpers of the kernels that split K over a thread-block cluster and add the partial tiles over distributed shared memory.
 #pragma once
 
+#include <limits.h>
+
 #include "common.cuh"
 
 namespace qmm {
@@ -75,13 +77,14 @@ inline void set_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], i
 
 // Resident clusters walk the tiles, so a launch takes as many rounds as the busiest cluster has tiles; a round costs its
 // stages and the hand-over of the partial tiles (about six stages).  resident(ks): clusters of ks CTAs held at once.
+// max_ctas: a caller's limit on the CTAs of the launch.
 constexpr int kRoundCost = 6;
 template <typename Fn>
-inline Grid choose_grid(int tiles, int stages_total, Fn resident) {
+inline Grid choose_grid(int tiles, int stages_total, Fn resident, int max_ctas = INT_MAX) {
   Grid best = {1, 1};
   long long best_cost = -1;
-  for (int ks = 1; ks <= kMaxCluster && ks <= stages_total; ++ks) {
-    const int c = resident(ks);
+  for (int ks = 1; ks <= kMaxCluster && ks <= stages_total && ks <= max_ctas; ++ks) {
+    const int held = resident(ks), c = held < max_ctas / ks ? held : max_ctas / ks;
     const int rounds = (tiles + c - 1) / c;
     const long long cost = static_cast<long long>(rounds) * ((stages_total + ks - 1) / ks + kRoundCost);
     if (best_cost < 0 || cost < best_cost) {

@@ -11,7 +11,7 @@ import sys
 import pytest
 import torch
 
-from jax_metallib_b200 import ops, quantized
+from jax_metallib_b200 import _lib, ops, quantized
 
 pytestmark = pytest.mark.gpu
 
@@ -156,6 +156,19 @@ def test_tiles_change_hands_int8_dot(cuda, m, k, n):
     for _ in range(4):
         a = torch.randint(-128, 128, (m, k), dtype=torch.int8, device="cuda", generator=g)
         assert torch.equal(ops.i8_dot(a, b)[0].double(), a.double() @ b.double())
+
+
+@pytest.mark.parametrize("limit", [1, 5, 147])
+def test_int8_dot_any_rows_cta_limit(cuda, limit):
+    lib, g = _lib.load(), _gen(limit)
+    a = torch.randint(-128, 128, (200, 331), dtype=torch.int8, device="cuda", generator=g)
+    b = torch.randint(-128, 128, (331, 1001), dtype=torch.int8, device="cuda", generator=g)
+    try:
+        _lib.check(lib.qmm_set_cta_limit(limit))
+        acc = ops.i8_dot(a, b)[0]
+    finally:
+        _lib.check(lib.qmm_set_cta_limit(0))
+    assert torch.equal(acc.double(), a.double() @ b.double())
 
 
 def _operator_weights(fmt, group, n, k, g):
