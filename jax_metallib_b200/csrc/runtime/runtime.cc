@@ -45,6 +45,7 @@ struct EventState {
   mutable std::mutex mu;
   mutable std::condition_variable cv;
   std::atomic<bool> ready{false};
+  bool of_launch = false;  // completes with the status that the kernels of an execution left
   int status = QMM_OK;
   std::string message;
   std::vector<std::function<void()>> callbacks;
@@ -838,9 +839,12 @@ static int read_to_host(qmm_rt_buffer* b, void* dst, int64_t offset, int64_t siz
   // A copy into pageable memory is complete when the call returns.  Then the event completes here: the host function
   // and the completion thread cost two thread wake-ups, 0.2-0.3 ms per result.
   if (cudaStreamQuery(dev->d2h) == cudaSuccess) {
-    // the producer is done too, but its own completion job may not have run yet: ask what that job would ask
-    if (producer && producer->ready.load() && producer->status != QMM_OK) st->finish(producer->status, producer->message);
-    else if (qmm_device_status() != 0) st->finish(QMM_ERR_TIMEOUT, "a kernel of this launch (or an earlier one) gave up waiting");
+    // The producer is done too.  What its completion recorded counts, not what another kernel did since; if that job has
+    // not run yet, ask what it would ask.
+    if (!producer) st->finish(QMM_OK, "");
+    else if (producer->ready.load()) st->finish(producer->status, producer->message);
+    else if (producer->of_launch && qmm_device_status() != 0)
+      st->finish(QMM_ERR_TIMEOUT, "a kernel of this launch (or an earlier one) gave up waiting");
     else st->finish(QMM_OK, "");
     return QMM_OK;
   }
@@ -901,6 +905,7 @@ int qmm_rt_buffer_copy_to_device(qmm_rt_buffer* b, qmm_rt_device* device, qmm_rt
       return rc;
     }
     auto done = std::make_shared<EventState>();
+    done->of_launch = true;
     EventRef d2 = done;
     if (after_stream(b->client, device->exec, [d2] { d2->finish(QMM_OK, ""); }) != QMM_OK) done = make_ready_event();
     mark_produced(copy, ev, done);

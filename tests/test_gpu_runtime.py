@@ -12,6 +12,7 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
 from jax_metallib_b200 import _lib, runtime, synthetic
 from oracle import qmm_oracle as O
@@ -62,6 +63,31 @@ def test_every_client_is_distinct_and_owns_its_handles_and_user_data(cuda):
     assert lib.qmm_rt_memory_get_user_data(b.memory_handle(0), 7) == 0x2002  # the other client is untouched
     b.destroy()
     assert destroyed == [0x1001, 0x1003, 0x2002]
+
+
+def test_buffers_that_are_done_read_back_after_another_kernel_gave_up(client, cuda):
+    lib = _lib.load()
+    x = np.arange(64 * 128, dtype=np.float32).reshape(64, 128)
+    up, done = client.buffer_from_host(x, want_event=True)
+    done.await_(5000)
+    exe = client.compile("""module @jit_f attributes {mhlo.num_partitions = 1 : i32, mhlo.num_replicas = 1 : i32} {
+  func.func public @main(%arg0: tensor<64x128xf32>) -> (tensor<64x128xf32>) {
+    %0 = stablehlo.add %arg0, %arg0 : tensor<64x128xf32>
+    return %0 : tensor<64x128xf32>
+  }
+}
+""")
+    outs, ready = exe.execute([up])
+    ready.await_(5000)
+    word = torch.zeros(1, dtype=torch.int32, device=cuda)
+    try:  # a word that nothing sets: the wait runs out after 50 ms and leaves the status word set
+        _lib.check(lib.qmm_wait_signals(word.data_ptr(), 1, 1, 50_000_000, torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert lib.qmm_device_status() != 0
+        np.testing.assert_array_equal(up.to_numpy(), x)
+        np.testing.assert_array_equal(outs[0].to_numpy(), 2 * x)
+    finally:
+        lib.qmm_clear_device_status()
 
 
 def test_strided_and_zero_element_uploads_and_raw_reads(client):
