@@ -140,6 +140,8 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     __syncwarp();
   } else if (warp < kConsumerWarps) {
     // ------------------------------ consumers -----------------------------
+    // The bounded waits for the ring begin when the activations can arrive: an earlier kernel may run for longer than they last.
+    dev::pdl_wait();
     const int cgrp = warp & 3, kh = warp >> 2;
     const int g8 = lane >> 2, t4 = lane & 3;
     // weights: lane l addresses packed row 32 kh + l, 16-byte chunks 2 cgrp and 2 cgrp + 1 (XOR-swizzled by the row)

@@ -68,6 +68,31 @@ def test_int4_weights(cuda, m, k, n, packed):
     assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + _sum_error(k, 4) * size * 1.01).all())
 
 
+def test_int4_weights_behind_a_long_kernel(cuda):
+    """A kernel that lets its successor start early and then runs for longer than the bounded waits (2 s) is no timeout."""
+    lib, g = _lib.load(), _gen(3)
+    a = torch.randint(-128, 128, (13000, 8193), dtype=torch.int8, device="cuda", generator=g)
+    b = torch.randint(-128, 128, (8193, 16385), dtype=torch.int8, device="cuda", generator=g)
+    x = torch.randn(8, 4096, device="cuda", generator=g).bfloat16()
+    wq = torch.randint(0, 256, (2048, 4096), dtype=torch.uint8, device="cuda", generator=g)
+    s = (torch.rand(32, 4096, device="cuda", generator=g) * 0.008 + 0.002).bfloat16()
+    zp = torch.randint(0, 256, (32, 2048), dtype=torch.uint8, device="cuda", generator=g)
+    y = ops.w4a16_g128(x, wq, s, zp, zeros_packed=True)
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    try:
+        _lib.check(lib.qmm_set_cta_limit(1))   # one persistent CTA: the other SMs are free for the successor
+        begin.record()
+        ops.i8_dot(a, b)
+    finally:
+        _lib.check(lib.qmm_set_cta_limit(0))
+    late = ops.w4a16_g128(x, wq, s, zp, zeros_packed=True)
+    end.record()
+    torch.cuda.synchronize()
+    assert lib.qmm_device_status() == 0
+    assert begin.elapsed_time(end) > 2200.0
+    assert torch.equal(y, late)
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 4, 16), (8, 100, 48), (9, 64, 128), (17, 1024, 1024), (33, 4, 16), (100, 2052, 400),
                                    (256, 512, 144)])
 def test_int8_weights_f32_rows(cuda, m, k, n):
