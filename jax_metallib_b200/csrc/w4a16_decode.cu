@@ -598,11 +598,11 @@ static int run(const char* name, const uint16_t* x, const uint8_t* wq, const uin
                const uint8_t* zeros, int zeros_packed, uint16_t* y, int64_t M, int64_t N, int64_t K,
                void* workspace, unsigned flags, int* status, cudaStream_t st) {
   // Few rows and columns: the kernel that splits K over a cluster and adds up in distributed shared memory.  This one
-  // streams wider rows and is ahead once N fills the device by itself: (this one, that one) at M = 8, 4096 x 6144 11.6,
-  // 9.7 us, 4096 x 28672 23.6, 28.0 us; at M = 16 17.0, 13.2 and 34.8, 41.1 us; at M = 32, 4096 x 6144 28.4, 31.5 us.
+  // streams wider rows and is ahead once N fills the device by itself: (this one, that one) at M = 8, 4096 x 6144 11.7,
+  // 9.1 us, 4096 x 28672 23.7, 25.7 us; at M = 32, 4096 x 6144 28.4, 31.5 us (that one with tiles of 32 rows).
   // It is ahead, too, where the weights are many and the start and the end of a call therefore little: at M = 3
-  // 14336 x 4096 16.4, 15.3 us, 8192 x 8192 16.2, 16.6 us, 16896 x 5888 20.5, 24.0 us; at M = 8 18.0, 16.7 us for
-  // 8192 x 8192, 20.2, 18.7 us for 14336 x 5120, 19.1, 20.8 us for 8192 x 9728, 22.8, 24.3 us for 16896 x 5888.
+  // 14336 x 4096 16.6, 14.1 us, 8192 x 8192 16.1, 15.2 us, 16896 x 5888 20.4, 22.1 us; at M = 8 18.0, 15.5 us for
+  // 8192 x 8192, 20.1, 17.3 us for 14336 x 5120, 19.1, 19.0 us for 8192 x 9728, 22.8, 22.2 us for 16896 x 5888.
   if (M <= 16 && N <= 16384 && N * K <= (M <= 4 ? 60000000 : 75000000))
     return w4a16_split(x, wq, scales, zeros, zeros_packed, y, M, N, K, (flags & QMM_W4_STATIC_WEIGHTS) ? 1 : 0, status, st);
   const int G = static_cast<int>(K / kGroup);

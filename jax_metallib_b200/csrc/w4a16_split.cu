@@ -7,15 +7,16 @@
 // the tiles, and warps of their own add the cluster's partial tiles over distributed shared memory in a fixed order.
 //
 // A consumer warp owns 32 columns and half of a group's k.  ldmatrix.trans hands it registers whose bytes are two packed
-// rows of two neighbouring columns; a shift and one logic operation per two weights leave the nibble in the top mantissa
-// bits of a bf16 (16 + q) * 2^-24, exactly (no activation overflows in the product; the scale makes up for it).  Low nibbles (even k) fill slots 0-7 of mma.sync.m16n8k16, high nibbles slots 8-15,
-// and the activations are paired to match.  A group is worth  s * (acc - (16 + z) * sum x):  the sums of the
-// activations come from the tensor core as well, as the product with a column of 2^-24.
+// rows of two neighbouring columns; a mask and one multiply-add per two weights make bf16 (q - z) * 2^-24 of them, exactly (no
+// activation overflows in the product; the scale makes up for it).  Low nibbles (even k) fill slots 0-7 of
+// mma.sync.m16n8k16, high nibbles slots 8-15, and the activations are paired to match.  Earlier, the codes went in as
+// 16 + q and (16 + z) * sum x was taken off afterwards: what cancels there cost precision where activations do not
+// average to zero (14336 x 4096, mean 1: 0.05 % of the results off by a rounding, 0.01 % now), and M = 16 took 21.2 us
+// for 14336 x 4096, 18.2 us now.
 //
-// Bound by the latency of a stage's chain (some 150 instructions a warp) and, for small matrices, by prologue and
+// Bound by the latency of a stage's chain and, for small matrices, by prologue and
 // hand-over, which this kernel has less of than the one that meets in global memory.  Measured (that kernel, this one) at
-// M = 8: 4096 x 6144 11.6, 9.7 us; 4096 x 4096 11.2, 7.9 us; 14336 x 4096 19.9, 15.5 us; 4096 x 28672 23.6, 28.0 us.
-// Tiles of 256 columns (24.4 us there, but 20.1 us for 14336 x 4096) were taken back.
+// M = 8: 4096 x 6144 11.7, 9.1 us; 4096 x 4096 11.2, 7.5 us; 14336 x 4096 19.6, 14.5 us; 4096 x 28672 23.7, 25.7 us.
 #include <cooperative_groups.h>
 
 #include "split_k.cuh"
@@ -59,10 +60,19 @@ __device__ __forceinline__ void bulk_copy_g2s(void* smem_dst, const void* gsrc, 
                "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(dev::smem_u32(bar))
                : "memory");
 }
-// The nibbles that `shifted` has at bits 3-6 of its halves -> bf16 (16 + q) * 2^-24 each.
-__device__ __forceinline__ uint32_t nibbles_to_bf16x2(uint32_t shifted) {
+// -z * 2^-24 as bf16, twice: z in the low byte of a bf16 reads as z * 2^-133 (a subnormal up to 127, the first binade above).
+__device__ __forceinline__ uint32_t minus_zero_point(uint32_t z) {
   uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(shifted), "r"(0x00780078u), "r"(0x35803580u));  // (t & m) | k
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(z * 0x00010001u), "r"(0xF600F600u));   // * -2^109
+  return r;
+}
+// The nibbles at bits SHIFT .. of w's halves -> (q - z) * 2^-24, exactly: q reads as q * 2^(SHIFT - 133) where it stands.
+template <int SHIFT>
+__device__ __forceinline__ uint32_t weights2(uint32_t w, uint32_t minus_z) {
+  uint32_t r;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;"
+      : "=r"(r)
+      : "r"(w & (0x000F000Fu << SHIFT)), "r"(SHIFT ? 0x74007400u : 0x76007600u), "r"(minus_z));
   return r;
 }
 
@@ -186,38 +196,19 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             xr[q][mt][0] = __byte_perm(lo, hi, 0x5410);   // (x0, x2): the low nibbles of two packed rows
             xr[q][mt][1] = __byte_perm(lo, hi, 0x7632);   // (x1, x3): the high nibbles
           }
-        // per-group constants of this thread's four columns: scale and 16 + zero point
-        float sc[2][2], zf[2][2];
+        // per-group constants of this thread's four columns: the scale, and -z * 2^-24 in bf16 twice
+        float sc[2][2];
+        uint32_t nz[2][2];
         const uint8_t* stp = smem + s * L::kStage;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const uint32_t s2 = *reinterpret_cast<const uint32_t*>(stp + L::kOffS + (lc + 16 * j) * 2);
           sc[j][0] = __uint_as_float(s2 << 16) * 16777216.f;
           sc[j][1] = __uint_as_float(s2 & 0xFFFF0000u) * 16777216.f;
-          dep ^= s2;
-          uint32_t z0, z1;
-          if (ZP) {
-            const uint32_t zb = stp[L::kOffZ + (lc + 16 * j) / 2];
-            dep ^= zb;
-            z0 = zb & 0xFu;
-            z1 = zb >> 4;
-          } else {
-            const uint32_t zb = *reinterpret_cast<const uint16_t*>(stp + L::kOffZ + lc + 16 * j);
-            dep ^= zb;
-            z0 = zb & 0xFFu;
-            z1 = zb >> 8;
-          }
-          zf[j][0] = __uint_as_float(0x4B000000u | (z0 + 16u)) - 8388608.f;
-          zf[j][1] = __uint_as_float(0x4B000000u | (z1 + 16u)) - 8388608.f;
-        }
-        float xs[MT][4];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) xs[mt][i] = 0.f;
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            mma_bf16_16816(xs[mt], 0x33803380u, 0x33803380u, 0x33803380u, 0x33803380u, xr[q][mt][0], xr[q][mt][1]);
+          const uint32_t zb = ZP ? stp[L::kOffZ + (lc + 16 * j) / 2] : *reinterpret_cast<const uint16_t*>(stp + L::kOffZ + lc + 16 * j);
+          nz[j][0] = minus_zero_point(ZP ? zb & 0xFu : zb & 0xFFu);
+          nz[j][1] = minus_zero_point(ZP ? zb >> 4 : zb >> 8);
+          dep ^= s2 ^ zb;
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -228,17 +219,17 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             for (int i = 0; i < 4; ++i) d[mt][i] = 0.f;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const uint32_t w = wr[j][q];
-            const uint32_t a0 = nibbles_to_bf16x2(w << 3), a2 = nibbles_to_bf16x2(w >> 1);    // column 2 g8: even k, odd k
-            const uint32_t a1 = nibbles_to_bf16x2(w >> 5), a3 = nibbles_to_bf16x2(w >> 9);    // column 2 g8 + 1
+            const uint32_t w = wr[j][q], w8 = w >> 8;
+            // columns 2 g8 and 2 g8 + 1: even k, odd k
+            const uint32_t a0 = weights2<0>(w, nz[j][0]), a2 = weights2<4>(w, nz[j][0]);
+            const uint32_t a1 = weights2<0>(w8, nz[j][1]), a3 = weights2<4>(w8, nz[j][1]);
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(d[mt], a0, a1, a2, a3, xr[q][mt][0], xr[q][mt][1]);
           }
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              acc[j][mt][i] = fmaf(sc[j][i >> 1], fmaf(-zf[j][i >> 1], xs[mt][i & 1], d[mt][i]), acc[j][mt][i]);
+            for (int i = 0; i < 4; ++i) acc[j][mt][i] = fmaf(sc[j][i >> 1], d[mt][i], acc[j][mt][i]);
         }
         release_slot(&empty[s], dep, never, lane);
         if (++s == S) { s = 0; ph ^= 1; }
