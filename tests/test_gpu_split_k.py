@@ -36,14 +36,15 @@ def _check(y, x, w, scale, rounding, steps):
 
 @pytest.mark.parametrize("m,k,n", [(1, 8, 16), (1, 4096, 4096), (8, 72, 144), (9, 1032, 1040), (16, 4096, 28672), (17, 64, 128),
                                    (32, 4096, 28672), (33, 520, 272), (64, 14336, 256), (97, 1000, 5632),
-                                   (97, 1000, 4736), (97, 2048, 5744), (1024, 248, 256)])
+                                   (97, 1000, 4736), (97, 2048, 5744), (1024, 248, 256), (1, 28672, 8192), (8, 33000, 16384)])
 def test_int8_weights_bf16_rows(cuda, m, k, n):
     g = _gen(m + k + n)
     x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
     w = torch.randint(-128, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
     s = torch.rand(n, device="cuda", generator=g) * 0.01 + 0.005
-    # one accumulator runs over a CTA's slice of K
-    _check(ops.w8a16_perchannel(x, w, s), x, w, s.double(), 2.0 ** -8, k // 16 + 1)
+    # one accumulator runs over a CTA's slice of K, over 16 stages of 64 k (two warps share them) where a slice is longer than 64
+    long = m <= 8 and k > 16384
+    _check(ops.w8a16_perchannel(x, w, s), x, w, s.double(), 2.0 ** -8, 32 if long else k // 16 + 1)
     wide = torch.zeros(m, n + 32, dtype=torch.bfloat16, device="cuda")
     ops.w8a16_perchannel(x, w, s, out=wide, out_col_offset=16)
     assert torch.equal(wide[:, 16:16 + n], ops.w8a16_perchannel(x, w, s))
