@@ -309,7 +309,8 @@ QMM_API int qmm_w4a16_g128_static_scratch(const uint16_t* x_bf16, const uint8_t*
  * group_size is 64 / 128 / 256 (4-bit) or 32 / 64 / 128 (8-bit) with a multiple
  * of 4 groups per row; MX: K is a multiple of 512 (mxfp4, mxfp8) or 256
  * (nvfp4).  Everything else with M >= 4, 16-byte aligned x and w_packed, K (and,
- * affine, group_size) a multiple of 32 runs a tcgen05 GEMM; what is left runs on
+ * affine, group_size) a multiple of 32 runs a tcgen05 GEMM where that is no
+ * slower (small N and M over a short K are left out); what remains runs on
  * CUDA-core kernels (scale * q + bias or scale * element in f32, f32
  * accumulation, one cast).  The tensor-core kernels apply the scale per group
  * instead of per weight: same result up to f32 rounding of the sums. */

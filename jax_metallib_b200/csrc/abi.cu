@@ -113,6 +113,11 @@ int env_int_once(const char* name, int dflt, std::atomic<int>& cache) {
   return v;
 }
 
+bool force_split_k() {
+  static std::atomic<int> cache{INT32_MIN};
+  return env_int_once("QMM_FORCE_SPLIT_K", 0, cache) != 0;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,

@@ -92,6 +92,9 @@ inline bool mark_device_once(std::atomic<uint64_t>& done, int ordinal) {
 int ensure_dynamic_smem(const void* func, int bytes, std::atomic<uint64_t>& done);
 // Environment switches are read once, when first asked for.
 int env_int_once(const char* name, int dflt, std::atomic<int>& cache);
+// QMM_FORCE_SPLIT_K=1: the kernels that split K and the operator GEMM take every shape that they can, whatever is faster (a
+// cross-check of small shapes on a GPU box; read once per process).
+bool force_split_k();
 int gemm_ctas();             // CTAs a persistent GEMM may launch: num_sms() unless qmm_set_cta_limit lowered it
 
 // 2-D tiled tensor map (TMA descriptor).  rows x cols elements of elem_bytes,

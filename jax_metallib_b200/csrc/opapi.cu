@@ -11,8 +11,8 @@
 // weight = scale * q + bias (affine) or scale * element (MX) in f32, product
 // and accumulation in f32, one final cast; NaN codes propagate.
 //
-// These CUDA-core kernels take any M and f32 or f16 activations, and run where nothing else does: up to three rows, K or
-// groups that are no multiple of 32, unaligned operands.  Decode-sized f16 problems (M <= 16) go to the TMA-ring
+// These CUDA-core kernels take any M and f32 or f16 activations, and run where nothing else does (K or groups that are no
+// multiple of 32, unaligned operands) or nothing else is faster (up to three rows, few columns and rows over a short K).  Decode-sized f16 problems (M <= 16) go to the TMA-ring
 // tensor-core kernels of opapi_tc.cu where the shape allows, then to affine_tc_kernel below; the rest goes to the
 // tcgen05 GEMM of opapi_gemm.cu.
 #include "opapi_decode.cuh"
@@ -29,7 +29,7 @@ int mx_ring_launch(int mode, const void* x, const void* w, const void* scales, v
                    void* stream);
 
 // the tcgen05 GEMM: any M, f16 or f32 activations
-bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, const void* x, const void* w, const void* y);
+bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, int f32, const void* x, const void* w, const void* y);
 int opgemm_launch(int fmt, const void* x, const void* w, const void* scales, const float* biases, void* y, int64_t M, int64_t N,
                   int64_t K, int64_t gs, int f32, void* stream);
 
@@ -549,7 +549,7 @@ int qmm_affine_matmul(const void* x, const void* w_packed, const float* scales, 
     return affine_ring_launch(bits, x, w_packed, scales, biases, y, M, N, K, group_size, stream);
   if (tcq::covers(M, N, K, bits, group_size, dtype, x, w_packed))
     return tcq::launch(bits, x, w_packed, scales, biases, y, M, N, K, group_size, stream);
-  if (opgemm_covers(M, N, K, bits == 4 ? 0 : 1, group_size, x, w_packed, y))
+  if (opgemm_covers(M, N, K, bits == 4 ? 0 : 1, group_size, dtype == QMM_F32, x, w_packed, y))
     return opgemm_launch(bits == 4 ? 0 : 1, x, w_packed, scales, biases, y, M, N, K, group_size, dtype == QMM_F32, stream);
   // rows of 16-byte words: the vectorised kernel
   if (aligned(w_packed, 16) && K % (bits == 4 ? 32 : 16) == 0) {
@@ -593,7 +593,7 @@ int qmm_mx_matmul(const void* x, const uint8_t* w_packed, const uint8_t* scales,
   static_assert(QMM_MXFP4 == 0 && QMM_MXFP8 == 1 && QMM_NVFP4 == 2, "mode numbering shared with the tensor-core kernel");
   if (mx_ring_covers(M, N, K, mode, dtype, x, w_packed, scales))   // decode-sized f16 problems: the tensor-core kernel
     return mx_ring_launch(mode, x, w_packed, scales, y, M, N, K, stream);
-  if (opgemm_covers(M, N, K, 2 + mode, gs, x, w_packed, y))
+  if (opgemm_covers(M, N, K, 2 + mode, gs, dtype == QMM_F32, x, w_packed, y))
     return opgemm_launch(2 + mode, x, w_packed, scales, nullptr, y, M, N, K, gs, dtype == QMM_F32, stream);
   if (aligned(w_packed, 16) && K % 32 == 0) {  // rows of 16-byte words: the vectorised kernel
     if (mode == QMM_MXFP4) {

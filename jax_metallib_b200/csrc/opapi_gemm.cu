@@ -833,17 +833,44 @@ static int resident_clusters(int ks) {
 // CTAs that share an output tile: the fewest rounds of resident clusters (six CTAs to a cluster, for one, leave SMs of
 // every GPC idle), a round costing its stages and, for the prologue and the hand-over, about as much as kRoundCost more.
 constexpr int kRoundCost = 16;
-template <int FMT, bool XF32, int BM>
-static int cluster_size(int tiles, int blocks, int stages) {
-  int best = 1;
+struct Rounds {
+  int ks, rounds, stages;   // CTAs to a cluster; rounds of clusters; stages of the longest slice
+};
+template <typename Fn>
+static Rounds choose_rounds(int tiles, int blocks, int stages, Fn resident) {
+  Rounds best = {1, 1, stages};
   long long best_cost = -1;
   for (int ks = 1; ks <= kMaxCluster && ks <= blocks; ++ks) {
-    const int c = resident_clusters<FMT, XF32, BM>(ks);
-    const int slice = (blocks + ks - 1) / ks;   // the longest slice, in blocks
-    const long long cost = static_cast<long long>((tiles + c - 1) / c) * (slice * ((stages + blocks - 1) / blocks) + kRoundCost);
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = ks; }
+    const int c = resident(ks);
+    const int slice = (blocks + ks - 1) / ks * ((stages + blocks - 1) / blocks);
+    const int rounds = (tiles + c - 1) / c;
+    const long long cost = static_cast<long long>(rounds) * (slice + kRoundCost);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = {ks, rounds, slice < stages ? slice : stages};
+    }
   }
   return best;
+}
+
+// How K is cut.  A unit is a scale group or a part of one, and no more than a stage: its MMAs come from one thread, and the
+// tensor core's own, truncated additions have to be cut short against f32 results (128 k: 2.5e-7 of the result, 64 k: 1e-7).
+// Slices of K begin on a box of raw weights and on a box of scales.
+struct Slicing {
+  int pu, sbox_k, block_k, blocks;
+};
+static Slicing slicing(int fmt, int K, int gs, bool scales_aligned) {
+  Slicing c;
+  const bool bias = fmt <= kAffine8;
+  c.pu = fmt == kNvfp4 || gs % 64 == 0 ? 64 : 32;
+  const bool boxed = fmt == kNvfp4 || !scales_aligned ? false
+                     : bias                           ? gs <= 128 && (K / gs) % 4 == 0 && 128 % gs == 0
+                                                      : K % 512 == 0 && K >= 2048;   // (slices of a short K stay fine)
+  c.sbox_k = !boxed ? 0 : (bias ? 4 * gs : 512);
+  const int box_k = fmt == kAffine8 || fmt == kMxfp8 ? 128 : 256;
+  c.block_k = c.sbox_k > box_k ? c.sbox_k : box_k;
+  c.blocks = (K + c.block_k - 1) / c.block_k;
+  return c;
 }
 
 template <int FMT, bool XF32, int BM>
@@ -861,17 +888,14 @@ static int launch(Args a, cudaStream_t stream) {
   static std::atomic<uint64_t> configured{0};
   auto kern = opgemm_kernel<FMT, XF32, BM>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), C::kSmem, configured)) return rc;
-  // A unit is a scale group or a part of one, and no more than a stage: its MMAs come from one thread, and the tensor
-  // core's own, truncated additions have to be cut short against f32 results (128 k: 2.5e-7 of the result, 64 k: 1e-7).
-  // Slices of K begin on a box of raw weights and on a box of scales.
-  a.pu = FMT == kNvfp4 || a.gs % 64 == 0 ? 64 : 32;
-  const bool boxed = FMT == kNvfp4 ? false
-                     : C::kBias    ? a.gs <= 128 && (a.K / a.gs) % 4 == 0 && 128 % a.gs == 0 && aligned(a.scales, 16) && aligned(a.biases, 16)
-                                   : a.K % 512 == 0 && a.K >= 2048 && aligned(a.scales, 16);   // (slices of a short K stay fine)
-  a.sbox_k = !boxed ? 0 : (C::kBias ? 4 * a.gs : 512);
-  a.block_k = a.sbox_k > C::kBoxK ? a.sbox_k : C::kBoxK;
+  const Slicing cut = slicing(FMT, a.K, a.gs, aligned(a.scales, 16) && (!C::kBias || aligned(a.biases, 16)));
+  a.pu = cut.pu;
+  a.sbox_k = cut.sbox_k;
+  a.block_k = cut.block_k;
+  a.blocks = cut.blocks;
+  static_assert(C::kBoxK == (FMT == kAffine8 || FMT == kMxfp8 ? 128 : 256), "box of raw weights");
   CUtensorMap smap = wmap, bmap = wmap;   // placeholders where they are not used
-  if (boxed) {
+  if (cut.sbox_k) {
     const uint64_t G = static_cast<uint64_t>(a.K / a.gs);
     const auto type = C::kBias ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
     const int esz = C::kBias ? 4 : 1;
@@ -881,11 +905,10 @@ static int launch(Args a, cudaStream_t stream) {
       if (int rc = make_tensor_map_2d(&bmap, a.biases, type, esz, (uint64_t)a.N, G, G * esz, BN, 16 / esz, CU_TENSOR_MAP_SWIZZLE_NONE))
         return rc;
   }
-  a.blocks = (a.K + a.block_k - 1) / a.block_k;
   a.idesc = dev::make_idesc(/*c=f32*/ 1, XF32 ? 1 : 0, XF32 ? 1 : 0, /*both K-major*/ 0, 0, BN, BM);
   a.status = device_status_word();
   const int nt = (a.N + BN - 1) / BN, mt = (a.M + BM - 1) / BM;
-  const int ks = cluster_size<FMT, XF32, BM>(nt * mt, a.blocks, (a.K + BK - 1) / BK);
+  const int ks = choose_rounds(nt * mt, a.blocks, (a.K + BK - 1) / BK, resident_clusters<FMT, XF32, BM>).ks;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ks, mt, nt);
   cfg.blockDim = dim3(C::kThreads);
@@ -907,18 +930,52 @@ static int launch_fmt(const Args& a, int f32, cudaStream_t stream) {
                    : (a.M <= 64 ? launch<FMT, false, 64>(a, stream) : launch<FMT, false, 128>(a, stream));
 }
 
+// Microseconds of a call, here and on the CUDA cores (one B200, calls of a graph on operands in L2; K and N from 64 to 4096,
+// M from 4 to 500, every format: here within 6 % in the mean, there within 9 %).
+//   here: rounds of clusters, each a start and a hand-over, and its stages
+//   there: a block of 16 columns and 8 rows runs over K by itself; three blocks fit an SM, and more of them queue
+static float gemm_us(int fmt, bool f32, int M, int N, int K, int gs) {
+  const int bm = M <= 32 ? 32 : (M <= 64 || f32 ? 64 : 128);
+  const int i = bm == 32 ? 0 : (bm == 64 ? 1 : 2);
+  static constexpr float kStart[3] = {4.2f, 5.5f, 7.5f};
+  // us per stage of 64 k: f16 activations at 32, 64 and 128 rows, f32 at 32 and 64
+  static constexpr float kStage[4][5] = {{1.33f, 1.71f, 3.5f, 1.48f, 1.84f},   // affine, units of 32 k
+                                         {0.91f, 1.12f, 2.0f, 1.12f, 1.32f},   // affine, 64 k
+                                         {0.72f, 0.77f, 1.02f, 1.11f, 1.26f},  // mxfp4, mxfp8
+                                         {0.59f, 0.57f, 0.55f, 0.92f, 1.01f}}; // nvfp4
+  const Slicing cut = slicing(fmt, K, gs, true);
+  const int kind = fmt == kNvfp4 ? 3 : (fmt > kAffine8 ? 2 : (cut.pu == 64 ? 1 : 0));
+  const int sms = num_sms();
+  const Rounds r = choose_rounds(((N + BN - 1) / BN) * ((M + bm - 1) / bm), cut.blocks, (K + BK - 1) / BK,
+                                 [&](int ks) { return sms / ks > 0 ? sms / ks : 1; });
+  return r.rounds * (kStart[i] + kStage[kind][f32 ? 3 + i : i] * r.stages);
+}
+static float cuda_core_us(int fmt, bool f32, int M, int N, int K) {
+  const bool wide = fmt == kAffine8 || fmt == kMxfp8;   // 8-bit codes take fewer instructions
+  const float least = f32 ? (wide ? 6.5f : 10.4f) : (wide ? 5.6f : 8.6f);
+  const float run = 3.f + K * (f32 ? (wide ? 0.0079f : 0.0089f) : (wide ? 0.0057f : 0.0056f));
+  float us = least > run ? least : run;
+  if (M <= 4) us *= 0.74f;
+  const float blocks = static_cast<float>((N + 15) / 16) * ((M + 7) / 8);
+  return blocks <= 3 * num_sms() ? us : us * (0.75f + blocks / (3.5f * num_sms()));
+}
+
 }  // namespace opg
 
-// Which calls come here.  Up to three rows the CUDA-core kernels, which read x from cache and split every column over a
-// warp, have less to set up (affine4, f32, 4096 x 8192: 30 us at one row, 62 at four, here 32 for any of them;
-// 4096 x 12288: 32, 63, here 58).
+// Which calls come here: those that take no longer than on the CUDA cores, by the estimates above.  Few blocks of columns
+// and rows over a short K stay there (affine8, f32, 512 x 1024 at M = 4: 5.1 us there, 8.3 here; at M = 64 12.9, 10.6), and
+// so do up to three rows, which the estimates do not cover (affine4, f32, 4096 x 8192: 30 us at one row, 62 at four, here
+// 32 for any of them).
+// QMM_FORCE_SPLIT_K=1 brings every call here that the kernel can take (a cross-check; read once per process).
 // fmt: 0 affine 4-bit, 1 affine 8-bit, 2 mxfp4, 3 mxfp8, 4 nvfp4.  K and the group a multiple of 32 (nvfp4: K), weights
 // and activations 16-byte aligned, results aligned for pairs.
-bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, const void* x, const void* w, const void* y) {
+bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, int f32, const void* x, const void* w, const void* y) {
   using namespace opg;
   if (M < 4 || K % 32 != 0 || (fmt <= kAffine8 && gs % 32 != 0)) return false;
   if (!aligned(x, 16) || !aligned(w, 16) || !aligned(y, 8)) return false;
-  return (M + 7) / 8 <= 65535 && (N + BN - 1) / BN <= 65535;
+  if ((M + 7) / 8 > 65535 || (N + BN - 1) / BN > 65535) return false;
+  const int m = static_cast<int>(M), n = static_cast<int>(N), k = static_cast<int>(K);
+  return force_split_k() || gemm_us(fmt, f32 != 0, m, n, k, static_cast<int>(gs)) <= cuda_core_us(fmt, f32 != 0, m, n, k);
 }
 
 int opgemm_launch(int fmt, const void* x, const void* w, const void* scales, const float* biases, void* y, int64_t M, int64_t N,

@@ -335,3 +335,11 @@ assert torch.equal(y, {call})
 """
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     subprocess.run([sys.executable, "-c", program], check=True, cwd=root, timeout=120)
+
+
+def test_forced_routes(cuda):
+    """The tests of this file once more with every shape on the kernels that split K or on the operator GEMM, small ones too."""
+    if os.environ.get("QMM_FORCE_SPLIT_K"):
+        pytest.skip("this is that run")
+    subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-k", "not first_call and not long_kernel", __file__],
+                   check=True, env=dict(os.environ, QMM_FORCE_SPLIT_K="1"), timeout=600)
