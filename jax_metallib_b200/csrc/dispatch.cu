@@ -143,14 +143,33 @@ static int force_simple() {
   return env_int_once("QMM_FORCE_SIMPLE", 0, cache);
 }
 
-// Which int8 dots take the kernel for few rows or rows that TMA cannot describe, instead of the GEMM.
+// Which int8 dots take the kernel that splits K, for few rows or rows that TMA cannot describe.  Measured in us (it, the
+// kernel that would run otherwise), operands in L2:
 static bool i8_skinny_covers(int64_t M, int64_t N, int64_t K, bool tma_ok) {
   if (M > 65535 || (N + 127) / 128 * ((M + 7) / 8) > (1ll << 30)) return false;
-  // The GEMM's tiles of 256 columns leave most SMs idle when there are few of them; this kernel splits K but reads b once
-  // per 64 rows.  Measured (this kernel, the GEMM): 64 x 4096 x 4096 14.0, 21.3 us; 128 x 4096 x 4096 20.0, 22.2 us;
-  // 256 x 4096 x 4096 30.8, 22.2 us; 64 x 8192 x 8192 30.5, 37.3 us; 128 x 8192 x 8192 50.4, 38.4 us;
-  // 256 x 1024 x 1024 9.8, 10.4 us.
-  return !tma_ok || (gemm_ctas() == num_sms() && (M <= 32 || (M + 63) / 64 * N <= 8192));
+  if (force_split_k()) return true;
+  const bool large = M * N >= 128 * 128;
+  if (!tma_ok) {
+    // else one thread per result: its time goes with K and, once the device is full, with M * N; this kernel has a start and
+    // a hand-over of 4 to 12 us.  M = 8, N = 255, K = 64: 5.8, 4.2; 128: 5.4, 5.9.  M = 64, N = 1023, K = 128: 11.5, 6.8;
+    // 256: 9.6, 11.3; N = 4095, K = 128: 11.7, 15.9.  M = 512, N = 4095, K = 32 25.2, 22.6; 64 25.6, 44.1.
+    const int64_t results = M * N;
+    if (K >= 256) return true;
+    if (K >= 128) return M <= 8 || results >= (M <= 32 ? 100000 : 200000);
+    return K >= 64 && results >= (M <= 32 ? 400000 : 900000);
+  }
+  if (!large) return K >= 256 || (K >= 128 && M <= 16);   // else one thread per result: M = 32, N = 256, K = 128 7.1, 6.1
+  if (gemm_ctas() != num_sms()) return false;             // a limit keeps the GEMM
+  // The GEMM's tiles of 256 columns leave most SMs idle when there are few of them; this kernel splits K, but reads b once
+  // per 64 rows and hands over 64 x 128 results at a time.  M = 32, N = 1024, K = 64: 8.5, 7.5; 128: 7.3, 7.5; N = 16384,
+  // K = 512 9.5, 9.0.
+  if (M <= 32) return M <= 16 || (K >= 128 && (N <= 8192 || K >= 1024));
+  // 64 x N and its likes: N = 1024, K = 256 9.0, 8.1; 512 8.2, 8.8; N = 2048, K = 512 9.5, 8.7; 1024 9.8, 10.2;
+  // N = 4096, K = 1024 10.7, 10.3; 2048 11.9, 13.0; N = 8192, K = 4096 20.5, 18.8 (8192 x 8192 from memory: 30.5, 37.3).
+  // The GEMM is quicker at a single tile of columns: M = 1024, N = 128, K = 1024 9.8, 8.9; 2048 10.7, 11.5.
+  const int64_t cols = (M + 63) / 64 * ((N + 127) / 128 * 128);
+  const int64_t least = cols <= 1024 ? 512 : (cols <= 2048 ? 1024 : (cols <= 4096 ? 2048 : 8192));
+  return cols <= 8192 && K >= (N <= 128 && least < 2048 ? 2048 : least);
 }
 
 }  // namespace qmm
