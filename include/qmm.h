@@ -118,8 +118,10 @@ QMM_API int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float* s
  * tcgen05 (kind::f16) GEMM with the int8->bf16 conversion done in shared
  * memory.  The tensor-core route needs K % 8 == 0, N % 16 == 0, an even ldy
  * and 16-byte aligned x and w (what TMA can address); any other shape runs on
- * a plain CUDA-core kernel.  On that route few rows (M <= 32, or ceil(M / 32) * N
- * <= 23000; 18944 for K < 2048, 8192 for K < 256) run a kernel that splits K over thread-block clusters. */
+ * a plain CUDA-core kernel, and so does M * N < 16384 with K < 128.  On that
+ * route few rows (M <= 32, or ceil(M / 32) * N <= 23000; 128 per SM for
+ * K < 2048, 8192 for K < 256) run a kernel that splits K over thread-block
+ * clusters. */
 QMM_API int qmm_w8a16_perchannel(const uint16_t* x_bf16, const int8_t* w, const float* scale,
                                  uint16_t* y_bf16, int64_t M, int64_t N, int64_t K, int64_t ldy,
                                  void* stream);

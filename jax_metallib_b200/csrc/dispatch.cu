@@ -254,9 +254,13 @@ static int w8a16_entry(const char* name, const uint16_t* x, const int8_t* w, con
   // 18432 columns (96 x 6144) 12.1 against 15.0 us, 20480 (320 x 2048) 16.9 against 14.5; K = 2048, 20480: 21.8 against 23.1.
   // Shorter still, the rows it reads again count: K = 128, 8192 columns (128 x 2048) 6.0 against 7.3 us, 16384 (512 x 1024)
   // 7.7 against 7.3.
+  // Results that are too few for the GEMM (M * N < 128 * 128) are one thread each otherwise, which is quicker for a short K:
+  // M = 32, N = 128, K = 64 6.8 against 3.8 us; K = 128 6.8 against 6.8.
   // (A caller that limits the GEMM's CTAs keeps the GEMM: the kernel for few rows fills the device.)
-  const int64_t few = K < 256 ? 8192 : K < 2048 ? 148 * 128 : 23000;
-  if (tma_ok && (M <= 32 || (M + 31) / 32 * N <= few) && gemm_ctas() == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr && !force_simple())
+  const int64_t few = K < 256 ? 8192 : K < 2048 ? num_sms() * 128 : 23000;
+  const bool pays = (M <= 32 || (M + 31) / 32 * N <= few) && (K >= 128 || M * N >= 128 * 128);
+  if (tma_ok && (pays || force_split_k()) && gemm_ctas() == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr &&
+      !force_simple())
     return w8a16_decode(x, w, scale, y, M, N, K, ldy, flags, s);
   if (tma_ok && M * N >= 128 * 128 && !force_simple())
     return w8a16_tcgen05(x, w, scale, y, M, N, K, ldy, flags, signal, arrive, s);
