@@ -103,8 +103,9 @@ QMM_API int qmm_set_cta_limit(int max_ctas);
  *  src/pjrt_plugin/ops/binary_ops.mm:165-193, :1006-1019).
  * The scale is applied once per output element.  With K % 4 == 0, N % 16 == 0,
  * 16-byte aligned x and w and 8-byte aligned y the activations go to the tensor
- * cores as three bf16 terms that hold all 24 bits (exact products, f32 sums);
- * any other shape runs in f32 FMA arithmetic on CUDA cores. */
+ * cores as three bf16 terms that hold all 24 bits (exact products, f32 sums;
+ * values too small for that are scaled first); any other shape, and a K below
+ * 128 unless M or N makes up for it, runs in f32 FMA arithmetic on CUDA cores. */
 QMM_API int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float* scale, float* y,
                                  int64_t M, int64_t N, int64_t K, void* stream);
 

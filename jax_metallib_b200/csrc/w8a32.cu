@@ -3,7 +3,7 @@
 //   y[M,N] = (x[M,K] @ float(w[K,N])) * scale[N]
 //
 // Rows that TMA can describe go to the tensor-core kernel of w8a16_decode.cu (three bf16 terms per activation); this
-// one takes the others (K no multiple of 4, N no multiple of 16, unaligned operands).
+// one takes the others (K no multiple of 4, N no multiple of 16, unaligned operands) and those of a short K.
 //
 // Exact f32 FMA arithmetic (int8 -> f32 is exact; the scale is applied once
 // per output element instead of once per weight, which differs from the
@@ -126,8 +126,11 @@ extern "C" int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float
               QMM_ERR_INVALID_ARGUMENT, "qmm_w8a32_perchannel: bad shape");
   if (M == 0 || N == 0) return QMM_OK;  // empty result: nothing to launch, pointers may be null
   QMM_REQUIRE(x && w && scale && y, QMM_ERR_INVALID_ARGUMENT, "qmm_w8a32_perchannel: null pointer");
-  // rows that TMA can describe: the tensor-core kernel
-  if (K > 0 && K % 4 == 0 && N % 16 == 0 && aligned(x, 16) && aligned(w, 16) && aligned(y, 8) && (M + TM - 1) / TM <= 65535 &&
+  // Rows that TMA can describe: the tensor-core kernel, whose start and hand-over pay from two stages of 64 k on.  Measured
+  // in us (that one, this one): M = 64, N = 1024: K = 32 6.4, 4.6; 64 6.4, 5.0; 128 5.8, 6.2.  M = 8, N = 1024: K = 16 4.5,
+  // 4.1; 32 4.5, 4.5; 64 4.7, 5.0; N = 16384, K = 16 4.9, 6.0.  M = 64, N = 8192: K = 32 8.1, 7.2; 64 8.0, 9.3.
+  const bool pays = K >= 128 || (M <= 8 && (K >= 32 || N >= 8192)) || (K >= 64 && M * N >= 250000) || force_split_k();
+  if (pays && K > 0 && K % 4 == 0 && N % 16 == 0 && aligned(x, 16) && aligned(w, 16) && aligned(y, 8) && (M + TM - 1) / TM <= 65535 &&
       N * ((M + 7) / 8) < (1ll << 36)) {
     if (int st = read_device_status())
       return set_error(QMM_ERR_TIMEOUT, "a previous kernel gave up waiting (status word 0x%x)", st);
