@@ -233,8 +233,9 @@ QMM_API int qmm_i8i8_i32(const void* a, const void* b, int32_t* acc, const float
  * Zero points are 4-bit values (0..15) in either form.
  * Requires group == 128, K % 128 == 0, N % 128 == 0, M >= 1.
  * M <= 32 runs an HBM-bound decode kernel (weights read once; K split over
- * thread-block clusters for M <= 16, N <= 16384 and N * K <= 60 million, or
- * 75 from M = 5 on, else over all SMs with the partial sums in the workspace); larger M runs a tcgen05 GEMM whose converter warps dequantise the
+ * thread-block clusters for M <= 16, N <= 16384 and N * K from 65536 to 75
+ * million, else over all SMs with the partial sums in the workspace); larger M
+ * runs a tcgen05 GEMM whose converter warps dequantise the
  * nibbles in shared memory: bf16((q - z) * s) per weight, which is what the
  * StableHLO chain computes in bf16, f32 accumulation, one rounding of the
  * result.  That route needs no workspace (qmm_w4a16_g128_workspace_bytes

@@ -603,7 +603,10 @@ static int run(const char* name, const uint16_t* x, const uint8_t* wq, const uin
   // It is ahead, too, where the weights are many and the start and the end of a call therefore little: at M = 3
   // 14336 x 4096 16.6, 14.1 us, 8192 x 8192 16.1, 15.2 us, 16896 x 5888 20.4, 22.1 us; at M = 8 18.0, 15.5 us for
   // 8192 x 8192, 20.1, 17.3 us for 14336 x 5120, 19.1, 19.0 us for 8192 x 9728, 22.8, 22.2 us for 16896 x 5888.
-  if (M <= 16 && N <= 16384 && N * K <= (M <= 4 ? 60000000 : 75000000))
+  // Both lines moved when that one took the zero point into the weight.  At the other end a call of one or two stages is
+  // all hand-over: M = 8, K = 128, N = 256 3.0, 4.1 us; 1024 6.1, 4.1 us.
+  const bool pays = N <= 16384 && N * K <= 75000000 && N * K >= 65536;
+  if (M <= 16 && (pays || force_split_k()))
     return w4a16_split(x, wq, scales, zeros, zeros_packed, y, M, N, K, (flags & QMM_W4_STATIC_WEIGHTS) ? 1 : 0, status, st);
   const int G = static_cast<int>(K / kGroup);
   const int C = col_blocks(N);

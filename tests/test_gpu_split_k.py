@@ -53,7 +53,7 @@ def test_int8_weights_bf16_rows(cuda, m, k, n):
 
 @pytest.mark.parametrize("packed", [True, False])
 @pytest.mark.parametrize("m,k,n", [(1, 128, 128), (8, 4096, 384), (9, 1280, 1536), (16, 14336, 256), (16, 384, 16384),
-                                   (4, 4864, 12416), (5, 4864, 12416)])
+                                   (4, 6016, 12416), (5, 6144, 12416)])
 def test_int4_weights(cuda, m, k, n, packed):
     g = _gen(m + k + n)
     x = (torch.randn(m, k, device="cuda", generator=g) * 3 + 1).bfloat16()
@@ -66,7 +66,7 @@ def test_int4_weights(cuda, m, k, n, packed):
     q = torch.stack((wq & 15, wq >> 4), 1).reshape(k, n).double()
     zr, sr = (v.double().repeat_interleave(128, 0) for v in (z, s))
     # the split kernel's products are x (q - z); the other one, which takes the large weights, takes z off afterwards
-    size = (q - zr).abs() if n * k <= (60_000_000 if m <= 4 else 75_000_000) else 32 + q + zr
+    size = (q - zr).abs() if 65536 <= n * k <= 75_000_000 else 32 + q + zr
     ref, size = x.double() @ ((q - zr) * sr), x.double().abs() @ (size * sr)
     assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + _sum_error(k, 4) * size * 1.01).all())
 
