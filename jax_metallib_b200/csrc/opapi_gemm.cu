@@ -386,9 +386,12 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         const uint32_t b_lo = XF32 ? a_lo + (kABytes >> 4) : x_lo + (st % C::kXRing) * (C::kXTile >> 4);
         for (int h = 0; h < units_per_stage; ++h) {
           const int u = st * units_per_stage + h;
-          if (u >= units) break;                                   // the zero half of a last stage
           const int buf = u % C::kAccBufs;
           if (!dev::mbar_wait(&tempty[buf], ((u / C::kAccBufs) & 1) ^ 1, a.status, 95)) { ok = false; break; }
+          if (u >= units) {   // the zero half of a last stage: no MMAs, but its buffer's barrier is the stage's
+            dev::tc_commit(&tfull[buf]);
+            break;
+          }
           dev::tc_fence_after();
           const uint32_t d = tmem_base + buf * BM;
           // the smallest terms first: the accumulator is still small when they are added
@@ -407,10 +410,11 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 dev::umma_f16_lh(d, a_lo + h * 4 + j * 2, kDescHi, b_lo + t * (C::kXTile >> 4) + h * 4 + j * 2, kDescHi, a.idesc,
                                  (t != C::kTerms - 1 || j != 0) ? 1u : 0u);
           }
-          // A commit costs the thread as much as an MMA: one for the units of a stage, on the barrier of the stage's last
-          // buffer even if its last unit does not exist.  That barrier completes once in every round of the buffers, as
-          // the parity that the promoters wait for takes for granted; the one of a stage's first buffer never completes.
-          if (h == units_per_stage - 1 || u == units - 1) dev::tc_commit(&tfull[buf | (units_per_stage - 1)]);
+          // A commit costs the thread as much as an MMA: one for the units of a stage, on the barrier of its last buffer.
+          // That barrier completes once in every round of the buffers, after the buffer was handed back in the round before
+          // (also where there is no unit for it), as the parity that the promoters wait for takes for granted; the one of
+          // a stage's first buffer never completes.
+          if (h == units_per_stage - 1) dev::tc_commit(&tfull[buf]);
         }
         if (ok) dev::tc_commit(&consumed[st % kConsumed]);
       }
@@ -693,12 +697,9 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) break;
         exact = *reinterpret_cast<const uint32_t*>(flags + slot * kGroupWarps) != 0u;
       }
-      // The units of a stage complete together, on the barrier of its last buffer.  It is waited for before the first of
-      // them is handed back: a last stage of one unit asks for that buffer alone, and its commit would otherwise complete
-      // the next round of a barrier that some promoter has still to see complete this one.
-      if ((u & (units_per_stage - 1)) == 0 &&
-          !dev::mbar_wait_relaxed_warp(&tfull[buf | (units_per_stage - 1)], phase, a.status, 100))
-        break;
+      // the units of a stage complete together, on the barrier of its last buffer
+      const int last = units_per_stage == 2 ? (u | 1) & (C::kAccBufs - 1) : buf;
+      if (!dev::mbar_wait_relaxed_warp(&tfull[last], phase, a.status, 100)) break;
       dev::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
       if (C::kUnitInfo && exact) {
