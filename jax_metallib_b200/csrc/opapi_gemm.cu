@@ -25,7 +25,8 @@
 //
 // What the split cannot represent takes an exact path: a unit whose activations are not finite (inf times
 // code plus inf times bias is not what inf times scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
-// the promoters from global memory with the arithmetic of the CUDA-core kernels.
+// the promoters from global memory with the arithmetic of the CUDA-core kernels; and so are affine results that are not
+// finite, because of their scales or biases.
 #include <cooperative_groups.h>
 
 #include "opapi_decode.cuh"
@@ -783,6 +784,12 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       const float2 p = *reinterpret_cast<const float2*>((KS > 1 ? cluster.map_shared_rank(tile, r) : tile) + m * BN + c);
       v.x += p.x;
       v.y += p.y;
+    }
+    if (C::kBias) {
+      // A scale or bias that is not finite leaves results that are not; which ones are infinities and which NaN, weight by
+      // weight, is not what the scaled sums give (an infinite scale times a code of 0).
+      if (!(fabsf(v.x) < INFINITY)) v.x = exact_unit<FMT, XF32>(a, m0 + m, n, 0, a.K);
+      if (!(fabsf(v.y) < INFINITY) && n + 1 < a.N) v.y = exact_unit<FMT, XF32>(a, m0 + m, n + 1, 0, a.K);
     }
     const size_t i = static_cast<size_t>(m0 + m) * a.N + n;
     if (XF32) {

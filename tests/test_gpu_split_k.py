@@ -295,6 +295,34 @@ def test_operator_matmul_special_values(cuda, fmt, group, m, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("fmt,group", [("affine4", 64), ("affine4", 32), ("affine8", 128)])
+@pytest.mark.parametrize("m", [20, 70, 300])
+def test_operator_matmul_infinite_weights(cuda, fmt, group, m, dtype):
+    """Infinite scales and biases: weight by weight, an infinity times a code of 0 is NaN, and so are infinities of both signs."""
+    g = _gen(m)
+    n, k, bits = 160, 2048, int(fmt[6:])
+    x = torch.randn(m, k, device="cuda", generator=g)
+    x[0] = x[0].abs() + 0.01
+    x = x.to(dtype)
+    q = torch.randint(0, 1 << bits, (n, k), device="cuda", generator=g)
+    q[4], q[8] = 3, 0
+    s = torch.rand(n, k // group, device="cuda", generator=g) * 0.01 + 0.002
+    b = torch.randn(n, k // group, device="cuda", generator=g) * 0.05
+    s[3, 1], s[4, 1], b[5, 2], b[6, 3], s[8, 0], s[9, 2] = (float(v) for v in ("inf", "inf", "inf", "-inf", "inf", "nan"))
+    packed = q.to(torch.uint8)
+    if bits == 4:
+        v = (q.view(n, k // 8, 8) << (4 * torch.arange(8, device="cuda"))).sum(-1)
+        packed = torch.where(v >= 2 ** 31, v - 2 ** 32, v).to(torch.int32)
+    y = quantized.affine_quantized_matmul(x, packed, s, b, bits=bits, group_size=group, K=k)
+    ref = x.double() @ (s.double().repeat_interleave(group, 1) * q.double() + b.double().repeat_interleave(group, 1)).T
+    assert torch.isinf(ref[0, 4:7]).all() and torch.isnan(ref[:, 8]).all() and torch.isnan(ref[1:, 5]).all()
+    assert torch.equal(torch.isnan(y), torch.isnan(ref)) and torch.equal(torch.isinf(y), torch.isinf(ref))
+    assert torch.equal(torch.sign(y)[torch.isinf(ref)], torch.sign(ref).to(dtype)[torch.isinf(ref)])
+    finite = torch.isfinite(ref)
+    assert ((y.double() - ref)[finite].norm() / ref[finite].norm()).item() < (1e-3 if dtype == torch.float16 else 1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("fmt,group", [("mxfp4", 32), ("mxfp8", 32), ("nvfp4", 16)])
 def test_operator_matmul_nan_codes(cuda, fmt, group, dtype):
     g = _gen(5)
