@@ -21,7 +21,7 @@
 // Measured (four linears of a layer, before: one warp per four columns on CUDA cores): mxfp8, f16, M = 512, 4096 / 14336
 // wide 15.2 -> 0.86 ms; affine 4-bit, f32, M = 48, 2048 / 5632 wide 597 -> 103 us.  Bound by latency, not by a unit: a
 // stage takes 0.5-1 us through issuer, tensor core and promoter (the two MMAs of a 32-k group are too little work to hide
-// a commit and a TMEM read), 0.18 of the bf16 rate at best.
+// a commit and a TMEM read), 0.16 of the measured bf16 rate at best (mxfp8, f16, M = 512, 4096 x 28672).
 //
 // What the split cannot represent takes an exact path: a unit whose activations are not finite (inf times
 // code plus inf times bias is not what inf times scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
