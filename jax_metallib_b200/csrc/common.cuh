@@ -93,7 +93,7 @@ int ensure_dynamic_smem(const void* func, int bytes, std::atomic<uint64_t>& done
 // Environment switches are read once, when first asked for.
 int env_int_once(const char* name, int dflt, std::atomic<int>& cache);
 // QMM_FORCE_SPLIT_K=1: the kernels that split K and the operator GEMM take every shape that they can, whatever is faster (a
-// cross-check of small shapes on a GPU box; read once per process).
+// cross-check of small shapes; read once per process).
 bool force_split_k();
 int gemm_ctas();             // CTAs a persistent GEMM may launch: num_sms() unless qmm_set_cta_limit lowered it
 
