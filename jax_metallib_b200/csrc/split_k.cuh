@@ -60,6 +60,22 @@ __device__ __forceinline__ bool wait_cluster_warp(uint64_t* bar, uint32_t parity
   return __all_sync(0xFFFFFFFFu, ok);
 }
 
+// Every thread of the cluster: what was written to shared memory before is visible to all of it afterwards.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p in the shared memory of CTA `rank`.
+__device__ __forceinline__ float2 load_peer(const float2* p, int rank) {
+  float2 v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %2, %3;\n\t"
+      "ld.shared::cluster.v2.f32 {%0, %1}, [ra];\n\t}"
+      : "=f"(v.x), "=f"(v.y)
+      : "r"(dev::smem_u32(p)), "r"(rank)
+      : "memory");
+  return v;
+}
+
 struct Grid {
   int ks, clusters;
 };
