@@ -4,8 +4,8 @@
 //
 // The weights are the 128-row operand of the MMA and go into it through TMEM: a converter thread owns one output column,
 // reads its packed codes from shared memory and writes them as f16 pairs into its own TMEM lane.  Nothing of a converted
-// weight crosses shared memory, which with both operands in it is what bounds such a kernel (a 64-k stage of 128 columns x
-// 192 rows moves 64 KB there in 384 clocks of MMA; with converted weights stored and read back it would be 96 KB).
+// weight crosses shared memory, which with both operands in it is what bounds such a kernel (64 k of 128 columns x
+// 192 rows move 64 KB there in 384 clocks of MMA; with converted weights stored and read back it would be 96 KB).
 //
 //   MX formats: element * scale goes in, exactly.  A significand has at most 6 bits; the power-of-two scales of a column are
 //     taken relative to the largest of 512 k (a unit), and f16 holds all bits of an element down to 2^-22 (mxfp8) or 2^-36
@@ -16,7 +16,7 @@
 //     acc += s * D + b * sum(x).  sum(x) comes from mma.sync against ones.  Results that are not finite are computed again.
 //
 // Persistent CTAs, one per SM.  Warps: TMA of activations, TMA of raw weights, the MMA issuer; two warpgroups of
-// converters that take the 64-k stages in turn; two warpgroups of promoters, a thread of which holds up to 96 rows of a
+// converters that take the 128-k stages in turn; two warpgroups of promoters, a thread of which holds up to 96 rows of a
 // column in registers (setmaxnreg: 144 for them, 72 for converters, 40 for the rest).  Two or more accumulators, so that
 // neither a promotion nor the store of a tile stops the tensor core.  Where tiles are few, the CTAs of a cluster share
 // one, each with a slice of K, and add their parts over distributed shared memory in a fixed order.
@@ -29,8 +29,7 @@ namespace opp {
 using namespace opg;
 
 constexpr int BN = 128;               // output columns per tile
-constexpr int BK = 64;                // k per stage
-constexpr int kStages = 4;            // converted weights in TMEM and activations in shared memory
+constexpr int BK = 128;               // k per stage: waits and arrivals cost a warp some 100 clocks each, a stage of 64 k was bound by them
 constexpr int kRawBoxes = 4;
 constexpr int kRawBox = BN * 128;     // 16 KB of raw weights
 constexpr int kUnitK = 512;           // k per accumulator, MX formats
@@ -47,18 +46,21 @@ struct Cfg {
   static constexpr bool kBias = FMT == kAffine4 || FMT == kAffine8;
   static constexpr bool kE8m0 = FMT == kMxfp4 || FMT == kMxfp8;
   static constexpr int kStagesPerBox = 128 * 8 / kBits / BK;
+  static constexpr int kSlots = kBias || CPT == 96 ? 2 : 4;      // stages of converted weights in TMEM
   static constexpr int kRows = 2 * CPT;
   static constexpr int kXBytes = kRows * BK * 2;
-  static constexpr int kAccBase = kStages * (BK / 2);            // first TMEM column of the accumulators
+  // activations in flight: a copy takes about 1 us from request to arrival, a stage's MMAs 0.02 - 0.2 us
+  static constexpr int kXStages = CPT == 96 ? 3 : (CPT == 64 ? 4 : 8);
+  static constexpr int kAccBase = kSlots * (BK / 2);            // first TMEM column of the accumulators
   static constexpr int kAccBufs = (512 - kAccBase) / kRows;
-  static constexpr int kOffRaw = kStages * kXBytes;
+  static constexpr int kOffRaw = kXStages * kXBytes;
   static constexpr int kOffInfo = kOffRaw + kRawBoxes * kRawBox;
   static constexpr int kOffBar = kOffInfo + (kBias ? kInfo * kRows * 4 : (kE8m0 ? kInfo * BN * 4 : 0));
   static constexpr int kSmem = kOffBar + 1024 + 1024;
   // scale that brings the largest element of a unit's largest scale just below f16's limit, and the smallest power of
   // two of a group's factor at which the last bit of an element is still there
   static constexpr int kUp = FMT == kMxfp8 ? 7 : 13, kLowest = FMT == kMxfp8 ? -15 : -23;
-  static_assert(kAccBufs >= 2 && kStages + kAccBufs + 2 <= kInfo && 2 * kStages + kAccBufs <= kInfo, "ring sizes");
+  static_assert(kAccBufs >= 2 && kSlots <= kXStages && kSlots + kAccBufs + 3 <= kInfo && (!kBias || 4 * kSlots + kAccBufs <= kInfo), "ring sizes");
   static_assert(kRows * BN * 4 <= kOffInfo, "the result tile reuses the rings");
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
@@ -87,6 +89,12 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
+}
+
+// A wait that usually finds its phase complete.
+__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, int* status, int tag) {
+  if (__all_sync(0xFFFFFFFFu, dev::mbar_try_wait(bar, parity))) return true;
+  return dev::mbar_wait_warp(bar, parity, status, tag);
 }
 
 // e8m0 scales of a column's unit: 16 bytes, 0 behind the end of the row
@@ -121,9 +129,9 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
   uint64_t* rfull = reinterpret_cast<uint64_t*>(smem + C::kOffBar);    // raw weights landed
   uint64_t* rempty = rfull + kRawBoxes;                                // and converted
   uint64_t* xfull = rempty + kRawBoxes;                                // activations landed
-  uint64_t* full = xfull + kStages;                                    // stage ready for its MMAs
-  uint64_t* consumed = full + kStages;                                 // and multiplied
-  uint64_t* dfull = consumed + kStages;                                // a unit's accumulator complete
+  uint64_t* full = xfull + C::kXStages;                                    // stage ready for its MMAs
+  uint64_t* consumed = full + C::kSlots;                                 // and multiplied (one per slot of the activations)
+  uint64_t* dfull = consumed + C::kXStages;                                // a unit's accumulator complete
   uint64_t* dempty = dfull + C::kAccBufs;                              // and drained
   uint64_t* info = dempty + C::kAccBufs;                               // activation sums of a unit / marks of a tile written
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(info + kInfo);
@@ -135,11 +143,12 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
   const int stages = (k_end - k_begin + BK - 1) / BK;
   const int boxes = (stages + C::kStagesPerBox - 1) / C::kStagesPerBox;
   const int units = (k_end - k_begin + a.pu - 1) / a.pu;
-  const int halves = C::kBias && a.pu < BK ? 2 : 1;   // units per stage, where a unit is no more than a stage
+  const int parts = C::kBias ? BK / a.pu : 1;   // units per stage, where a unit is no more than a stage
 
   if (warp == 0) {
     if (lane < kRawBoxes) { dev::mbar_init(&rfull[lane], 1); dev::mbar_init(&rempty[lane], C::kStagesPerBox * 4); }
-    if (lane < kStages) { dev::mbar_init(&xfull[lane], 1); dev::mbar_init(&full[lane], 4); dev::mbar_init(&consumed[lane], 1); }
+    if (lane < C::kXStages) { dev::mbar_init(&xfull[lane], 1); dev::mbar_init(&consumed[lane], 1); }
+    if (lane < C::kSlots) dev::mbar_init(&full[lane], 4);
     if (lane < C::kAccBufs) { dev::mbar_init(&dfull[lane], 1); dev::mbar_init(&dempty[lane], 8); }
     if (lane < kInfo) dev::mbar_init(&info[lane], C::kBias ? 4 : 8);
     dev::fence_mbar_init();
@@ -172,15 +181,16 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         for (int t = blockIdx.y; ok && t < a.tiles; t += gridDim.y) {
           const int m0 = (t % a.mt) * a.bm;
           for (int st = 0; st < stages; ++st, ++cnt) {
-            const uint32_t s = cnt % kStages;
-            if (!dev::mbar_wait_relaxed(&consumed[s], ((cnt / kStages) & 1) ^ 1, a.status, 111)) { ok = false; break; }
+            const uint32_t s = cnt % C::kXStages;
+            if (!dev::mbar_wait_relaxed(&consumed[s], ((cnt / C::kXStages) & 1) ^ 1, a.status, 111)) { ok = false; break; }
             dev::mbar_expect_tx(&xfull[s], a.bm * BK * 2);
             dev::tma_load_2d(smem + s * C::kXBytes, &xmap, &xfull[s], k_begin + st * BK, m0);
+            dev::tma_load_2d(smem + s * C::kXBytes + C::kXBytes / 2, &xmap, &xfull[s], k_begin + st * BK + 64, m0);
           }
         }
         // every copy has landed before this CTA's shared memory is reused, whatever the other warps did
-        for (uint32_t i = cnt > kStages ? cnt - kStages : 0; i < cnt; ++i)
-          if (!dev::mbar_wait_relaxed(&xfull[i % kStages], (i / kStages) & 1, a.status, 112)) break;
+        for (uint32_t i = cnt > C::kXStages ? cnt - C::kXStages : 0; i < cnt; ++i)
+          if (!dev::mbar_wait_relaxed(&xfull[i % C::kXStages], (i / C::kXStages) & 1, a.status, 112)) break;
       }
     } else if (warp == 1) {
       // ------------------------ TMA producer: raw weights --------------------
@@ -201,29 +211,32 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
       }
     } else if (warp == 2) {
       // ------------------------------ MMA issuer -----------------------------
-      if (lane == 0) {
+      if (dev::elect_one()) {
         constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // SBO, version, 128-byte swizzle
         const uint32_t x_lo = ((dev::smem_u32(smem) >> 4) & 0x3FFF) | ((16u >> 4) << 16);
-        uint32_t cnt = 0, buf = 0, bpar = 1;   // bpar: parity of the wait for the accumulator, flips with every round
+        uint32_t cnt = 0, xs = 0, buf = 0, bpar = 1;   // bpar: parity of the wait for the accumulator, flips with every round
         bool ok = true;
         for (int t = blockIdx.y; ok && t < a.tiles; t += gridDim.y) {
           for (int st = 0; ok && st < stages; ++st, ++cnt) {
-            const uint32_t s = cnt % kStages;
-            if (!dev::mbar_wait(&full[s], (cnt / kStages) & 1, a.status, 115)) { ok = false; break; }
-            const uint32_t at = tmem_base + s * (BK / 2), b_lo = x_lo + s * (C::kXBytes >> 4);
+            const uint32_t s = cnt % C::kSlots;
+            if (!dev::mbar_wait(&full[s], (cnt / C::kSlots) & 1, a.status, 115)) { ok = false; break; }
+            const uint32_t at = tmem_base + s * (BK / 2), b_lo = x_lo + xs * (C::kXBytes >> 4);
+            // a step of 16 k: 8 columns of TMEM, 32 bytes of a row; 64 k of activations are one swizzled tile
+            auto step = [&](uint32_t d, int j, uint32_t accumulate) {
+              dev::umma_f16_ts(d, at + j * 8, b_lo + (j >> 2) * (C::kXBytes >> 5) + (j & 3) * 2, kDescHi, a.idesc, accumulate);
+            };
             if (C::kBias) {
-              for (int h = 0; h < halves; ++h) {
-                if (st * halves + h >= units) break;
+              for (int h = 0; h < parts; ++h) {
+                if (st * parts + h >= units) break;
                 if (!dev::mbar_wait(&dempty[buf], bpar, a.status, 116)) { ok = false; break; }
                 dev::tc_fence_after();
                 const uint32_t d = tmem_base + C::kAccBase + buf * C::kRows;
-                if (halves == 1) {
+                if (parts == 2) {
 #pragma unroll
-                  for (int j = 0; j < 4; ++j) dev::umma_f16_ts(d, at + j * 8, b_lo + j * 2, kDescHi, a.idesc, j != 0);
+                  for (int j = 0; j < 4; ++j) step(d, h * 4 + j, j != 0);
                 } else {
 #pragma unroll
-                  for (int j = 0; j < 2; ++j)
-                    dev::umma_f16_ts(d, at + h * 16 + j * 8, b_lo + h * 4 + j * 2, kDescHi, a.idesc, j != 0);
+                  for (int j = 0; j < 2; ++j) step(d, h * 2 + j, j != 0);
                 }
                 dev::tc_commit(&dfull[buf]);
                 if (++buf == C::kAccBufs) { buf = 0; bpar ^= 1; }
@@ -234,13 +247,14 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
               dev::tc_fence_after();
               const uint32_t d = tmem_base + C::kAccBase + buf * C::kRows;
 #pragma unroll
-              for (int j = 0; j < 4; ++j) dev::umma_f16_ts(d, at + j * 8, b_lo + j * 2, kDescHi, a.idesc, !first || j != 0);
+              for (int j = 0; j < 8; ++j) step(d, j, !first || j != 0);
               if (st % (kUnitK / BK) == kUnitK / BK - 1 || st == stages - 1) {
                 dev::tc_commit(&dfull[buf]);
                 if (++buf == C::kAccBufs) { buf = 0; bpar ^= 1; }
               }
             }
-            if (ok) dev::tc_commit(&consumed[s]);
+            if (ok) dev::tc_commit(&consumed[xs]);
+            if (++xs == C::kXStages) xs = 0;
           }
         }
       }
@@ -256,71 +270,75 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
     bool ok = true;
     for (int t = blockIdx.y; ok && t < a.tiles; t += gridDim.y, cnt0 += stages, box0 += boxes, unit0 += units, ++tile_no) {
       const int n = min((t / a.mt) * BN + row, a.N - 1);
-      // MX: scales of the unit, the largest of them; nvfp4: the four scales of the next stage
+      // MX: scales of the unit, the largest of them; nvfp4: the eight scales of the next stage
       const int G = C::kE8m0 ? a.K / 32 : a.K / 16;
       const uint8_t* srow = static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(n) * (C::kBias ? 0 : G);
       const bool vec = C::kE8m0 && G % 16 == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 15) == 0;
-      const bool quad = FMT == kNvfp4 && G % 4 == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 3) == 0;
-      uint4 us = make_uint4(0u, 0u, 0u, 0u);
-      int ref = 0, unit = -1;
-      uint32_t nv = 0u;
+      const bool pairs8 = FMT == kNvfp4 && G % 8 == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 7) == 0;
+      uint4 us = make_uint4(0u, 0u, 0u, 0u), next_us = us;
+      int ref = 0;
+      uint2 nv = make_uint2(0u, 0u);
       auto load_nv = [&](int st) {
         const int g = (k_begin + st * BK) / 16;
-        if (quad) return __ldg(reinterpret_cast<const uint32_t*>(srow + g));
-        uint32_t r = 0u;
+        if (pairs8) return __ldg(reinterpret_cast<const uint2*>(srow + g));
+        uint2 r = make_uint2(0u, 0u);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (g + i < G) r |= static_cast<uint32_t>(__ldg(srow + g + i)) << (8 * i);
+        for (int i = 0; i < 4; ++i) {
+          if (g + i < G) r.x |= static_cast<uint32_t>(__ldg(srow + g + i)) << (8 * i);
+          if (g + 4 + i < G) r.y |= static_cast<uint32_t>(__ldg(srow + g + 4 + i)) << (8 * i);
+        }
         return r;
       };
+      if (C::kE8m0) next_us = unit_scales(srow, k_begin / 32, G, vec);
       if (FMT == kNvfp4 && grp < stages) nv = load_nv(grp);
       for (int st = grp; st < stages; st += 2) {
-        const uint32_t c = cnt0 + st, s = c % kStages, par = (c / kStages) & 1;
+        const uint32_t c = cnt0 + st, s = c % C::kSlots, xs = c % C::kXStages;
         const uint32_t box = box0 + st / C::kStagesPerBox, rs = box % kRawBoxes;
         const int sub = st % C::kStagesPerBox;
-        if (C::kE8m0 && st / (kUnitK / BK) != unit) {
-          unit = st / (kUnitK / BK);
-          us = unit_scales(srow, (k_begin + unit * kUnitK) / 32, G, vec);
+        if (C::kE8m0 && st % (kUnitK / BK) == grp) {   // the group's first stage of a unit
+          us = next_us;
           ref = unit_largest(us);
+          const int next = (k_begin + (st / (kUnitK / BK) + 1) * kUnitK) / 32;
+          if (next < G) next_us = unit_scales(srow, next, G, vec);
         }
-        const uint32_t nv_now = nv;
+        const uint2 nv_now = nv;
         if (FMT == kNvfp4 && st + 2 < stages) nv = load_nv(st + 2);
-        if (!dev::mbar_wait_warp(&rfull[rs], (box / kRawBoxes) & 1, a.status, 117)) { ok = false; break; }
+        if (!wait_warp(&rfull[rs], (box / kRawBoxes) & 1, a.status, 117)) { ok = false; break; }
         const uint8_t* raw = smem + C::kOffRaw + rs * kRawBox + row * 128;
-        constexpr int kPieces = C::kBits == 4 ? 2 : 4;   // 16-byte pieces of this column's 64 k
-        uint4 v[kPieces];
+        if (c >= C::kSlots) {   // the MMAs that read this slot's TMEM before have retired
+          const uint32_t p = c - C::kSlots;
+          if (!wait_warp(&consumed[p % C::kXStages], (p / C::kXStages) & 1, a.status, 118)) { ok = false; break; }
+          dev::tc_fence_after();
+        }
+        constexpr int kPieces = C::kBits / 4;   // 16-byte pieces of a column's 32 k
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i) v[i] = *reinterpret_cast<const uint4*>(raw + (((sub * kPieces + i) ^ (row & 7)) << 4));
-        // the MMAs that read this stage's TMEM before have retired
-        if (!dev::mbar_wait_warp(&consumed[s], par ^ 1, a.status, 118)) { ok = false; break; }
-        dev::tc_fence_after();
+        for (int h = 0; h < 4; ++h) {   // 32 k: 16 TMEM columns
+          uint4 v[kPieces];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {   // 32 k: 16 TMEM columns
+          for (int i = 0; i < kPieces; ++i)
+            v[i] = *reinterpret_cast<const uint4*>(raw + ((((sub * 4 + h) * kPieces + i) ^ (row & 7)) << 4));
           uint32_t f0 = 0u, f1 = 0u;    // factors of its two halves
           if (C::kE8m0) {
-            const int g = (st % (kUnitK / BK)) * 2 + h;
-            const uint32_t word = g < 4 ? us.x : (g < 8 ? us.y : (g < 12 ? us.z : us.w));
-            const int code = (word >> (8 * (g & 3))) & 0xFF;
+            const int quad = st % (kUnitK / BK);
+            const uint32_t word = quad < 2 ? (quad == 0 ? us.x : us.y) : (quad == 2 ? us.z : us.w);
+            const int code = (word >> (8 * h)) & 0xFF;
             const int e = C::kUp - (ref - code);
             __half2 f = __float2half2_rn(e < C::kLowest ? 0.f : __uint_as_float(static_cast<uint32_t>(127 + e) << 23));
             f0 = f1 = code == 255 ? 0x7E007E00u : *reinterpret_cast<uint32_t*>(&f);
             if (e < C::kLowest) {
               uint32_t any = 0u;
 #pragma unroll
-              for (int i = 0; i < kPieces / 2; ++i) {
-                const uint4 p = v[h * (kPieces / 2) + i];
-                any |= p.x | p.y | p.z | p.w;
-              }
-              if (any & 0x7F7F7F7Fu & (C::kBits == 4 ? 0x77777777u : 0xFFFFFFFFu)) marks[(tile_no % kInfo) * BN + row] = tile_no + 1;
+              for (int i = 0; i < kPieces; ++i) any |= v[i].x | v[i].y | v[i].z | v[i].w;
+              if (any & (C::kBits == 4 ? 0x77777777u : 0x7F7F7F7Fu)) marks[(tile_no % kInfo) * BN + row] = tile_no + 1;
             }
           } else if (FMT == kNvfp4) {
-            f0 = e4m3_pair<false>((nv_now >> (16 * h)) & 0xFFu);
-            f1 = e4m3_pair<false>((nv_now >> (16 * h + 8)) & 0xFFu);
+            const uint32_t word = h < 2 ? nv_now.x : nv_now.y;
+            f0 = e4m3_pair<false>((word >> (16 * (h & 1))) & 0xFFu);
+            f1 = e4m3_pair<false>((word >> (16 * (h & 1) + 8)) & 0xFFu);
           }
           uint32_t o[16];
           if (C::kBits == 4) {
-            const uint4 p = v[h];
-            const uint32_t in[4] = {p.x, p.y, p.z, p.w};
+            const uint32_t in[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const uint4 r = convert8<FMT, false>(in[i], 0u, i < 2 ? f0 : f1, false);
@@ -328,9 +346,8 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const uint4 p = v[2 * h + i];
-              const uint4 r = convert8<FMT, false>(p.x, p.y, 0u, false), u = convert8<FMT, false>(p.z, p.w, 0u, false);
+            for (int i = 0; i < kPieces; ++i) {
+              const uint4 r = convert8<FMT, false>(v[i].x, v[i].y, 0u, false), u = convert8<FMT, false>(v[i].z, v[i].w, 0u, false);
               o[8 * i] = r.x; o[8 * i + 1] = r.y; o[8 * i + 2] = r.z; o[8 * i + 3] = r.w;
               o[8 * i + 4] = u.x; o[8 * i + 5] = u.y; o[8 * i + 6] = u.z; o[8 * i + 7] = u.w;
             }
@@ -341,29 +358,34 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
           }
           dev::tmem_st_32x16(a_lane + s * (BK / 2) + h * 16, o);
         }
-        if (!dev::mbar_wait_warp(&xfull[s], par, a.status, 119)) { ok = false; break; }
+        if (!wait_warp(&xfull[xs], (c / C::kXStages) & 1, a.status, 119)) { ok = false; break; }
         if (C::kBias) {
           // activation sums of the stage's units: 16 rows at a time against a column of ones
-          const uint32_t unit_no = unit0 + st * halves;
-          const uint32_t xt = dev::smem_u32(smem + s * C::kXBytes);
+          const uint32_t unit_no = unit0 + st * parts;
+          const uint32_t xt = dev::smem_u32(smem + xs * C::kXBytes);
           for (int rb = ww; rb * 16 < a.bm; rb += 4) {
             const int r = rb * 16 + (lane & 15);
-            float d[2][4] = {};
+            float d[4][4] = {};   // one per 32 k
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < 8; ++j) {
               uint32_t f[4];
-              ldmatrix_x4(xt + r * 128 + (((2 * j + (lane >> 4)) ^ (r & 7)) << 4), f);
-              if (halves == 1 || j < 2) mma_f16_ones(d[0], f);
-              else mma_f16_ones(d[1], f);
+              ldmatrix_x4(xt + (j >> 2) * (C::kXBytes / 2) + r * 128 + (((2 * (j & 3) + (lane >> 4)) ^ (r & 7)) << 4), f);
+              mma_f16_ones(d[j >> 1], f);
             }
             if ((lane & 3) == 0) {
-              float* dst = xsum + (unit_no % kInfo) * C::kRows + rb * 16 + (lane >> 2);
-              dst[0] = d[0][0];
-              dst[8] = d[0][2];
-              if (halves == 2 && st * 2 + 1 < units) {
-                dst = xsum + ((unit_no + 1) % kInfo) * C::kRows + rb * 16 + (lane >> 2);
-                dst[0] = d[1][0];
-                dst[8] = d[1][2];
+              const int at = rb * 16 + (lane >> 2);
+              if (parts == 2) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  float* dst = xsum + ((unit_no + h) % kInfo) * C::kRows + at;
+                  if (st * 2 + h < units) { dst[0] = d[2 * h][0] + d[2 * h + 1][0]; dst[8] = d[2 * h][2] + d[2 * h + 1][2]; }
+                }
+              } else {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                  float* dst = xsum + ((unit_no + h) % kInfo) * C::kRows + at;
+                  if (st * 4 + h < units) { dst[0] = d[h][0]; dst[8] = d[h][2]; }
+                }
               }
             }
           }
@@ -372,14 +394,10 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         dev::tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          dev::mbar_arrive(&rempty[rs]);
           dev::mbar_arrive(&full[s]);
-          if (C::kBias) {
-            const uint32_t unit_no = unit0 + st * halves;
-            dev::mbar_arrive(&info[unit_no % kInfo]);
-            if (halves == 2 && st * 2 + 1 < units) dev::mbar_arrive(&info[(unit_no + 1) % kInfo]);
-          }
+          dev::mbar_arrive(&rempty[rs]);
         }
+        if (C::kBias && lane < parts && st * parts + lane < units) dev::mbar_arrive(&info[(unit0 + st * parts + lane) % kInfo]);
       }
       // the last box of an odd number of stages: what the other stages of the box would have handed back
       if (ok) {
@@ -436,7 +454,7 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
           s0 = s1; b0 = b1;
           next_scale(s1, b1);
           // the bias's share first: it needs no accumulator
-          if (!dev::mbar_wait_warp(&info[unit_no % kInfo], (unit_no / kInfo) & 1, a.status, 120)) { ok = false; break; }
+          if (!wait_warp(&info[unit_no % kInfo], (unit_no / kInfo) & 1, a.status, 120)) { ok = false; break; }
           const float* xs = xsum + (unit_no % kInfo) * C::kRows + c0;
 #pragma unroll
           for (int c = 0; c < CPT; c += 8) {
@@ -449,7 +467,7 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
             }
           }
         }
-        if (!dev::mbar_wait_warp(&dfull[buf], bpar, a.status, 121)) { ok = false; break; }
+        if (!wait_warp(&dfull[buf], bpar, a.status, 121)) { ok = false; break; }
         dev::tc_fence_after();
         const uint64_t s2 = pack2(s, s);
         const uint32_t taddr = d_lane + buf * C::kRows;
@@ -620,7 +638,7 @@ static int launch(Args a, const Cut& cut, cudaStream_t stream) {
                                   CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
   if (int rc = make_tensor_map_2d(&xmap, a.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)a.M, (uint64_t)a.K, (uint64_t)a.K * 2,
-                                  a.bm, BK, CU_TENSOR_MAP_SWIZZLE_128B))
+                                  a.bm, 64, CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
   static std::atomic<uint64_t> configured{0};
   auto kern = op_prefill_kernel<FMT, CPT>;
