@@ -15,9 +15,9 @@
 //   affine: the codes q go in, exactly, one scale group (at most 64 k) per accumulator; promoters apply s and b in f32:
 //     acc += s * D + b * sum(x).  sum(x) comes from mma.sync against ones.  Results that are not finite are computed again.
 //
-// Persistent CTAs, one per SM.  Warps: TMA of activations, TMA of raw weights, the MMA issuer; two warpgroups of
+// Persistent CTAs, one per SM.  Warps: TMA of activations, TMA of raw weights, the MMA issuer; three warpgroups of
 // converters that take the 128-k stages in turn; two warpgroups of promoters, a thread of which holds up to 96 rows of a
-// column in registers (setmaxnreg: 144 for them, 72 for converters, 40 for the rest).  Two or more accumulators, so that
+// column in registers (setmaxnreg).  Two or more accumulators, so that
 // neither a promotion nor the store of a tile stops the tensor core.  Where tiles are few, the CTAs of a cluster share
 // one, each with a slice of K, and add their parts over distributed shared memory in a fixed order.
 #include "opapi_convert.cuh"
@@ -30,14 +30,16 @@ using namespace opg;
 
 constexpr int BN = 128;               // output columns per tile
 constexpr int BK = 128;               // k per stage: waits and arrivals cost a warp some 100 clocks each, a stage of 64 k was bound by them
-constexpr int kRawBoxes = 4;
 constexpr int kRawBox = BN * 128;     // 16 KB of raw weights
 constexpr int kUnitK = 512;           // k per accumulator, MX formats
 constexpr int kInfo = 16;             // units whose activation sums are kept; tiles whose columns may be marked
 constexpr int kMaxRows = 192;
 constexpr int kMaxCluster = 8;
-constexpr int kFirstConverter = 4, kFirstPromoter = 12, kThreads = 640;
-constexpr int kMiscRegs = 40, kConverterRegs = 72, kPromoterRegs = 144;
+constexpr int kGroups = 3;            // warpgroups of converters
+constexpr int kFirstConverter = 4, kFirstPromoter = kFirstConverter + 4 * kGroups, kThreads = (kFirstPromoter + 8) * 32;
+constexpr int kLaunchRegs = 65536 / kThreads / 8 * 8;
+constexpr int kSBoxes = 4;            // affine: boxes of scales and biases (four groups each) on their way to the promoters
+constexpr int kSBoxBytes = 2 * BN * 16;
 constexpr uint32_t kMarked = 0x7FC0F1A6u;   // partial result of a column that has to be computed again
 
 template <int FMT, int CPT>   // CPT: rows of a tile (accumulator columns) per promoter thread, at most
@@ -53,18 +55,23 @@ struct Cfg {
   static constexpr int kXStages = CPT == 96 ? 3 : (CPT == 64 ? 4 : 8);
   static constexpr int kAccBase = kSlots * (BK / 2);            // first TMEM column of the accumulators
   static constexpr int kAccBufs = (512 - kAccBase) / kRows;
+  static constexpr int kRawBoxes = kBias || kBits == 8 ? 3 : 4;
   static constexpr int kOffRaw = kXStages * kXBytes;
   static constexpr int kOffInfo = kOffRaw + kRawBoxes * kRawBox;
-  static constexpr int kOffBar = kOffInfo + (kBias ? kInfo * kRows * 4 : (kE8m0 ? kInfo * BN * 4 : 0));
+  static constexpr int kOffS = kOffInfo + (kBias ? kInfo * kRows * 4 : (kE8m0 ? kInfo * BN * 4 : 0));
+  static constexpr int kOffBar = kOffS + (kBias ? kSBoxes * kSBoxBytes : 0);
   static constexpr int kSmem = kOffBar + 1024 + 1024;
   // scale that brings the largest element of a unit's largest scale just below f16's limit, and the smallest power of
   // two of a group's factor at which the last bit of an element is still there
   static constexpr int kUp = FMT == kMxfp8 ? 7 : 13, kLowest = FMT == kMxfp8 ? -15 : -23;
   static_assert(kAccBufs >= 2 && kSlots <= kXStages && kSlots + kAccBufs + 3 <= kInfo && (!kBias || 4 * kSlots + kAccBufs <= kInfo), "ring sizes");
+  // registers of a thread: producers and issuer, converters, promoters
+  static constexpr int kMiscRegs = kBias && CPT == 96 ? 40 : 32, kConverterRegs = kBias && CPT == 96 ? 56 : 64;
+  static constexpr int kPromoterRegs = kBias && CPT == 96 ? 136 : 128;
+  static_assert(128 * kMiscRegs + kGroups * 128 * kConverterRegs + 256 * kPromoterRegs <= kThreads * kLaunchRegs, "registers of the launch");
   static_assert(kRows * BN * 4 <= kOffInfo, "the result tile reuses the rings");
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
-static_assert(4 * 32 * kMiscRegs + 8 * 32 * (kConverterRegs + kPromoterRegs) <= kThreads * 96, "registers of the launch");
 
 struct Args {
   const void* x;
@@ -75,6 +82,7 @@ struct Args {
   int M, N, K, gs, pu;       // pu: k per accumulator
   int bm, mt, tiles;         // rows per tile, tiles along M, tiles in all
   int blocks, block_k;       // K in blocks of the slice granularity
+  int sbox_k;                // affine: k per box of scales; 0: promoters read them from global memory
   uint32_t idesc;
   int* status;
 };
@@ -120,21 +128,24 @@ __device__ __forceinline__ int unit_largest(const uint4& s) {
 
 template <int FMT, int CPT>
 __global__ void __launch_bounds__(kThreads, 1)
-op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ Args a) {
+op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+                  const __grid_constant__ CUtensorMap smap, const __grid_constant__ CUtensorMap bmap, const __grid_constant__ Args a) {
   using C = Cfg<FMT, CPT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   float* xsum = reinterpret_cast<float*>(smem + C::kOffInfo);          // [kInfo][kRows], affine
   uint32_t* marks = reinterpret_cast<uint32_t*>(smem + C::kOffInfo);   // [kInfo][BN], MX: number of the tile that marked the column
   uint64_t* rfull = reinterpret_cast<uint64_t*>(smem + C::kOffBar);    // raw weights landed
-  uint64_t* rempty = rfull + kRawBoxes;                                // and converted
-  uint64_t* xfull = rempty + kRawBoxes;                                // activations landed
+  uint64_t* rempty = rfull + C::kRawBoxes;                                // and converted
+  uint64_t* xfull = rempty + C::kRawBoxes;                                // activations landed
   uint64_t* full = xfull + C::kXStages;                                    // stage ready for its MMAs
   uint64_t* consumed = full + C::kSlots;                                 // and multiplied (one per slot of the activations)
   uint64_t* dfull = consumed + C::kXStages;                                // a unit's accumulator complete
   uint64_t* dempty = dfull + C::kAccBufs;                              // and drained
   uint64_t* info = dempty + C::kAccBufs;                               // activation sums of a unit / marks of a tile written
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(info + kInfo);
+  uint64_t* sfull = info + kInfo;                                      // a box of scales landed
+  uint64_t* sempty = sfull + kSBoxes;                                  // and read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sempty + kSBoxes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KS = gridDim.x, rank = blockIdx.x;
@@ -146,11 +157,12 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
   const int parts = C::kBias ? BK / a.pu : 1;   // units per stage, where a unit is no more than a stage
 
   if (warp == 0) {
-    if (lane < kRawBoxes) { dev::mbar_init(&rfull[lane], 1); dev::mbar_init(&rempty[lane], C::kStagesPerBox * 4); }
+    if (lane < C::kRawBoxes) { dev::mbar_init(&rfull[lane], 1); dev::mbar_init(&rempty[lane], C::kStagesPerBox * 4); }
     if (lane < C::kXStages) { dev::mbar_init(&xfull[lane], 1); dev::mbar_init(&consumed[lane], 1); }
     if (lane < C::kSlots) dev::mbar_init(&full[lane], 4);
     if (lane < C::kAccBufs) { dev::mbar_init(&dfull[lane], 1); dev::mbar_init(&dempty[lane], 8); }
-    if (lane < kInfo) dev::mbar_init(&info[lane], C::kBias ? 4 : 8);
+    if (lane < kInfo) dev::mbar_init(&info[lane], C::kBias ? 4 : 4 * kGroups);
+    if (lane < kSBoxes) { dev::mbar_init(&sfull[lane], 1); dev::mbar_init(&sempty[lane], 8); }
     dev::fence_mbar_init();
   } else if (warp == 2 && lane == 0) {
     dev::tma_prefetch_desc(&wmap);
@@ -172,7 +184,7 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
   float* tile_out = reinterpret_cast<float*>(smem);   // [bm][BN] partial results, once the rings are idle (KS > 1)
 
   if (warp < kFirstConverter) {
-    dev::reg_dealloc<kMiscRegs>();
+    dev::reg_dealloc<C::kMiscRegs>();
     if (warp == 0) {
       // ------------------------ TMA producer: activations --------------------
       if (lane == 0) {
@@ -199,15 +211,33 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         bool ok = true;
         for (int t = blockIdx.y; ok && t < a.tiles; t += gridDim.y) {
           const int n0 = (t / a.mt) * BN;
-          for (int b = 0; b < boxes; ++b, ++cnt) {
-            const uint32_t s = cnt % kRawBoxes;
-            if (!dev::mbar_wait_relaxed(&rempty[s], ((cnt / kRawBoxes) & 1) ^ 1, a.status, 113)) { ok = false; break; }
+          for (int b = 0; ok && b < boxes; ++b, ++cnt) {
+            const uint32_t s = cnt % C::kRawBoxes;
+            if (!dev::mbar_wait_relaxed(&rempty[s], ((cnt / C::kRawBoxes) & 1) ^ 1, a.status, 113)) { ok = false; break; }
             dev::mbar_expect_tx(&rfull[s], kRawBox);
             dev::tma_load_2d(smem + C::kOffRaw + s * kRawBox, &wmap, &rfull[s], k_begin / 8 * C::kBits + b * 128, n0);
           }
         }
-        for (uint32_t i = cnt > kRawBoxes ? cnt - kRawBoxes : 0; i < cnt; ++i)
-          if (!dev::mbar_wait_relaxed(&rfull[i % kRawBoxes], (i / kRawBoxes) & 1, a.status, 114)) break;
+        for (uint32_t i = cnt > C::kRawBoxes ? cnt - C::kRawBoxes : 0; i < cnt; ++i)
+          if (!dev::mbar_wait_relaxed(&rfull[i % C::kRawBoxes], (i / C::kRawBoxes) & 1, a.status, 114)) break;
+      }
+    } else if (warp == 3) {
+      // ------------------- TMA producer: affine scales and biases ------------
+      if (C::kBias && a.sbox_k && lane == 0) {
+        uint32_t cnt = 0;
+        bool ok = true;
+        for (int t = blockIdx.y; ok && t < a.tiles; t += gridDim.y) {
+          for (int k = k_begin; k < k_end; k += a.sbox_k, ++cnt) {
+            const uint32_t s = cnt % kSBoxes;
+            if (!dev::mbar_wait_relaxed(&sempty[s], ((cnt / kSBoxes) & 1) ^ 1, a.status, 109)) { ok = false; break; }
+            uint8_t* dst = smem + C::kOffS + s * kSBoxBytes;
+            dev::mbar_expect_tx(&sfull[s], kSBoxBytes);
+            dev::tma_load_2d(dst, &smap, &sfull[s], k / a.gs, (t / a.mt) * BN);
+            dev::tma_load_2d(dst + BN * 16, &bmap, &sfull[s], k / a.gs, (t / a.mt) * BN);
+          }
+        }
+        for (uint32_t i = cnt > kSBoxes ? cnt - kSBoxes : 0; i < cnt; ++i)
+          if (!dev::mbar_wait_relaxed(&sfull[i % kSBoxes], (i / kSBoxes) & 1, a.status, 110)) break;
       }
     } else if (warp == 2) {
       // ------------------------------ MMA issuer -----------------------------
@@ -262,7 +292,7 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
     __syncwarp();
   } else if (warp < kFirstPromoter) {
     // ------------------------------ converters -----------------------------
-    dev::reg_dealloc<kConverterRegs>();
+    dev::reg_dealloc<C::kConverterRegs>();
     const int grp = (warp - kFirstConverter) >> 2, ww = warp & 3;
     const int row = ww * 32 + lane;
     const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(ww * 32) << 16);
@@ -276,7 +306,7 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
       const bool vec = C::kE8m0 && G % 16 == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 15) == 0;
       const bool pairs8 = FMT == kNvfp4 && G % 8 == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 7) == 0;
       uint4 us = make_uint4(0u, 0u, 0u, 0u), next_us = us;
-      int ref = 0;
+      int ref = 0, unit = -1;
       uint2 nv = make_uint2(0u, 0u);
       auto load_nv = [&](int st) {
         const int g = (k_begin + st * BK) / 16;
@@ -290,20 +320,24 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         return r;
       };
       if (C::kE8m0) next_us = unit_scales(srow, k_begin / 32, G, vec);
-      if (FMT == kNvfp4 && grp < stages) nv = load_nv(grp);
-      for (int st = grp; st < stages; st += 2) {
+      // The groups take the stages of all tiles in turn, so that a group has seen, with its stage before, the phase ahead of
+      // the one that it waits for next (a parity says no more than that).
+      const int first = static_cast<int>((grp + kGroups - cnt0 % kGroups) % kGroups);
+      if (FMT == kNvfp4 && first < stages) nv = load_nv(first);
+      for (int st = first; st < stages; st += kGroups) {
         const uint32_t c = cnt0 + st, s = c % C::kSlots, xs = c % C::kXStages;
-        const uint32_t box = box0 + st / C::kStagesPerBox, rs = box % kRawBoxes;
+        const uint32_t box = box0 + st / C::kStagesPerBox, rs = box % C::kRawBoxes;
         const int sub = st % C::kStagesPerBox;
-        if (C::kE8m0 && st % (kUnitK / BK) == grp) {   // the group's first stage of a unit
+        if (C::kE8m0 && st / (kUnitK / BK) != unit) {
+          unit = st / (kUnitK / BK);
           us = next_us;
           ref = unit_largest(us);
-          const int next = (k_begin + (st / (kUnitK / BK) + 1) * kUnitK) / 32;
+          const int next = (k_begin + (unit + 1) * kUnitK) / 32;   // every group has a stage in every unit
           if (next < G) next_us = unit_scales(srow, next, G, vec);
         }
         const uint2 nv_now = nv;
-        if (FMT == kNvfp4 && st + 2 < stages) nv = load_nv(st + 2);
-        if (!wait_warp(&rfull[rs], (box / kRawBoxes) & 1, a.status, 117)) { ok = false; break; }
+        if (FMT == kNvfp4 && st + kGroups < stages) nv = load_nv(st + kGroups);
+        if (!wait_warp(&rfull[rs], (box / C::kRawBoxes) & 1, a.status, 117)) { ok = false; break; }
         const uint8_t* raw = smem + C::kOffRaw + rs * kRawBox + row * 128;
         if (c >= C::kSlots) {   // the MMAs that read this slot's TMEM before have retired
           const uint32_t p = c - C::kSlots;
@@ -399,24 +433,24 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         }
         if (C::kBias && lane < parts && st * parts + lane < units) dev::mbar_arrive(&info[(unit0 + st * parts + lane) % kInfo]);
       }
-      // the last box of an odd number of stages: what the other stages of the box would have handed back
+      // a last box that is not full: what its other stages would have handed back
       if (ok) {
         const int missing = boxes * C::kStagesPerBox - stages;
         __syncwarp();
         if (lane == 0) {
-          if (grp == 0)
-            for (int i = 0; i < missing; ++i) dev::mbar_arrive(&rempty[(box0 + boxes - 1) % kRawBoxes]);
+          if ((cnt0 + stages - 1) % kGroups == grp)
+            for (int i = 0; i < missing; ++i) dev::mbar_arrive(&rempty[(box0 + boxes - 1) % C::kRawBoxes]);
           if (C::kE8m0) dev::mbar_arrive(&info[tile_no % kInfo]);
         }
       }
     }
   } else {
     // ------------------------------ promoters ------------------------------
-    dev::reg_alloc<kPromoterRegs>();
+    dev::reg_alloc<C::kPromoterRegs>();
     const int q = warp & 3, part = (warp - kFirstPromoter) >> 2;
     const int hc = a.bm / 2, c0 = part * hc;   // this thread's rows of the tile: c0 .. c0 + hc - 1
     const uint32_t d_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + C::kAccBase + c0;
-    uint32_t buf = 0, bpar = 0, unit_no = 0, tile_no = 0;
+    uint32_t buf = 0, bpar = 0, unit_no = 0, tile_no = 0, sb = 0, sb_par = 0;
     bool ok = true;
     uint64_t acc[CPT / 2];
     for (int t = blockIdx.y; ok && t < a.tiles; t += gridDim.y, ++tile_no) {
@@ -426,22 +460,21 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
       const int G = C::kBias ? a.K / a.gs : (C::kE8m0 ? a.K / 32 : 0);
       const uint8_t* srow = static_cast<const uint8_t*>(a.scales) + static_cast<size_t>(nc) * (C::kE8m0 ? G : 0);
       const bool vec = C::kE8m0 && G % 16 == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 15) == 0;
-      // affine: scale and bias two units ahead (a load from L2 takes longer than a unit)
+      // affine, scales that do not come in boxes: read one unit ahead
       const float* sp = static_cast<const float*>(a.scales) + static_cast<size_t>(nc) * (C::kBias ? G : 0);
       const float* bp = C::kBias ? a.biases + static_cast<size_t>(nc) * G : nullptr;
       const int units_per_group = C::kBias ? a.gs / a.pu : 1;
       int gi = C::kBias ? k_begin / a.gs : 0, gu = C::kBias ? (k_begin % a.gs) / a.pu : 0;   // group and unit of the next load
-      float s0 = 1.f, b0 = 0.f, s1 = 1.f, b1 = 0.f;
-      auto next_scale = [&](float& s, float& b) {
+      float s0 = 1.f, b0 = 0.f;
+      auto next_scale = [&]() {
         const int g = min(gi, G - 1);
-        s = __ldg(sp + g);
-        b = __ldg(bp + g);
+        s0 = __ldg(sp + g);
+        b0 = __ldg(bp + g);
         if (++gu == units_per_group) { gu = 0; ++gi; }
       };
-      if (C::kBias) {
-        next_scale(s0, b0);
-        next_scale(s1, b1);
-      }
+      const int units_per_box = C::kBias && a.sbox_k ? a.sbox_k / a.pu : 0;
+      int in_box = 0;
+      if (C::kBias && units_per_box == 0) next_scale();
       for (int u = 0; u < units; ++u, ++unit_no) {
         float s = 1.f;
         if (C::kE8m0) {
@@ -449,10 +482,22 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
           s = opapi::decode_e8m0(ref) * __uint_as_float(static_cast<uint32_t>(127 - C::kUp) << 23);
         }
         if (C::kBias) {
+          float b = b0;
           s = s0;
-          const uint64_t b2 = pack2(b0, b0);
-          s0 = s1; b0 = b1;
-          next_scale(s1, b1);
+          if (units_per_box) {
+            if (in_box == 0 && !wait_warp(&sfull[sb], sb_par, a.status, 108)) { ok = false; break; }
+            const uint8_t* at = smem + C::kOffS + sb * kSBoxBytes + (q * 32 + lane) * 16 + in_box / units_per_group * 4;
+            s = *reinterpret_cast<const float*>(at);
+            b = *reinterpret_cast<const float*>(at + BN * 16);
+            if (++in_box == units_per_box || u == units - 1) {
+              split::release_slot(&sempty[sb], __float_as_uint(s) ^ __float_as_uint(b), a.M < 0, lane);
+              in_box = 0;
+              if (++sb == kSBoxes) { sb = 0; sb_par ^= 1; }
+            }
+          } else {
+            next_scale();
+          }
+          const uint64_t b2 = pack2(b, b);
           // the bias's share first: it needs no accumulator
           if (!wait_warp(&info[unit_no % kInfo], (unit_no / kInfo) & 1, a.status, 120)) { ok = false; break; }
           const float* xs = xsum + (unit_no % kInfo) * C::kRows + c0;
@@ -471,19 +516,21 @@ op_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         dev::tc_fence_after();
         const uint64_t s2 = pack2(s, s);
         const uint32_t taddr = d_lane + buf * C::kRows;
+        constexpr int kLd = CPT == 96 ? 16 : 32;   // values in flight beside the sums, as registers allow
 #pragma unroll
-        for (int c = 0; c < CPT; c += 32) {
+        for (int c = 0; c < CPT; c += kLd) {
           if (c < hc) {
-            uint32_t r[32];
-            dev::tmem_ld_32x32(taddr + c, r);
+            uint32_t r[kLd];
+            if constexpr (kLd == 16) dev::tmem_ld_32x16(taddr + c, r);
+            else dev::tmem_ld_32x32(taddr + c, r);
             dev::tc_wait_ld();
-            if (c + 32 >= hc) {   // the last values are in registers: the buffer goes back
+            if (c + kLd >= hc) {   // the last values are in registers: the buffer goes back
               dev::tc_fence_before();
               __syncwarp();
               if (lane == 0) dev::mbar_arrive(&dempty[buf]);
             }
 #pragma unroll
-            for (int e = 0; e < 16; ++e)
+            for (int e = 0; e < kLd / 2; ++e)
               fma2(acc[c / 2 + e], s2, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
           }
         }
@@ -627,7 +674,15 @@ static Cut choose_cut(int fmt, int M, int N, int K, int pu, int blocks, Fn held)
   return best;
 }
 static int unit_k(int fmt, int gs) { return fmt >= kMxfp4 ? kUnitK : (gs % 64 == 0 ? 64 : 32); }
-static int slice_k(int fmt) { return fmt >= kMxfp4 ? kUnitK : (fmt == kAffine4 ? 256 : 128); }
+// k per box of affine scales (16 bytes of a column: four groups), where rows of them are made of such pieces
+static int scale_box_k(int fmt, int K, int gs, const void* scales, const void* biases) {
+  if (fmt >= kMxfp4 || !aligned(scales, 16) || !aligned(biases, 16)) return 0;
+  return gs <= 128 && 128 % gs == 0 && (K / gs) % 4 == 0 ? 4 * gs : 0;
+}
+static int slice_k(int fmt, int sbox_k) {
+  const int box_k = fmt >= kMxfp4 ? kUnitK : (fmt == kAffine4 ? 256 : 128);
+  return sbox_k > box_k ? sbox_k : box_k;
+}
 
 template <int FMT, int CPT>
 static int launch(Args a, const Cut& cut, cudaStream_t stream) {
@@ -640,6 +695,16 @@ static int launch(Args a, const Cut& cut, cudaStream_t stream) {
   if (int rc = make_tensor_map_2d(&xmap, a.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)a.M, (uint64_t)a.K, (uint64_t)a.K * 2,
                                   a.bm, 64, CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
+  CUtensorMap smap = wmap, bmap = wmap;   // placeholders where they are not used
+  if (a.sbox_k) {
+    const uint64_t G = static_cast<uint64_t>(a.K / a.gs);
+    if (int rc = make_tensor_map_2d(&smap, a.scales, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)a.N, G, G * 4, BN, 4,
+                                    CU_TENSOR_MAP_SWIZZLE_NONE))
+      return rc;
+    if (int rc = make_tensor_map_2d(&bmap, a.biases, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)a.N, G, G * 4, BN, 4,
+                                    CU_TENSOR_MAP_SWIZZLE_NONE))
+      return rc;
+  }
   static std::atomic<uint64_t> configured{0};
   auto kern = op_prefill_kernel<FMT, CPT>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), C::kSmem, configured)) return rc;
@@ -651,7 +716,7 @@ static int launch(Args a, const Cut& cut, cudaStream_t stream) {
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   split::set_attrs(cfg, attr, cut.ks);
-  QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, a));
+  QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, smap, bmap, a));
   return QMM_OK;
 }
 
@@ -700,7 +765,8 @@ int op_prefill_launch(int fmt, const void* x, const void* w, const void* scales,
   a.K = static_cast<int>(K);
   a.gs = static_cast<int>(gs);
   a.pu = unit_k(fmt, a.gs);
-  a.block_k = slice_k(fmt);
+  a.sbox_k = scale_box_k(fmt, a.K, a.gs, scales, biases);
+  a.block_k = slice_k(fmt, a.sbox_k);
   a.blocks = (a.K + a.block_k - 1) / a.block_k;
   a.status = device_status_word();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
