@@ -33,10 +33,9 @@ bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, int f32
 int opgemm_launch(int fmt, const void* x, const void* w, const void* scales, const float* biases, void* y, int64_t M, int64_t N,
                   int64_t K, int64_t gs, int f32, void* stream);
 
-// the same with f16 activations at prompt sizes: weights converted into TMEM
-bool op_prefill_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, const void* x, const void* w, const void* y);
-int op_prefill_launch(int fmt, const void* x, const void* w, const void* scales, const float* biases, void* y, int64_t M,
-                      int64_t N, int64_t K, int64_t gs, void* stream);
+// MX formats, f16 activations, prompt sizes: weights converted into TMEM
+bool mx_prefill(int mode, const void* x, const void* w, const void* scales, void* y, int64_t M, int64_t N, int64_t K,
+                void* stream, int* rc);
 
 namespace opapi {
 
@@ -554,8 +553,6 @@ int qmm_affine_matmul(const void* x, const void* w_packed, const float* scales, 
     return affine_ring_launch(bits, x, w_packed, scales, biases, y, M, N, K, group_size, stream);
   if (tcq::covers(M, N, K, bits, group_size, dtype, x, w_packed))
     return tcq::launch(bits, x, w_packed, scales, biases, y, M, N, K, group_size, stream);
-  if (dtype == QMM_F16 && op_prefill_covers(M, N, K, bits == 4 ? 0 : 1, group_size, x, w_packed, y))
-    return op_prefill_launch(bits == 4 ? 0 : 1, x, w_packed, scales, biases, y, M, N, K, group_size, stream);
   if (opgemm_covers(M, N, K, bits == 4 ? 0 : 1, group_size, dtype == QMM_F32, x, w_packed, y))
     return opgemm_launch(bits == 4 ? 0 : 1, x, w_packed, scales, biases, y, M, N, K, group_size, dtype == QMM_F32, stream);
   // rows of 16-byte words: the vectorised kernel
@@ -600,10 +597,10 @@ int qmm_mx_matmul(const void* x, const uint8_t* w_packed, const uint8_t* scales,
   static_assert(QMM_MXFP4 == 0 && QMM_MXFP8 == 1 && QMM_NVFP4 == 2, "mode numbering shared with the tensor-core kernel");
   if (mx_ring_covers(M, N, K, mode, dtype, x, w_packed, scales))   // decode-sized f16 problems: the tensor-core kernel
     return mx_ring_launch(mode, x, w_packed, scales, y, M, N, K, stream);
-  if (dtype == QMM_F16 && op_prefill_covers(M, N, K, 2 + mode, gs, x, w_packed, y))
-    return op_prefill_launch(2 + mode, x, w_packed, scales, nullptr, y, M, N, K, gs, stream);
-  if (opgemm_covers(M, N, K, 2 + mode, gs, dtype == QMM_F32, x, w_packed, y))
-    return opgemm_launch(2 + mode, x, w_packed, scales, nullptr, y, M, N, K, gs, dtype == QMM_F32, stream);
+  int rc = QMM_OK;
+  if (dtype == QMM_F16 && mx_prefill(mode, x, w_packed, scales, y, M, N, K, stream, &rc)) return rc;
+  if (dtype == QMM_F32 && opgemm_covers(M, N, K, 2 + mode, gs, 1, x, w_packed, y))
+    return opgemm_launch(2 + mode, x, w_packed, scales, nullptr, y, M, N, K, gs, 1, stream);
   if (aligned(w_packed, 16) && K % 32 == 0) {  // rows of 16-byte words: the vectorised kernel
     if (mode == QMM_MXFP4) {
       VMx<0> d{w_packed, scales, k};

@@ -1,5 +1,5 @@
-// Operator-API matmuls (weights [N, K], K contiguous) on the 5th-generation tensor cores: any number of rows,
-// f16 or f32 activations, all five weight formats.
+// Operator-API matmuls (weights [N, K], K contiguous) on the 5th-generation tensor cores: any number of rows, f32
+// activations and all five weight formats, f16 activations and the affine formats (the MX formats go to mx_prefill.cu).
 //
 //   y[m,n] = sum over groups g of  s[n,g] * sum_{k in g} x[m,k] c[n,k]  (+ b[n,g] * sum_{k in g} x[m,k])
 //
@@ -18,10 +18,9 @@
 // activations into their three terms, and sum the activations of a unit for the biases) and four to
 // sixteen promoters that drain the accumulators.
 //
-// Measured (four linears of a layer, before: one warp per four columns on CUDA cores): mxfp8, f16, M = 512, 4096 / 14336
-// wide 15.2 -> 0.86 ms; affine 4-bit, f32, M = 48, 2048 / 5632 wide 597 -> 103 us.  Bound by latency, not by a unit: a
-// stage takes 0.5-1 us through issuer, tensor core and promoter (the two MMAs of a 32-k group are too little work to hide
-// a commit and a TMEM read), 0.16 of the measured bf16 rate at best (mxfp8, f16, M = 512, 4096 x 28672).
+// Measured (four linears of a layer, before: one warp per four columns on CUDA cores): affine 4-bit, f32, M = 48, 2048 / 5632
+// wide 597 -> 103 us.  Bound by latency, not by a unit: a stage takes 0.9-1.3 us through workers, issuer, tensor core and
+// promoter.
 //
 // What the split cannot represent takes an exact path: a unit whose activations are not finite (inf times
 // code plus inf times bias is not what inf times scale * code + bias gives), or, for f32, lie outside 2^-100 .. 2^100, is computed by
@@ -463,64 +462,6 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     };
     // Scales come in boxes (one TMA copy for all promoters), else each promoter reads its lanes' values ahead.
     const int units_per_box = FMT != kNvfp4 && a.sbox_k ? a.sbox_k / a.pu : 0;
-    if constexpr ((FMT == kMxfp4 || FMT == kMxfp8) && !XF32) {
-      // Two units a stage and nothing but a scale to each: one wait, one look at the scales and one hand-back for both.
-      float nx[2] = {1.f, 1.f}, unused;
-      if (units_per_box == 0) {
-        load_scale(0, nx[0], unused);
-        load_scale(1, nx[1], unused);
-      }
-      int in_box = 0;
-      uint32_t sb = 0, sb_phase = 0, phase = 0;
-      for (int u = 0; u < units; u += 2) {
-        const int buf = u & (C::kAccBufs - 1);
-        const bool both = u + 1 < units;
-        float s0 = nx[0], s1 = nx[1];
-        if (units_per_box) {
-          if (in_box == 0 && !dev::mbar_wait_relaxed_warp(&sfull[sb], sb_phase, a.status, 101)) break;
-          const uint32_t two = *reinterpret_cast<const uint16_t*>(smem + C::kOffS + sb * kSBoxBytes + (q * 32 + lane) * 16 + in_box);
-          s0 = opapi::decode_e8m0(two & 0xFFu);
-          s1 = opapi::decode_e8m0(two >> 8);
-        } else {
-          load_scale(u + 2, nx[0], unused);
-          load_scale(u + 3, nx[1], unused);
-        }
-        if (!dev::mbar_wait_relaxed_warp(&tfull[buf + 1], phase, a.status, 100)) break;   // the stage's barrier, also for one unit
-        dev::tc_fence_after();
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
-        const uint64_t s02 = pack2(s0, s0), s12 = pack2(s1, s1);
-#pragma unroll
-        for (int c = 0; c < C::kCols; c += 16) {
-          uint32_t r[16];
-          dev::tmem_ld_32x16(taddr + c, r);
-          dev::tc_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            fma2(acc[c / 2 + e], s02, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
-          if (both) {
-            dev::tmem_ld_32x16(taddr + BM + c, r);
-            dev::tc_wait_ld();
-          }
-          if (c + 16 == C::kCols) {
-            dev::tc_fence_before();
-            __syncwarp();
-            if (lane < 2) dev::mbar_arrive(&tempty[buf + lane]);
-          }
-          if (both) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              fma2(acc[c / 2 + e], s12, pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
-          }
-        }
-        if (buf == C::kAccBufs - 2) phase ^= 1;
-        in_box += 2;
-        if (units_per_box && in_box == units_per_box) {
-          split::release_slot(&sempty[sb], __float_as_uint(s0) ^ __float_as_uint(s1), a.M < 0, lane);
-          in_box = 0;
-          if (++sb == kSBoxes) { sb = 0; sb_phase ^= 1; }
-        }
-      }
-    } else {
     float s_next = 1.f, b_next = 0.f;
     if (units_per_box == 0) load_scale(0, s_next, b_next);
     int in_box = 0, in_group = 0, comp = 0;   // unit of the box, unit of the group, group of the box
@@ -602,7 +543,6 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         in_box = comp = 0;
         if (++sb == kSBoxes) { sb = 0; sb_phase ^= 1; }
       }
-    }
     }
     // ---- this slice's results, [row][column], into the idle rings (after every warp is done with them)
     dev::tc_fence_before();
@@ -787,8 +727,10 @@ static int launch_fmt(const Args& a, int f32, cudaStream_t stream) {
     // a stage of 128 rows would need 64 KB for the three terms of the activations alone
     return a.M <= 32 ? launch<FMT, true, 32>(a, stream) : launch<FMT, true, 64>(a, stream);
   }
-  return a.M <= 32 ? launch<FMT, false, 32>(a, stream)
-                   : (a.M <= 64 ? launch<FMT, false, 64>(a, stream) : launch<FMT, false, 128>(a, stream));
+  if constexpr (FMT <= kAffine8)
+    return a.M <= 32 ? launch<FMT, false, 32>(a, stream)
+                     : (a.M <= 64 ? launch<FMT, false, 64>(a, stream) : launch<FMT, false, 128>(a, stream));
+  return set_error(QMM_ERR_UNSUPPORTED, "opgemm: MX formats take f32 activations here");
 }
 
 // Microseconds of a call, here and on the CUDA cores (one B200, calls of a graph on operands in L2; K and N from 64 to 4096,
@@ -811,7 +753,7 @@ static float gemm_us(int fmt, bool f32, int M, int N, int K, int gs) {
                                  [&](int ks) { return sms / ks > 0 ? sms / ks : 1; });
   return r.rounds * (kStart[i] + kStage[kind][f32 ? 3 + i : i] * r.stages);
 }
-static float cuda_core_us(int fmt, bool f32, int M, int N, int K) {
+float cuda_core_us(int fmt, bool f32, int M, int N, int K) {
   const bool wide = fmt == kAffine8 || fmt == kMxfp8;   // 8-bit codes take fewer instructions
   const float least = f32 ? (wide ? 6.5f : 10.4f) : (wide ? 5.6f : 8.6f);
   const float run = 3.f + K * (f32 ? (wide ? 0.0079f : 0.0089f) : (wide ? 0.0057f : 0.0056f));
