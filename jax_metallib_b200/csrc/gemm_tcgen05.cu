@@ -14,14 +14,16 @@
 //      epilogue warps (optional int32 store and/or float(acc) * row[m] * col[n]).
 //
 //  (2) w8a16: y[M,N] = bf16((x[M,K] @ float(w[K,N])) * scale[N]), bf16
-//      activations, int8 weights.  The weight tile is the 128-row MMA operand
-//      (MN-major: its 128 output channels are contiguous in memory), the
-//      activation tile the 256-column operand; a CTA runs two weight blocks
-//      against one activation tile (256 channels x 256 rows).  Warps: a TMA
+//      activations, int8 weights.  The weight tile is the 128-row MMA operand and goes
+//      into it through TMEM, the activation tile (up to 192 rows) is the other one; a CTA
+//      runs two weight blocks against one activation tile (256 channels x 192 rows).
+//      With the converted weights in shared memory (written, and read by the MMA) a 64-k
+//      stage of 256 x 256 moved 192 KB there in 1024 clocks of MMA, at 128 bytes a clock:
+//      0.66 of the MMA rate, as measured; now 104 KB in 768 clocks.  Warps: a TMA
 //      producer for activations, one for raw int8 weights, two MMA issuers and
-//      24 worker warps in three groups that take every third 64-k stage: a
-//      group reads the raw tile, converts it to bf16 (exactly) and writes the
-//      MMA's swizzled layout; when a tile's stages are done the same 24 warps
+//      16 worker warps in two groups that take every other 64-k stage: a
+//      group reads the raw tile (ldmatrix.trans pairs the k of a channel), converts it to
+//      bf16 (exactly) and stores it to TMEM; when a tile's stages are done the same warps
 //      drain its accumulators.  The accumulator holds the transposed tile
 //      (lane = output channel), so the per-channel scale is one register per
 //      thread.  Leftover tiles of the last round are cut into halves or
@@ -301,20 +303,16 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
 // ============================================================================
 namespace w8 {
 constexpr int BNW = 128;   // output channels per MMA (its M); a full tile has two such blocks
-constexpr int BMX = 256;   // activation rows per tile (MMA N)
-constexpr int BK = 64;     // k per TMA stage
-constexpr int BKS = 32;    // k per converted sub-block
-constexpr int kXStages = 3;    // activation ring, held until the MMAs that read a stage retire
-constexpr int kWStages = 4;    // raw-weight ring, held only until a stage is in the converters' registers
-constexpr int kCvtBufs = 4;    // converted sub-blocks between the converter warps and the MMA
+constexpr int kMaxRows = 192;   // activation rows per tile (MMA N), at most: two accumulators of 192 columns leave 128 for the weights
+constexpr int BK = 64;     // k per stage
+constexpr int kXStages = 4;    // activation ring, held until the MMAs that read a stage retire
+constexpr int kWStages = 6;    // raw-weight ring (a multiple of the converter groups), held only until a stage is in registers
 constexpr int kCvtWarps = 8;    // converter warps per group
-constexpr int kCvtGroups = 3;   // group g converts the stages with cnt % 3 == g
-constexpr int kCvtSlots = 2;    // converted stages in flight (two sub-block buffers each)
-// Warp roles: 0 TMA (activations), 1 MMA issue for channel block 0, 2-25 workers (convert the
-// stages of a tile, then drain its accumulators), 26 TMA (raw weights), 27 MMA issue for channel
-// block 1.  One thread needs ~85 cycles to issue a tcgen05.mma and about as much per wait and per
-// commit, about what the MMAs themselves take; two issuing threads (one per accumulator) leave the
-// tensor pipe as the limit.
+constexpr int kCvtGroups = 2;   // group g converts the stages with cnt % 2 == g
+constexpr int kCvtSlots = 2;    // converted stages in TMEM
+// Warp roles: 0 TMA (activations), 1 MMA issue for channel block 0, 2-17 workers (convert the
+// stages of a tile, then drain its accumulators), 18 TMA (raw weights), 19 MMA issue for channel
+// block 1.
 constexpr int kFirstCvtWarp = 2;
 constexpr int kWorkerWarps = kCvtGroups * kCvtWarps;
 constexpr int kWProducerWarp = kFirstCvtWarp + kWorkerWarps;
@@ -322,54 +320,49 @@ constexpr int kSecondMmaWarp = kWProducerWarp + 1;
 constexpr int kWarps = kSecondMmaWarp + 1;
 constexpr int kRawBlock = BK * BNW;               // 8 KB  int8 [k][128 n]
 constexpr int kRawBytes = 2 * kRawBlock;          // 16 KB: both channel blocks
-constexpr int kXBytes = BMX * BK * 2;             // 32 KB bf16 [m][k]
-constexpr int kCvtBlock = BKS * BNW * 2;          // 8 KB bf16: two 64-channel halves of [32 k][128 B]
-constexpr int kCvtBytes = 2 * kCvtBlock;          // 16 KB: both channel blocks
+constexpr int kXBytes = kMaxRows * BK * 2;        // 24 KB bf16 [m][k]
 constexpr int kRawBase = kXStages * kXBytes;                 // 96 KB
-constexpr int kCvtBase = kRawBase + kWStages * kRawBytes;    // 160 KB
-constexpr int kBarBase = kCvtBase + kCvtBufs * kCvtBytes;    // 224 KB
+constexpr int kBarBase = kRawBase + kWStages * kRawBytes;    // 192 KB
 constexpr int kThreads = kWarps * 32;
 constexpr int kSmemBytes = kBarBase + 256 + 1024;
+constexpr int kSlotCols = 2 * BK / 2;             // TMEM columns of a converted stage: both channel blocks, two k to a column
+constexpr int kAccBase = kCvtSlots * kSlotCols;   // first TMEM column of the accumulators
+static_assert(kAccBase + 2 * kMaxRows <= 512, "TMEM");
+static_assert(kWStages % kCvtGroups == 0, "a group has seen the phase ahead of the one that it waits for");
 constexpr int kPanelTiles = 8;  // most activation tiles swept together (fewer when K is long: a panel should stay in L2)
-// One "consumed" barrier per stage in a ring of 6 (a multiple of both the activation ring and the
-// two converted stage slots): the activation producer waits for stage cnt - 3, the converters for
+// One "consumed" barrier per stage in a ring: the activation producer waits for stage cnt - 4, the converters for
 // stage cnt - 2, and the issuing threads commit once per stage.
 constexpr int kConsumed = 6;
 
 
-// Eight int8 (one 8-byte read) -> eight bf16, exactly, in 16 instructions.
-// For a byte b (two's complement v): A = 0x4300 | (b & 0x7F) is the bf16
-// 128 + (b & 0x7F); C = 0xC300 | (b & 0x80) is -128 for v >= 0 and -256 for
-// v < 0; A + C = v, exact in bf16 (|v| <= 128 has 8 significant bits).  One
-// byte-permute spreads two bytes over the two halves of a register, two
-// logic ops build A and C for both, one packed add finishes the pair.  The MMA
-// needs both operands in one 16-bit format (an f16 weight operand against bf16
-// activations raises an illegal-instruction error on sm_100a), so the weights
-// follow the activations.
+// Two int8 -> two bf16, exactly, over 64.  `word` holds u = v + 128 in each byte: u in the low bits of a half reads as the bf16
+// u * 2^-133 (a subnormal up to 127, the first binade above), and one fused multiply-add makes u / 64 - 2 = v / 64 of it (|v| <=
+// 128 has 8 significant bits).  The epilogue multiplies by 64.
 __device__ __forceinline__ uint32_t convert2(uint32_t word, uint32_t selector) {
-  const uint32_t t = __byte_perm(word, 0u, selector);  // 0x00bb00aa
-  uint32_t a, c, r;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(a) : "r"(t), "r"(0x007F007Fu), "r"(0x43004300u));  // (t & m) | k
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(c) : "r"(t), "r"(0x00800080u), "r"(0xC300C300u));
-  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(c));
+  uint32_t r;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(__byte_perm(word, 0u, selector)), "r"(0x7F007F00u), "r"(0xC000C000u));
   return r;
 }
-__device__ __forceinline__ uint4 convert8(const uint2& in) {
-  return make_uint4(convert2(in.x, 0x4140), convert2(in.x, 0x4342), convert2(in.y, 0x4140), convert2(in.y, 0x4342));
+// 8 x 8 tiles of 16-bit units, transposed: a unit is one k (or one packed pair of k) of two neighbouring channels.
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
 }
 
-// The work of one launch.  A full tile is 256 channels x 256 rows: two channel
-// blocks share one activation tile, so a CTA stages 48 KB per 64 k for
-// 2 x 128 x 256 outputs.  CTA c takes tiles c, c + G, ... for `full_waves`
+// The work of one launch.  A full tile is 256 channels x `rows` rows: two channel
+// blocks share one activation tile, so a CTA stages up to 40 KB per 64 k for
+// 2 x 128 x 192 outputs.  CTA c takes tiles c, c + G, ... for `full_waves`
 // rounds; the tiles left over (fewer than G) are cut into `tail_div` parts each
-// (1: whole, 2: one channel block, 4: one channel block x 128 rows) and dealt
+// (1: whole, 2: one channel block, 4: one channel block x half of the rows) and dealt
 // round-robin, so that the last round costs 1 / tail_div of a tile.
 struct Sched {
   int tiles_n2, tiles_m, full_waves, tail_tiles, tail_div;
   int panel;  // activation tiles per panel
+  int rows;   // rows per tile, a multiple of 32
 };
 struct Work {
-  int tn2, tm;   // tile coordinates (256-channel, 256-row units)
+  int tn2, tm;   // tile coordinates (units of 256 channels, of `rows` rows)
   int h0, nh;    // channel blocks [h0, h0 + nh); nh == 0: nothing to do
   int m_off, m_cols;  // rows [m_off, m_off + m_cols) of the activation tile
 };
@@ -414,17 +407,17 @@ __device__ __forceinline__ bool get_work(const Sched& sc, int i, int M, int N, W
     if (len == div) len = 0;
   }
   tile_coords(tile, sc.tiles_m, sc.tiles_n2, sc.panel, w.tm, w.tn2);
-  w.h0 = 0; w.nh = 2; w.m_off = 0; w.m_cols = BMX;
+  w.h0 = 0; w.nh = 2; w.m_off = 0; w.m_cols = sc.rows;
   if (len != 0) {
     if (div == 2) { w.h0 = sub; w.nh = 1; }
     if (div == 4) {
       w.h0 = sub >> 1; w.nh = 1;
-      if (len == 1) { w.m_off = (sub & 1) * (BMX / 2); w.m_cols = BMX / 2; }
+      if (len == 1) { w.m_off = (sub & 1) * (sc.rows / 2); w.m_cols = sc.rows / 2; }
     }
   }
   const int blocks_left = (N - w.tn2 * 2 * BNW + BNW - 1) / BNW - w.h0;  // channel blocks that exist
   w.nh = max(0, min(w.nh, blocks_left));
-  if (w.tm * BMX + w.m_off >= M) w.nh = 0;
+  if (w.tm * sc.rows + w.m_off >= M) w.nh = 0;
   return true;
 }
 
@@ -435,18 +428,16 @@ struct GroupQuant {
   int packed;
 };
 
-// Four packed weights (the two k of two neighbouring channels, one byte per channel, low nibble =
-// even k) -> the bf16 pairs (q - z) * s of the even and of the odd k.  0x4300 | q is the bf16
-// 128 + q exactly, zz holds 128 + z, so the subtraction is exact and the product is rounded to
-// bf16 once: bit for bit what the StableHLO chain convert -> subtract -> multiply computes in bf16.
-__device__ __forceinline__ void dequant4(uint32_t t, uint32_t zz, uint32_t ss, uint32_t& even_k, uint32_t& odd_k) {
-  uint32_t lo, hi;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(lo) : "r"(t), "r"(0x000F000Fu), "r"(0x43004300u));
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(hi) : "r"(t >> 4), "r"(0x000F000Fu), "r"(0x43004300u));
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(lo), "r"(zz));
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"(hi), "r"(zz));
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(even_k) : "r"(lo), "r"(ss));
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(odd_k) : "r"(hi), "r"(ss));
+// One packed byte (two k of one channel, low nibble = even k) -> the bf16 pair (q - z) * s.  `w` holds the byte at
+// position BYTE, `w4` is w >> 4.  0x4300 | q is the bf16 128 + q exactly, zz holds 128 + z twice, so the subtraction is exact
+// and the product is rounded to bf16 once: bit for bit what the StableHLO chain convert -> subtract -> multiply computes in bf16.
+template <int BYTE>
+__device__ __forceinline__ uint32_t dequant2(uint32_t w, uint32_t w4, uint32_t zz, uint32_t ss) {
+  uint32_t t;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(t) : "r"(__byte_perm(w, w4, BYTE | (4 + BYTE) << 8)), "r"(0x000F000Fu), "r"(0x43004300u));
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(t), "r"(zz));
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(t), "r"(ss));
+  return t;
 }
 
 // WBITS = 8: int8 weights [K, N], per-channel f32 scale applied in the epilogue.
@@ -456,7 +447,7 @@ template <int WBITS>
 __global__ void __launch_bounds__(kThreads, 1)
 w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
              const float* __restrict__ scale, const GroupQuant gq, uint16_t* __restrict__ y, int M, int N, int K,
-             long long ldy, uint32_t idesc256, uint32_t idesc128, const Sched sc, uint32_t flags,
+             long long ldy, uint32_t idesc_full, uint32_t idesc_half, const Sched sc, uint32_t flags,
              uint32_t* signal, uint32_t* arrive, int* status) {
   // a raw stage holds 64 k of both channel blocks: 64 byte-rows of int8, 32 of packed int4
   constexpr int kRawRows = (WBITS == 8) ? BK : BK / 2;
@@ -508,8 +499,8 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
   }
   const bool mc_store = (flags & QMM_GEMM_STORE_MULTIMEM) != 0;
 
-  // Stage `cnt` (counted over the whole launch) uses activation slot cnt % 3,
-  // raw-weight slot cnt % 4 and converted buffers 2 (cnt % 2) and 2 (cnt % 2) + 1.
+  // Stage `cnt` (counted over the whole launch) uses activation slot cnt % 4,
+  // raw-weight slot cnt % 6 and the converted stage cnt % 2 in TMEM.
   if (warp == 0) {
     // ------------------------ TMA producer: activations --------------------
     if (lane == 0) {
@@ -525,8 +516,8 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
             const unsigned prev = cnt - kXStages;
             if (!dev::mbar_wait(&consumed[prev % kConsumed], (prev / kConsumed) & 1, status, 21)) { ok = false; break; }
           }
-          dev::mbar_expect_tx(&xfull[xs], kXBytes);
-          dev::tma_load_2d(smem + xs * kXBytes, &xmap, &xfull[xs], kb * BK, w.tm * BMX);
+          dev::mbar_expect_tx(&xfull[xs], sc.rows * BK * 2);
+          dev::tma_load_2d(smem + xs * kXBytes, &xmap, &xfull[xs], kb * BK, w.tm * sc.rows);
         }
       }
     }
@@ -540,7 +531,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       for (int i = 0; ok && get_work(sc, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
         for (int kb = 0; kb < kblocks; ++kb, ++cnt) {
-          const int ws = cnt & (kWStages - 1);
+          const int ws = cnt % kWStages;
           if (!dev::mbar_wait(&wempty[ws], ((cnt / kWStages) & 1) ^ 1, status, 20)) { ok = false; break; }
           uint8_t* raw = smem + kRawBase + ws * kRawBytes;
           dev::mbar_expect_tx(&wfull[ws], w.nh * kRawBlockW);
@@ -560,34 +551,35 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       const int me = (warp == 1) ? 0 : 1;
       // descriptor halves: the high half is constant, the low half carries the start address
       constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (kSwizzle128 << 29);  // SBO, version, swizzle
-      constexpr uint32_t kAStepK = (16 * 128) >> 4, kAStepH = kCvtBlock >> 4, kAStepBuf = kCvtBytes >> 4;
       constexpr uint32_t kBStepK = 32 >> 4, kBStepStage = kXBytes >> 4;
-      const uint32_t a_lo0 = (((dev::smem_u32(smem + kCvtBase) >> 4) & 0x3FFF) | (((BKS * 128u) >> 4) << 16)) +
-                             me * kAStepH;
+      const uint32_t a_t0 = tmem_base + me * (BK / 2);
       const uint32_t b_lo0 = ((dev::smem_u32(smem) >> 4) & 0x3FFF) | ((16u >> 4) << 16);
-      const uint32_t d = tmem_base + me * BMX;
+      const uint32_t d = tmem_base + kAccBase + me * kMaxRows;
       uint32_t g = 0, gpar = 0;   // converted-stage slot and the parity of its use
       uint32_t xs = 0;            // activation slot
       uint32_t c6 = 0;            // consumed-ring index
       int items = 0;
-      bool ok = true;
+      bool ok = true, ready = false;
       Work w;
       for (int i = 0; ok && get_work(sc, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
         if (!dev::mbar_wait(tempty, (items & 1) ^ 1, status, 22)) break;
         dev::tc_fence_after();
-        const uint32_t idesc = (w.m_cols == BMX) ? idesc256 : idesc128;
+        const uint32_t idesc = (w.m_cols == sc.rows) ? idesc_full : idesc_half;
         const uint32_t b_item = b_lo0 + ((w.m_off * 128) >> 4);
         const uint32_t mine = (me >= w.h0) && (me < w.h0 + w.nh);
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!dev::mbar_wait(&sfull[g], gpar, status, 23)) { ok = false; break; }
+          // whether the next stage is ready is asked while this one's MMAs are still being issued: behind them a question
+          // waits for its turn
+          if (!ready && !dev::mbar_wait(&sfull[g], gpar, status, 23)) { ok = false; break; }
           dev::tc_fence_after();
-          const uint32_t a_c = a_lo0 + g * (2 * kAStepBuf);
+          const uint32_t a_c = a_t0 + g * kSlotCols;   // 16 k: eight columns
           const uint32_t b_s = b_item + xs * kBStepStage;
-          dev::umma_f16_lh_if(mine, d, a_c, kDescHi, b_s, kDescHi, idesc, kb != 0);
-          dev::umma_f16_lh_if(mine, d, a_c + kAStepK, kDescHi, b_s + kBStepK, kDescHi, idesc, 1);
-          dev::umma_f16_lh_if(mine, d, a_c + kAStepBuf, kDescHi, b_s + 2 * kBStepK, kDescHi, idesc, 1);
-          dev::umma_f16_lh_if(mine, d, a_c + kAStepBuf + kAStepK, kDescHi, b_s + 3 * kBStepK, kDescHi, idesc, 1);
+          dev::umma_f16_ts_if(mine, d, a_c, b_s, kDescHi, idesc, kb != 0);
+          dev::umma_f16_ts_if(mine, d, a_c + 8, b_s + kBStepK, kDescHi, idesc, 1);
+          dev::umma_f16_ts_if(mine, d, a_c + 16, b_s + 2 * kBStepK, kDescHi, idesc, 1);
+          ready = dev::mbar_test(&sfull[g ^ 1], gpar ^ g);
+          dev::umma_f16_ts_if(mine, d, a_c + 24, b_s + 3 * kBStepK, kDescHi, idesc, 1);
           dev::tc_commit(&consumed[c6]);  // second arrival: the other issuer
           gpar ^= g;  // the parity flips after slot 1's stage
           g ^= 1;
@@ -600,190 +592,155 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     }
   } else {
     // ------------------------------ workers --------------------------------
-    // Conversion: a half-warp reads one 128-byte raw row, 8 bytes per lane (conflict-free in any
-    // permutation); each lane writes the 16-byte bf16 chunk it made, so a quarter-warp store
-    // covers the eight chunks of one 128-byte row of one 64-channel half: conflict-free as well,
-    // with no divergence.  One warp needs ~1000 cycles for its share of a stage (dependent ALU
-    // chains), as long as the MMAs of the stage take, so three groups of eight warps take every
-    // third stage.  The raw slot is handed back as soon as its bytes are in registers.
-    // Epilogue: when the tile's stages are converted the same 24 warps drain its accumulators
-    // (warp & 3 selects the 32 TMEM lanes = channels a warp may read; the six warps of a lane
+    // Conversion: a warp takes one lane quarter (32 channels) of one channel block, all 64 k of a stage.  ldmatrix.trans
+    // on 16-bit units leaves, for two neighbouring channels, two k (int8) or two packed pairs of k (int4) in a register;
+    // converted, they have the layout of the 16-lane TMEM stores, with channel 2 i in lane i and channel 2 i + 1 in lane
+    // i + 8 of the 16.  Two groups of eight warps take every other stage.
+    // Epilogue: when the tile's stages are converted the same 16 warps drain its accumulators
+    // (warp & 3 selects the 32 TMEM lanes = channels a warp may read; the four warps of a lane
     // quarter share the 32-row chunks).
     const int o = warp - kFirstCvtWarp;
     const int grp = o / kCvtWarps, cw = o % kCvtWarps;
     const int q = warp & 3, esub = o >> 2;
-    const int piece = lane & 15;         // 8 channels: [8*piece, 8*piece+8)
-    const int rsub = lane >> 4;          // row within a pair
+    const int hh = cw >> 2;              // channel block of the item that this warp converts
+    const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     unsigned cnt = 0;  // stages since the start of the launch
-    int r3 = 0;        // cnt % 3
+    int turn = 0;      // cnt % kCvtGroups
     int items = 0;
     bool ok = true;
     Work w;
     for (int i = 0; ok && get_work(sc, i, M, N, w); ++i) {
       if (w.nh == 0) continue;
-      for (int kb = 0; kb < kblocks; ++kb, ++cnt, r3 = (r3 == 2) ? 0 : r3 + 1) {
-        if (r3 != grp) continue;
-        const int ws = cnt & (kWStages - 1);
-        const int slot = cnt & 1, c0 = 2 * slot;  // the stage's two converted buffers
-        const uint8_t* raw = smem + kRawBase + ws * kRawBytes;
-        if constexpr (WBITS == 4) {
-          // ---- packed int4: a lane owns 8 channels of each channel block; a byte-row of the raw
-          // tile (two k per byte) becomes two k-rows of the converted tile.  Scales and zero points
-          // of the stage's 128-k group are fetched before the wait for the weights.
-          const int grp_q = kb >> 1;
-          uint4 sv[2];
-          uint2 zv[2];
+      const int h = w.h0 + hh;
+      const bool mine = hh < w.nh;
+      uint32_t sv_next[2] = {0u, 0u}, zv_next[2] = {0u, 0u};
+      auto load_scales = [&](int kb, int h) {
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            sv[hh] = make_uint4(0, 0, 0, 0);
-            zv[hh] = make_uint2(0, 0);
-            if (hh < w.nh) {
-              const long long n0 = static_cast<long long>(w.tn2 * 2 + w.h0 + hh) * BNW + piece * 8;
-              sv[hh] = __ldg(reinterpret_cast<const uint4*>(gq.scales + static_cast<long long>(grp_q) * N + n0));
-              if (gq.packed) zv[hh].x = __ldg(reinterpret_cast<const uint32_t*>(gq.zeros + (static_cast<long long>(grp_q) * N + n0) / 2));
-              else zv[hh] = __ldg(reinterpret_cast<const uint2*>(gq.zeros + static_cast<long long>(grp_q) * N + n0));
-            }
-          }
-          if (!dev::mbar_wait_warp(&wfull[ws], (cnt / kWStages) & 1, status, 26)) { ok = false; break; }
-          uint2 in[4];  // [sub-block][channel block]
-#pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            const int sb = p >> 1, hh = p & 1;
-            const int brow = sb * (BKS / 2) + cw * 2 + rsub;  // byte-row 0..31 of the stage
-            in[p] = make_uint2(0, 0);
-            if (hh < w.nh)
-              in[p] = *reinterpret_cast<const uint2*>(raw + (w.h0 + hh) * kRawBlockW + brow * 128 +
-                                                      (((piece >> 1) ^ (brow & 7)) << 4) + ((piece & 1) << 3));
-          }
-          __syncwarp();
-          if (lane == 0) dev::mbar_arrive(&wempty[ws]);  // every raw byte of the stage is in registers
-          bool waited = false;
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            if (hh >= w.nh) continue;
-            // 128 + z and s of the lane's four channel pairs
-            uint32_t zz[4], ss[4] = {sv[hh].x, sv[hh].y, sv[hh].z, sv[hh].w};
-            if (gq.packed) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint32_t b = (zv[hh].x >> (8 * j)) & 0xFFu;  // channels 2j (low nibble), 2j+1 (high)
-                zz[j] = 0x43004300u | (b & 0xFu) | ((b >> 4) << 16);
-              }
-            } else {
-              zz[0] = __byte_perm(zv[hh].x, 0x43004300u, 0x7150);
-              zz[1] = __byte_perm(zv[hh].x, 0x43004300u, 0x7352);
-              zz[2] = __byte_perm(zv[hh].y, 0x43004300u, 0x7150);
-              zz[3] = __byte_perm(zv[hh].y, 0x43004300u, 0x7352);
-            }
-#pragma unroll
-            for (int sb = 0; sb < 2; ++sb) {
-              const uint2 v = in[sb * 2 + hh];
-              uint4 ev, od;
-              dequant4(__byte_perm(v.x, 0u, 0x4140), zz[0], ss[0], ev.x, od.x);
-              dequant4(__byte_perm(v.x, 0u, 0x4342), zz[1], ss[1], ev.y, od.y);
-              dequant4(__byte_perm(v.y, 0u, 0x4140), zz[2], ss[2], ev.z, od.z);
-              dequant4(__byte_perm(v.y, 0u, 0x4342), zz[3], ss[3], ev.w, od.w);
-              if (!waited) {
-                waited = true;
-                if (cnt >= 2) {  // the MMAs of the stage that used these buffers before must have retired
-                  const unsigned prev = cnt - 2;
-                  if (!dev::mbar_wait_warp(&consumed[prev % kConsumed], (prev / kConsumed) & 1, status, 27)) ok = false;
-                }
-              }
-              if (ok) {
-                uint8_t* cvt = smem + kCvtBase + (c0 + sb) * kCvtBytes + (w.h0 + hh) * kCvtBlock +
-                               (piece >> 3) * (BKS * 128);
-                const int r = 2 * (cw * 2 + rsub);  // k-row of the even k inside the 32-k sub-block
-                *reinterpret_cast<uint4*>(cvt + r * 128 + (((piece & 7) ^ (r & 7)) << 4)) = ev;
-                *reinterpret_cast<uint4*>(cvt + (r + 1) * 128 + (((piece & 7) ^ ((r + 1) & 7)) << 4)) = od;
-              }
-            }
-          }
-          if (!ok) break;
-        } else {
-        if (!dev::mbar_wait_warp(&wfull[ws], (cnt / kWStages) & 1, status, 26)) { ok = false; break; }
-        // tasks of this warp: per sub-block and channel block 16 row pairs, two per warp
-        uint2 in[8];
-#pragma unroll
-        for (int p = 0; p < 8; ++p) {
-          const int sb = p >> 2, hh = (p >> 1) & 1;  // sub-block; 0: first block of the item, 1: second
-          const int r = ((p & 1) * kCvtWarps + cw) * 2 + rsub;  // row 0..31 of the sub-block
-          const int krow = sb * BKS + r;
-          if (hh < w.nh)
-            in[p] = *reinterpret_cast<const uint2*>(raw + (w.h0 + hh) * kRawBlockW + krow * 128 +
-                                                    (((piece >> 1) ^ (krow & 7)) << 4) + ((piece & 1) << 3));
+        for (int c = 0; c < 2; ++c) {
+          const long long at = static_cast<long long>(kb >> 1) * N + (w.tn2 * 2 + h) * BNW + q * 32 + c * 16 + 2 * (lane >> 2);
+          sv_next[c] = __ldg(reinterpret_cast<const uint32_t*>(gq.scales + at));
+          zv_next[c] = gq.packed ? __ldg(gq.zeros + at / 2) : __ldg(reinterpret_cast<const uint16_t*>(gq.zeros + at));
         }
-        // sub-block 0 is converted before the wait for its buffers, sub-block 1 after its stores
-        uint4 out[4];
+      };
+      if (WBITS == 4 && mine) {
+        const int first = (grp + kCvtGroups - turn) % kCvtGroups;   // the group's first stage of the item
+        if (first < kblocks) load_scales(first, h);
+      }
+      for (int kb = 0; kb < kblocks; ++kb, ++cnt, turn = (turn == kCvtGroups - 1) ? 0 : turn + 1) {
+        if (turn != grp) continue;
+        const int ws = cnt % kWStages;
+        const uint32_t raw = dev::smem_u32(smem + kRawBase + ws * kRawBytes + h * kRawBlockW) + lane * 128;
+        const uint32_t a_slot = a_lane + (cnt & 1) * kSlotCols + h * (BK / 2);
+        // scales and zero points of the stage's 128-k group and this lane's two channel pairs, read one stage of the group's ahead
+        uint32_t sv[2] = {sv_next[0], sv_next[1]}, zv[2] = {zv_next[0], zv_next[1]};
+        if (WBITS == 4 && mine && kb + kCvtGroups < kblocks) load_scales(kb + kCvtGroups, h);
+        if (!dev::mbar_wait_warp(&wfull[ws], (cnt / kWStages) & 1, status, 26)) { ok = false; break; }
+        // 16 channels x 64 k -> 16 registers
+        auto convert = [&](int c, uint32_t (&out)[16]) {
+          const uint32_t at = raw + (((q * 2 + c) ^ (lane & 7)) << 4);
+          if (WBITS == 4) {
+            uint32_t in[4];
+            ldmatrix_x4_trans(at, in);
+            const uint32_t s0 = __byte_perm(sv[c], 0u, 0x1010), s1 = __byte_perm(sv[c], 0u, 0x3232);
+            // the two zero points: nibbles of a byte, or two bytes
+            const uint32_t z0 = 0x43004300u | (gq.packed ? (zv[c] & 0xFu) * 0x10001u : __byte_perm(zv[c], 0u, 0x4040));
+            const uint32_t z1 = 0x43004300u | (gq.packed ? (zv[c] >> 4) * 0x10001u : __byte_perm(zv[c], 0u, 0x4141));
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
-          if ((p >> 1) < w.nh) out[p] = convert8(in[p]);
-        if (cnt >= 2) {  // the MMAs of the stage that used these buffers before must have retired
+            for (int m = 0; m < 4; ++m) {
+              const uint32_t v = in[m], v4 = in[m] >> 4;
+              out[4 * m] = dequant2<0>(v, v4, z0, s0);
+              out[4 * m + 1] = dequant2<2>(v, v4, z0, s0);
+              out[4 * m + 2] = dequant2<1>(v, v4, z1, s1);
+              out[4 * m + 3] = dequant2<3>(v, v4, z1, s1);
+            }
+          } else {
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              uint32_t in[4];
+              ldmatrix_x4_trans(at + g * 32 * 128, in);
+#pragma unroll
+              for (int m = 0; m < 4; ++m) {
+                const uint32_t u = in[m] ^ 0x80808080u;
+                out[8 * g + 2 * m] = convert2(u, 0x4240);
+                out[8 * g + 2 * m + 1] = convert2(u, 0x4341);
+              }
+            }
+          }
+        };
+        auto store = [&](int c, const uint32_t (&out)[16]) {
+          if (WBITS == 4) dev::tmem_st_16x256b_x4(a_slot + (static_cast<uint32_t>(c * 16) << 16), out);
+          else dev::tmem_st_16x128b_x8(a_slot + (static_cast<uint32_t>(c * 16) << 16), out);
+        };
+        // Everything is converted before the wait for the slot: from the end of the MMAs that read it to the start of those
+        // that read it next there are only two stores to TMEM.
+        uint32_t out[2][16];
+        if (mine) {
+          convert(0, out[0]);
+          convert(1, out[1]);
+        }
+        // the issuing threads wait only for this group: make sure the activations are there too
+        if (!dev::mbar_wait_warp(&xfull[cnt % kXStages], (cnt / kXStages) & 1, status, 28)) { ok = false; break; }
+        if (cnt >= 2) {  // the MMAs of the stage that used the slot before must have retired
           const unsigned prev = cnt - 2;
           if (!dev::mbar_wait_warp(&consumed[prev % kConsumed], (prev / kConsumed) & 1, status, 27)) { ok = false; break; }
+          dev::tc_fence_after();
         }
-#pragma unroll
-        for (int sb = 0; sb < 2; ++sb) {
-          uint8_t* cvt = smem + kCvtBase + (c0 + sb) * kCvtBytes;
-#pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            const int hh = p >> 1;
-            const int r = ((p & 1) * kCvtWarps + cw) * 2 + rsub;
-            if (hh < w.nh)
-              *reinterpret_cast<uint4*>(cvt + (w.h0 + hh) * kCvtBlock + (piece >> 3) * (BKS * 128) + r * 128 +
-                                        (((piece & 7) ^ (r & 7)) << 4)) = out[p];
-          }
-          if (sb == 0) {
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-              if ((p >> 1) < w.nh) out[p] = convert8(in[4 + p]);
-            // every raw byte of the stage is in registers: hand the slot back
-            __syncwarp();
-            if (lane == 0) dev::mbar_arrive(&wempty[ws]);
-          }
+        if (mine) {
+          store(0, out[0]);
+          store(1, out[1]);
+          dev::tc_wait_st();
         }
-        }
-        dev::fence_proxy_async();
-        // the issuing threads wait only for this barrier: make sure the activations are there too
-        if (!dev::mbar_wait_warp(&xfull[cnt % kXStages], (cnt / kXStages) & 1, status, 28)) { ok = false; break; }
+        dev::tc_fence_before();
         __syncwarp();
-        if (lane == 0) dev::mbar_arrive(&sfull[slot]);
+        if (lane == 0) {
+          dev::mbar_arrive(&sfull[cnt & 1]);
+          dev::mbar_arrive(&wempty[ws]);   // the raw bytes went through registers into TMEM
+        }
       }
       if (!ok) break;
       // ---- epilogue of this item
       if (!dev::mbar_wait_relaxed_warp(tfull, items & 1, status, 25)) break;
       dev::tc_fence_after();
-      const int chunks = w.m_cols / 32;
+      const int chunks = (w.m_cols + 31) / 32;
+      const int m_end = min(M, w.tm * sc.rows + w.m_off + w.m_cols);
 #pragma unroll 1
       for (int idx = esub; idx < w.nh * chunks; idx += kWorkerWarps / 4) {
         const int h = w.h0 + idx / chunks, ch = idx % chunks;
-        const int n = (w.tn2 * 2 + h) * BNW + q * 32 + lane;  // this thread's output channel
+        // this thread's output channel: of 16 lanes, the first eight hold the even ones
+        const int n = (w.tn2 * 2 + h) * BNW + q * 32 + (lane & 16) + 2 * (lane & 7) + ((lane >> 3) & 1);
         const float scl = (WBITS == 4) ? 1.f : ((n < N) ? __ldg(scale + n) : 0.f);
         uint32_t r[32];
-        dev::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + h * BMX + ch * 32, r);
+        dev::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + kAccBase + h * kMaxRows + ch * 32, r);
         dev::tc_wait_ld();
-        const int m0 = w.tm * BMX + w.m_off + ch * 32;
-        // pair neighbouring channels so that every lane stores 4 bytes: even
-        // lanes write rows m0+2j, odd lanes rows m0+2j+1
+        if (idx + kWorkerWarps / 4 >= w.nh * chunks) {   // the last values are in registers: the next item may start
+          dev::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) dev::mbar_arrive(tempty);
+        }
+        const int m0 = w.tm * sc.rows + w.m_off + ch * 32;
+        // pair neighbouring channels so that every lane stores 4 bytes: lanes of the
+        // even channels write rows m0+2j, those of the odd ones rows m0+2j+1
+        const bool odd = (lane & 8) != 0;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const float a = __uint_as_float(r[2 * j]) * scl;
-          const float b = __uint_as_float(r[2 * j + 1]) * scl;
-          const float send = (lane & 1) ? a : b;
-          const float got = __shfl_xor_sync(0xFFFFFFFFu, send, 1);
-          const int m = m0 + 2 * j + (lane & 1);
-          const uint32_t packed = (lane & 1) ? dev::pack_bf16x2(got, b) : dev::pack_bf16x2(a, got);
+          const float a = (WBITS == 8 ? 64.f * __uint_as_float(r[2 * j]) : __uint_as_float(r[2 * j])) * scl;
+          const float b = (WBITS == 8 ? 64.f * __uint_as_float(r[2 * j + 1]) : __uint_as_float(r[2 * j + 1])) * scl;
+          const float send = odd ? a : b;
+          const float got = __shfl_xor_sync(0xFFFFFFFFu, send, 8);
+          const int m = m0 + 2 * j + odd;
+          const uint32_t packed = odd ? dev::pack_bf16x2(got, b) : dev::pack_bf16x2(a, got);
           const int n_even = n & ~1;
-          if (m < M && n_even < N) {
+          if (m < m_end && n_even < N) {
             uint16_t* dst = y + static_cast<size_t>(m) * ldy + n_even;
             if (mc_store) dev::multimem_st_b32(dst, packed);  // the same offset of every rank's buffer
             else *reinterpret_cast<uint32_t*>(dst) = packed;
           }
         }
       }
-      dev::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) dev::mbar_arrive(tempty);
+      if (esub >= w.nh * chunks) {   // a warp without a share
+        __syncwarp();
+        if (lane == 0) dev::mbar_arrive(tempty);
+      }
       ++items;
     }
   }
@@ -853,59 +810,80 @@ int i8gemm_tcgen05(const void* a, const void* b, int32_t* acc, const float* row_
   return QMM_OK;
 }
 
+// How M x N is cut into tiles for `sms` CTAs: rows per tile (as few tiles as there may be, or up to three more, of equal
+// height) and the parts of the tiles that are left after the last full round.  Parts pay where each CTA has one at most.
+// The costs are a fit to 600 calls of a graph (M 64 to 3000, K 1024 to 14336, N 1536 to 28672, every cut: 4 to 6 % off in the
+// mean): microseconds per 64 k of a whole tile and of one channel block, with a floor (the chain converter - MMA - converter of
+// two stages in TMEM) and a slope per row, and per piece for its first stages and its results.  What they choose is 0.2 %
+// slower than the best cut in the mean (4096 x 4096, M = 777, int4: 47 us; cut in quarters, which cost no fewer clocks, 72).
+static tc::w8::Sched schedule(int64_t M, int64_t N, int64_t K, int wbits, int sms) {
+  using namespace tc::w8;
+  struct Cost { float floor, row, piece; };
+  static constexpr Cost kWhole[2] = {{0.43f, 0.0030f, 6.6f}, {0.59f, 0.0033f, 5.9f}};   // int8, int4
+  static constexpr Cost kBlock[2] = {{0.39f, 0.0022f, 5.0f}, {0.48f, 0.00265f, 4.8f}};
+  const float stages = static_cast<float>((K + BK - 1) / BK);
+  auto us = [&](const Cost& c, int rows) { return (rows * c.row > c.floor ? rows * c.row : c.floor) * stages + c.piece; };
+  Sched best = {};
+  float best_cost = -1.f;
+  const int least = static_cast<int>((M + kMaxRows - 1) / kMaxRows);
+  for (int tiles_m = least; tiles_m <= least + 3; ++tiles_m) {
+    Sched sc = {};
+    sc.tiles_n2 = static_cast<int>((N + 2 * BNW - 1) / (2 * BNW));
+    sc.rows = static_cast<int>(((M + tiles_m - 1) / tiles_m + 31) / 32 * 32);
+    sc.tiles_m = static_cast<int>((M + sc.rows - 1) / sc.rows);
+    const int tiles = sc.tiles_n2 * sc.tiles_m;
+    sc.full_waves = tiles / sms;
+    sc.tail_tiles = tiles - sc.full_waves * sms;
+    // a panel of activation tiles (K bf16 a row) should fit in half of L2 (measured at K = 28672, N = 8192, tiles of 256 rows:
+    // panels of 8 / 4 / 3 / 2 tiles give 1180 / 1218 / 1149 / 1134 TFLOP/s)
+    const long long tile_bytes = 2ll * sc.rows * K;
+    const long long pt = (64ll << 20) / (tile_bytes > 0 ? tile_bytes : 1);
+    sc.panel = static_cast<int>(pt < 2 ? 2 : (pt > kPanelTiles ? kPanelTiles : pt));
+    const float whole = us(kWhole[wbits == 4], sc.rows);
+    for (sc.tail_div = 1; sc.tail_div <= 4; sc.tail_div *= 2) {
+      if (sc.tail_div > 1 && (sc.tail_tiles == 0 || sc.tail_tiles * sc.tail_div > sms)) break;
+      const float tail = sc.tail_tiles == 0 ? 0.f
+                         : sc.tail_div == 1 ? whole
+                                            : us(kBlock[wbits == 4], sc.tail_div == 2 ? sc.rows : sc.rows / 2);
+      const float cost = sc.full_waves * whole + tail;
+      if (best_cost < 0.f || cost < best_cost) {
+        best_cost = cost;
+        best = sc;
+      }
+    }
+  }
+  return best;
+}
+
 // Shared launch path of the weight-only GEMMs (int8 per-channel, int4 group-wise).
 template <int WBITS>
 static int launch_weight_only(const uint16_t* x, const void* w, const float* scale, const tc::w8::GroupQuant& gq,
                               uint16_t* y, int64_t M, int64_t N, int64_t K, int64_t ldy, uint32_t flags,
                               uint32_t* signal, uint32_t* arrive, cudaStream_t stream) {
   using namespace tc::w8;
+  const int sms = gemm_ctas();  // persistent CTAs of this launch
+  const Sched sc = schedule(M, N, K, WBITS, sms);
   CUtensorMap wmap, xmap;
   constexpr int kRawRows = (WBITS == 8) ? BK : BK / 2;
   if (int rc = make_tensor_map_2d(&wmap, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)(WBITS == 8 ? K : K / 2),
                                   (uint64_t)N, (uint64_t)N, kRawRows, BNW, CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
   if (int rc = make_tensor_map_2d(&xmap, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M,
-                                  (uint64_t)K, (uint64_t)K * 2, BMX, BK, CU_TENSOR_MAP_SWIZZLE_128B))
+                                  (uint64_t)K, (uint64_t)K * 2, sc.rows, BK, CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
   static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
   auto kern = w8a16_kernel<WBITS>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes, configured)) return rc;
-  // operand "a" of the MMA = weights (bf16, MN-major), "b" = activations (bf16, K-major)
-  const uint32_t idesc256 = dev::make_idesc(/*c=f32*/ 1, /*bf16*/ 1, /*bf16*/ 1,
-                                            /*a MN-major*/ 1, /*b K-major*/ 0, BNW, BMX);
-  const uint32_t idesc128 = dev::make_idesc(1, 1, 1, 1, 0, BNW, BMX / 2);
-  Sched sc;
-  sc.tiles_n2 = static_cast<int>((N + 2 * BNW - 1) / (2 * BNW));
-  sc.tiles_m = static_cast<int>((M + BMX - 1) / BMX);
-  const int tiles = sc.tiles_n2 * sc.tiles_m;
-  {
-    // a panel of activation tiles (256 rows x K bf16 each) should fit in half of L2 (measured at
-    // K = 28672, N = 8192: panels of 8 / 4 / 3 / 2 tiles give 1180 / 1218 / 1149 / 1134 TFLOP/s)
-    const long long tile_bytes = 2ll * BMX * K;
-    long long pt = (64ll << 20) / (tile_bytes > 0 ? tile_bytes : 1);
-    sc.panel = static_cast<int>(pt < 2 ? 2 : (pt > kPanelTiles ? kPanelTiles : pt));
-  }
-  const int sms = gemm_ctas();  // persistent CTAs of this launch
-  sc.full_waves = tiles / sms;
-  sc.tail_tiles = tiles - sc.full_waves * sms;
-  // cut the leftover tiles as finely as shortens the last round
-  sc.tail_div = 1;
-  int best_num = 1, best_den = 1;  // cost of the last round = rounds / parts, in tiles
-  for (int d = 2; d <= 4 && sc.tail_tiles > 0; d *= 2) {
-    const int rounds = (sc.tail_tiles * d + sms - 1) / sms;
-    if (rounds * best_den < best_num * d) {
-      best_num = rounds;
-      best_den = d;
-      sc.tail_div = d;
-    }
-  }
+  // operand "a" of the MMA = weights (bf16, from TMEM), "b" = activations (bf16, K-major)
+  const uint32_t idesc_full = dev::make_idesc(/*c=f32*/ 1, /*bf16*/ 1, /*bf16*/ 1, 0, /*b K-major*/ 0, BNW, sc.rows);
+  const uint32_t idesc_half = dev::make_idesc(1, 1, 1, 0, 0, BNW, sc.rows / 2);
   const int grid = sc.full_waves > 0 ? sms : (sc.tail_tiles * sc.tail_div < sms ? sc.tail_tiles * sc.tail_div : sms);
   // Programmatic stream serialization: the CTAs of this launch may become resident while the
   // kernel ahead of it drains; they order themselves behind it inside the kernel (or not at all
   // when the caller states independence, which fills the last, partly idle round of one launch
   // with the first tiles of the next).
   QMM_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, wmap, xmap, scale, gq, y, (int)M,
-                          (int)N, (int)K, (long long)ldy, idesc256, idesc128, sc, flags, signal, arrive,
+                          (int)N, (int)K, (long long)ldy, idesc_full, idesc_half, sc, flags, signal, arrive,
                           device_status_word()));
   return QMM_OK;
 }
