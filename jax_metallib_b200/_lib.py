@@ -218,6 +218,14 @@ def load():
     return lib
 
 
+def bind_calls() -> None:
+    """Give the compiled calls (``_calls``) the entry points of the library that this process has loaded."""
+    from . import _calls
+
+    lib = load()
+    _calls.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in _calls.ENTRY_POINTS.split()))
+
+
 def last_error() -> str:
     lib = load()
     buf = ctypes.create_string_buffer(512)

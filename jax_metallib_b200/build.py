@@ -1,4 +1,4 @@
-"""Build ``libqmm.so`` (the C-ABI kernel library) in-tree with nvcc for sm_100a.
+"""Build ``libqmm.so`` (the C-ABI kernel library) in-tree with nvcc for sm_100a, and ``_calls.so`` (the torch-facing calls).
 
     python -m jax_metallib_b200.build [--force]
 
@@ -18,6 +18,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libqmm.so")
+CALLS_SRC = os.path.join(HERE, "binding", "calls.cc")
+CALLS = os.path.join(HERE, "_calls.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -56,7 +58,30 @@ def _headers_mtime() -> float:
     return latest
 
 
+def build_calls(force: bool = False) -> str:
+    """The extension module of ops.py and quantized.py: C++ against the headers of the torch that is installed."""
+    header = os.path.join(os.path.dirname(HERE), "include", "qmm.h")
+    if not force and os.path.exists(CALLS) and os.path.getmtime(CALLS) >= max(os.path.getmtime(CALLS_SRC), os.path.getmtime(header)):
+        return CALLS
+    import importlib.util
+    import sysconfig
+
+    torch = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    include = [os.path.join(torch, "include"), os.path.join(torch, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    # the C++ ABI must be torch's: its compiler leaves the choice in libtorch's own flags (new ABI since torch 2.6)
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=1",
+           *[f"-isystem{d}" for d in include], CALLS_SRC, "-o", CALLS, f"-L{os.path.join(torch, 'lib')}",
+           "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return CALLS
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_calls(force)
     os.makedirs(OBJ, exist_ok=True)
     nvcc = _nvcc()
     hdr = _headers_mtime()

@@ -115,11 +115,11 @@ inline Grid choose_grid(int tiles, int stages_total, Fn resident, int max_ctas =
 // Clusters of `ks` CTAs of a kernel that the current device holds at once; `cache` belongs to the kernel.
 template <typename Kern>
 inline int resident_clusters(Kern kern, int threads, int smem, int per_sm, int ks, std::atomic<int> (&cache)[kMaxDevices][kMaxCluster + 1]) {
+  int dev = 0, n = 0;
+  const bool tracked = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices;
+  if (tracked && (n = cache[dev][ks].load(std::memory_order_relaxed)) > 0) return n;
   const int guess = per_sm * num_sms() / ks > 0 ? per_sm * num_sms() / ks : 1;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return guess;
-  int n = cache[dev][ks].load(std::memory_order_relaxed);
-  if (n > 0) return n;
+  if (!tracked) return guess;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(ks, 1024);

@@ -2,16 +2,31 @@
 
 Each function checks shapes and dtypes, hands raw device pointers and the
 current CUDA stream to ``libqmm.so`` and returns a torch tensor that owns the
-output memory.  PyTorch is only the allocator and the stream here; all
+output memory.  Ordinary calls go through ``_calls`` (the same in C++); what it
+declines by returning ``None`` is done, or refused, here.  PyTorch is only the allocator and the stream here; all
 arithmetic happens in the library's kernels, and a missing library or a
 non-CUDA tensor is an error (there is no fallback path).
 """
 
 from __future__ import annotations
 
+import functools
+
 import torch
 
-from . import _lib
+from . import _calls, _lib
+
+
+@functools.cache
+def _bind() -> None:
+    _lib.bind_calls()
+
+
+def _done(y):
+    """A result of ``_calls``: a status that is not QMM_OK is an int."""
+    if type(y) is int:
+        _lib.check(y)
+    return y
 
 
 def _stream_ptr() -> int:
@@ -36,6 +51,10 @@ def w8a32_perchannel(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor) -> t
     multiply / dot_general chain (src/pjrt_plugin/ops/shape_ops.mm:793-829,
     ops/binary_ops.mm:165-193, :1006-1019).
     """
+    y = _calls.w8a32(x, w, scale)
+    if y is not None:
+        return _done(y)
+    _bind()
     _need_cuda(x, w, scale)
     if x.dtype != torch.float32 or w.dtype != torch.int8 or scale.dtype != torch.float32:
         raise TypeError("expected x float32, w int8, scale float32")
@@ -62,6 +81,11 @@ def w8a16_perchannel(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor, out:
     the output (``QMM_GEMM_INDEPENDENT``): the launch is not ordered behind
     its predecessor.
     """
+    if out is None and not independent:
+        y = _calls.w8a16(x, w, scale)
+        if y is not None:
+            return _done(y)
+    _bind()
     _need_cuda(x, w, scale, out)
     if x.dtype != torch.bfloat16 or w.dtype != torch.int8 or scale.dtype != torch.float32:
         raise TypeError("expected x bfloat16, w int8, scale float32")
@@ -96,6 +120,10 @@ def i8_dot(a: torch.Tensor, b: torch.Tensor, row_scale: torch.Tensor | None = No
     Returns ``(acc_int32 or None, out_f32 or None)``.  Replaces the reference's
     IntegerMatMul emulation (src/pjrt_plugin/ops/binary_ops.mm:433-475).
     """
+    pair = _calls.i8_dot(a, b, row_scale, col_scale, want_acc)
+    if pair is not None:
+        return _done(pair)
+    _bind()
     _need_cuda(a, b, row_scale, col_scale)
     if a.dtype not in (torch.int8, torch.uint8) or b.dtype not in (torch.int8, torch.uint8):
         raise TypeError("operands must be int8 or uint8")
@@ -150,6 +178,11 @@ def w4a16_g128(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, zeros: t
     the kernel that nothing queued earlier on the stream writes the weights,
     so it may fetch them while the previous kernel is still finishing.
     """
+    if out is None and workspace is None:
+        y = _calls.w4a16(x, wq, scales, zeros, zeros_packed, group, static_weights, _w4_workspaces)
+        if y is not None:
+            return _done(y)
+    _bind()
     _need_cuda(x, wq, scales, zeros, out, workspace)
     if x.dtype != torch.bfloat16 or wq.dtype != torch.uint8 or scales.dtype != torch.bfloat16 or zeros.dtype != torch.uint8:
         raise TypeError("expected x bfloat16, wq uint8, scales bfloat16, zeros uint8")

@@ -19,6 +19,8 @@ torch tensors, no host copies).
 
 from __future__ import annotations
 
+import functools
+
 import numpy as np
 
 from . import _lib
@@ -283,6 +285,18 @@ def _to_device(a, torch, device, dtype=None):
     return t.contiguous()
 
 
+def _finished(y):
+    """A result of ``_calls``, which takes ordinary calls in C++ and declines others (``None``): an int is a status."""
+    if type(y) is int:
+        _lib.check(y)
+    return y
+
+
+@functools.cache
+def _bind() -> None:
+    _lib.bind_calls()
+
+
 def _launch_matmul(x, call, N, K, out_dtype):
     """Shared driver: flatten batch dims, run the kernel in x's dtype, cast, restore dims."""
     import torch
@@ -290,7 +304,7 @@ def _launch_matmul(x, call, N, K, out_dtype):
     is_t = _is_torch(x)
     if not (is_t and x.is_cuda) and not torch.cuda.is_available():
         raise RuntimeError("quantized matmul needs a CUDA device: this build has no CPU fallback")
-    _lib.load()
+    _bind()
     device = x.device if (is_t and x.is_cuda) else torch.device("cuda", torch.cuda.current_device())
     xt = _to_device(x, torch, device)
     if xt.dtype == torch.float32:
@@ -317,6 +331,12 @@ def _launch_matmul(x, call, N, K, out_dtype):
 def quantized_matmul(x, w_packed, scales, *, mode: str = "mxfp4", K: int, out_dtype=None):
     """``x[..., M, K] @ dequant(w_packed[N, K//pack], scales[N, K//group])^T`` (reference: quantized.py:995-1074)."""
     cfg = _mode(mode)
+    if out_dtype is None and _is_torch(x):
+        from . import _calls
+
+        y = _calls.mx_matmul(x, w_packed, scales, cfg["bits"], cfg["group_size"], _lib.MX_MODE_IDS[mode] + 1, K)
+        if y is not None:
+            return _finished(y)
     N = w_packed.shape[0]
     if K % cfg["group_size"] != 0:
         raise ValueError(f"K ({K}) must be divisible by group_size ({cfg['group_size']})")
@@ -337,6 +357,12 @@ def affine_quantized_matmul(x, w_packed, scales, biases, *, bits: int = 4, group
                             out_dtype=None):
     """``x[..., M, K] @ dequant(w_packed, scales, biases)^T`` for 4- and 8-bit affine weights
     (reference: quantized.py:1077-1152)."""
+    if out_dtype is None and _is_torch(x):
+        from . import _calls
+
+        y = _calls.affine_matmul(x, w_packed, scales, biases, bits, group_size, K)
+        if y is not None:
+            return _finished(y)
     _bits_ok(bits)
     if bits not in (4, 8):
         raise ValueError(f"fused affine matmul kernels exist for bits 4 and 8; got {bits}")
