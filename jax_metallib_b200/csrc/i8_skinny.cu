@@ -8,11 +8,15 @@
 // column, and mma.sync.m16n8k32 takes b as its 16-row operand and a as its 8-column operand.  The partial tiles of the
 // cluster meet in distributed shared memory.
 //
-// Row pitches that are no multiple of 16 bytes (K or N odd, a view at an odd offset) have no tensor map.  There, loader
-// warps fetch the aligned 32-bit words around each 16-byte piece, shift the bytes into place and store the piece where
-// TMA would have put it, with the next stage's words on their way.  Only words that hold a byte of the tensor are read.
-// Measured (one thread per result before, without the prefetch, now): 65 x 2048 x 1000 90, 21, 12.9 us; 64 x 4095 x 4097
-// 437, 63, 26 us; 4000 x 4097 x 4095 22.7 ms, 2.0 ms, 0.86 ms.  Bound by those loads: five per 16 bytes.
+// Row pitches that are no multiple of 16 bytes (K or N odd, a view at an odd offset) have no tensor map.  Where they and
+// the addresses are multiples of 8, loader warps copy pieces of 8 or 16 bytes asynchronously to where TMA would have put
+// them, a whole ring of stages ahead.  Elsewhere they fetch the aligned 32-bit words around each 16-byte piece, shift the
+// bytes into place and store the piece, with the next stage's words on their way.  Only words that hold a byte of the tensor
+// are read.
+// Measured (shifted words, copies): 65 x 2048 x 1000 13.1, 11.4 us (9.8 with 1024 columns, by TMA); 1000 x 2056 x 2056 69, 53 us.
+// Pieces of 4 bytes lost where there is more to do (33 x 4100 x 4100 19.9, 22.8 us).  Shifted words (one thread per result before, without the
+// prefetch, now): 64 x 4095 x 4097 437, 63, 26 us; 4000 x 4097 x 4095 22.7 ms, 2.0 ms, 0.86 ms; bound by their loads: five
+// per 16 bytes.
 #include <cooperative_groups.h>
 
 #include "split_k.cuh"
@@ -84,12 +88,32 @@ struct Piece {
   }
 };
 
+// Copies a stage's [ROWS][BYTES] part in pieces of W bytes by the 128 loader threads: rows row0 + r, columns col0 + c of a
+// tensor of `rows` x `cols` bytes whose pitch, address and col0 are multiples of W; zeros beyond its ends.  place(r, c): offset
+// of a byte in the stage.
+template <int W, int ROWS, int BYTES, typename Place>
+__device__ __forceinline__ void copy_pieces(uint32_t dst, const uint8_t* src, int row0, int rows, int col0, int cols, int lt, Place place) {
+  constexpr int kPer = BYTES / W, kStep = kLoaderWarps * 32 / kPer;
+  const int c = (lt % kPer) * W;
+#pragma unroll 4
+  for (int r = lt / kPer; r < ROWS; r += kStep) {
+    const bool in = row0 + r < rows && col0 + c < cols;
+    const uint8_t* from = in ? src + static_cast<size_t>(row0 + r) * cols + col0 + c : src;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst + place(r, c)), "l"(from), "n"(W), "r"(in ? W : 0) : "memory");
+  }
+}
+template <int ROWS, int BYTES, typename Place>
+__device__ __forceinline__ void copy_part(int w, uint32_t dst, const uint8_t* src, int row0, int rows, int col0, int cols, int lt, Place place) {
+  if (w == 16) copy_pieces<16, ROWS, BYTES>(dst, src, row0, rows, col0, cols, lt, place);
+  else copy_pieces<8, ROWS, BYTES>(dst, src, row0, rows, col0, cols, lt, place);
+}
+
 template <int MT, bool AU, bool BU, bool TMA>
 __global__ void __launch_bounds__(Smem<MT, TMA>::kThreads, Smem<MT, TMA>::kPerSm)
 i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ a,
                  const uint8_t* __restrict__ b, int32_t* __restrict__ acc_out, float* __restrict__ out,
                  const float* __restrict__ row_scale, const float* __restrict__ col_scale, int M, int N, int K, int stages_total,
-                 int pairs, int* status) {
+                 int pairs, int a_piece, int b_piece, int* status) {
   using L = Smem<MT, TMA>;
   constexpr int S = L::kStages, PB = L::kPartBufs;
   extern __shared__ uint8_t smem_raw[];
@@ -112,7 +136,7 @@ i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       dev::tma_prefetch_desc(&xmap);
     }
     for (int s = 0; s < S; ++s) {
-      dev::mbar_init(&full[s], TMA ? 1 : kLoaderWarps);
+      dev::mbar_init(&full[s], TMA ? 1 : kLoaderWarps * (a_piece ? 32 : 1));
       dev::mbar_init(&empty[s], kConsumerWarps);
     }
     for (int b = 0; b < PB; ++b) {
@@ -149,6 +173,23 @@ i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
           if (!dev::mbar_wait_relaxed(&full[i % S], (i / S) & 1, status, 111)) break;
       }
       __syncwarp();
+    } else if (a_piece) {
+      const int lt = threadIdx.x - kConsumerWarps * 32;   // 0 .. 127
+      for (int t = blockIdx.y; ok && t < tiles; t += gridDim.y) {
+        const int col0 = (t / row_tiles) * kCols, row0 = (t % row_tiles) * MT * 8;
+        for (int it = it_begin; it < it_end; ++it, ++n) {
+          const int s = n % S;
+          if (!dev::mbar_wait_relaxed_warp(&empty[s], ((n / S) & 1) ^ 1, status, 110)) { ok = false; break; }
+          const uint32_t st = dev::smem_u32(smem + s * L::kStage);
+          copy_part<kBK, kCols>(b_piece, st, b, it * kBK, K, col0, N, lt,
+                                [](int r, int c) { return r * 128 + (((c >> 4) ^ (r & 7)) << 4) + (c & 15); });
+          copy_part<MT * 8, kBK>(a_piece, st + kWBytes, a, row0, M, it * kBK, K, lt,
+                                 [](int r, int c) { return r * 64 + (((c >> 4) ^ ((r >> 1) & 3)) << 4) + (c & 15); });
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(dev::smem_u32(&full[s])) : "memory");
+        }
+      }
+      // no copy may still be on its way into this CTA's shared memory when it leaves
+      asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
       const int lt = threadIdx.x - kConsumerWarps * 32;   // 0 .. 127
       const uint8_t* a_end = a + static_cast<size_t>(M) * K;
@@ -369,8 +410,14 @@ static int launch(const Args& p, cudaStream_t stream) {
   cfg.stream = stream;
   set_attrs(cfg, attr, g.ks);
   const int pairs = p.N % 2 == 0 && aligned(p.acc, 8) && aligned(p.out, 8);
+  // the largest piece that a pitch and an address are made of, 8 or 16 bytes; one operand without one: shifted words for both
+  auto piece = [](const uint8_t* at, int pitch) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(at) | static_cast<uintptr_t>(pitch);
+    return bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : 0;
+  };
+  const int pa = TMA ? 0 : piece(p.a, p.K), pb = TMA ? 0 : piece(p.b, p.N);
   QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, p.a, p.b, p.acc, p.out, p.rs, p.cs, p.M, p.N, p.K, stages_total, pairs,
-                                  device_status_word()));
+                                  pb ? pa : 0, pa ? pb : 0, device_status_word()));
   return QMM_OK;
 }
 
