@@ -135,7 +135,7 @@ __device__ __forceinline__ void add2(uint64_t& acc, uint64_t a) { asm("add.rn.f3
 
 // sum_{k in [k0, k1)} x[m,k] * weight[n,k], as the CUDA-core kernels compute it
 template <int FMT, bool XF32>
-__device__ __noinline__ float exact_dot(const void* x, const uint8_t* w, const void* scales, const float* biases, int K, int gs,
+__device__ __forceinline__ float exact_dot_here(const void* x, const uint8_t* w, const void* scales, const float* biases, int K, int gs,
                                         int m, int n, int k0, int k1) {
   float acc = 0.f;
   for (int k = k0; k < k1; k += 8) {
@@ -158,6 +158,12 @@ __device__ __noinline__ float exact_dot(const void* x, const uint8_t* w, const v
     }
   }
   return acc;
+}
+// The same as a call: it is rare, and its registers are not to weigh on the code around it.
+template <int FMT, bool XF32>
+__device__ __noinline__ float exact_dot(const void* x, const uint8_t* w, const void* scales, const float* biases, int K, int gs,
+                                        int m, int n, int k0, int k1) {
+  return exact_dot_here<FMT, XF32>(x, w, scales, biases, K, gs, m, n, k0, k1);
 }
 
 }  // namespace opg
