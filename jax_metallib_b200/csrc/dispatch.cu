@@ -247,22 +247,28 @@ static int w8a16_entry(const char* name, const uint16_t* x, const int8_t* w, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool tma_ok = K > 0 && K % 8 == 0 && N % 16 == 0 && ldy % 2 == 0 && aligned(x, 16) &&
                       aligned(w, 16) && aligned(y, 4);
-  // Few rows, results that stay on this GPU: the HBM-bound kernel.  It reads the weights once per 32 rows; the GEMM reads
-  // them once but does not split K, so that a narrow N leaves SMs idle: measured at M = 64, 4096 x 4096: 16 against 39 us,
-  // 14336 x 4096: 39 against 121 us, 4096 x 28672: 85 against 62 us; at M = 128, 8192 x 8192: 81 against 74 us.
-  // Its blocks are 32 rows x 128 columns.  Where K is short, a second one per CTA is what the GEMM does not have: K = 1024,
-  // 18432 columns (96 x 6144) 12.1 against 15.0 us, 20480 (320 x 2048) 16.9 against 14.5; K = 2048, 20480: 21.8 against 23.1.
-  // Shorter still, the rows it reads again count: K = 128, 8192 columns (128 x 2048) 6.0 against 7.3 us, 16384 (512 x 1024)
-  // 7.7 against 7.3.
+  // Few rows, results that stay on this GPU: the HBM-bound kernel.  It reads the weights once per 32 rows, over all SMs; the
+  // GEMM reads them once, but its blocks are 256 columns wide and go through all of K, so that a narrow N leaves SMs idle:
+  // M = 64, 4096 x 4096: 16.3 against 29.6 us, 14336 x 4096: 40 against 90 us.
+  // Both take a time that grows with K, so that the line is a number of columns, counted once per 32 rows: 128 for each SM.
+  // K = 4096, 18944 columns (M = 32) 27.0 against 30.8 us, 20480: 34.9 against 34.5, 28672: 46 against 35; M = 64, 14336: 46
+  // against 31; M = 128, 4096: 26 against 31, 6144: 39 against 30; K = 8192, M = 64, 8192: 45 against 54, 10240: 59 against 55.
+  // Where K is short, what each kernel does before and after its loop counts, and the GEMM does that once per SM:
+  // K = 1024, 12288 columns (M = 32) 11.8 against 11.9 us, 16384 (64 x 8192) 12.1 against 11.7, 24576 (96 x 8192) 17.6
+  // against 12.0; K = 768, 8192 (32 x 8192) 9.1 against 10.2, 16384 (64 x 8192) 10.9 against 10.2; K = 256, 4096 6.2 against
+  // 7.1, 8192 8.2 against 7.1; K = 64, 4096 6.9 against 5.9.
+  // A single tile of 16 rows is the quicker one for every N: M = 16, 4096 x 28672: 30.5 against 34.3 us, 8192 x 57344: 101
+  // against 117; only where K is below 256 and N above 32000 it is the slower one by a microsecond or two.
   // Results that are too few for the GEMM (M * N < 128 * 128) are one thread each otherwise, which is quicker for a short K:
   // M = 32, N = 128, K = 64 6.8 against 3.8 us; K = 128 6.8 against 6.8.
   // (A caller that limits the GEMM's CTAs keeps the GEMM: the kernel for few rows fills the device.)
-  const int64_t few = K < 256 ? 8192 : K < 2048 ? num_sms() * 128 : 23000;
-  const bool pays = (M <= 32 || (M + 31) / 32 * N <= few) && (K >= 128 || M * N >= 128 * 128);
+  const int64_t few = num_sms() * (K < 128 ? 0 : K < 512 ? 32 : K < 1024 ? 64 : K < 2048 ? 96 : 128);
+  const bool gemm = M * N >= 128 * 128;
+  const bool pays = gemm ? M <= 16 || (M + 31) / 32 * N <= few : K >= 128;
   if (tma_ok && (pays || force_split_k()) && gemm_ctas() == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr &&
       !force_simple())
     return w8a16_decode(x, w, scale, y, M, N, K, ldy, flags, s);
-  if (tma_ok && M * N >= 128 * 128 && !force_simple())
+  if (tma_ok && gemm && !force_simple())
     return w8a16_tcgen05(x, w, scale, y, M, N, K, ldy, flags, signal, arrive, s);
   QMM_REQUIRE(!(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr, QMM_ERR_UNSUPPORTED,
               "%s: multicast stores and completion signals need the tensor-core route "

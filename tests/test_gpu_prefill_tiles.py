@@ -15,8 +15,12 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(33, 64, 24576), (96, 1024, 8192), (161, 1160, 8208), (192, 256, 16384), (193, 640, 8320), (224, 512, 5392),
           (385, 2048, 4096), (777, 384, 6144), (1025, 136, 2064), (1500, 512, 10240)]
 
+# where the kernel for few rows and the GEMM meet, by columns per SM and the length of K
+LINE = [(16, 64, 18960), (17, 8, 1024), (17, 64, 976), (20, 72, 4112), (32, 128, 4736), (32, 136, 4752), (31, 520, 9488),
+        (33, 1016, 4752), (17, 1032, 14224), (64, 1536, 7120), (17, 2048, 18944), (25, 2056, 18960), (65, 2048, 6336)]
 
-@pytest.mark.parametrize("m,k,n", SHAPES)
+
+@pytest.mark.parametrize("m,k,n", SHAPES + LINE)
 def test_int8_weights(cuda, m, k, n):
     g = torch.Generator(device="cuda").manual_seed(m + k + n)
     x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
