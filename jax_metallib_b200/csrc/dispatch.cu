@@ -247,24 +247,22 @@ static int w8a16_entry(const char* name, const uint16_t* x, const int8_t* w, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool tma_ok = K > 0 && K % 8 == 0 && N % 16 == 0 && ldy % 2 == 0 && aligned(x, 16) &&
                       aligned(w, 16) && aligned(y, 4);
-  // Few rows, results that stay on this GPU: the HBM-bound kernel.  It reads the weights once per 32 rows, over all SMs; the
-  // GEMM reads them once, but its blocks are 256 columns wide and go through all of K, so that a narrow N leaves SMs idle:
-  // M = 64, 4096 x 4096: 16.3 against 29.6 us, 14336 x 4096: 40 against 90 us.
-  // Both take a time that grows with K, so that the line is a number of columns, counted once per 32 rows: 128 for each SM.
-  // K = 4096, 18944 columns (M = 32) 27.0 against 30.8 us, 20480: 34.9 against 34.5, 28672: 46 against 35; M = 64, 14336: 46
-  // against 31; M = 128, 4096: 26 against 31, 6144: 39 against 30; K = 8192, M = 64, 8192: 45 against 54, 10240: 59 against 55.
-  // Where K is short, what each kernel does before and after its loop counts, and the GEMM does that once per SM:
-  // K = 1024, 12288 columns (M = 32) 11.8 against 11.9 us, 16384 (64 x 8192) 12.1 against 11.7, 24576 (96 x 8192) 17.6
-  // against 12.0; K = 768, 8192 (32 x 8192) 9.1 against 10.2, 16384 (64 x 8192) 10.9 against 10.2; K = 256, 4096 6.2 against
-  // 7.1, 8192 8.2 against 7.1; K = 64, 4096 6.9 against 5.9.
-  // A single tile of 16 rows is the quicker one for every N: M = 16, 4096 x 28672: 30.5 against 34.3 us, 8192 x 57344: 101
-  // against 117; only where K is below 256 and N above 32000 it is the slower one by a microsecond or two.
+  // Few rows, results that stay on this GPU: the HBM-bound kernel, which reads the weights once per 32 rows and splits K over
+  // clusters.  So does the GEMM where its tiles are few, and it reads them once: up to 16 rows the other one is ahead by its
+  // shorter start and end (M = 16, 4096 x 4096 8.8 against 12.5 us, 14336 x 4096 16.4 against 23.5, 8192 x 57344 96 against
+  // 117), with more rows while a call is short: while fewer than 15 M weights are read, over all passes (M = 32: 14336 x 1024
+  // 16.1 against 17.8 us, 4096 x 4096 14.1 against 12.7, 8192 x 8192 25.8 against 22.0; M = 64: 4096 x 1024 10.9 against 11.0,
+  // 2048 x 4096 11.9 against 11.5, 8192 x 8192 45 against 23.5), ...
+  // ... and while its columns, over all passes, are fewer than 64 for each SM, or 32 where K is short (1024 x 8192, M = 32 9.8
+  // against 10.0 us, M = 64 12.2 against 11.2; 512 x 16384, M = 32 9.8 against 9.1; 256 x 4096, M = 32 6.3 against 7.1, M = 64
+  // 8.1 against 7.0); K = 64: 4096 columns, M = 32 6.9 against 6.0, none.
   // Results that are too few for the GEMM (M * N < 128 * 128) are one thread each otherwise, which is quicker for a short K:
   // M = 32, N = 128, K = 64 6.8 against 3.8 us; K = 128 6.8 against 6.8.
   // (A caller that limits the GEMM's CTAs keeps the GEMM: the kernel for few rows fills the device.)
-  const int64_t few = num_sms() * (K < 128 ? 0 : K < 512 ? 32 : K < 1024 ? 64 : K < 2048 ? 96 : 128);
+  const int64_t columns = (M + 31) / 32 * N;
   const bool gemm = M * N >= 128 * 128;
-  const bool pays = gemm ? M <= 16 || (M + 31) / 32 * N <= few : K >= 128;
+  const bool brief = columns <= num_sms() * (K < 128 ? 0 : K < 512 ? 32 : 64) && columns * K < 15000000;
+  const bool pays = gemm ? M <= 16 || brief : K >= 128;
   if (tma_ok && (pays || force_split_k()) && gemm_ctas() == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr &&
       !force_simple())
     return w8a16_decode(x, w, scale, y, M, N, K, ldy, flags, s);

@@ -27,13 +27,14 @@
 //      drain its accumulators.  The accumulator holds the transposed tile
 //      (lane = output channel), so the per-channel scale is one register per
 //      thread.  Leftover tiles of the last round are cut into halves or
-//      quarters.  The output may be stored with multimem.st to a multicast
-//      address (one store reaches the same offset of every rank's buffer:
-//      the all-gather of a column-sharded linear happens in the epilogue), and
-//      the launch can signal its completion to every rank.
+//      quarters.  Where the tiles are few, a cluster of up to eight CTAs takes one, each a share of its K, and adds the
+//      accumulators up over distributed shared memory: M = 64, int8 4096 x 4096 29.6 us in one CTA to a tile, 14.3 now;
+//      14336 x 4096 89, 25.5; int4 14336 x 2048 112, 26.6; M = 320, 8192 x 8192 59, 44.  The output may be stored with
+//      multimem.st to a multicast address (one store reaches the same offset of every rank's buffer: the all-gather of a
+//      column-sharded linear happens in the epilogue), and the launch can signal its completion to every rank.
 #include <cstdlib>
 
-#include "common.cuh"
+#include "split_k.cuh"
 
 namespace qmm {
 namespace tc {
@@ -360,6 +361,7 @@ struct Sched {
   int tiles_n2, tiles_m, full_waves, tail_tiles, tail_div;
   int panel;  // activation tiles per panel
   int rows;   // rows per tile, a multiple of 32
+  int ks;     // CTAs that share the K of a piece
 };
 struct Work {
   int tn2, tm;   // tile coordinates (units of 256 channels, of `rows` rows)
@@ -378,21 +380,20 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tm = p * panel + r % rows;
 }
 
-// Item `i` of this CTA; false when the CTA is done.  After its full-wave tiles a CTA takes a
+// Item `i` of CTA `cta` of `G`; false when the CTA is done.  After its full-wave tiles a CTA takes a
 // contiguous run of the tail's parts (tile-major: part 2h + mh of a tile cut in four is channel
 // block h, row half mh) and works it off in the largest aligned pieces: a whole tile, a channel
 // block with all its rows, or a single part, so that neighbouring parts cost one pipeline fill
 // and use the full-width MMA.
-__device__ __forceinline__ bool get_work(const Sched& sc, int i, int M, int N, Work& w) {
-  const int G = gridDim.x;
+__device__ __forceinline__ bool get_work(const Sched& sc, int cta, int G, int i, int M, int N, Work& w) {
   int tile, sub = 0, len = 0;  // len: parts covered, in units of 1 / tail_div tile; 0 = whole tile
   const int div = sc.tail_div;
   if (i < sc.full_waves) {
-    tile = blockIdx.x + i * G;
+    tile = cta + i * G;
   } else {
     const long long total = static_cast<long long>(sc.tail_tiles) * div;
-    int pos = static_cast<int>(blockIdx.x * total / G);
-    const int end = static_cast<int>((blockIdx.x + 1) * total / G);
+    int pos = static_cast<int>(cta * total / G);
+    const int end = static_cast<int>((cta + 1) * total / G);
     for (int skip = i - sc.full_waves;; --skip) {
       if (pos >= end) return false;
       const int r = pos % div;
@@ -443,7 +444,9 @@ __device__ __forceinline__ uint32_t dequant2(uint32_t w, uint32_t w4, uint32_t z
 // WBITS = 8: int8 weights [K, N], per-channel f32 scale applied in the epilogue.
 // WBITS = 4: packed int4 weights [K/2, N] (byte = two k of one channel), per-(128-k group, channel)
 //            bf16 scale and zero point applied by the converter warps; K % 128 == 0.
-template <int WBITS>
+// SPLIT: a piece of work is one cluster's; its CTAs take a share of K each and add their accumulators up over distributed
+// shared memory, in CTA order.  One piece a cluster, so that the rings are free for the sums when the last MMA has retired.
+template <int WBITS, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
              const float* __restrict__ scale, const GroupQuant gq, uint16_t* __restrict__ y, int M, int N, int K,
@@ -469,7 +472,10 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kblocks = (K + BK - 1) / BK;
+  const int all_kblocks = (K + BK - 1) / BK;
+  const int kb_begin = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * blockIdx.x / gridDim.x) : 0;
+  const int kb_end = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * (blockIdx.x + 1) / gridDim.x) : all_kblocks;
+  const int cta = SPLIT ? blockIdx.y : blockIdx.x, ctas = SPLIT ? gridDim.y : gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kXStages; ++s) dev::mbar_init(&xfull[s], 1);
@@ -508,9 +514,9 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       unsigned cnt = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work(sc, i, M, N, w); ++i) {
+      for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
-        for (int kb = 0; kb < kblocks; ++kb, ++cnt) {
+        for (int kb = kb_begin; kb < kb_end; ++kb, ++cnt) {
           const int xs = cnt % kXStages;
           if (cnt >= kXStages) {  // the slot's previous stage must have been multiplied
             const unsigned prev = cnt - kXStages;
@@ -528,9 +534,9 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       unsigned cnt = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work(sc, i, M, N, w); ++i) {
+      for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
-        for (int kb = 0; kb < kblocks; ++kb, ++cnt) {
+        for (int kb = kb_begin; kb < kb_end; ++kb, ++cnt) {
           const int ws = cnt % kWStages;
           if (!dev::mbar_wait(&wempty[ws], ((cnt / kWStages) & 1) ^ 1, status, 20)) { ok = false; break; }
           uint8_t* raw = smem + kRawBase + ws * kRawBytes;
@@ -561,21 +567,21 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       int items = 0;
       bool ok = true, ready = false;
       Work w;
-      for (int i = 0; ok && get_work(sc, i, M, N, w); ++i) {
+      for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
         if (!dev::mbar_wait(tempty, (items & 1) ^ 1, status, 22)) break;
         dev::tc_fence_after();
         const uint32_t idesc = (w.m_cols == sc.rows) ? idesc_full : idesc_half;
         const uint32_t b_item = b_lo0 + ((w.m_off * 128) >> 4);
         const uint32_t mine = (me >= w.h0) && (me < w.h0 + w.nh);
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb = kb_begin; kb < kb_end; ++kb) {
           // whether the next stage is ready is asked while this one's MMAs are still being issued: behind them a question
           // waits for its turn
           if (!ready && !dev::mbar_wait(&sfull[g], gpar, status, 23)) { ok = false; break; }
           dev::tc_fence_after();
           const uint32_t a_c = a_t0 + g * kSlotCols;   // 16 k: eight columns
           const uint32_t b_s = b_item + xs * kBStepStage;
-          dev::umma_f16_ts_if(mine, d, a_c, b_s, kDescHi, idesc, kb != 0);
+          dev::umma_f16_ts_if(mine, d, a_c, b_s, kDescHi, idesc, kb != kb_begin);
           dev::umma_f16_ts_if(mine, d, a_c + 8, b_s + kBStepK, kDescHi, idesc, 1);
           dev::umma_f16_ts_if(mine, d, a_c + 16, b_s + 2 * kBStepK, kDescHi, idesc, 1);
           ready = dev::mbar_test(&sfull[g ^ 1], gpar ^ g);
@@ -609,7 +615,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     int items = 0;
     bool ok = true;
     Work w;
-    for (int i = 0; ok && get_work(sc, i, M, N, w); ++i) {
+    for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
       if (w.nh == 0) continue;
       const int h = w.h0 + hh;
       const bool mine = hh < w.nh;
@@ -623,17 +629,17 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         }
       };
       if (WBITS == 4 && mine) {
-        const int first = (grp + kCvtGroups - turn) % kCvtGroups;   // the group's first stage of the item
-        if (first < kblocks) load_scales(first, h);
+        const int first = kb_begin + (grp + kCvtGroups - turn) % kCvtGroups;   // the group's first stage of the item
+        if (first < kb_end) load_scales(first, h);
       }
-      for (int kb = 0; kb < kblocks; ++kb, ++cnt, turn = (turn == kCvtGroups - 1) ? 0 : turn + 1) {
+      for (int kb = kb_begin; kb < kb_end; ++kb, ++cnt, turn = (turn == kCvtGroups - 1) ? 0 : turn + 1) {
         if (turn != grp) continue;
         const int ws = cnt % kWStages;
         const uint32_t raw = dev::smem_u32(smem + kRawBase + ws * kRawBytes + h * kRawBlockW) + lane * 128;
         const uint32_t a_slot = a_lane + (cnt & 1) * kSlotCols + h * (BK / 2);
         // scales and zero points of the stage's 128-k group and this lane's two channel pairs, read one stage of the group's ahead
         uint32_t sv[2] = {sv_next[0], sv_next[1]}, zv[2] = {zv_next[0], zv_next[1]};
-        if (WBITS == 4 && mine && kb + kCvtGroups < kblocks) load_scales(kb + kCvtGroups, h);
+        if (WBITS == 4 && mine && kb + kCvtGroups < kb_end) load_scales(kb + kCvtGroups, h);
         if (!dev::mbar_wait_warp(&wfull[ws], (cnt / kWStages) & 1, status, 26)) { ok = false; break; }
         // 16 channels x 64 k -> 16 registers
         auto convert = [&](int c, uint32_t (&out)[16]) {
@@ -712,6 +718,12 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         uint32_t r[32];
         dev::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + kAccBase + h * kMaxRows + ch * 32, r);
         dev::tc_wait_ld();
+        if (SPLIT) {   // the sums of this CTA's share of K, [row][channel], over the rings
+          float* mine = reinterpret_cast<float*>(smem) + (h - w.h0) * BNW + (n & (BNW - 1));
+#pragma unroll
+          for (int j = 0; j < 32; ++j) mine[(ch * 32 + j) * (w.nh * BNW)] = __uint_as_float(r[j]);
+          continue;
+        }
         if (idx + kWorkerWarps / 4 >= w.nh * chunks) {   // the last values are in registers: the next item may start
           dev::tc_fence_before();
           __syncwarp();
@@ -737,12 +749,51 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
           }
         }
       }
+      if (SPLIT) break;
       if (esub >= w.nh * chunks) {   // a warp without a share
         __syncwarp();
         if (lane == 0) dev::mbar_arrive(tempty);
       }
       ++items;
     }
+  }
+  if (SPLIT) {
+    // Every CTA of the cluster sums every gridDim.x-th run of the results, four channels to a thread.
+    __syncwarp();
+    split::cluster_sync();
+    Work w;
+    if (get_work(sc, cta, ctas, 0, M, N, w) && w.nh > 0) {
+      const int quads = w.nh * (BNW / 4), m_first = w.tm * sc.rows + w.m_off;
+      const int rows = min(M - m_first, w.m_cols), n_first = (w.tn2 * 2 + w.h0) * BNW;
+      for (int e = blockIdx.x * kThreads + threadIdx.x; e < rows * quads; e += gridDim.x * kThreads) {
+        const int row = e / quads, c = e % quads * 4, n = n_first + c;
+        if (n >= N) continue;
+        float4 v[split::kMaxCluster];
+#pragma unroll
+        for (int p = 0; p < split::kMaxCluster; ++p)
+          if (p < gridDim.x) v[p] = split::load_peer(reinterpret_cast<const float4*>(smem + (row * quads * 4 + c) * 4), p);
+        float4 sum = v[0];
+#pragma unroll
+        for (int p = 1; p < split::kMaxCluster; ++p)
+          if (p < gridDim.x) {
+            sum.x += v[p].x;
+            sum.y += v[p].y;
+            sum.z += v[p].z;
+            sum.w += v[p].w;
+          }
+        if (WBITS == 8) {
+          sum.x = 64.f * sum.x * __ldg(scale + n);
+          sum.y = 64.f * sum.y * __ldg(scale + n + 1);
+          sum.z = 64.f * sum.z * __ldg(scale + n + 2);
+          sum.w = 64.f * sum.w * __ldg(scale + n + 3);
+        }
+        uint32_t* dst = reinterpret_cast<uint32_t*>(y + static_cast<size_t>(m_first + row) * ldy + n);
+        dst[0] = dev::pack_bf16x2(sum.x, sum.y);
+        dst[1] = dev::pack_bf16x2(sum.z, sum.w);
+      }
+    }
+    __syncwarp();
+    split::cluster_sync();   // peers keep their shared memory alive until it has been read
   }
   // Completion signal: every thread that stored makes its stores visible system-wide, the CTAs
   // count themselves on a local counter (which wraps back to zero), and the last one adds 1 to
@@ -816,19 +867,30 @@ int i8gemm_tcgen05(const void* a, const void* b, int32_t* acc, const float* row_
 // mean): microseconds per 64 k of a whole tile and of one channel block, with a floor (the chain converter - MMA - converter of
 // two stages in TMEM) and a slope per row, and per piece for its first stages and its results.  What they choose is 0.2 %
 // slower than the best cut in the mean (4096 x 4096, M = 777, int4: 47 us; cut in quarters, which cost no fewer clocks, 72).
-static tc::w8::Sched schedule(int64_t M, int64_t N, int64_t K, int wbits, int sms) {
+// Tiles, or channel blocks, that a share of the SMs holds go to clusters where that is estimated to be quicker; those costs are
+// a fit to 3600 calls (M 33 to 512, K 512 to 14336, N 1024 to 14336, every cut and cluster size: 5 to 7 % off).
+// `resident(ks)`: clusters of ks CTAs that the device holds at once, 0 where K must not be split.
+template <typename Fn>
+static tc::w8::Sched schedule(int64_t M, int64_t N, int64_t K, int wbits, int sms, Fn resident) {
   using namespace tc::w8;
   struct Cost { float floor, row, piece; };
   static constexpr Cost kWhole[2] = {{0.43f, 0.0030f, 6.6f}, {0.59f, 0.0033f, 5.9f}};   // int8, int4
   static constexpr Cost kBlock[2] = {{0.39f, 0.0022f, 5.0f}, {0.48f, 0.00265f, 4.8f}};
+  static constexpr Cost kSplitWhole[2] = {{0.43f, 0.0027f, 5.6f}, {0.59f, 0.0032f, 5.2f}};
+  static constexpr Cost kSplitBlock[2] = {{0.36f, 0.0021f, 5.9f}, {0.47f, 0.0025f, 5.6f}};
+  constexpr float kSumCta = 0.18f, kSumRow = 0.036f;   // the sums: per CTA of a cluster, per row of 256 channels
   const float stages = static_cast<float>((K + BK - 1) / BK);
-  auto us = [&](const Cost& c, int rows) { return (rows * c.row > c.floor ? rows * c.row : c.floor) * stages + c.piece; };
+  auto us = [&](const Cost& c, int rows, int ks = 1) {
+    const int share = (static_cast<int>(stages) + ks - 1) / ks;
+    return (rows * c.row > c.floor ? rows * c.row : c.floor) * share + c.piece;
+  };
   Sched best = {};
   float best_cost = -1.f;
   const int least = static_cast<int>((M + kMaxRows - 1) / kMaxRows);
   for (int tiles_m = least; tiles_m <= least + 3; ++tiles_m) {
     Sched sc = {};
     sc.tiles_n2 = static_cast<int>((N + 2 * BNW - 1) / (2 * BNW));
+    sc.ks = 1;
     sc.rows = static_cast<int>(((M + tiles_m - 1) / tiles_m + 31) / 32 * 32);
     sc.tiles_m = static_cast<int>((M + sc.rows - 1) / sc.rows);
     const int tiles = sc.tiles_n2 * sc.tiles_m;
@@ -851,6 +913,19 @@ static tc::w8::Sched schedule(int64_t M, int64_t N, int64_t K, int wbits, int sm
         best = sc;
       }
     }
+    // pieces that a share of the SMs holds at once: clusters of CTAs, each with a part of K
+    sc.full_waves = 0;
+    sc.tail_tiles = tiles;
+    for (sc.tail_div = 1; sc.tail_div <= 2 && tiles * sc.tail_div <= sms / 2; sc.tail_div *= 2)
+      for (sc.ks = 2; sc.ks <= split::kMaxCluster && sc.ks <= stages; ++sc.ks) {
+        if (tiles * sc.tail_div * sc.ks > sms || tiles * sc.tail_div > resident(sc.ks)) break;
+        const float cost = us((sc.tail_div == 1 ? kSplitWhole : kSplitBlock)[wbits == 4], sc.rows, sc.ks) + kSumCta * sc.ks +
+                           kSumRow * sc.rows / sc.tail_div;
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = sc;
+        }
+      }
   }
   return best;
 }
@@ -862,7 +937,17 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
                               uint32_t* signal, uint32_t* arrive, cudaStream_t stream) {
   using namespace tc::w8;
   const int sms = gemm_ctas();  // persistent CTAs of this launch
-  const Sched sc = schedule(M, N, K, WBITS, sms);
+  static std::atomic<int> resident[kMaxDevices][split::kMaxCluster + 1];
+  static std::atomic<uint64_t> configured[2] = {};  // per device (one mask per instance of the kernel)
+  auto kern = w8a16_kernel<WBITS, false>;
+  auto split_kern = w8a16_kernel<WBITS, true>;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes, configured[0])) return rc;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(split_kern), kSmemBytes, configured[1])) return rc;
+  // results that go to several GPUs or are announced, and callers with a limit on the CTAs, keep one CTA to a piece
+  const bool may_split = sms == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr;
+  const Sched sc = schedule(M, N, K, WBITS, sms, [&](int ks) {
+    return may_split ? split::resident_clusters(split_kern, kThreads, kSmemBytes, 1, ks, resident) : 0;
+  });
   CUtensorMap wmap, xmap;
   constexpr int kRawRows = (WBITS == 8) ? BK : BK / 2;
   if (int rc = make_tensor_map_2d(&wmap, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)(WBITS == 8 ? K : K / 2),
@@ -871,12 +956,21 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
   if (int rc = make_tensor_map_2d(&xmap, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M,
                                   (uint64_t)K, (uint64_t)K * 2, sc.rows, BK, CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
-  static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
-  auto kern = w8a16_kernel<WBITS>;
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes, configured)) return rc;
   // operand "a" of the MMA = weights (bf16, from TMEM), "b" = activations (bf16, K-major)
   const uint32_t idesc_full = dev::make_idesc(/*c=f32*/ 1, /*bf16*/ 1, /*bf16*/ 1, 0, /*b K-major*/ 0, BNW, sc.rows);
   const uint32_t idesc_half = dev::make_idesc(1, 1, 1, 0, 0, BNW, sc.rows / 2);
+  if (sc.ks > 1) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    cfg.gridDim = dim3(sc.ks, sc.tail_tiles * sc.tail_div);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.stream = stream;
+    split::set_attrs(cfg, attr, sc.ks);
+    QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kern, wmap, xmap, scale, gq, y, (int)M, (int)N, (int)K, (long long)ldy, idesc_full,
+                                    idesc_half, sc, flags, signal, arrive, device_status_word()));
+    return QMM_OK;
+  }
   const int grid = sc.full_waves > 0 ? sms : (sc.tail_tiles * sc.tail_div < sms ? sc.tail_tiles * sc.tail_div : sms);
   // Programmatic stream serialization: the CTAs of this launch may become resident while the
   // kernel ahead of it drains; they order themselves behind it inside the kernel (or not at all

@@ -75,6 +75,16 @@ __device__ __forceinline__ float2 load_peer(const float2* p, int rank) {
       : "memory");
   return v;
 }
+__device__ __forceinline__ float4 load_peer(const float4* p, int rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(dev::smem_u32(p)), "r"(rank)
+      : "memory");
+  return v;
+}
 
 struct Grid {
   int ks, clusters;
