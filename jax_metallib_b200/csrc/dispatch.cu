@@ -160,16 +160,15 @@ static bool i8_skinny_covers(int64_t M, int64_t N, int64_t K, bool tma_ok) {
   }
   if (!large) return K >= 256 || (K >= 128 && M <= 16);   // else one thread per result: M = 32, N = 256, K = 128 7.1, 6.1
   if (gemm_ctas() != num_sms()) return false;             // a limit keeps the GEMM
-  // The GEMM's tiles of 256 columns leave most SMs idle when there are few of them; this kernel splits K, but reads b once
-  // per 64 rows and hands over 64 x 128 results at a time.  M = 32, N = 1024, K = 64: 8.5, 7.5; 128: 7.3, 7.5; N = 16384,
-  // K = 512 9.5, 9.0.
-  if (M <= 32) return M <= 16 || (K >= 128 && (N <= 8192 || K >= 1024));
-  // 64 x N and its likes: N = 1024, K = 256 9.0, 8.1; 512 8.2, 8.8; N = 2048, K = 512 9.5, 8.7; 1024 9.8, 10.2;
-  // N = 4096, K = 1024 10.7, 10.3; 2048 11.9, 13.0; N = 8192, K = 4096 20.5, 18.8 (8192 x 8192 from memory: 30.5, 37.3).
-  // The GEMM is quicker at a single tile of columns: M = 1024, N = 128, K = 1024 9.8, 8.9; 2048 10.7, 11.5.
-  const int64_t cols = (M + 63) / 64 * ((N + 127) / 128 * 128);
-  const int64_t least = cols <= 1024 ? 512 : (cols <= 2048 ? 1024 : (cols <= 4096 ? 2048 : 8192));
-  return cols <= 8192 && K >= (N <= 128 && least < 2048 ? 2048 : least);
+  // Both split K.  This kernel reads b once per 64 rows and hands over 64 x 128 results at a time, the GEMM once per 128 and
+  // 128 x 256.  M = 16, 4096 x 4096 8.0, 9.1; 8192 x 8192 14.3, 12.4, M = 8 13.1, 15.4.
+  // M = 32, K = 128, N = 4096 7.6, 7.4 (M = 20 6.5, 7.6); 64: 8.5, 7.5; 512 x 1024 6.2, 6.5; 512 x 4096 8.0, 6.7; 2048 x 1024
+  // 7.0, 7.5; 2048 x 2048 7.9, 7.7; 4096 x 1024 7.6, 8.0; 4096 x 4096 9.8, 8.9; 8192 x 1024 9.6, 9.5.
+  if (M <= 32) return M <= 16 || (K >= 128 && (K < 256 ? N <= 8192 : N <= 2048 && N * K <= 4 << 20));
+  // M = 64, 512 x 512 8.1, 7.9; 2048 x 2048 10.9, 8.8; 8192 x 8192 30, 14.  With more rows, only few columns suit it: M = 128,
+  // 512 x 512 8.2, 9.2; 2048 x 512 9.3, 10.0; 1024 x 1024 9.7, 9.7; M = 192, 2048 x 512 9.7, 10.1; M = 256, 1024 x 256 8.6, 9.5;
+  // 2048 x 512 10.4, 10.2; M = 512, 1024 x 256 9.7, 9.7.
+  return M > 64 && (M + 63) / 64 * ((N + 127) / 128 * 128) <= 1536 && K >= 512;
 }
 
 }  // namespace qmm

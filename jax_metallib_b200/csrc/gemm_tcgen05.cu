@@ -12,6 +12,9 @@
 //      transposed copy of b is ever made.  Tile 256 (m, two accumulators) x
 //      256 (n) x 128 (k).  Warps: one TMA producer, two MMA issuers, eight
 //      epilogue warps (optional int32 store and/or float(acc) * row[m] * col[n]).
+//      Where the tiles are few, a cluster of up to eight CTAs takes a 128 x 256 block, each a share of its K, and adds the
+//      accumulators up over distributed shared memory: M = 64, 4096 x 4096 18.3 us in one CTA to a block, 9.7 now; 8192 x 8192
+//      30, 14; M = 512, 8192 x 1024 30, 14.
 //
 //  (2) w8a16: y[M,N] = bf16((x[M,K] @ float(w[K,N])) * scale[N]), bf16
 //      activations, int8 weights.  The weight tile is the 128-row MMA operand and goes
@@ -73,8 +76,17 @@ static_assert(BK == 128, "the issue loop is written out for four 32-byte k-steps
 struct Work {
   int tm2, tn, h0, nh;
 };
-__device__ __forceinline__ bool get_work(int i, int tiles_m2, int tiles_n, int halves, int M, Work& w) {
-  const int v = blockIdx.x + i * gridDim.x;
+template <bool SPLIT>
+__device__ __forceinline__ bool get_work(int cta, int ctas, int i, int tiles_m2, int tiles_n, int halves, int M, Work& w) {
+  if (SPLIT) {   // row block `cta`, one to a cluster
+    const int blocks_m = (M + BMB - 1) / BMB, bm = cta % blocks_m;
+    w.tm2 = bm >> 1;
+    w.tn = cta / blocks_m;
+    w.h0 = bm & 1;
+    w.nh = 1;
+    return i == 0;
+  }
+  const int v = cta + i * ctas;
   const int total = tiles_m2 * tiles_n * (halves ? 2 : 1);
   if (v >= total) return false;
   const int tile = halves ? (v >> 1) : v;
@@ -87,6 +99,9 @@ __device__ __forceinline__ bool get_work(int i, int tiles_m2, int tiles_n, int h
   return true;
 }
 
+// SPLIT (with halves): a row block is one cluster's; its CTAs take a share of K each and add their accumulators up over
+// distributed shared memory.  One block a cluster, so that the ring is free for the sums when the last MMA has retired.
+template <bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap,
               const __grid_constant__ CUtensorMap accmap, const __grid_constant__ CUtensorMap outmap,
@@ -104,7 +119,10 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m2 = (M + 2 * BMB - 1) / (2 * BMB), tiles_n = (N + BN - 1) / BN;
-  const int kblocks = (K + BK - 1) / BK;
+  const int all_kblocks = (K + BK - 1) / BK;
+  const int kb_begin = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * blockIdx.x / gridDim.x) : 0;
+  const int kb_end = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * (blockIdx.x + 1) / gridDim.x) : all_kblocks;
+  const int cta = SPLIT ? blockIdx.y : blockIdx.x, ctas = SPLIT ? gridDim.y : gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -132,9 +150,9 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
       uint32_t s = 0, ph = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work(i, tiles_m2, tiles_n, halves, M, w); ++i) {
+      for (int i = 0; ok && get_work<SPLIT>(cta, ctas, i, tiles_m2, tiles_n, halves, M, w); ++i) {
         if (w.nh == 0) continue;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!dev::mbar_wait(&empty[s], ph ^ 1, status, 11)) { ok = false; break; }
           uint8_t* st = smem + s * kStageBytes;
           dev::mbar_expect_tx(&full[s], w.nh * kABlock + kBBytes);
@@ -166,16 +184,16 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
       int items = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work(i, tiles_m2, tiles_n, halves, M, w); ++i) {
+      for (int i = 0; ok && get_work<SPLIT>(cta, ctas, i, tiles_m2, tiles_n, halves, M, w); ++i) {
         if (w.nh == 0) continue;
         if (!dev::mbar_wait(tempty, (items & 1) ^ 1, status, 12)) break;
         dev::tc_fence_after();
         const uint32_t mine = (me >= w.h0) && (me < w.h0 + w.nh);
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!dev::mbar_wait(&full[s], ph, status, 13)) { ok = false; break; }
           dev::tc_fence_after();
           const uint32_t a_s = a_lo0 + s * kStageStep, b_s = b_lo0 + s * kStageStep;
-          dev::umma_i8_lh_if(mine, d_tmem, a_s, kDescHi, b_s, kDescHi, idesc, kb != 0);
+          dev::umma_i8_lh_if(mine, d_tmem, a_s, kDescHi, b_s, kDescHi, idesc, kb != kb_begin);
           dev::umma_i8_lh_if(mine, d_tmem, a_s + kAStepK, kDescHi, b_s + kBStepK, kDescHi, idesc, 1);
           dev::umma_i8_lh_if(mine, d_tmem, a_s + 2 * kAStepK, kDescHi, b_s + 2 * kBStepK, kDescHi, idesc, 1);
           dev::umma_i8_lh_if(mine, d_tmem, a_s + 3 * kAStepK, kDescHi, b_s + 3 * kBStepK, kDescHi, idesc, 1);
@@ -194,7 +212,7 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
     const uint64_t store_policy = dev::policy_evict_first();
     int items = 0;
     Work w;
-    for (int i = 0; get_work(i, tiles_m2, tiles_n, halves, M, w); ++i) {
+    for (int i = 0; get_work<SPLIT>(cta, ctas, i, tiles_m2, tiles_n, halves, M, w); ++i) {
       if (w.nh == 0) continue;
       if (!dev::mbar_wait_relaxed_warp(tfull, items & 1, status, 14)) break;
       dev::tc_fence_after();
@@ -206,21 +224,29 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
       // has been consumed once the accumulators are complete); earlier items overlap their plain stores with the
       // loads of the next item, which the producer has already started into the ring
       Work w_next;
-      const bool staged = staged_store && !get_work(i + 1, tiles_m2, tiles_n, halves, M, w_next);
-      const int row0 = (w.tm2 * 2 + j) * BMB + q * 32;
+      const bool staged = staged_store && !get_work<SPLIT>(cta, ctas, i + 1, tiles_m2, tiles_n, halves, M, w_next);
+      const int block = SPLIT ? w.h0 : j;   // (a single block's chunks are shared out among all warps)
+      const int row0 = (w.tm2 * 2 + block) * BMB + q * 32;
       const int row = row0 + lane;
       const bool mine = (j >= w.h0) && (j < w.h0 + w.nh) && row < M;
       const float rs = (f_out && mine) ? __ldg(row_scale + row) : 0.f;
       uint8_t* stage = smem + kOutBase + (warp - 2) * kOutStage;
       uint8_t* my_row = stage + lane * 128;
-      if (j >= w.h0 && j < w.h0 + w.nh && row0 < M) {
+      if (block >= w.h0 && block < w.h0 + w.nh && row0 < M) {
 #pragma unroll 1
-        for (int ch = 0; ch < BN / 32; ++ch) {
+        for (int ch = SPLIT ? j : 0; ch < BN / 32; ch += SPLIT ? 2 : 1) {
           const int col0 = w.tn * BN + ch * 32;
           if (col0 >= N) break;
           uint32_t r[32];
-          dev::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + j * BN + ch * 32, r);
+          dev::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + block * BN + ch * 32, r);
           dev::tc_wait_ld();
+          if (SPLIT) {   // the sums of this CTA's share of K, [row][256 columns], 16-byte pieces swizzled by the row
+#pragma unroll
+            for (int i4 = 0; i4 < 8; ++i4)
+              *reinterpret_cast<uint4*>(smem + (q * 32 + lane) * (BN * 4) + (((ch * 8 + i4) ^ (lane & 7)) << 4)) =
+                  make_uint4(r[4 * i4], r[4 * i4 + 1], r[4 * i4 + 2], r[4 * i4 + 3]);
+            continue;
+          }
           if (!staged) {
             // straight from registers: 16-byte stores of 32 different rows per instruction
             if (mine) {
@@ -292,6 +318,55 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
       ++items;
     }
     if (lane == 0) dev::tma_store_wait_read();   // no store still reads this CTA's shared memory
+  }
+  if (SPLIT) {
+    // Every CTA of the cluster sums every gridDim.x-th run of the results, four columns to a thread.
+    __syncwarp();
+    split::cluster_sync();
+    Work w;
+    if (get_work<SPLIT>(cta, ctas, 0, tiles_m2, tiles_n, halves, M, w) && w.nh > 0) {
+      const int row0 = (w.tm2 * 2 + w.h0) * BMB, rows = min(M - row0, BMB);
+      const int step = gridDim.x * kThreads, end = rows * (BN / 4);
+      for (int e0 = blockIdx.x * kThreads + threadIdx.x; e0 < end; e0 += 2 * step) {
+        float4 v[2][split::kMaxCluster];   // two runs at a time: a load from a peer takes about 0.5 us
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int e = min(e0 + k * step, end - 1), r = e / (BN / 4), c = e % (BN / 4);
+          const float4* at = reinterpret_cast<const float4*>(smem + r * (BN * 4) + ((c ^ (r & 7)) << 4));
+#pragma unroll
+          for (int p = 0; p < split::kMaxCluster; ++p)
+            if (p < gridDim.x) v[k][p] = split::load_peer(at, p);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int e = e0 + k * step, r = e / (BN / 4), col = w.tn * BN + e % (BN / 4) * 4;
+          if (e >= end || col >= N) continue;
+          uint32_t sum[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+          for (int p = 0; p < split::kMaxCluster; ++p)
+            if (p < gridDim.x) {
+              sum[0] += __float_as_uint(v[k][p].x);
+              sum[1] += __float_as_uint(v[k][p].y);
+              sum[2] += __float_as_uint(v[k][p].z);
+              sum[3] += __float_as_uint(v[k][p].w);
+            }
+          const size_t to = static_cast<size_t>(row0 + r) * N + col;
+          if (acc_out) *reinterpret_cast<uint4*>(acc_out + to) = make_uint4(sum[0], sum[1], sum[2], sum[3]);
+          if (f_out) {
+            const float rs = __ldg(row_scale + row0 + r);
+            const float4 cs = __ldg(reinterpret_cast<const float4*>(col_scale + col));
+            float4 o;
+            o.x = static_cast<float>(static_cast<int32_t>(sum[0])) * rs * cs.x;
+            o.y = static_cast<float>(static_cast<int32_t>(sum[1])) * rs * cs.y;
+            o.z = static_cast<float>(static_cast<int32_t>(sum[2])) * rs * cs.z;
+            o.w = static_cast<float>(static_cast<int32_t>(sum[3])) * rs * cs.w;
+            *reinterpret_cast<float4*>(f_out + to) = o;
+          }
+        }
+      }
+    }
+    __syncwarp();
+    split::cluster_sync();   // peers keep their shared memory alive until it has been read
   }
   dev::tc_fence_before();
   __syncthreads();
@@ -822,6 +897,24 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
 // ----------------------------------------------------------------------------
 namespace qmm {
 
+// CTAs that share the K of a 128 x 256 block.  The costs are a fit to 1200 calls (M 2 to 1024, K 64 to 16384, N 256 to 16384,
+// every cluster size: 3 % off in the median): microseconds per 128 k, and per call for its start, its rows and the sums.
+template <typename Fn>
+static int split_of(int64_t M, int blocks, int stages, Fn resident) {
+  const float rows = M < 128 ? static_cast<float>(M) : 128.f;
+  int best = 1;
+  float best_cost = 0.34f * stages + 6.9f + 0.009f * rows;
+  for (int ks = 2; ks <= split::kMaxCluster && ks <= stages && blocks * ks <= num_sms(); ++ks) {
+    if (blocks > resident(ks)) continue;
+    const float cost = 0.34f * ((stages + ks - 1) / ks) + 4.6f + 0.2f * ks + (0.023f + 0.03f / ks) * rows;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = ks;
+    }
+  }
+  return best;
+}
+
 int i8gemm_tcgen05(const void* a, const void* b, int32_t* acc, const float* row_scale,
                    const float* col_scale, float* out, int64_t M, int64_t N, int64_t K,
                    int a_unsigned, int b_unsigned, cudaStream_t stream) {
@@ -843,8 +936,12 @@ int i8gemm_tcgen05(const void* a, const void* b, int32_t* acc, const float* row_
     if (int rc = make_tensor_map_2d(&outmap, out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)M, (uint64_t)N,
                                     (uint64_t)N * 4, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B))
       return rc;
-  static std::atomic<uint64_t> configured{0};  // per device
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(i8gemm_kernel), kSmemBytes, configured)) return rc;
+  static std::atomic<uint64_t> configured[2] = {};  // per device
+  static std::atomic<int> resident[kMaxDevices][split::kMaxCluster + 1];
+  auto kern = i8gemm_kernel<false>;
+  auto split_kern = i8gemm_kernel<true>;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes, configured[0])) return rc;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(split_kern), kSmemBytes, configured[1])) return rc;
   const uint32_t idesc = dev::make_idesc(/*c=s32*/ 2, a_unsigned ? 0 : 1, b_unsigned ? 0 : 1,
                                          /*a K-major*/ 0, /*b MN-major*/ 1, BMB, BN);
   const int tiles = static_cast<int>(((M + 2 * BMB - 1) / (2 * BMB)) * ((N + BN - 1) / BN));
@@ -852,9 +949,31 @@ int i8gemm_tcgen05(const void* a, const void* b, int32_t* acc, const float* row_
   const int halves = (tiles * 2 <= ctas) ? 1 : 0;  // few tiles: one row block per CTA
   const int items = tiles * (halves ? 2 : 1);
   const int grid = items < ctas ? items : ctas;
+  const int blocks = static_cast<int>((M + BMB - 1) / BMB * ((N + BN - 1) / BN));
+  int ks = 1;   // callers with a limit on the CTAs keep one to a block
+  if (ctas == num_sms())
+    ks = split_of(M, blocks, static_cast<int>((K + BK - 1) / BK),
+                  [&](int n) { return split::resident_clusters(split_kern, kThreads, kSmemBytes, 1, n, resident); });
+  if (ks > 1) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ks, blocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kern, amap, bmap, accmap, outmap, acc, out, row_scale, col_scale, (int)M, (int)N,
+                                    (int)K, idesc, 1, 0, device_status_word()));
+    return QMM_OK;
+  }
   static std::atomic<int> staged_cache{INT32_MIN};
   const int staged = env_int_once("QMM_I8_STAGED_STORE", 1, staged_cache);   // 0: results stored straight from registers
-  i8gemm_kernel<<<grid, kThreads, kSmemBytes, stream>>>(amap, bmap, accmap, outmap, acc, out, row_scale, col_scale,
+  kern<<<grid, kThreads, kSmemBytes, stream>>>(amap, bmap, accmap, outmap, acc, out, row_scale, col_scale,
                                                         (int)M, (int)N, (int)K, idesc, halves, staged,
                                                         device_status_word());
   QMM_CHECK_LAUNCH("i8gemm_kernel");
