@@ -599,14 +599,20 @@ static int run(const char* name, const uint16_t* x, const uint8_t* wq, const uin
                void* workspace, unsigned flags, int* status, cudaStream_t st) {
   // Few rows and columns: the kernel that splits K over a cluster and adds up in distributed shared memory.  This one
   // streams wider rows and is ahead once N fills the device by itself: (this one, that one) at M = 8, 4096 x 6144 11.7,
-  // 9.1 us, 4096 x 28672 23.7, 25.7 us; at M = 32, 4096 x 6144 28.4, 31.5 us (that one with tiles of 32 rows).
+  // 9.1 us, 4096 x 28672 23.7, 25.7 us.
   // It is ahead, too, where the weights are many and the start and the end of a call therefore little: at M = 3
   // 14336 x 4096 16.6, 14.1 us, 8192 x 8192 16.1, 15.2 us, 16896 x 5888 20.4, 22.1 us; at M = 8 18.0, 15.5 us for
   // 8192 x 8192, 20.1, 17.3 us for 14336 x 5120, 19.1, 19.0 us for 8192 x 9728, 22.8, 22.2 us for 16896 x 5888.
   // Both lines moved when that one took the zero point into the weight.  At the other end a call of one or two stages is
   // all hand-over: M = 8, K = 128, N = 256 3.0, 4.1 us; 1024 6.1, 4.1 us.
-  const bool pays = N <= 16384 && N * K <= 75000000 && N * K >= 65536;
-  if (M <= 16 && (pays || force_split_k()))
+  // With 9 to 16 rows it is ahead for all but the widest matrices, and with 17 to 32, which that one takes as two tiles of 16,
+  // for narrow ones and short K: M = 16 28672 x 4096 38.8, 31.4 us, 4096 x 18944 23.6, 20.7, 2048 x 20480 20.2, 21.0, 8192 x
+  // 57344 97, 123; M = 32 512 x 512 11.1, 4.8, 4096 x 4096 23.3, 12.9, 4096 x 10240 33.5, 26.5, 14336 x 4096 44.8, 30.9,
+  // 2048 x 20480 31.2, 24.7; 4096 x 12288 34.3, 35.2, 8192 x 14336 63.1, 63.9, 4096 x 28672 63.1, 65.2.
+  const bool pays = N * K >= 65536 && (M <= 8    ? N <= 16384 && N * K <= 75000000
+                                       : M <= 16 ? N <= num_sms() * kColsPerBlock / 2
+                                                 : N <= 10240 || K <= 2048);
+  if (pays || force_split_k())
     return w4a16_split(x, wq, scales, zeros, zeros_packed, y, M, N, K, (flags & QMM_W4_STATIC_WEIGHTS) ? 1 : 0, status, st);
   const int G = static_cast<int>(K / kGroup);
   const int C = col_blocks(N);

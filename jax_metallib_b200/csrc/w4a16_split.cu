@@ -1,4 +1,4 @@
-// int4 group-wise (g128, asymmetric) weight-only matmul at decode sizes (M <= 16), K split over a cluster.
+// int4 group-wise (g128, asymmetric) weight-only matmul at decode sizes (M <= 32), K split over a cluster.
 //
 //   y[M,N] = bf16( x[M,K] @ ((q[K,N] - z[K/128,N]) * s[K/128,N]) )
 //
@@ -17,6 +17,8 @@
 // Bound by the latency of a stage's chain and, for small matrices, by prologue and
 // hand-over, which this kernel has less of than the one that meets in global memory.  Measured (that kernel, this one) at
 // M = 8: 4096 x 6144 11.7, 9.1 us; 4096 x 4096 11.2, 7.5 us; 14336 x 4096 19.6, 14.5 us; 4096 x 28672 23.7, 25.7 us.
+// 17 to 32 rows are two tiles of 16, side by side in the walk: one tile of 32 has registers for one CTA per SM only (earlier:
+// 4096 x 6144 31.5 us, now 19.9).
 #include <cooperative_groups.h>
 
 #include "split_k.cuh"
@@ -91,7 +93,9 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
   uint64_t* vacant = ready + PB;     // every CTA of the cluster has read this CTA's partial tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KS = gridDim.x, rank = blockIdx.x;      // the cluster is the grid's x extent
-  const int tiles = N / kCols;
+  // 17 to 32 rows: a tile's two halves of 16 rows are tiles of their own, next to each other in the walk (the second finds the
+  // weights in L2)
+  const int two = M > 16, tiles = N / kCols << two;
   const int it_begin = (groups * rank) / KS, it_end = (groups * (rank + 1)) / KS;
   cg::cluster_group cluster = cg::this_cluster();
 
@@ -117,7 +121,7 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
       const uint64_t policy = dev::policy_evict_first();
       auto issue_weights = [&](int s, int t, int it) {
         uint8_t* st = smem + s * L::kStage;
-        const size_t col0 = static_cast<size_t>(t) * kCols, row = static_cast<size_t>(it) * N;
+        const size_t col0 = static_cast<size_t>(t >> two) * kCols, row = static_cast<size_t>(it) * N;
         dev::mbar_expect_tx(&full[s], kWBytes + 256 + L::kZBytes);
         dev::tma_load_2d_hint(st, &wmap, &full[s], static_cast<int>(col0), it * (kGroup / 2), policy);
         bulk_copy_g2s(st + L::kOffS, scales + row + col0, 256, &full[s]);
@@ -140,8 +144,8 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
           }
           uint8_t* st = smem + s * L::kStage;
           dev::mbar_expect_tx(&full[s], 2 * L::kXBox);   // rows past M arrive as zeros
-          dev::tma_load_2d(st + L::kOffX, &xmap, &full[s], it * kGroup, 0);
-          dev::tma_load_2d(st + L::kOffX + L::kXBox, &xmap, &full[s], it * kGroup + 64, 0);
+          dev::tma_load_2d(st + L::kOffX, &xmap, &full[s], it * kGroup, (t & two) * 16);
+          dev::tma_load_2d(st + L::kOffX + L::kXBox, &xmap, &full[s], it * kGroup + 64, (t & two) * 16);
         }
       // no copy may still be on its way into this CTA's shared memory when it leaves, whatever the consumers did
       for (int i = n > S ? n - S : 0; i < n; ++i)
@@ -263,7 +267,8 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
       const int b = tile % PB;
       const float* part = reinterpret_cast<const float*>(smem + L::kOffPart + b * 2 * L::kPart);
       if (!wait_cluster_warp(&ready[b], (tile / PB) & 1, status, 124)) break;
-      for (int e = rank * kR + tid; e < M * (kCols / 2); e += KS * kR) {
+      const int first = (t & two) * 16, rows = min(M - first, MT * 8);
+      for (int e = rank * kR + tid; e < rows * (kCols / 2); e += KS * kR) {
         const int m = e / (kCols / 2), c = (e % (kCols / 2)) * 2;
         float2 lo[kMaxCluster], hi[kMaxCluster];
 #pragma unroll
@@ -280,7 +285,7 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             v.x += lo[r].x + hi[r].x;
             v.y += lo[r].y + hi[r].y;
           }
-        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(m) * N + static_cast<size_t>(t) * kCols + c) =
+        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(first + m) * N + static_cast<size_t>(t >> two) * kCols + c) =
             dev::pack_bf16x2(v.x, v.y);
       }
       __syncwarp();
@@ -298,7 +303,7 @@ static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const uint16
   static std::atomic<int> resident[kMaxDevices][kMaxCluster + 1];
   auto kern = w4a16_split_kernel<MT, ZP>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
-  const Grid g = choose_grid(N / kCols, groups,
+  const Grid g = choose_grid(N / kCols << (M > 16), groups,
                              [&](int ks) { return resident_clusters(kern, L::kThreads, L::kTotal, L::kPerSm, ks, resident); });
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
@@ -313,7 +318,7 @@ static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const uint16
 
 }  // namespace w4s
 
-// 1 <= M <= 16, N and K multiples of 128, operands 16-byte aligned (checked by the caller).
+// 1 <= M <= 32, N and K multiples of 128, operands 16-byte aligned (checked by the caller).
 int w4a16_split(const uint16_t* x, const uint8_t* wq, const uint16_t* scales, const uint8_t* zeros, int zeros_packed, uint16_t* y,
                 int64_t M, int64_t N, int64_t K, int static_weights, int* status, cudaStream_t stream) {
   using namespace w4s;
