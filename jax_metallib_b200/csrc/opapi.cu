@@ -12,9 +12,9 @@
 // and accumulation in f32, one final cast; NaN codes propagate.
 //
 // These CUDA-core kernels take any M and f32 or f16 activations, and run where nothing else does (K or groups that are no
-// multiple of 32, unaligned operands) or nothing else is faster (up to three rows, few columns and rows over a short K).  Decode-sized f16 problems (M <= 16) go to the TMA-ring
-// tensor-core kernels of opapi_tc.cu where the shape allows, then to affine_tc_kernel below; the rest goes to the
-// tcgen05 GEMM of opapi_gemm.cu.
+// multiple of 32, unaligned operands) or nothing else is faster (up to three rows, few columns and rows over a short K).
+// Decode-sized f16 problems (M <= 16) go to the TMA-ring tensor-core kernels of opapi_tc.cu where the shape allows, then to
+// affine_tc_kernel below; of the rest, MX formats with f16 activations go to mx_prefill.cu, the others to opapi_gemm.cu.
 #include "opapi_decode.cuh"
 
 namespace qmm {

@@ -19,7 +19,7 @@
 // sixteen promoters that drain the accumulators.
 //
 // Measured (four linears of a layer, before: one warp per four columns on CUDA cores): affine 4-bit, f32, M = 48, 2048 / 5632
-// wide 597 -> 103 us.  Bound by latency, not by a unit: a stage takes 0.9-1.3 us through workers, issuer, tensor core and
+// wide 597 -> 98 us.  Bound by latency, not by a unit: a stage takes 0.9-1.3 us through workers, issuer, tensor core and
 // promoter.
 //
 // What the split cannot represent takes an exact path: a unit whose activations are not finite (inf times

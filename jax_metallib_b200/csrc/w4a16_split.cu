@@ -78,7 +78,9 @@ __device__ __forceinline__ uint32_t weights2(uint32_t w, uint32_t minus_z) {
   return r;
 }
 
-template <int MT, bool ZP>
+// TWO: 17 to 32 rows.  A tile's two halves of 16 rows are tiles of their own, next to each other in the walk (the second finds the
+// weights in L2).
+template <int MT, bool ZP, int TWO>
 __global__ void __launch_bounds__(Smem<MT, ZP>::kThreads, Smem<MT, ZP>::kPerSm)
 w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                    const uint16_t* __restrict__ scales, const uint8_t* __restrict__ zeros, uint16_t* __restrict__ y, int M, int N,
@@ -93,9 +95,7 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
   uint64_t* vacant = ready + PB;     // every CTA of the cluster has read this CTA's partial tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KS = gridDim.x, rank = blockIdx.x;      // the cluster is the grid's x extent
-  // 17 to 32 rows: a tile's two halves of 16 rows are tiles of their own, next to each other in the walk (the second finds the
-  // weights in L2)
-  const int two = M > 16, tiles = N / kCols << two;
+  const int tiles = N / kCols << TWO;
   const int it_begin = (groups * rank) / KS, it_end = (groups * (rank + 1)) / KS;
   cg::cluster_group cluster = cg::this_cluster();
 
@@ -121,7 +121,7 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
       const uint64_t policy = dev::policy_evict_first();
       auto issue_weights = [&](int s, int t, int it) {
         uint8_t* st = smem + s * L::kStage;
-        const size_t col0 = static_cast<size_t>(t >> two) * kCols, row = static_cast<size_t>(it) * N;
+        const size_t col0 = static_cast<size_t>(t >> TWO) * kCols, row = static_cast<size_t>(it) * N;
         dev::mbar_expect_tx(&full[s], kWBytes + 256 + L::kZBytes);
         dev::tma_load_2d_hint(st, &wmap, &full[s], static_cast<int>(col0), it * (kGroup / 2), policy);
         bulk_copy_g2s(st + L::kOffS, scales + row + col0, 256, &full[s]);
@@ -144,8 +144,8 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
           }
           uint8_t* st = smem + s * L::kStage;
           dev::mbar_expect_tx(&full[s], 2 * L::kXBox);   // rows past M arrive as zeros
-          dev::tma_load_2d(st + L::kOffX, &xmap, &full[s], it * kGroup, (t & two) * 16);
-          dev::tma_load_2d(st + L::kOffX + L::kXBox, &xmap, &full[s], it * kGroup + 64, (t & two) * 16);
+          dev::tma_load_2d(st + L::kOffX, &xmap, &full[s], it * kGroup, (t & TWO) * 16);
+          dev::tma_load_2d(st + L::kOffX + L::kXBox, &xmap, &full[s], it * kGroup + 64, (t & TWO) * 16);
         }
       // no copy may still be on its way into this CTA's shared memory when it leaves, whatever the consumers did
       for (int i = n > S ? n - S : 0; i < n; ++i)
@@ -267,7 +267,7 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
       const int b = tile % PB;
       const float* part = reinterpret_cast<const float*>(smem + L::kOffPart + b * 2 * L::kPart);
       if (!wait_cluster_warp(&ready[b], (tile / PB) & 1, status, 124)) break;
-      const int first = (t & two) * 16, rows = min(M - first, MT * 8);
+      const int first = (t & TWO) * 16, rows = min(M - first, MT * 8);
       for (int e = rank * kR + tid; e < rows * (kCols / 2); e += KS * kR) {
         const int m = e / (kCols / 2), c = (e % (kCols / 2)) * 2;
         float2 lo[kMaxCluster], hi[kMaxCluster];
@@ -285,7 +285,7 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             v.x += lo[r].x + hi[r].x;
             v.y += lo[r].y + hi[r].y;
           }
-        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(first + m) * N + static_cast<size_t>(t >> two) * kCols + c) =
+        *reinterpret_cast<uint32_t*>(y + static_cast<size_t>(first + m) * N + static_cast<size_t>(t >> TWO) * kCols + c) =
             dev::pack_bf16x2(v.x, v.y);
       }
       __syncwarp();
@@ -295,15 +295,15 @@ w4a16_split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
   cluster.sync();   // peers keep their shared memory alive until it has been read
 }
 
-template <int MT, bool ZP>
+template <int MT, bool ZP, int TWO>
 static int launch(const CUtensorMap& wmap, const CUtensorMap& xmap, const uint16_t* scales, const uint8_t* zeros, uint16_t* y, int M,
                   int N, int groups, int static_weights, int* status, cudaStream_t stream) {
   using L = Smem<MT, ZP>;
   static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
   static std::atomic<int> resident[kMaxDevices][kMaxCluster + 1];
-  auto kern = w4a16_split_kernel<MT, ZP>;
+  auto kern = w4a16_split_kernel<MT, ZP, TWO>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
-  const Grid g = choose_grid(N / kCols << (M > 16), groups,
+  const Grid g = choose_grid(N / kCols << TWO, groups,
                              [&](int ks) { return resident_clusters(kern, L::kThreads, L::kTotal, L::kPerSm, ks, resident); });
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
@@ -331,11 +331,12 @@ int w4a16_split(const uint16_t* x, const uint8_t* wq, const uint16_t* scales, co
                                   64, CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
   const int m = static_cast<int>(M), n = static_cast<int>(N), g = static_cast<int>(K / kGroup);
-#define QMM_W4S_LAUNCH(MT)                                                                              \
-  (zeros_packed ? launch<MT, true>(wmap, xmap, scales, zeros, y, m, n, g, static_weights, status, stream) \
-                : launch<MT, false>(wmap, xmap, scales, zeros, y, m, n, g, static_weights, status, stream))
-  if (mt == 1) return QMM_W4S_LAUNCH(1);
-  return QMM_W4S_LAUNCH(2);
+#define QMM_W4S_LAUNCH(MT, TWO)                                                                               \
+  (zeros_packed ? launch<MT, true, TWO>(wmap, xmap, scales, zeros, y, m, n, g, static_weights, status, stream) \
+                : launch<MT, false, TWO>(wmap, xmap, scales, zeros, y, m, n, g, static_weights, status, stream))
+  if (mt == 1) return QMM_W4S_LAUNCH(1, 0);
+  if (m <= 16) return QMM_W4S_LAUNCH(2, 0);
+  return QMM_W4S_LAUNCH(2, 1);
 #undef QMM_W4S_LAUNCH
 }
 
