@@ -77,16 +77,16 @@ struct Work {
   int tm2, tn, h0, nh;
 };
 template <bool SPLIT>
-__device__ __forceinline__ bool get_work(int cta, int ctas, int i, int tiles_m2, int tiles_n, int halves, int M, Work& w) {
-  if (SPLIT) {   // row block `cta`, one to a cluster
-    const int blocks_m = (M + BMB - 1) / BMB, bm = cta % blocks_m;
+__device__ __forceinline__ bool get_work(int i, int tiles_m2, int tiles_n, int halves, int M, Work& w) {
+  if (SPLIT) {   // one row block to a cluster
+    const int blocks_m = (M + BMB - 1) / BMB, bm = blockIdx.y % blocks_m;
     w.tm2 = bm >> 1;
-    w.tn = cta / blocks_m;
+    w.tn = blockIdx.y / blocks_m;
     w.h0 = bm & 1;
     w.nh = 1;
     return i == 0;
   }
-  const int v = cta + i * ctas;
+  const int v = blockIdx.x + i * gridDim.x;
   const int total = tiles_m2 * tiles_n * (halves ? 2 : 1);
   if (v >= total) return false;
   const int tile = halves ? (v >> 1) : v;
@@ -122,7 +122,6 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
   const int all_kblocks = (K + BK - 1) / BK;
   const int kb_begin = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * blockIdx.x / gridDim.x) : 0;
   const int kb_end = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * (blockIdx.x + 1) / gridDim.x) : all_kblocks;
-  const int cta = SPLIT ? blockIdx.y : blockIdx.x, ctas = SPLIT ? gridDim.y : gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -150,7 +149,7 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
       uint32_t s = 0, ph = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work<SPLIT>(cta, ctas, i, tiles_m2, tiles_n, halves, M, w); ++i) {
+      for (int i = 0; ok && get_work<SPLIT>(i, tiles_m2, tiles_n, halves, M, w); ++i) {
         if (w.nh == 0) continue;
         for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!dev::mbar_wait(&empty[s], ph ^ 1, status, 11)) { ok = false; break; }
@@ -184,7 +183,7 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
       int items = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work<SPLIT>(cta, ctas, i, tiles_m2, tiles_n, halves, M, w); ++i) {
+      for (int i = 0; ok && get_work<SPLIT>(i, tiles_m2, tiles_n, halves, M, w); ++i) {
         if (w.nh == 0) continue;
         if (!dev::mbar_wait(tempty, (items & 1) ^ 1, status, 12)) break;
         dev::tc_fence_after();
@@ -212,7 +211,7 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
     const uint64_t store_policy = dev::policy_evict_first();
     int items = 0;
     Work w;
-    for (int i = 0; get_work<SPLIT>(cta, ctas, i, tiles_m2, tiles_n, halves, M, w); ++i) {
+    for (int i = 0; get_work<SPLIT>(i, tiles_m2, tiles_n, halves, M, w); ++i) {
       if (w.nh == 0) continue;
       if (!dev::mbar_wait_relaxed_warp(tfull, items & 1, status, 14)) break;
       dev::tc_fence_after();
@@ -224,7 +223,7 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
       // has been consumed once the accumulators are complete); earlier items overlap their plain stores with the
       // loads of the next item, which the producer has already started into the ring
       Work w_next;
-      const bool staged = staged_store && !get_work<SPLIT>(cta, ctas, i + 1, tiles_m2, tiles_n, halves, M, w_next);
+      const bool staged = staged_store && !get_work<SPLIT>(i + 1, tiles_m2, tiles_n, halves, M, w_next);
       const int block = SPLIT ? w.h0 : j;   // (a single block's chunks are shared out among all warps)
       const int row0 = (w.tm2 * 2 + block) * BMB + q * 32;
       const int row = row0 + lane;
@@ -324,7 +323,7 @@ i8gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ 
     __syncwarp();
     split::cluster_sync();
     Work w;
-    if (get_work<SPLIT>(cta, ctas, 0, tiles_m2, tiles_n, halves, M, w) && w.nh > 0) {
+    if (get_work<SPLIT>(0, tiles_m2, tiles_n, halves, M, w) && w.nh > 0) {
       const int row0 = (w.tm2 * 2 + w.h0) * BMB, rows = min(M - row0, BMB);
       const int step = gridDim.x * kThreads, end = rows * (BN / 4);
       for (int e0 = blockIdx.x * kThreads + threadIdx.x; e0 < end; e0 += 2 * step) {
@@ -455,12 +454,14 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tm = p * panel + r % rows;
 }
 
-// Item `i` of CTA `cta` of `G`; false when the CTA is done.  After its full-wave tiles a CTA takes a
+// Item `i` of this CTA (of its cluster); false when there is none.  After its full-wave tiles a CTA takes a
 // contiguous run of the tail's parts (tile-major: part 2h + mh of a tile cut in four is channel
 // block h, row half mh) and works it off in the largest aligned pieces: a whole tile, a channel
 // block with all its rows, or a single part, so that neighbouring parts cost one pipeline fill
 // and use the full-width MMA.
-__device__ __forceinline__ bool get_work(const Sched& sc, int cta, int G, int i, int M, int N, Work& w) {
+template <bool SPLIT>
+__device__ __forceinline__ bool get_work(const Sched& sc, int i, int M, int N, Work& w) {
+  const int cta = SPLIT ? blockIdx.y : blockIdx.x, G = SPLIT ? gridDim.y : gridDim.x;
   int tile, sub = 0, len = 0;  // len: parts covered, in units of 1 / tail_div tile; 0 = whole tile
   const int div = sc.tail_div;
   if (i < sc.full_waves) {
@@ -550,7 +551,6 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
   const int all_kblocks = (K + BK - 1) / BK;
   const int kb_begin = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * blockIdx.x / gridDim.x) : 0;
   const int kb_end = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * (blockIdx.x + 1) / gridDim.x) : all_kblocks;
-  const int cta = SPLIT ? blockIdx.y : blockIdx.x, ctas = SPLIT ? gridDim.y : gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kXStages; ++s) dev::mbar_init(&xfull[s], 1);
@@ -589,7 +589,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       unsigned cnt = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
+      for (int i = 0; ok && get_work<SPLIT>(sc, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
         for (int kb = kb_begin; kb < kb_end; ++kb, ++cnt) {
           const int xs = cnt % kXStages;
@@ -609,7 +609,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       unsigned cnt = 0;
       bool ok = true;
       Work w;
-      for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
+      for (int i = 0; ok && get_work<SPLIT>(sc, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
         for (int kb = kb_begin; kb < kb_end; ++kb, ++cnt) {
           const int ws = cnt % kWStages;
@@ -642,7 +642,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       int items = 0;
       bool ok = true, ready = false;
       Work w;
-      for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
+      for (int i = 0; ok && get_work<SPLIT>(sc, i, M, N, w); ++i) {
         if (w.nh == 0) continue;
         if (!dev::mbar_wait(tempty, (items & 1) ^ 1, status, 22)) break;
         dev::tc_fence_after();
@@ -690,7 +690,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     int items = 0;
     bool ok = true;
     Work w;
-    for (int i = 0; ok && get_work(sc, cta, ctas, i, M, N, w); ++i) {
+    for (int i = 0; ok && get_work<SPLIT>(sc, i, M, N, w); ++i) {
       if (w.nh == 0) continue;
       const int h = w.h0 + hh;
       const bool mine = hh < w.nh;
@@ -837,7 +837,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     __syncwarp();
     split::cluster_sync();
     Work w;
-    if (get_work(sc, cta, ctas, 0, M, N, w) && w.nh > 0) {
+    if (get_work<SPLIT>(sc, 0, M, N, w) && w.nh > 0) {
       const int quads = w.nh * (BNW / 4), m_first = w.tm * sc.rows + w.m_off;
       const int rows = min(M - m_first, w.m_cols), n_first = (w.tn2 * 2 + w.h0) * BNW;
       for (int e = blockIdx.x * kThreads + threadIdx.x; e < rows * quads; e += gridDim.x * kThreads) {
