@@ -436,6 +436,7 @@ struct Sched {
   int panel;  // activation tiles per panel
   int rows;   // rows per tile, a multiple of 32
   int ks;     // CTAs that share the K of a piece
+  float cost;   // estimate in microseconds
 };
 struct Work {
   int tn2, tm;   // tile coordinates (units of 256 channels, of `rows` rows)
@@ -1030,6 +1031,7 @@ static tc::w8::Sched schedule(int64_t M, int64_t N, int64_t K, int wbits, int sm
       if (best_cost < 0.f || cost < best_cost) {
         best_cost = cost;
         best = sc;
+        best.cost = cost;
       }
     }
     // pieces that a share of the SMs holds at once: clusters of CTAs, each with a part of K
@@ -1043,6 +1045,7 @@ static tc::w8::Sched schedule(int64_t M, int64_t N, int64_t K, int wbits, int sm
         if (cost < best_cost) {
           best_cost = cost;
           best = sc;
+          best.cost = cost;
         }
       }
   }
@@ -1055,7 +1058,7 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
                               uint16_t* y, int64_t M, int64_t N, int64_t K, int64_t ldy, uint32_t flags,
                               uint32_t* signal, uint32_t* arrive, cudaStream_t stream) {
   using namespace tc::w8;
-  const int sms = gemm_ctas();  // persistent CTAs of this launch
+  const int sms = gemm_ctas();  // persistent CTAs of a launch
   static std::atomic<int> resident[kMaxDevices][split::kMaxCluster + 1];
   static std::atomic<uint64_t> configured[2] = {};  // per device (one mask per instance of the kernel)
   auto kern = w8a16_kernel<WBITS, false>;
@@ -1064,41 +1067,68 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(split_kern), kSmemBytes, configured[1])) return rc;
   // results that go to several GPUs or are announced, and callers with a limit on the CTAs, keep one CTA to a piece
   const bool may_split = sms == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr;
-  const Sched sc = schedule(M, N, K, WBITS, sms, [&](int ks) {
-    return may_split ? split::resident_clusters(split_kern, kThreads, kSmemBytes, 1, ks, resident) : 0;
-  });
-  CUtensorMap wmap, xmap;
-  constexpr int kRawRows = (WBITS == 8) ? BK : BK / 2;
-  if (int rc = make_tensor_map_2d(&wmap, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)(WBITS == 8 ? K : K / 2),
-                                  (uint64_t)N, (uint64_t)N, kRawRows, BNW, CU_TENSOR_MAP_SWIZZLE_128B))
-    return rc;
-  if (int rc = make_tensor_map_2d(&xmap, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M,
-                                  (uint64_t)K, (uint64_t)K * 2, sc.rows, BK, CU_TENSOR_MAP_SWIZZLE_128B))
-    return rc;
-  // operand "a" of the MMA = weights (bf16, from TMEM), "b" = activations (bf16, K-major)
-  const uint32_t idesc_full = dev::make_idesc(/*c=f32*/ 1, /*bf16*/ 1, /*bf16*/ 1, 0, /*b K-major*/ 0, BNW, sc.rows);
-  const uint32_t idesc_half = dev::make_idesc(1, 1, 1, 0, 0, BNW, sc.rows / 2);
-  if (sc.ks > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[2];
-    cfg.gridDim = dim3(sc.ks, sc.tail_tiles * sc.tail_div);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemBytes;
-    cfg.stream = stream;
-    split::set_attrs(cfg, attr, sc.ks);
-    QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kern, wmap, xmap, scale, gq, y, (int)M, (int)N, (int)K, (long long)ldy, idesc_full,
-                                    idesc_half, sc, flags, signal, arrive, device_status_word()));
-    return QMM_OK;
+  auto plan = [&](int64_t rows) {
+    return schedule(rows, N, K, WBITS, sms, [&](int ks) {
+      return may_split ? split::resident_clusters(split_kern, kThreads, kSmemBytes, 1, ks, resident) : 0;
+    });
+  };
+  Sched sc = plan(M), rest = {};
+  // Few rounds of tiles that fill the SMs badly: the first rows go in one launch and the others in a second, which splits K where
+  // its tiles are few, if that is estimated to be quicker by more than the estimate's error.  One launch, two: 14336 x 4096, M = 777
+  // int8 117 -> 95 us, int4 141 -> 105; 8192 x 8192, M = 777 137 -> 106, 167 -> 119; 16128 x 5120, M = 1587 242 -> 205, 285 -> 232;
+  // 4096 x 4096, M = 2048 68 -> 62, 81 -> 70.  With more than three rounds the gaps are small and the estimate is off by as much:
+  // 5120 x 32256, M = 2048, int4 626 -> 682.  Independent launches fill one another's gaps and stay whole.
+  int64_t first = M;
+  if (may_split && !(flags & QMM_GEMM_INDEPENDENT) && sc.full_waves <= 3 && sc.cost > 30.f) {
+    const int64_t tiles_m = (M + kMaxRows - 1) / kMaxRows;
+    float best = 0.96f * sc.cost;
+    for (int64_t t = tiles_m > 6 ? tiles_m - 5 : 1; t < tiles_m; ++t) {
+      const Sched head = plan(t * kMaxRows), tail = plan(M - t * kMaxRows);
+      if (head.cost + tail.cost + 2.f < best) {
+        best = head.cost + tail.cost + 2.f;
+        first = t * kMaxRows;
+        sc = head;
+        rest = tail;
+      }
+    }
   }
-  const int grid = sc.full_waves > 0 ? sms : (sc.tail_tiles * sc.tail_div < sms ? sc.tail_tiles * sc.tail_div : sms);
-  // Programmatic stream serialization: the CTAs of this launch may become resident while the
-  // kernel ahead of it drains; they order themselves behind it inside the kernel (or not at all
-  // when the caller states independence, which fills the last, partly idle round of one launch
-  // with the first tiles of the next).
-  QMM_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, wmap, xmap, scale, gq, y, (int)M,
-                          (int)N, (int)K, (long long)ldy, idesc_full, idesc_half, sc, flags, signal, arrive,
-                          device_status_word()));
-  return QMM_OK;
+  auto launch = [&](const Sched& sc, int64_t row, int64_t rows) -> int {
+    uint16_t* out = y + row * ldy;
+    CUtensorMap wmap, xmap;
+    constexpr int kRawRows = (WBITS == 8) ? BK : BK / 2;
+    if (int rc = make_tensor_map_2d(&wmap, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)(WBITS == 8 ? K : K / 2),
+                                    (uint64_t)N, (uint64_t)N, kRawRows, BNW, CU_TENSOR_MAP_SWIZZLE_128B))
+      return rc;
+    if (int rc = make_tensor_map_2d(&xmap, x + row * K, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)rows,
+                                    (uint64_t)K, (uint64_t)K * 2, sc.rows, BK, CU_TENSOR_MAP_SWIZZLE_128B))
+      return rc;
+    // operand "a" of the MMA = weights (bf16, from TMEM), "b" = activations (bf16, K-major)
+    const uint32_t idesc_full = dev::make_idesc(/*c=f32*/ 1, /*bf16*/ 1, /*bf16*/ 1, 0, /*b K-major*/ 0, BNW, sc.rows);
+    const uint32_t idesc_half = dev::make_idesc(1, 1, 1, 0, 0, BNW, sc.rows / 2);
+    if (sc.ks > 1) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[2];
+      cfg.gridDim = dim3(sc.ks, sc.tail_tiles * sc.tail_div);
+      cfg.blockDim = dim3(kThreads);
+      cfg.dynamicSmemBytes = kSmemBytes;
+      cfg.stream = stream;
+      split::set_attrs(cfg, attr, sc.ks);
+      QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kern, wmap, xmap, scale, gq, out, (int)rows, (int)N, (int)K, (long long)ldy, idesc_full,
+                                      idesc_half, sc, flags, signal, arrive, device_status_word()));
+      return QMM_OK;
+    }
+    const int grid = sc.full_waves > 0 ? sms : (sc.tail_tiles * sc.tail_div < sms ? sc.tail_tiles * sc.tail_div : sms);
+    // Programmatic stream serialization: the CTAs of this launch may become resident while the
+    // kernel ahead of it drains; they order themselves behind it inside the kernel (or not at all
+    // when the caller states independence, which fills the last, partly idle round of one launch
+    // with the first tiles of the next).
+    QMM_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, wmap, xmap, scale, gq, out, (int)rows,
+                            (int)N, (int)K, (long long)ldy, idesc_full, idesc_half, sc, flags, signal, arrive,
+                            device_status_word()));
+    return QMM_OK;
+  };
+  if (int rc = launch(sc, 0, first)) return rc;
+  return first < M ? launch(rest, first, M - first) : QMM_OK;
 }
 
 int w8a16_tcgen05(const uint16_t* x, const int8_t* w, const float* scale, uint16_t* y, int64_t M,

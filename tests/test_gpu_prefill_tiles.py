@@ -22,9 +22,11 @@ LINE = [(16, 64, 18960), (17, 8, 1024), (17, 64, 976), (20, 72, 4112), (32, 128,
 # K split over clusters: few pieces, shares of one stage and of different lengths, edges of rows and columns
 SPLIT = [(33, 16384, 128), (40, 8200, 144), (160, 4096, 400), (192, 14336, 1040), (193, 2048, 1792), (300, 1032, 768),
          (500, 5120, 512), (64, 14336, 4096), (1200, 2048, 256)]
+# rows in two launches
+TWO = [(777, 14336, 4096), (1587, 8192, 5120), (801, 8200, 4112)]
 
 
-@pytest.mark.parametrize("m,k,n", SHAPES + LINE + SPLIT)
+@pytest.mark.parametrize("m,k,n", SHAPES + LINE + SPLIT + TWO)
 def test_int8_weights(cuda, m, k, n):
     g = torch.Generator(device="cuda").manual_seed(m + k + n)
     x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
@@ -39,7 +41,7 @@ def test_int8_weights(cuda, m, k, n):
 
 
 @pytest.mark.parametrize("packed", [True, False])
-@pytest.mark.parametrize("m,k,n", [(m, max(128, k // 128 * 128), (n + 127) // 128 * 128) for m, k, n in SHAPES + SPLIT])
+@pytest.mark.parametrize("m,k,n", [(m, max(128, k // 128 * 128), (n + 127) // 128 * 128) for m, k, n in SHAPES + SPLIT + TWO])
 def test_int4_weights(cuda, m, k, n, packed):
     g = torch.Generator(device="cuda").manual_seed(m + k + n)
     x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
