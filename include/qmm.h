@@ -116,13 +116,13 @@ QMM_API int qmm_w8a32_perchannel(const float* x, const int8_t* w, const float* s
  * bf16 operands, f32 accumulation, one rounding to the declared result type).
  * ldy is the row stride of y in elements (>= N), so that a rank holding a
  * column shard can write straight into its slice of the gathered output.
- * tcgen05 (kind::f16) GEMM with the int8->bf16 conversion done in shared
- * memory.  The tensor-core route needs K % 8 == 0, N % 16 == 0, an even ldy
+ * tcgen05 (kind::f16) GEMM whose weights are converted to bf16 on their way
+ * into tensor memory; K is split over thread-block clusters where its tiles are
+ * few.  The tensor-core route needs K % 8 == 0, N % 16 == 0, an even ldy
  * and 16-byte aligned x and w (what TMA can address); any other shape runs on
  * a plain CUDA-core kernel, and so does M * N < 16384 with K < 128.  On that
- * route few rows (M <= 32, or ceil(M / 32) * N <= 23000; 128 per SM for
- * K < 2048, 8192 for K < 256) run a kernel that splits K over thread-block
- * clusters. */
+ * route few rows (M <= 16; more for few columns and weights) run an HBM-bound
+ * kernel that splits K over clusters as well. */
 QMM_API int qmm_w8a16_perchannel(const uint16_t* x_bf16, const int8_t* w, const float* scale,
                                  uint16_t* y_bf16, int64_t M, int64_t N, int64_t K, int64_t ldy,
                                  void* stream);
@@ -233,10 +233,10 @@ QMM_API int qmm_i8i8_i32(const void* a, const void* b, int32_t* acc, const float
  * Zero points are 4-bit values (0..15) in either form.
  * Requires group == 128, K % 128 == 0, N % 128 == 0, M >= 1.
  * M <= 32 runs an HBM-bound decode kernel (weights read once; K split over
- * thread-block clusters for M <= 16, N <= 16384 and N * K from 65536 to 75
- * million, else over all SMs with the partial sums in the workspace); larger M
+ * thread-block clusters for all but the widest and the smallest matrices, else
+ * over all SMs with the partial sums in the workspace); larger M
  * runs a tcgen05 GEMM whose converter warps dequantise the
- * nibbles in shared memory: bf16((q - z) * s) per weight, which is what the
+ * nibbles into tensor memory: bf16((q - z) * s) per weight, which is what the
  * StableHLO chain computes in bf16, f32 accumulation, one rounding of the
  * result.  That route needs no workspace (qmm_w4a16_g128_workspace_bytes
  * returns 0 for M > 32 and workspace may be NULL) and ignores flags.
