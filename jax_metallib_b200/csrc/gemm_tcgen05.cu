@@ -1075,11 +1075,13 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
   Sched sc = plan(M), rest = {};
   // Few rounds of tiles that fill the SMs badly: the first rows go in one launch and the others in a second, which splits K where
   // its tiles are few, if that is estimated to be quicker by more than the estimate's error.  One launch, two: 14336 x 4096, M = 777
-  // int8 117 -> 95 us, int4 141 -> 105; 8192 x 8192, M = 777 137 -> 106, 167 -> 119; 16128 x 5120, M = 1587 242 -> 205, 285 -> 232;
-  // 4096 x 4096, M = 2048 68 -> 62, 81 -> 70.  With more than three rounds the gaps are small and the estimate is off by as much:
-  // 5120 x 32256, M = 2048, int4 626 -> 682.  Independent launches fill one another's gaps and stay whole.
+  // int8 108 -> 95 us, int4 138 -> 105; 8192 x 8192, M = 777 123 -> 99, 148 -> 112; 16128 x 5120, M = 1587 243 -> 204, 288 -> 232;
+  // 4096 x 4096, M = 2048 68 -> 62, 81 -> 70.  The worst of 200 calls (M 400 to 3333) is 2 % slower (4096 x 6144, M = 2048 80.4,
+  // 82.2).  Below 50 us the second launch costs too much (2048 x 11264, M = 640, int4 47.7, 51.3), and with more than three rounds
+  // the gaps are small and the estimate is off by as much (5120 x 32256, M = 2048, int4 626, 682).  Independent launches fill one
+  // another's gaps and stay whole.
   int64_t first = M;
-  if (may_split && !(flags & QMM_GEMM_INDEPENDENT) && sc.full_waves <= 3 && sc.cost > 30.f) {
+  if (may_split && !(flags & QMM_GEMM_INDEPENDENT) && sc.full_waves <= 3 && sc.cost > 50.f) {
     const int64_t tiles_m = (M + kMaxRows - 1) / kMaxRows;
     float best = 0.96f * sc.cost;
     for (int64_t t = tiles_m > 6 ? tiles_m - 5 : 1; t < tiles_m; ++t) {
