@@ -108,12 +108,15 @@ __device__ __forceinline__ void copy_part(int w, uint32_t dst, const uint8_t* sr
   else copy_pieces<8, ROWS, BYTES>(dst, src, row0, rows, col0, cols, lt, place);
 }
 
-template <int MT, bool AU, bool BU, bool TMA>
-__global__ void __launch_bounds__(Smem<MT, TMA>::kThreads, Smem<MT, TMA>::kPerSm)
+// LOAD: how a stage arrives.
+enum Load { kWords, kPieces, kTma };
+template <int MT, bool AU, bool BU, Load LOAD>
+__global__ void __launch_bounds__(Smem<MT, LOAD == kTma>::kThreads, Smem<MT, LOAD == kTma>::kPerSm)
 i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ a,
                  const uint8_t* __restrict__ b, int32_t* __restrict__ acc_out, float* __restrict__ out,
                  const float* __restrict__ row_scale, const float* __restrict__ col_scale, int M, int N, int K, int stages_total,
                  int pairs, int a_piece, int b_piece, int* status) {
+  constexpr bool TMA = LOAD == kTma;
   using L = Smem<MT, TMA>;
   constexpr int S = L::kStages, PB = L::kPartBufs;
   extern __shared__ uint8_t smem_raw[];
@@ -136,7 +139,7 @@ i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       dev::tma_prefetch_desc(&xmap);
     }
     for (int s = 0; s < S; ++s) {
-      dev::mbar_init(&full[s], TMA ? 1 : kLoaderWarps * (a_piece ? 32 : 1));
+      dev::mbar_init(&full[s], TMA ? 1 : kLoaderWarps * (LOAD == kPieces ? 32 : 1));
       dev::mbar_init(&empty[s], kConsumerWarps);
     }
     for (int b = 0; b < PB; ++b) {
@@ -173,7 +176,7 @@ i8_skinny_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
           if (!dev::mbar_wait_relaxed(&full[i % S], (i / S) & 1, status, 111)) break;
       }
       __syncwarp();
-    } else if (a_piece) {
+    } else if (LOAD == kPieces) {
       const int lt = threadIdx.x - kConsumerWarps * 32;   // 0 .. 127
       for (int t = blockIdx.y; ok && t < tiles; t += gridDim.y) {
         const int col0 = (t / row_tiles) * kCols, row0 = (t % row_tiles) * MT * 8;
@@ -380,8 +383,15 @@ struct Args {
   int M, N, K;
 };
 
-template <int MT, bool AU, bool BU, bool TMA>
+// The largest piece that a pitch and an address are made of, 8 or 16 bytes, or 0.
+static int piece(const uint8_t* at, int pitch) {
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(at) | static_cast<uintptr_t>(pitch);
+  return bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : 0;
+}
+
+template <int MT, bool AU, bool BU, Load LOAD>
 static int launch(const Args& p, cudaStream_t stream) {
+  constexpr bool TMA = LOAD == kTma;
   using L = Smem<MT, TMA>;
   CUtensorMap wmap = {}, xmap = {};
   if (TMA) {
@@ -394,7 +404,7 @@ static int launch(const Args& p, cudaStream_t stream) {
   }
   static std::atomic<uint64_t> configured{0};  // per device (one mask per template instance)
   static std::atomic<int> resident[kMaxDevices][kMaxCluster + 1];
-  auto kern = i8_skinny_kernel<MT, AU, BU, TMA>;
+  auto kern = i8_skinny_kernel<MT, AU, BU, LOAD>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kTotal, configured)) return rc;
   const int stages_total = (p.K + kBK - 1) / kBK;
   // a limit leaves SMs to a collective: one CTA to each of the others
@@ -410,28 +420,22 @@ static int launch(const Args& p, cudaStream_t stream) {
   cfg.stream = stream;
   set_attrs(cfg, attr, g.ks);
   const int pairs = p.N % 2 == 0 && aligned(p.acc, 8) && aligned(p.out, 8);
-  // the largest piece that a pitch and an address are made of, 8 or 16 bytes; one operand without one: shifted words for both
-  auto piece = [](const uint8_t* at, int pitch) {
-    const uintptr_t bits = reinterpret_cast<uintptr_t>(at) | static_cast<uintptr_t>(pitch);
-    return bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : 0;
-  };
-  const int pa = TMA ? 0 : piece(p.a, p.K), pb = TMA ? 0 : piece(p.b, p.N);
   QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, wmap, xmap, p.a, p.b, p.acc, p.out, p.rs, p.cs, p.M, p.N, p.K, stages_total, pairs,
-                                  pb ? pa : 0, pa ? pb : 0, device_status_word()));
+                                  piece(p.a, p.K), piece(p.b, p.N), device_status_word()));
   return QMM_OK;
 }
 
-template <bool AU, bool BU, bool TMA>
+template <bool AU, bool BU, Load LOAD>
 static int launch_rows(const Args& p, cudaStream_t stream) {
-  if (p.M <= 8) return launch<1, AU, BU, TMA>(p, stream);
-  if (p.M <= 16) return launch<2, AU, BU, TMA>(p, stream);
-  if (p.M <= 32) return launch<4, AU, BU, TMA>(p, stream);
-  return launch<8, AU, BU, TMA>(p, stream);
+  if (p.M <= 8) return launch<1, AU, BU, LOAD>(p, stream);
+  if (p.M <= 16) return launch<2, AU, BU, LOAD>(p, stream);
+  if (p.M <= 32) return launch<4, AU, BU, LOAD>(p, stream);
+  return launch<8, AU, BU, LOAD>(p, stream);
 }
-template <bool TMA>
+template <Load LOAD>
 static int launch_types(const Args& p, int au, int bu, cudaStream_t stream) {
-  if (au) return bu ? launch_rows<true, true, TMA>(p, stream) : launch_rows<true, false, TMA>(p, stream);
-  return bu ? launch_rows<false, true, TMA>(p, stream) : launch_rows<false, false, TMA>(p, stream);
+  if (au) return bu ? launch_rows<true, true, LOAD>(p, stream) : launch_rows<true, false, LOAD>(p, stream);
+  return bu ? launch_rows<false, true, LOAD>(p, stream) : launch_rows<false, false, LOAD>(p, stream);
 }
 
 }  // namespace i8s
@@ -441,8 +445,10 @@ int i8_skinny(const void* a, const void* b, int32_t* acc, const float* row_scale
               int64_t N, int64_t K, int a_unsigned, int b_unsigned, bool aligned_rows, cudaStream_t stream) {
   const i8s::Args p = {static_cast<const uint8_t*>(a), static_cast<const uint8_t*>(b), acc, out, row_scale, col_scale,
                        static_cast<int>(M), static_cast<int>(N), static_cast<int>(K)};
-  return aligned_rows ? i8s::launch_types<true>(p, a_unsigned, b_unsigned, stream)
-                      : i8s::launch_types<false>(p, a_unsigned, b_unsigned, stream);
+  if (aligned_rows) return i8s::launch_types<i8s::kTma>(p, a_unsigned, b_unsigned, stream);
+  // one operand without pieces: shifted words for both
+  if (i8s::piece(p.a, p.K) && i8s::piece(p.b, p.N)) return i8s::launch_types<i8s::kPieces>(p, a_unsigned, b_unsigned, stream);
+  return i8s::launch_types<i8s::kWords>(p, a_unsigned, b_unsigned, stream);
 }
 
 }  // namespace qmm
