@@ -278,7 +278,7 @@ def build_weights(torch, synthetic, device, rank, world, layers):
 # (K, N), from the ncu captures summarised in profiles/w8a16_kernel_dram_traffic.md.  Shapes that
 # were not captured are scaled by FLOPs from the nearest captured shape of the same K and said so.
 MEASURED_TRAFFIC = {
-    (8192, 10240): 417.29e6, (8192, 8192): 339.71e6, (8192, 57344): 2020.91e6, (28672, 8192): 1304.28e6,  # full width
+    (8192, 10240): 457.78e6, (8192, 8192): 363.96e6, (8192, 57344): 2193.87e6, (28672, 8192): 1491.95e6,  # full width
     (8192, 5120): 231.95e6, (8192, 4096): 199.90e6, (8192, 28672): 1065.67e6, (28672, 4096): 794.24e6,    # N / 2
     (8192, 2560): 115.98e6, (8192, 2048): 85.28e6, (8192, 14336): 545.10e6, (28672, 2048): 295.03e6,      # N / 4
     (8192, 1280): 164.82e6, (8192, 1024): 77.20e6, (8192, 7168): 295.67e6, (28672, 1024): 266.00e6,       # N / 8
