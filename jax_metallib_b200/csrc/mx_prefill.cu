@@ -24,6 +24,7 @@
 // column in registers (setmaxnreg).  Two or more accumulators, so that neither a promotion nor the store of a tile stops the
 // tensor core.  Where tiles are few, the CTAs of a cluster share one, each with a slice of K, and add their parts over
 // distributed shared memory in a fixed order.
+#include "mx_rings.h"
 #include "opapi_convert.cuh"
 #include "split_k.cuh"
 
@@ -36,13 +37,11 @@ namespace mxp {
 using namespace opg;
 
 constexpr int BN = 128;               // output columns per tile
-constexpr int BK = 128;               // k per stage: waits and arrivals cost a warp some 100 clocks each, a stage of 64 k was bound by them
+constexpr int BK = kStageK;
 constexpr int kRawBox = BN * 128;     // 16 KB of raw weights
 constexpr int kUnitK = 512;           // k per accumulator, MX formats
 constexpr int kInfo = 16;             // tiles whose columns may be marked
-constexpr int kConsumed = 8;          // stages whose retirement can be asked for
 constexpr int kMaxRows = 192;
-constexpr int kGroups = 2;            // warpgroups of converters
 constexpr int kFirstConverter = 4, kFirstPromoter = kFirstConverter + 4 * kGroups, kThreads = (kFirstPromoter + 8) * 32;
 constexpr int kLaunchRegs = 65536 / kThreads / 8 * 8;
 constexpr uint32_t kMarked = 0x7FC0F1A6u;   // partial result of a column that has to be computed again
@@ -51,13 +50,11 @@ template <int FMT, int CPT>   // CPT: rows of a tile (accumulator columns) per p
 struct Cfg {
   static constexpr int kBits = FMT == kMxfp8 ? 8 : 4;
   static constexpr bool kE8m0 = FMT == kMxfp4 || FMT == kMxfp8;
-  static constexpr int kStagesPerBox = 128 * 8 / kBits / BK;
-  static constexpr int kSlots = CPT == 96 ? 2 : 4;      // stages of converted weights in TMEM
+  static constexpr Rings kRings = rings(kBits, CPT);
+  static_assert(sound(kRings), "waits by parity");
+  static constexpr int kStagesPerBox = kRings.stages_per_box, kSlots = kRings.slots, kXStages = kRings.x_stages, kRawBoxes = kRings.raw_boxes;
   static constexpr int kRows = 2 * CPT;
   static constexpr int kXBytes = kRows * BK * 2;
-  // activations and raw weights in flight: a copy takes about 1 us from request to arrival, a stage's MMAs 0.1 - 0.4 us
-  static constexpr int kXStages = CPT == 96 ? 3 : (CPT == 64 ? (kBits == 8 ? 3 : 4) : (kBits == 8 ? 6 : 8));
-  static constexpr int kRawBoxes = CPT == 96 || kBits == 4 ? 4 : 6;
   static constexpr int kAccBase = kSlots * (BK / 2);            // first TMEM column of the accumulators
   static constexpr int kAccBufs = (512 - kAccBase) / kRows;
   static constexpr int kOffRaw = kXStages * kXBytes;
@@ -68,7 +65,7 @@ struct Cfg {
   // scale that brings the largest element of a unit's largest scale just below f16's limit, and the smallest power of
   // two of a group's factor at which the last bit of an element is still there
   static constexpr int kUp = FMT == kMxfp8 ? 7 : 13, kLowest = FMT == kMxfp8 ? -15 : -23;
-  static_assert(kAccBufs >= 2 && kSlots <= kConsumed && kXStages <= kConsumed && kRawBoxes % kGroups == 0 && kSlots + kAccBufs + 3 <= kInfo, "ring sizes");
+  static_assert(kAccBufs >= 2 && kSlots + kAccBufs + 3 <= kInfo, "ring sizes");
   // registers of a thread: producers and issuer, converters, promoters
   static constexpr int kMiscRegs = 40, kPromoterRegs = CPT == 96 ? 136 : 120, kConverterRegs = 216 - kPromoterRegs;
   static_assert(kMiscRegs <= kLaunchRegs && kConverterRegs <= kLaunchRegs && kPromoterRegs >= kLaunchRegs, "what shrinks and what grows");
@@ -298,8 +295,7 @@ mx_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
       const uint8_t* srow = row_of(t);
       uint4 us = make_uint4(0u, 0u, 0u, 0u);
       int ref = 0, unit = -1;
-      // The groups take the stages of all tiles in turn, so that a group has seen, with its stage before, the phase ahead of
-      // the one that it waits for next (a parity says no more than that).
+      // The groups take the stages of all tiles in turn.  What their waits by parity rely on: mx_rings.h.
       const int first = first_stage(cnt0);
       if (first >= stages) ask_tile(t + gridDim.y, cnt0 + stages);
       for (int st = first; st < stages; st += kGroups) {
