@@ -1,5 +1,5 @@
 // The torch-facing calls of ops.py and quantized.py in the form that programs make in earnest: plain, contiguous CUDA
-// tensors of the right types and shapes.  Each function checks its arguments, allocates the result, hands raw pointers and
+// tensors of the right types and shapes, all on the current device.  Each function checks its arguments, allocates the result, hands raw pointers and
 // the current stream to libqmm.so and returns the result.  What it does not recognise it declines (returns None): the Python
 // code behind it then takes the call, with its conversions and its error messages.  A status other than QMM_OK comes back as
 // an int.
@@ -9,7 +9,9 @@
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Device.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <initializer_list>
@@ -38,8 +40,25 @@ const at::Tensor* plain(PyObject* o) {
   if (!t.defined() || !t.is_cuda() || t.layout() != c10::kStrided || t.key_set().has_any(special) || !t.is_contiguous()) return nullptr;
   return &t;
 }
+// Whether all of them are CUDA device number `current`: the library works with the current device's stream, SMs and status word,
+// and another device's memory is nothing that it may be pointed at.
+bool all_on(const c10::Device* devices, size_t n, c10::DeviceIndex current) {
+  for (size_t i = 0; i < n; ++i)
+    if (!devices[i].is_cuda() || devices[i].index() != current) return false;
+  return true;
+}
+constexpr size_t kMaxOperands = 4;
+// The tensors behind a[0 .. n), if a kernel may be pointed at all of them.
+bool operands(PyObject* const* a, size_t n, const at::Tensor** t) {
+  c10::Device devices[kMaxOperands] = {c10::kCPU, c10::kCPU, c10::kCPU, c10::kCPU};
+  for (size_t i = 0; i < n; ++i) {
+    if (!(t[i] = plain(a[i]))) return false;
+    devices[i] = t[i]->device();
+  }
+  return all_on(devices, n, c10::cuda::current_device());
+}
 bool is(const at::Tensor* t, c10::ScalarType type, std::initializer_list<int64_t> shape) {
-  return t != nullptr && t->scalar_type() == type && t->sizes() == c10::IntArrayRef(shape);
+  return t->scalar_type() == type && t->sizes() == c10::IntArrayRef(shape);
 }
 // No mode is to see the allocation (it would be Python's call otherwise), and the library is there.
 bool ready() {
@@ -72,8 +91,10 @@ PyObject* guarded(Fn fn) {
 PyObject* w8a32(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     if (n != 3 || !ready()) Py_RETURN_NONE;
-    const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *s = plain(a[2]);
-    if (!x || !w || !s || x->scalar_type() != c10::kFloat || x->dim() < 1 || w->dim() != 2 || x->numel() == 0) Py_RETURN_NONE;
+    const at::Tensor* t[3];
+    if (!operands(a, 3, t)) Py_RETURN_NONE;
+    const at::Tensor *x = t[0], *w = t[1], *s = t[2];
+    if (x->scalar_type() != c10::kFloat || x->dim() < 1 || w->dim() != 2 || x->numel() == 0) Py_RETURN_NONE;
     const int64_t K = x->size(-1), N = w->size(1), M = x->numel() / K;
     if (!is(w, c10::kChar, {K, N}) || !is(s, c10::kFloat, {N})) Py_RETURN_NONE;
     at::Tensor y = result(*x, N, c10::kFloat);
@@ -87,8 +108,10 @@ PyObject* w8a32(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* w8a16(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     if (n != 3 || !ready()) Py_RETURN_NONE;
-    const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *s = plain(a[2]);
-    if (!x || !w || !s || x->scalar_type() != c10::kBFloat16 || x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
+    const at::Tensor* t[3];
+    if (!operands(a, 3, t)) Py_RETURN_NONE;
+    const at::Tensor *x = t[0], *w = t[1], *s = t[2];
+    if (x->scalar_type() != c10::kBFloat16 || x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
     const int64_t M = x->size(0), K = x->size(1), N = w->size(1);
     if (!is(w, c10::kChar, {K, N}) || !is(s, c10::kFloat, {N})) Py_RETURN_NONE;
     at::Tensor y = result(*x, N, c10::kBFloat16);
@@ -106,17 +129,18 @@ PyObject* i8_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n != 5 || !ready()) Py_RETURN_NONE;
     const bool rescale = a[2] != Py_None, want = a[4] == Py_True;
     if ((a[3] != Py_None) != rescale || (!want && a[4] != Py_False) || (!rescale && !want)) Py_RETURN_NONE;
-    const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
-    if (!x || !w || x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
+    const at::Tensor* t[4];
+    if (!operands(a, rescale ? 4 : 2, t)) Py_RETURN_NONE;
+    const at::Tensor *x = t[0], *w = t[1];
+    if (x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
     const c10::ScalarType tx = x->scalar_type(), tw = w->scalar_type();
     const int64_t M = x->size(0), K = x->size(1), N = w->size(1);
     if ((tx != c10::kChar && tx != c10::kByte) || (tw != c10::kChar && tw != c10::kByte) || w->size(0) != K) Py_RETURN_NONE;
     const float *row = nullptr, *col = nullptr;
     if (rescale) {
-      const at::Tensor *r = plain(a[2]), *c = plain(a[3]);
-      if (!is(r, c10::kFloat, {M}) || !is(c, c10::kFloat, {N})) Py_RETURN_NONE;
-      row = r->const_data_ptr<float>();
-      col = c->const_data_ptr<float>();
+      if (!is(t[2], c10::kFloat, {M}) || !is(t[3], c10::kFloat, {N})) Py_RETURN_NONE;
+      row = t[2]->const_data_ptr<float>();
+      col = t[3]->const_data_ptr<float>();
     }
     at::Tensor acc, out;
     if (want) acc = result(*x, N, c10::kInt);
@@ -142,8 +166,10 @@ PyObject* w4a16(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n != 8 || !ready() || !PyLong_CheckExact(a[5]) || !PyDict_CheckExact(a[7])) Py_RETURN_NONE;
     if ((a[4] != Py_True && a[4] != Py_False) || (a[6] != Py_True && a[6] != Py_False)) Py_RETURN_NONE;
     const bool packed = a[4] == Py_True;
-    const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *s = plain(a[2]), *z = plain(a[3]);
-    if (!x || !w || !s || !z || x->scalar_type() != c10::kBFloat16 || x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
+    const at::Tensor* op[4];
+    if (!operands(a, 4, op)) Py_RETURN_NONE;
+    const at::Tensor *x = op[0], *w = op[1], *s = op[2], *z = op[3];
+    if (x->scalar_type() != c10::kBFloat16 || x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
     const long long group = PyLong_AsLongLong(a[5]);
     const int64_t M = x->size(0), K = x->size(1), N = w->size(1);
     if (group <= 0 || K % group != 0 || K % 2 != 0) {
@@ -167,7 +193,7 @@ PyObject* w4a16(PyObject*, PyObject* const* a, Py_ssize_t n) {
       const at::Tensor* t = plain(buf);
       if (t) ws = *t;
       Py_DECREF(buf);
-      if (!t || t->scalar_type() != c10::kByte || static_cast<size_t>(ws.numel()) < need) Py_RETURN_NONE;
+      if (!t || t->device() != x->device() || t->scalar_type() != c10::kByte || static_cast<size_t>(ws.numel()) < need) Py_RETURN_NONE;
     }
     at::Tensor y = result(*x, N, c10::kBFloat16);
     void* st = stream();
@@ -182,7 +208,7 @@ PyObject* w4a16(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // Activations of the operator API: f16 or f32, [..., K].
 bool activations(const at::Tensor* x, int64_t K, int* dtype) {
-  if (!x || x->dim() < 1 || x->numel() == 0 || x->size(-1) != K) return false;
+  if (x->dim() < 1 || x->numel() == 0 || x->size(-1) != K) return false;
   *dtype = x->scalar_type() == c10::kFloat ? QMM_F32 : QMM_F16;
   return x->scalar_type() == c10::kFloat || x->scalar_type() == c10::kHalf;
 }
@@ -202,10 +228,12 @@ PyObject* mx_matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     long long v[4];   // bits, group, mode + 1, K
     if (n != 7 || !ready() || !integers(a, 3, 7, v) || v[3] % v[1] != 0) Py_RETURN_NONE;
-    const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *s = plain(a[2]);
+    const at::Tensor* t[3];
+    if (!operands(a, 3, t)) Py_RETURN_NONE;
+    const at::Tensor *x = t[0], *w = t[1], *s = t[2];
     const int64_t K = v[3];
     int dtype;
-    if (!activations(x, K, &dtype) || !w || w->dim() != 2) Py_RETURN_NONE;
+    if (!activations(x, K, &dtype) || w->dim() != 2) Py_RETURN_NONE;
     const int64_t N = w->size(0), M = x->numel() / K;
     if (!is(w, c10::kByte, {N, v[0] == 4 ? K / 2 : K}) || !is(s, c10::kByte, {N, K / v[1]})) Py_RETURN_NONE;
     at::Tensor y = result(*x, N, x->scalar_type());
@@ -222,10 +250,12 @@ PyObject* affine_matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     long long v[3];   // bits, group, K
     if (n != 7 || !ready() || !integers(a, 4, 7, v) || (v[0] != 4 && v[0] != 8) || v[2] % v[1] != 0) Py_RETURN_NONE;
-    const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *s = plain(a[2]), *b = plain(a[3]);
+    const at::Tensor* t[4];
+    if (!operands(a, 4, t)) Py_RETURN_NONE;
+    const at::Tensor *x = t[0], *w = t[1], *s = t[2], *b = t[3];
     const int64_t K = v[2];
     int dtype;
-    if (!activations(x, K, &dtype) || !w || w->dim() != 2) Py_RETURN_NONE;
+    if (!activations(x, K, &dtype) || w->dim() != 2) Py_RETURN_NONE;
     const int64_t N = w->size(0), M = x->numel() / K, G = K / v[1];
     if (!(v[0] == 4 ? is(w, c10::kInt, {N, K / 8}) : is(w, c10::kByte, {N, K})) || !is(s, c10::kFloat, {N, G}) || !is(b, c10::kFloat, {N, G}))
       Py_RETURN_NONE;
@@ -235,6 +265,27 @@ PyObject* affine_matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return p_affine(x->const_data_ptr(), w->const_data_ptr(), s->const_data_ptr<float>(), b->const_data_ptr<float>(),
                       y.mutable_data_ptr(), M, N, K, static_cast<int>(v[0]), v[1], dtype, st);
     }), y);
+  });
+}
+
+// one_device(number of the current device, torch.device, ...): what every call above asks of its operands
+PyObject* one_device(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    c10::Device devices[kMaxOperands] = {c10::kCPU, c10::kCPU, c10::kCPU, c10::kCPU};
+    if (n < 1 || n > static_cast<Py_ssize_t>(kMaxOperands) + 1) {
+      PyErr_SetString(PyExc_TypeError, "one_device() takes a number and up to four devices");
+      return nullptr;
+    }
+    const long current = PyLong_AsLong(a[0]);
+    if (current == -1 && PyErr_Occurred()) return nullptr;
+    for (Py_ssize_t i = 1; i < n; ++i) {
+      if (!THPDevice_Check(a[i])) {
+        PyErr_SetString(PyExc_TypeError, "one_device() takes devices");
+        return nullptr;
+      }
+      devices[i - 1] = reinterpret_cast<THPDevice*>(a[i])->device;
+    }
+    return PyBool_FromLong(all_on(devices, static_cast<size_t>(n - 1), static_cast<c10::DeviceIndex>(current)));
   });
 }
 
@@ -267,7 +318,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {METHOD(bind), METHOD(w8a32), METHOD(w8a16), METHOD(i8_dot), METHOD(w4a16), METHOD(mx_matmul),
-                         METHOD(affine_matmul), {nullptr, nullptr, 0, nullptr}};
+                         METHOD(affine_matmul), METHOD(one_device), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

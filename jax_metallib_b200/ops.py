@@ -42,6 +42,13 @@ def _need_cuda(*tensors: torch.Tensor) -> None:
             raise TypeError("quantized-matmul operators run on CUDA tensors only (no CPU fallback)")
         if not t.is_contiguous():
             raise ValueError("tensors must be contiguous (row-major)")
+        if t.device != tensors[0].device:
+            raise ValueError(f"tensors must be on one device, got {tensors[0].device} and {t.device}")
+
+
+def _elsewhere(x: torch.Tensor) -> bool:
+    """Whether a call belongs on another device than the current one: the library works with the current device and its stream."""
+    return x.device.index != torch.cuda.current_device()
 
 
 def w8a32_perchannel(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
@@ -56,6 +63,9 @@ def w8a32_perchannel(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor) -> t
         return _done(y)
     _bind()
     _need_cuda(x, w, scale)
+    if _elsewhere(x):
+        with torch.cuda.device(x.device):
+            return w8a32_perchannel(x, w, scale)
     if x.dtype != torch.float32 or w.dtype != torch.int8 or scale.dtype != torch.float32:
         raise TypeError("expected x float32, w int8, scale float32")
     lead = x.shape[:-1]
@@ -87,6 +97,9 @@ def w8a16_perchannel(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor, out:
             return _done(y)
     _bind()
     _need_cuda(x, w, scale, out)
+    if _elsewhere(x):
+        with torch.cuda.device(x.device):
+            return w8a16_perchannel(x, w, scale, out, out_col_offset, independent)
     if x.dtype != torch.bfloat16 or w.dtype != torch.int8 or scale.dtype != torch.float32:
         raise TypeError("expected x bfloat16, w int8, scale float32")
     if x.ndim != 2 or w.ndim != 2 or x.shape[1] != w.shape[0] or scale.shape != (w.shape[1],):
@@ -125,6 +138,9 @@ def i8_dot(a: torch.Tensor, b: torch.Tensor, row_scale: torch.Tensor | None = No
         return _done(pair)
     _bind()
     _need_cuda(a, b, row_scale, col_scale)
+    if _elsewhere(a):
+        with torch.cuda.device(a.device):
+            return i8_dot(a, b, row_scale, col_scale, want_acc)
     if a.dtype not in (torch.int8, torch.uint8) or b.dtype not in (torch.int8, torch.uint8):
         raise TypeError("operands must be int8 or uint8")
     if a.ndim != 2 or b.ndim != 2 or a.shape[1] != b.shape[0]:
@@ -184,6 +200,10 @@ def w4a16_g128(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, zeros: t
             return _done(y)
     _bind()
     _need_cuda(x, wq, scales, zeros, out, workspace)
+    if _elsewhere(x):
+        with torch.cuda.device(x.device):
+            return w4a16_g128(x, wq, scales, zeros, zeros_packed=zeros_packed, group=group, out=out, workspace=workspace,
+                              static_weights=static_weights)
     if x.dtype != torch.bfloat16 or wq.dtype != torch.uint8 or scales.dtype != torch.bfloat16 or zeros.dtype != torch.uint8:
         raise TypeError("expected x bfloat16, wq uint8, scales bfloat16, zeros uint8")
     if x.ndim != 2 or wq.ndim != 2 or 2 * wq.shape[0] != x.shape[1]:

@@ -318,7 +318,8 @@ def _launch_matmul(x, call, N, K, out_dtype):
     x2 = xt.reshape(-1, K)
     M = x2.shape[0]
     y = torch.empty((M, N), dtype=xt.dtype, device=device)
-    call(x2, y, M, tag, device, torch)
+    with torch.cuda.device(device):   # the library works with the current device and its stream
+        call(x2, y, M, tag, device, torch)
     y = y.reshape(*xt.shape[:-1], N)
     if is_t:
         if out_dtype is not None and not isinstance(out_dtype, torch.dtype):
