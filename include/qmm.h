@@ -242,7 +242,9 @@ QMM_API int qmm_i8i8_i32(const void* a, const void* b, int32_t* acc, const float
  * returns 0 for M > 32 and workspace may be NULL) and ignores flags.
  * workspace (M <= 32): qmm_w4a16_g128_workspace_bytes(M, N, K) bytes, 256-byte
  * aligned, zero-filled before its first use; the kernel leaves it zero-filled,
- * so back-to-back calls on one stream may share it.
+ * so back-to-back calls on one stream may share it.  With
+ * QMM_W4_CLEAR_WORKSPACE its contents do not matter: what has to be zero is
+ * cleared on the stream first, where a kernel runs that uses it.
  * flags: 0, or QMM_W4_STATIC_WEIGHTS when wq, scales and zeros are not written
  * by any work queued earlier on the stream (the usual case for model weights).
  * The kernel is launched with programmatic stream serialization: its blocks
@@ -251,6 +253,7 @@ QMM_API int qmm_i8i8_i32(const void* a, const void* b, int32_t* acc, const float
  * QMM_W4_STATIC_WEIGHTS the first weight tiles are fetched before that point,
  * which hides the launch gap in a decode loop. */
 #define QMM_W4_STATIC_WEIGHTS 1u
+#define QMM_W4_CLEAR_WORKSPACE 2u
 QMM_API size_t qmm_w4a16_g128_workspace_bytes(int64_t M, int64_t N, int64_t K);
 QMM_API int qmm_w4a16_g128(const uint16_t* x_bf16, const uint8_t* wq, const uint16_t* scales_bf16,
                            const uint8_t* zeros, int zeros_packed, uint16_t* y_bf16, int64_t M,

@@ -16,6 +16,7 @@ LIB_PATH = os.environ.get("QMM_LIBRARY_PATH", os.path.join(HERE, "libqmm.so"))
 QMM_F32, QMM_F16, QMM_BF16, QMM_S8, QMM_U8, QMM_S32, QMM_U4, QMM_U32 = range(8)
 QMM_MXFP4, QMM_MXFP8, QMM_NVFP4 = range(3)
 QMM_W4_STATIC_WEIGHTS = 1
+QMM_W4_CLEAR_WORKSPACE = 2
 QMM_ATTN_STATIC_CACHE = 1
 MX_MODE_IDS = {"mxfp4": QMM_MXFP4, "mxfp8": QMM_MXFP8, "nvfp4": QMM_NVFP4}
 

@@ -10,6 +10,7 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -160,7 +161,8 @@ PyObject* i8_dot(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// (x, wq, scales, zeros, zeros_packed, group, static_weights, {(device index,): object whose .buf is the device's workspace})
+// (x, wq, scales, zeros, zeros_packed, group, static_weights, {(device index, stream): object whose .buf is the
+// stream's workspace})
 PyObject* w4a16(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     if (n != 8 || !ready() || !PyLong_CheckExact(a[5]) || !PyDict_CheckExact(a[7])) Py_RETURN_NONE;
@@ -180,8 +182,10 @@ PyObject* w4a16(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!is(w, c10::kByte, {K / 2, N}) || !is(s, c10::kBFloat16, {G, N}) || !is(z, c10::kByte, {G, packed ? N / 2 : N})) Py_RETURN_NONE;
     const size_t need = p_w4_workspace(M, N, K);
     at::Tensor ws;
-    if (need > 0) {   // the device's workspace, if it is there and large enough
-      PyObject* key = Py_BuildValue("(i)", static_cast<int>(x->device().index()));
+    if (need > 0) {   // the stream's workspace, if it is there and large enough; a captured call has its own
+      if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) Py_RETURN_NONE;
+      PyObject* key = Py_BuildValue("(iK)", static_cast<int>(x->device().index()),
+                                    static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream())));
       PyObject* holder = key ? PyDict_GetItemWithError(a[7], key) : nullptr;   // borrowed
       Py_XDECREF(key);
       if (!holder) {

@@ -623,6 +623,7 @@ static int run(const char* name, const uint16_t* x, const uint8_t* wq, const uin
   const size_t counters = counter_bytes(C);
   int* ws_counter = static_cast<int*>(workspace);
   float* ws_partial = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + counters);
+  if (flags & QMM_W4_CLEAR_WORKSPACE) QMM_CUDA_TRY(cudaMemsetAsync(ws_counter, 0, counters, st));
 
   CUtensorMap wmap, xmap;
   if (int rc = make_tensor_map_2d(&wmap, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1,

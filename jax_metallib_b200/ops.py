@@ -11,6 +11,7 @@ non-CUDA tensor is an error (there is no fallback path).
 from __future__ import annotations
 
 import functools
+import threading
 
 import torch
 
@@ -168,7 +169,7 @@ def i8_dot(a: torch.Tensor, b: torch.Tensor, row_scale: torch.Tensor | None = No
 
 
 class W4Workspace:
-    """Scratch for the split-K int4 decode kernel: zeroed once, left zeroed by every call."""
+    """Scratch of one stream for the split-K int4 decode kernel: zeroed once, left zeroed by every call."""
 
     def __init__(self, device: torch.device):
         self.device = device
@@ -180,7 +181,22 @@ class W4Workspace:
         return self.buf
 
 
-_w4_workspaces: dict = {}
+_MAX_W4_WORKSPACES = 32
+_w4_workspaces: dict = {}   # (device index, stream) -> W4Workspace; calls on one stream follow one another and share it
+_w4_lock = threading.Lock()
+
+
+def _w4_workspace(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
+    """The workspace of a stream, allocated with that stream as the current one: what is dropped or replaced goes back to the
+    stream's own pool, where work in flight is ahead of whatever uses the memory next."""
+    key = (device.index, stream)
+    with _w4_lock:
+        ws = _w4_workspaces.get(key)
+        if ws is None:
+            while len(_w4_workspaces) >= _MAX_W4_WORKSPACES:
+                del _w4_workspaces[next(iter(_w4_workspaces))]
+            ws = _w4_workspaces[key] = W4Workspace(device)
+        return ws.get(nbytes)
 
 
 def w4a16_g128(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, zeros: torch.Tensor, *,
@@ -217,16 +233,18 @@ def w4a16_g128(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, zeros: t
         raise ValueError(f"scales/zeros shapes do not match: {tuple(scales.shape)}, {tuple(zeros.shape)}")
     lib = _lib.load()
     need = lib.qmm_w4a16_g128_workspace_bytes(M, N, K)  # 0 for M > 32: the prefill GEMM needs no scratch
+    flags = _lib.QMM_W4_STATIC_WEIGHTS if static_weights else 0
     if workspace is None and need > 0:
-        key = (x.device.index,)
-        ws = _w4_workspaces.setdefault(key, W4Workspace(x.device))
-        workspace = ws.get(need)
+        if torch.cuda.is_current_stream_capturing():   # a graph may run beside its stream's calls and beside other graphs
+            workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
+            flags |= _lib.QMM_W4_CLEAR_WORKSPACE
+        else:
+            workspace = _w4_workspace(x.device, _stream_ptr(), need)
     if out is None:
         out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
     _lib.check(lib.qmm_w4a16_g128(x.data_ptr(), wq.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
                                   1 if zeros_packed else 0, out.data_ptr(), M, N, K, group,
                                   workspace.data_ptr() if workspace is not None else None,
                                   workspace.numel() if workspace is not None else 0,
-                                  _lib.QMM_W4_STATIC_WEIGHTS if static_weights else 0,
-                                  _stream_ptr()))
+                                  flags, _stream_ptr()))
     return out
