@@ -7,7 +7,9 @@ raises.  There is no CPU or framework fallback behind these calls.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
+import warnings
 from ctypes import c_char_p, c_int, c_int64, c_size_t, c_uint, c_void_p
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -219,12 +221,36 @@ def load():
     return lib
 
 
-def bind_calls() -> None:
-    """Give the compiled calls (``_calls``) the entry points of the library that this process has loaded."""
-    from . import _calls
+class _Declines:
+    """In the place of ``_calls`` where there is none: everything is done in Python."""
 
-    lib = load()
-    _calls.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in _calls.ENTRY_POINTS.split()))
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+@functools.cache
+def calls():
+    """The compiled calls of ``ops`` and ``quantized``, for the torch that they were built against."""
+    import torch
+
+    try:
+        from . import _calls
+    except ImportError as e:
+        why = str(e)
+    else:
+        if _calls.TORCH == torch.__version__:
+            return _calls
+        why = f"it was built for torch {_calls.TORCH}"
+    warnings.warn(f"_calls.so is not used ({why}): calls take some 5 us longer; python -m jax_metallib_b200.build builds it",
+                  RuntimeWarning, stacklevel=2)
+    return _Declines()
+
+
+def bind_calls() -> None:
+    """Give the compiled calls the entry points of the library that this process has loaded."""
+    lib, compiled = load(), calls()
+    if not isinstance(compiled, _Declines):
+        compiled.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in compiled.ENTRY_POINTS.split()))
 
 
 def last_error() -> str:

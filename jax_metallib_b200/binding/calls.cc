@@ -329,6 +329,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, methods, nul
 
 PyMODINIT_FUNC PyInit__calls() {
   PyObject* m = PyModule_Create(&module);
-  if (m && PyModule_AddStringConstant(m, "ENTRY_POINTS", kNames) != 0) Py_CLEAR(m);
+  // the torch whose headers this was compiled with; another one lays its classes out as it likes
+  if (m && (PyModule_AddStringConstant(m, "ENTRY_POINTS", kNames) != 0 || PyModule_AddStringConstant(m, "TORCH", QMM_TORCH_VERSION) != 0))
+    Py_CLEAR(m);
   return m;
 }

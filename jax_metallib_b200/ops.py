@@ -15,7 +15,9 @@ import threading
 
 import torch
 
-from . import _calls, _lib
+from . import _lib
+
+_calls = _lib.calls()
 
 
 @functools.cache

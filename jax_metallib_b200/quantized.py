@@ -333,9 +333,7 @@ def quantized_matmul(x, w_packed, scales, *, mode: str = "mxfp4", K: int, out_dt
     """``x[..., M, K] @ dequant(w_packed[N, K//pack], scales[N, K//group])^T`` (reference: quantized.py:995-1074)."""
     cfg = _mode(mode)
     if out_dtype is None and _is_torch(x):
-        from . import _calls
-
-        y = _calls.mx_matmul(x, w_packed, scales, cfg["bits"], cfg["group_size"], _lib.MX_MODE_IDS[mode] + 1, K)
+        y = _lib.calls().mx_matmul(x, w_packed, scales, cfg["bits"], cfg["group_size"], _lib.MX_MODE_IDS[mode] + 1, K)
         if y is not None:
             return _finished(y)
     N = w_packed.shape[0]
@@ -359,9 +357,7 @@ def affine_quantized_matmul(x, w_packed, scales, biases, *, bits: int = 4, group
     """``x[..., M, K] @ dequant(w_packed, scales, biases)^T`` for 4- and 8-bit affine weights
     (reference: quantized.py:1077-1152)."""
     if out_dtype is None and _is_torch(x):
-        from . import _calls
-
-        y = _calls.affine_matmul(x, w_packed, scales, biases, bits, group_size, K)
+        y = _lib.calls().affine_matmul(x, w_packed, scales, biases, bits, group_size, K)
         if y is not None:
             return _finished(y)
     _bits_ok(bits)
