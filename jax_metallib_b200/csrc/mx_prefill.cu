@@ -11,13 +11,14 @@
 // element * scale goes in exactly.  A significand has at most 6 bits; the power-of-two scales of a column are taken relative
 // to the largest of 512 k (a unit), and f16 holds all bits of an element down to 2^-22 (mxfp8) or 2^-36 (mxfp4) of that scale.
 // nvfp4's scale * element always fits.  One accumulator runs over a unit; promoters then add it, times the unit's scale, to f32
-// registers, so that the tensor core's truncated additions stay short.  A column with a group below that range that is not
-// zero is computed again from global memory, with the CUDA cores' arithmetic.
+// registers, so that the tensor core's truncated additions stay short.  A group below that range that is not zero goes in
+// as zeros, and its 32 k are added to the column's sums in f32, from global memory, before the result is rounded.
 //
 // Measured (mxfp8, f16, M = 512; before: a scale group of 32 k per accumulator, both operands in shared memory): four linears
 // of 4096 / 14336 wide 857 -> 296 us; 4096 x 28672 462 -> 122 us, 0.60 of the measured bf16 rate; M = 17, 14336 x 4096 36.9 ->
-// 17.8 us.  Bound by the converters where rows are few (a stage of 128 k takes 0.47 us, their instructions half of it) and near
-// the MMA rate at 192 rows (0.65 us a stage, 0.40 of it MMAs at 1.9 GHz).
+// 17.8 us.  Bound by the converters where rows are few (a stage of 128 k takes 0.47 us, their instructions half of it); at 192 rows
+// MMAs are 0.40 of a stage's 0.65 us at 1.9 GHz.  Groups below the range, mxfp8, M = 512, 14336 x 4096 (none: 65 us): one in every
+// 128th column 69 us, in every 16th 73, in every column 162; 4096 x 28672 (119 us): 155, 178, 724.
 //
 // Persistent CTAs, one per SM.  Warps: TMA of activations, TMA of raw weights, the MMA issuer; two warpgroups of
 // converters that take the 128-k stages in turn; two warpgroups of promoters, a thread of which holds up to 96 rows of a
@@ -44,7 +45,6 @@ constexpr int kInfo = 16;             // tiles whose columns may be marked
 constexpr int kMaxRows = 192;
 constexpr int kFirstConverter = 4, kFirstPromoter = kFirstConverter + 4 * kGroups, kThreads = (kFirstPromoter + 8) * 32;
 constexpr int kLaunchRegs = 65536 / kThreads / 8 * 8;
-constexpr uint32_t kMarked = 0x7FC0F1A6u;   // partial result of a column that has to be computed again
 
 template <int FMT, int CPT>   // CPT: rows of a tile (accumulator columns) per promoter thread, at most
 struct Cfg {
@@ -126,6 +126,142 @@ __device__ __forceinline__ int unit_largest(const uint4& s) {
     m[i] = __vmaxu2(((w[i] & 0x00FF00FFu) + 0x00010001u) & 0x00FF00FFu, (((w[i] >> 8) & 0x00FF00FFu) + 0x00010001u) & 0x00FF00FFu);
   const uint32_t best = __vmaxu2(__vmaxu2(m[0], m[1]), __vmaxu2(m[2], m[3]));
   return max(static_cast<int>(max(best & 0xFFFFu, best >> 16)) - 1, 0);
+}
+
+// What the groups below the range of their unit, which go into the MMAs as zeros, contribute to column n, rows m0 .. m0 + 32 * TIMES
+// - 1: v[t] of a lane, to row m0 + 32 t + lane.  The whole warp does a column: each lane looks for such groups among 16 scales, then
+// takes its rows of each group, 32 k in f32.  Where such a group meets an activation that is not finite, the MMAs' zero times
+// that is not what it should be: bit t of the result says that v[t] is the dot product over k_begin .. k_end itself.
+template <int FMT, int TIMES>
+__device__ __forceinline__ uint32_t small_groups(const __half* x, const uint8_t* w, const uint8_t* scales, int M, int K, int n, int m0,
+                                                 int k_begin, int k_end, float (&v)[TIMES]) {
+  using C = Cfg<FMT, 96>;
+  const int lane = threadIdx.x & 31, G = K / 32, g_end = k_end / 32;
+  const bool vec = G % 16 == 0 && (reinterpret_cast<uintptr_t>(scales) & 15) == 0;
+  const uint8_t* srow = scales + static_cast<size_t>(n) * G;
+  uint32_t lost = 0u;
+#pragma unroll
+  for (int t = 0; t < TIMES; ++t) v[t] = 0.f;
+  for (int first = k_begin / 32; first < g_end; first += 32 * 16) {
+    const int g0 = first + lane * 16;
+    uint32_t mine = 0u;
+    if (g0 < g_end) {
+      const uint4 us = unit_scales(srow, g0, G, vec);
+      const uint32_t word[4] = {us.x, us.y, us.z, us.w};
+      const int ref = unit_largest(us);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int code = (word[j / 4] >> (8 * (j % 4))) & 0xFF;
+        if (g0 + j < g_end && code != 255 && C::kUp - (ref - code) < C::kLowest) mine |= 1u << j;
+      }
+    }
+    for (uint32_t lanes = __ballot_sync(0xFFFFFFFFu, mine != 0u); lanes != 0u; lanes &= lanes - 1u) {
+      const int from = __ffs(lanes) - 1;
+      for (uint32_t groups = __shfl_sync(0xFFFFFFFFu, mine, from); groups != 0u; groups &= groups - 1u) {
+        const int g = first + from * 16 + __ffs(groups) - 1;
+        const uint4* codes = reinterpret_cast<const uint4*>(w + (static_cast<size_t>(n) * K + g * 32) / 8 * C::kBits);
+        uint4 c[C::kBits / 4];
+        uint32_t any = 0u;
+#pragma unroll
+        for (int i = 0; i < C::kBits / 4; ++i) {
+          c[i] = __ldg(codes + i);
+          any |= c[i].x | c[i].y | c[i].z | c[i].w;
+        }
+        if (!(any & (C::kBits == 4 ? 0x77777777u : 0x7F7F7F7Fu))) continue;
+        const float scale = opapi::decode_e8m0(__ldg(srow + g));
+        float sum[TIMES];
+#pragma unroll
+        for (int t = 0; t < TIMES; ++t) sum[t] = 0.f;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {   // 8 k
+          uint4 xv[TIMES];
+#pragma unroll
+          for (int t = 0; t < TIMES; ++t)
+            xv[t] = __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(min(m0 + 32 * t + lane, M - 1)) * K + g * 32) + p);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {   // 2 k
+            const int bit = (p * 8 + i * 2) * C::kBits;
+            const uint4& piece = c[bit / 128];
+            const uint32_t words[4] = {piece.x, piece.y, piece.z, piece.w};
+            const uint32_t two = words[bit / 32 % 4] >> (bit % 32);
+            const float w0 = scale * (C::kBits == 8 ? opapi::decode_e4m3(two & 0xFFu) : opapi::kE2M1[two & 0xFu]);
+            const float w1 = scale * (C::kBits == 8 ? opapi::decode_e4m3(two >> 8 & 0xFFu) : opapi::kE2M1[two >> 4 & 0xFu]);
+#pragma unroll
+            for (int t = 0; t < TIMES; ++t) {
+              const uint32_t h[4] = {xv[t].x, xv[t].y, xv[t].z, xv[t].w};
+              const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[i]));
+              sum[t] = fmaf(f.y, w1, fmaf(f.x, w0, sum[t]));
+            }
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < TIMES; ++t) {
+          v[t] += sum[t];
+          if (!(fabsf(sum[t]) < INFINITY)) lost |= 1u << t;   // finite activations cannot: the scale is far below the largest
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < TIMES; ++t)
+    if (lost >> t & 1u) v[t] = exact_dot_here<FMT, false>(x, w, scales, nullptr, K, 32, min(m0 + 32 * t + lane, M - 1), n, k_begin, k_end);
+  return lost;
+}
+// For a warp's columns n0 .. n0 + 31, those of `columns`, whose sums are in TMEM (lane = column, `rows` rows from m0 on), and into y.
+template <int FMT, int TIMES>
+__device__ __noinline__ void add_small_groups(const __half* x, const uint8_t* w, const uint8_t* scales, __half* y, int M, int N, int K,
+                                              uint32_t taddr, uint32_t columns, int n0, int m0, int rows) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t left = columns; left != 0u; left &= left - 1u) {
+    const int owner = __ffs(left) - 1;
+    float v[TIMES];
+    const uint32_t lost = small_groups<FMT, TIMES>(x, w, scales, M, K, n0 + owner, m0, 0, K, v);
+#pragma unroll
+    for (int t = 0; t < TIMES; ++t) {
+      const uint32_t replaced = __ballot_sync(0xFFFFFFFFu, lost >> t & 1u);
+#pragma unroll 1
+      for (int b = 0; b < 32 && 32 * t + b < rows; b += 8) {
+        uint32_t r[8];
+        dev::tmem_ld_32x8(taddr + 32 * t + b, r);
+        dev::tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float sum = __shfl_sync(0xFFFFFFFFu, v[t], b + i);
+          if (lane == owner) r[i] = __float_as_uint(replaced >> (b + i) & 1u ? sum : __uint_as_float(r[i]) + sum);
+        }
+        dev::tmem_st_32x8(taddr + 32 * t + b, r);
+      }
+    }
+    dev::tc_wait_st();
+  }
+#pragma unroll 1
+  for (int b = 0; b < rows; b += 8) {
+    uint32_t r[8];
+    dev::tmem_ld_32x8(taddr + b, r);
+    dev::tc_wait_ld();
+    if (columns >> lane & 1u) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (m0 + b + i < M) y[static_cast<size_t>(m0 + b + i) * N + n0 + lane] = __float2half_rn(__uint_as_float(r[i]));
+    }
+    __syncwarp();
+  }
+}
+// The same for a slice of K whose sums are in shared memory, [row][BN columns].
+template <int FMT, int TIMES>
+__device__ __noinline__ void add_small_groups(const __half* x, const uint8_t* w, const uint8_t* scales, float* part, int M, int K,
+                                              uint32_t columns, int n0, int m0, int rows, int k_begin, int k_end) {
+  const int lane = threadIdx.x & 31;
+  for (; columns != 0u; columns &= columns - 1u) {
+    const int owner = __ffs(columns) - 1;
+    float v[TIMES];
+    const uint32_t lost = small_groups<FMT, TIMES>(x, w, scales, M, K, n0 + owner, m0, k_begin, k_end, v);
+#pragma unroll
+    for (int t = 0; t < TIMES; ++t) {
+      float* at = part + (32 * t + lane) * BN + owner;
+      if (32 * t + lane < rows) *at = lost >> t & 1u ? v[t] : *at + v[t];
+    }
+  }
 }
 
 template <int FMT, int CPT>
@@ -446,7 +582,7 @@ mx_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
             if (c + kLd >= hc) {   // the last values are in registers: the buffer goes back
               dev::tc_fence_before();
               __syncwarp();
-              if (lane == 0) dev::mbar_arrive(&dempty[buf]);
+              if (lane == 0 && (!C::kE8m0 || u < units - 1)) dev::mbar_arrive(&dempty[buf]);
             }
 #pragma unroll
             for (int e = 0; e < kLd / 2; ++e)
@@ -456,10 +592,15 @@ mx_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         if (++buf == C::kAccBufs) { buf = 0; bpar ^= 1; }
       }
       if (!ok) break;
-      bool marked = false;
-      if (C::kE8m0) {
+      // The last accumulator goes back when it is clear that no column misses groups; else it takes the tile's sums.
+      [[maybe_unused]] uint32_t marked = 0u;
+      [[maybe_unused]] const uint32_t last = buf == 0 ? C::kAccBufs - 1 : buf - 1;
+      if constexpr (C::kE8m0) {
         if (!dev::mbar_wait_warp(&info[tile_no % kInfo], (tile_no / kInfo) & 1, a.status, 122)) { ok = false; break; }
-        marked = marks[(tile_no % kInfo) * BN + q * 32 + lane] == tile_no + 1;
+        marked = __ballot_sync(0xFFFFFFFFu, marks[(tile_no % kInfo) * BN + q * 32 + lane] == tile_no + 1);
+        if (marked == 0u) {
+          if (lane == 0) dev::mbar_arrive(&dempty[last]);
+        }
       }
       if (KS > 1) break;   // one tile per cluster: it is put together below
       // ---- results: two rows at a time, neighbouring lanes exchange so that each stores two columns of one row
@@ -482,12 +623,33 @@ mx_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
           }
         }
       }
-      if (C::kE8m0) {
-        __syncwarp();   // a neighbour has stored half of the column
-        if (marked && n < a.N) {
-#pragma unroll 1
-          for (int m = m0 + c0; m < min(a.M, m0 + c0 + hc); ++m)
-            y[static_cast<size_t>(m) * a.N + n] = __float2half_rn(exact_dot<FMT, false>(a.x, a.w, a.scales, nullptr, a.K, 32, m, n, 0, a.K));
+      if constexpr (C::kE8m0) {
+        if (marked != 0u) {
+#pragma unroll
+          for (int c = 0; c < CPT; c += 8) {
+            if (c < hc) {
+              uint32_t r[8];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                float v0, v1;
+                unpack2(acc[c / 2 + i], v0, v1);
+                r[2 * i] = __float_as_uint(v0);
+                r[2 * i + 1] = __float_as_uint(v1);
+              }
+              dev::tmem_st_32x8(d_lane + last * C::kRows + c, r);
+            }
+          }
+          dev::tc_wait_st();
+          __syncwarp();   // a neighbour has stored half of the column
+          add_small_groups<FMT, CPT / 32>(static_cast<const __half*>(a.x), a.w, static_cast<const uint8_t*>(a.scales), y, a.M, a.N, a.K,
+                                          d_lane + last * C::kRows, marked, (t / a.mt) * BN + q * 32, m0 + c0, hc);
+          dev::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) dev::mbar_arrive(&dempty[last]);
+          // not live across the call, around which they would be spilled (40 to 470 bytes, in the loop too: 4096 x 28672, M = 100
+          // 46.8 us without any such column, 41.8 so)
+#pragma unroll
+          for (int i = 0; i < CPT / 2; ++i) acc[i] = 0ull;
         }
       }
     }
@@ -495,19 +657,24 @@ mx_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
     __syncthreads();   // every warp is done with the rings and with TMEM
     if (KS == 1) return;
     // ---- this slice's results, [row][column], into the idle rings; the cluster's CTAs add up a share of the rows each
-    const bool marked = C::kE8m0 && ok && marks[q * 32 + lane] == 1u;
 #pragma unroll
     for (int i = 0; i < CPT / 2; ++i) {
       if (2 * i < hc) {
         float v0, v1;
         unpack2(acc[i], v0, v1);
-        if (marked) v0 = v1 = __uint_as_float(kMarked);
         tile_out[(c0 + 2 * i) * BN + q * 32 + lane] = v0;
         tile_out[(c0 + 2 * i + 1) * BN + q * 32 + lane] = v1;
       }
     }
-    split::cluster_sync();
     const int m0 = (blockIdx.y % a.mt) * a.bm, n0 = (blockIdx.y / a.mt) * BN;
+    if constexpr (C::kE8m0) {
+      const uint32_t marked = __ballot_sync(0xFFFFFFFFu, ok && marks[q * 32 + lane] == 1u);
+      __syncwarp();
+      if (marked != 0u)
+        add_small_groups<FMT, CPT / 32>(static_cast<const __half*>(a.x), a.w, static_cast<const uint8_t*>(a.scales), tile_out + c0 * BN + q * 32,
+                                        a.M, a.K, marked, n0 + q * 32, m0 + c0, hc, k_begin, k_end);
+    }
+    split::cluster_sync();
     const int rows = min(a.bm, a.M - m0);
     const bool pairs = (a.N & 1) == 0;
     constexpr int kAdders = kThreads - kFirstPromoter * 32;
@@ -515,19 +682,10 @@ mx_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
       const int m = e / (BN / 2), c = (e % (BN / 2)) * 2, n = n0 + c;
       if (n >= a.N) continue;
       float2 v = make_float2(0.f, 0.f);
-      bool redo_x = false, redo_y = false;
       for (int r = 0; r < KS; ++r) {
         const float2 p = split::load_peer(reinterpret_cast<const float2*>(tile_out + m * BN + c), r);
-        if (C::kE8m0) {
-          redo_x |= __float_as_uint(p.x) == kMarked;
-          redo_y |= __float_as_uint(p.y) == kMarked;
-        }
         v.x += p.x;
         v.y += p.y;
-      }
-      if (C::kE8m0) {
-        if (redo_x) v.x = exact_dot<FMT, false>(a.x, a.w, a.scales, nullptr, a.K, 32, m0 + m, n, 0, a.K);
-        if (redo_y && n + 1 < a.N) v.y = exact_dot<FMT, false>(a.x, a.w, a.scales, nullptr, a.K, 32, m0 + m, n + 1, 0, a.K);
       }
       __half* y = static_cast<__half*>(a.y) + static_cast<size_t>(m0 + m) * a.N + n;
       if (pairs) *reinterpret_cast<__half2*>(y) = __floats2half2_rn(v.x, v.y);
