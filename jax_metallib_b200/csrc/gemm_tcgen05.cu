@@ -404,6 +404,13 @@ constexpr int kSlotCols = 2 * BK / 2;             // TMEM columns of a converted
 constexpr int kAccBase = kCvtSlots * kSlotCols;   // first TMEM column of the accumulators
 static_assert(kAccBase + 2 * kMaxRows <= 512, "TMEM");
 static_assert(kWStages % kCvtGroups == 0, "a group has seen the phase ahead of the one that it waits for");
+// Tiles of up to 96 rows leave accumulators unused: with int8 weights, K goes into two to six of them one after the other, and the
+// epilogue adds them up in f32, rounded.  The tensor core cuts off what it adds to an accumulator, and a long K in one shows.  Outputs
+// that a rounding to bf16 puts elsewhere than it puts the sum in 64 bits, M = 32: 4.0e-4 -> 2.1e-4 for 8192 x 8192, 6.7e-4 -> 3.1e-4 for
+// 14336 x 4096, 2.1e-3 -> 2.9e-4 for 28672 x 8192 (the kernel for few rows: 2.4e-4, 1.5e-4, 9.5e-4).  It costs 1 to 3 % (8192 x 8192,
+// M = 32 22.1 -> 22.5 us, M = 64 23.5 -> 24.1), 4 % where few rows meet many columns (8192 x 57344 118.1 -> 123.3).  int4 weights, which
+// come here from 33 rows on and are rounded themselves, keep one.
+constexpr int kLeastPart = 16;   // stages that are worth an accumulator
 constexpr int kPanelTiles = 8;  // most activation tiles swept together (fewer when K is long: a panel should stay in L2)
 // One "consumed" barrier per stage in a ring: the activation producer waits for stage cnt - 4, the converters for
 // stage cnt - 2, and the issuing threads commit once per stage.
@@ -523,7 +530,8 @@ __device__ __forceinline__ uint32_t dequant2(uint32_t w, uint32_t w4, uint32_t z
 //            bf16 scale and zero point applied by the converter warps; K % 128 == 0.
 // SPLIT: a piece of work is one cluster's; its CTAs take a share of K each and add their accumulators up over distributed
 // shared memory, in CTA order.  One piece a cluster, so that the rings are free for the sums when the last MMA has retired.
-template <int WBITS, bool SPLIT>
+// PARTS: K in several accumulators.
+template <int WBITS, bool SPLIT, bool PARTS>
 __global__ void __launch_bounds__(kThreads, 1)
 w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
              const float* __restrict__ scale, const GroupQuant gq, uint16_t* __restrict__ y, int M, int N, int K,
@@ -552,6 +560,8 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
   const int all_kblocks = (K + BK - 1) / BK;
   const int kb_begin = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * blockIdx.x / gridDim.x) : 0;
   const int kb_end = SPLIT ? static_cast<int>(static_cast<long long>(all_kblocks) * (blockIdx.x + 1) / gridDim.x) : all_kblocks;
+  // stages that go into one accumulator
+  const int spare = PARTS ? kMaxRows / sc.rows : 1, part = PARTS ? max((kb_end - kb_begin + spare - 1) / spare, kLeastPart) : kb_end - kb_begin;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kXStages; ++s) dev::mbar_init(&xfull[s], 1);
@@ -650,23 +660,31 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         const uint32_t idesc = (w.m_cols == sc.rows) ? idesc_full : idesc_half;
         const uint32_t b_item = b_lo0 + ((w.m_off * 128) >> 4);
         const uint32_t mine = (me >= w.h0) && (me < w.h0 + w.nh);
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          // whether the next stage is ready is asked while this one's MMAs are still being issued: behind them a question
-          // waits for its turn
-          if (!ready && !dev::mbar_wait(&sfull[g], gpar, status, 23)) { ok = false; break; }
-          dev::tc_fence_after();
-          const uint32_t a_c = a_t0 + g * kSlotCols;   // 16 k: eight columns
-          const uint32_t b_s = b_item + xs * kBStepStage;
-          dev::umma_f16_ts_if(mine, d, a_c, b_s, kDescHi, idesc, kb != kb_begin);
-          dev::umma_f16_ts_if(mine, d, a_c + 8, b_s + kBStepK, kDescHi, idesc, 1);
-          dev::umma_f16_ts_if(mine, d, a_c + 16, b_s + 2 * kBStepK, kDescHi, idesc, 1);
-          ready = dev::mbar_test(&sfull[g ^ 1], gpar ^ g);
-          dev::umma_f16_ts_if(mine, d, a_c + 24, b_s + 3 * kBStepK, kDescHi, idesc, 1);
-          dev::tc_commit(&consumed[c6]);  // second arrival: the other issuer
-          gpar ^= g;  // the parity flips after slot 1's stage
-          g ^= 1;
-          xs = (xs == kXStages - 1) ? 0 : xs + 1;
-          c6 = (c6 == kConsumed - 1) ? 0 : c6 + 1;
+        auto multiply = [&](uint32_t d, int begin, int end) {
+          for (int kb = begin; kb < end; ++kb) {
+            // whether the next stage is ready is asked while this one's MMAs are still being issued: behind them a question
+            // waits for its turn
+            if (!ready && !dev::mbar_wait(&sfull[g], gpar, status, 23)) { ok = false; break; }
+            dev::tc_fence_after();
+            const uint32_t a_c = a_t0 + g * kSlotCols;   // 16 k: eight columns
+            const uint32_t b_s = b_item + xs * kBStepStage;
+            dev::umma_f16_ts_if(mine, d, a_c, b_s, kDescHi, idesc, kb != begin);
+            dev::umma_f16_ts_if(mine, d, a_c + 8, b_s + kBStepK, kDescHi, idesc, 1);
+            dev::umma_f16_ts_if(mine, d, a_c + 16, b_s + 2 * kBStepK, kDescHi, idesc, 1);
+            ready = dev::mbar_test(&sfull[g ^ 1], gpar ^ g);
+            dev::umma_f16_ts_if(mine, d, a_c + 24, b_s + 3 * kBStepK, kDescHi, idesc, 1);
+            dev::tc_commit(&consumed[c6]);  // second arrival: the other issuer
+            gpar ^= g;  // the parity flips after slot 1's stage
+            g ^= 1;
+            xs = (xs == kXStages - 1) ? 0 : xs + 1;
+            c6 = (c6 == kConsumed - 1) ? 0 : c6 + 1;
+          }
+        };
+        if (PARTS) {
+          uint32_t d_part = d;
+          for (int kb = kb_begin; ok && kb < kb_end; kb += part, d_part += sc.rows) multiply(d_part, kb, min(kb + part, kb_end));
+        } else {
+          multiply(d, kb_begin, kb_end);
         }
         if (ok) dev::tc_commit(tfull);
         ++items;
@@ -792,8 +810,22 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         const int n = (w.tn2 * 2 + h) * BNW + q * 32 + (lane & 16) + 2 * (lane & 7) + ((lane >> 3) & 1);
         const float scl = (WBITS == 4) ? 1.f : ((n < N) ? __ldg(scale + n) : 0.f);
         uint32_t r[32];
-        dev::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + kAccBase + h * kMaxRows + ch * 32, r);
+        const uint32_t at = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + kAccBase + h * kMaxRows + ch * 32;
+        dev::tmem_ld_32x32(at, r);
         dev::tc_wait_ld();
+        if (PARTS) {
+#pragma unroll 1
+          for (int k = part, p = sc.rows; k < kb_end - kb_begin; k += part, p += sc.rows) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 8) {   // (16 at a time spill)
+              uint32_t more[8];
+              dev::tmem_ld_32x8(at + p + e, more);
+              dev::tc_wait_ld();
+#pragma unroll
+              for (int j = 0; j < 8; ++j) r[e + j] = __float_as_uint(__uint_as_float(r[e + j]) + __uint_as_float(more[j]));
+            }
+          }
+        }
         if (SPLIT) {   // the sums of this CTA's share of K, [row][channel], over the rings
           float* mine = reinterpret_cast<float*>(smem) + (h - w.h0) * BNW + (n & (BNW - 1));
 #pragma unroll
@@ -1060,16 +1092,18 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
   using namespace tc::w8;
   const int sms = gemm_ctas();  // persistent CTAs of a launch
   static std::atomic<int> resident[kMaxDevices][split::kMaxCluster + 1];
-  static std::atomic<uint64_t> configured[2] = {};  // per device (one mask per instance of the kernel)
-  auto kern = w8a16_kernel<WBITS, false>;
-  auto split_kern = w8a16_kernel<WBITS, true>;
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes, configured[0])) return rc;
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(split_kern), kSmemBytes, configured[1])) return rc;
+  static std::atomic<uint64_t> configured[4] = {};  // per device (one mask per instance of the kernel)
+  decltype(&w8a16_kernel<WBITS, false, false>) kerns[2] = {w8a16_kernel<WBITS, false, false>, w8a16_kernel<WBITS, false, WBITS == 8>};
+  decltype(&w8a16_kernel<WBITS, false, false>) split_kerns[2] = {w8a16_kernel<WBITS, true, false>, w8a16_kernel<WBITS, true, WBITS == 8>};
+  for (int i = 0; i < 2; ++i) {
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kerns[i]), kSmemBytes, configured[i])) return rc;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(split_kerns[i]), kSmemBytes, configured[2 + i])) return rc;
+  }
   // results that go to several GPUs or are announced, and callers with a limit on the CTAs, keep one CTA to a piece
   const bool may_split = sms == num_sms() && !(flags & QMM_GEMM_STORE_MULTIMEM) && signal == nullptr;
   auto plan = [&](int64_t rows) {
     return schedule(rows, N, K, WBITS, sms, [&](int ks) {
-      return may_split ? split::resident_clusters(split_kern, kThreads, kSmemBytes, 1, ks, resident) : 0;
+      return may_split ? split::resident_clusters(split_kerns[0], kThreads, kSmemBytes, 1, ks, resident) : 0;
     });
   };
   Sched sc = plan(M), rest = {};
@@ -1107,6 +1141,7 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
     // operand "a" of the MMA = weights (bf16, from TMEM), "b" = activations (bf16, K-major)
     const uint32_t idesc_full = dev::make_idesc(/*c=f32*/ 1, /*bf16*/ 1, /*bf16*/ 1, 0, /*b K-major*/ 0, BNW, sc.rows);
     const uint32_t idesc_half = dev::make_idesc(1, 1, 1, 0, 0, BNW, sc.rows / 2);
+    const bool parts = WBITS == 8 && 2 * sc.rows <= kMaxRows && (K + BK - 1) / BK > static_cast<int64_t>(kLeastPart) * sc.ks;
     if (sc.ks > 1) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute attr[2];
@@ -1115,7 +1150,7 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
       cfg.dynamicSmemBytes = kSmemBytes;
       cfg.stream = stream;
       split::set_attrs(cfg, attr, sc.ks);
-      QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kern, wmap, xmap, scale, gq, out, (int)rows, (int)N, (int)K, (long long)ldy, idesc_full,
+      QMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kerns[parts], wmap, xmap, scale, gq, out, (int)rows, (int)N, (int)K, (long long)ldy, idesc_full,
                                       idesc_half, sc, flags, signal, arrive, device_status_word()));
       return QMM_OK;
     }
@@ -1124,7 +1159,7 @@ static int launch_weight_only(const uint16_t* x, const void* w, const float* sca
     // kernel ahead of it drains; they order themselves behind it inside the kernel (or not at all
     // when the caller states independence, which fills the last, partly idle round of one launch
     // with the first tiles of the next).
-    QMM_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, wmap, xmap, scale, gq, out, (int)rows,
+    QMM_CUDA_TRY(launch_pdl(kerns[parts], dim3(grid), dim3(kThreads), kSmemBytes, stream, wmap, xmap, scale, gq, out, (int)rows,
                             (int)N, (int)K, (long long)ldy, idesc_full, idesc_half, sc, flags, signal, arrive,
                             device_status_word()));
     return QMM_OK;
