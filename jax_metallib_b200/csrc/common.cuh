@@ -279,21 +279,9 @@ __device__ __forceinline__ uint64_t policy_evict_first() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ uint64_t policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
 // 2-D tile store, this CTA's shared memory -> global, tracked by the issuing thread's bulk group.  Parts of the
-// box outside the tensor are not written.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* smem_src, int32_t c0, int32_t c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(m)),
-               "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
-               : "memory");
-}
-// The same with an L2 eviction-priority hint (createpolicy value): results that nothing reads back soon should
-// not push the operands of the next launch out of L2.
+// box outside the tensor are not written.  The L2 eviction-priority hint is a createpolicy value: results that nothing reads
+// back soon should not push the operands of the next launch out of L2.
 __device__ __forceinline__ void tma_store_2d_hint(const CUtensorMap* m, const void* smem_src, int32_t c0, int32_t c1,
                                                   uint64_t policy) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;" ::"l"(
@@ -326,14 +314,6 @@ __device__ __forceinline__ void multimem_red_release_add_u32(uint32_t* mc_addr, 
 }
 __device__ __forceinline__ void red_release_sys_add_u32(uint32_t* addr, uint32_t v) {
   asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* addr) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_gpu_u32(uint32_t* addr, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ uint32_t ld_acquire_sys_u32(const uint32_t* addr) {
   uint32_t v;
@@ -371,30 +351,12 @@ __device__ __forceinline__ void tc_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                        uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same MMAs with each descriptor given as its two 32-bit halves.  The start
-// address (in 16-byte units) is the low 14 bits of the low half, so a descriptor
-// is advanced with one 32-bit add.  The thread that issues the MMAs is the
-// serial resource of a tcgen05 kernel: a tcgen05.mma costs it about 110 cycles
-// and whatever it executes between two MMAs is added to that, so descriptors are
-// never rebuilt inside the issue loop.
+// D[tmem] (+)= A[smem desc] * B[smem desc], each shared-memory matrix descriptor (sm_100 format) given as its two 32-bit
+// halves.  Low: start address and leading byte offset in 16-byte units, at bits 0 and 16.  High: stride byte offset in 16-byte
+// units, descriptor version 1 at bit 14, swizzle mode at bit 29 (0 none, 2 = 128B, 4 = 64B, 6 = 32B).  A descriptor is
+// advanced with one 32-bit add: the thread that issues the MMAs is the serial resource of a tcgen05 kernel, a tcgen05.mma
+// costs it about 110 cycles and whatever it executes between two MMAs is added to that, so descriptors are never rebuilt
+// inside the issue loop.
 __device__ __forceinline__ void umma_f16_lh(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
                                             uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -404,26 +366,7 @@ __device__ __forceinline__ void umma_f16_lh(uint32_t d_tmem, uint32_t a_lo, uint
       "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The same, issued only when `enable` is non-zero (a predicated instruction, no branch).
-__device__ __forceinline__ void umma_f16_lh_if(uint32_t enable, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
-                                               uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
-      "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(enable)
-      : "memory");
-}
-__device__ __forceinline__ void umma_i8_lh(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
-                                           uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\t"
-      "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
+// 8-bit integers; issued only when `enable` is non-zero (a predicated instruction, no branch)
 __device__ __forceinline__ void umma_i8_lh_if(uint32_t enable, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
                                               uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -454,20 +397,6 @@ __device__ __forceinline__ void umma_f16_ts_if(uint32_t enable, uint32_t d_tmem,
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
       "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(enable)
       : "memory");
-}
-
-// Shared-memory matrix descriptor (sm_100 format): start address, leading and
-// stride byte offsets in 16-byte units, descriptor version 1, swizzle mode in
-// bits 61..63 (0 none, 2 = 128B, 4 = 64B, 6 = 32B).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes,
-                                                   uint32_t sbo_bytes, uint32_t layout_type) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFF);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= static_cast<uint64_t>(1) << 46;  // descriptor version for sm_100
-  d |= static_cast<uint64_t>(layout_type & 7) << 61;
-  return d;
 }
 
 // Instruction descriptor for kind::f16 / kind::i8 (dense, no negate, no saturate).

@@ -425,12 +425,6 @@ __device__ __forceinline__ uint32_t convert2(uint32_t word, uint32_t selector) {
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(__byte_perm(word, 0u, selector)), "r"(0x7F007F00u), "r"(0xC000C000u));
   return r;
 }
-// 8 x 8 tiles of 16-bit units, transposed: a unit is one k (or one packed pair of k) of two neighbouring channels.
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
 
 // The work of one launch.  A full tile is 256 channels x `rows` rows: two channel
 // blocks share one activation tile, so a CTA stages up to 40 KB per 64 k for
@@ -740,7 +734,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
           const uint32_t at = raw + (((q * 2 + c) ^ (lane & 7)) << 4);
           if (WBITS == 4) {
             uint32_t in[4];
-            ldmatrix_x4_trans(at, in);
+            split::ldmatrix_x4_trans(at, in);
             const uint32_t s0 = __byte_perm(sv[c], 0u, 0x1010), s1 = __byte_perm(sv[c], 0u, 0x3232);
             // the two zero points: nibbles of a byte, or two bytes
             const uint32_t z0 = 0x43004300u | (gq.packed ? (zv[c] & 0xFu) * 0x10001u : __byte_perm(zv[c], 0u, 0x4040));
@@ -757,7 +751,7 @@ w8a16_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
               uint32_t in[4];
-              ldmatrix_x4_trans(at + g * 32 * 128, in);
+              split::ldmatrix_x4_trans(at + g * 32 * 128, in);
 #pragma unroll
               for (int m = 0; m < 4; ++m) {
                 const uint32_t u = in[m] ^ 0x80808080u;

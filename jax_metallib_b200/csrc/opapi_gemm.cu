@@ -51,7 +51,7 @@ template <int FMT, bool XF32, int BM>
 struct Cfg {
   static constexpr int kBits = (FMT == kAffine8 || FMT == kMxfp8) ? 8 : 4;
   static constexpr bool kBias = FMT == kAffine4 || FMT == kAffine8;
-  static constexpr bool kUnitInfo = kBias || XF32;          // sums and / or flags travel with a unit
+  static_assert(kBias || XF32, "MX formats with f16 activations: mx_prefill.cu");   // sums and / or flags travel with a unit
   static constexpr int kTerms = XF32 ? 3 : 1;
   static constexpr int kBoxK = 128 * 8 / kBits;             // k per raw box
   static constexpr int kStagesPerBox = kBoxK / BK;          // 4 or 2
@@ -366,7 +366,7 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
       const int xs = st % C::kXRing;
       if (!dev::mbar_wait_relaxed_warp(&xfull[xs], (st / C::kXRing) & 1, a.status, 98)) break;
       const int slot = (units_per_stage * st) % kInfo;   // first unit of this stage (a unit with sums is at most a stage)
-      if (C::kUnitInfo) {
+      {
         const uint8_t* xt = smem + C::kOffX + xs * C::kXBytes;
         uint32_t bad = 0;   // bit 0: first half of the stage, bit 1: second half
         auto rows16 = [&](int i) {
@@ -464,10 +464,8 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         dev::mbar_arrive(&wempty[rs]);
         if (XF32) dev::mbar_arrive(&xempty[xs]);
         dev::mbar_arrive(&full[op]);
-        if (C::kUnitInfo) {
-          dev::mbar_arrive(&ifull[slot]);
-          if (units_per_stage == 2) dev::mbar_arrive(&ifull[(slot + 1) % kInfo]);
-        }
+        dev::mbar_arrive(&ifull[slot]);
+        if (units_per_stage == 2) dev::mbar_arrive(&ifull[(slot + 1) % kInfo]);
       }
     }
   } else {
@@ -521,17 +519,14 @@ opgemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         if (centred<FMT>(s, b, shifted)) b = shifted;
       }
       if (FMT == kAffine8 && XF32) s *= 64.f;
-      bool exact = false;
-      if (C::kUnitInfo) {
-        if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) break;
-        exact = *reinterpret_cast<const uint32_t*>(flags + slot * kGroupWarps) != 0u;
-      }
+      if (!dev::mbar_wait_relaxed_warp(&ifull[slot], (u / kInfo) & 1, a.status, 99)) break;
+      const bool exact = *reinterpret_cast<const uint32_t*>(flags + slot * kGroupWarps) != 0u;
       // the units of a stage complete together, on the barrier of its last buffer
       const int last = units_per_stage == 2 ? (u | 1) & (C::kAccBufs - 1) : buf;
       if (!dev::mbar_wait_relaxed_warp(&tfull[last], phase, a.status, 100)) break;
       dev::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BM + c0;
-      if (C::kUnitInfo && exact) {
+      if (exact) {
         // the unit's exact sums take the accumulator's place (registers cannot be indexed)
         const int k0 = k_begin + u * a.pu, k1 = min(a.K, k0 + a.pu);
 #pragma unroll 1
@@ -756,15 +751,15 @@ static int launch(Args a, cudaStream_t stream) {
 }
 
 template <int FMT>
-static int launch_fmt(const Args& a, int f32, cudaStream_t stream) {
-  if (f32) {
-    // a stage of 128 rows would need 64 KB for the three terms of the activations alone
-    return a.M <= 32 ? launch<FMT, true, 32>(a, stream) : launch<FMT, true, 64>(a, stream);
-  }
-  if constexpr (FMT <= kAffine8)
-    return a.M <= 32 ? launch<FMT, false, 32>(a, stream)
-                     : (a.M <= 64 ? launch<FMT, false, 64>(a, stream) : launch<FMT, false, 128>(a, stream));
-  return set_error(QMM_ERR_UNSUPPORTED, "opgemm: MX formats take f32 activations here");
+static int launch_f32(const Args& a, cudaStream_t stream) {
+  // a stage of 128 rows would need 64 KB for the three terms of the activations alone
+  return a.M <= 32 ? launch<FMT, true, 32>(a, stream) : launch<FMT, true, 64>(a, stream);
+}
+template <int FMT>
+static int launch_affine(const Args& a, int f32, cudaStream_t stream) {
+  if (f32) return launch_f32<FMT>(a, stream);
+  return a.M <= 32 ? launch<FMT, false, 32>(a, stream)
+                   : (a.M <= 64 ? launch<FMT, false, 64>(a, stream) : launch<FMT, false, 128>(a, stream));
 }
 
 // Microseconds of a call, here and on the CUDA cores (one B200, calls of a graph on operands in L2; K and N from 64 to 4096,
@@ -775,17 +770,18 @@ static float gemm_us(int fmt, bool f32, int M, int N, int K, int gs) {
   const int bm = M <= 32 ? 32 : (M <= 64 || f32 ? 64 : 128);
   const int i = bm == 32 ? 0 : (bm == 64 ? 1 : 2);
   static constexpr float kStart[3] = {4.2f, 5.5f, 7.5f};
-  // us per stage of 64 k: f16 activations at 32, 64 and 128 rows, f32 at 32 and 64
-  static constexpr float kStage[4][5] = {{1.33f, 1.71f, 3.5f, 1.48f, 1.84f},   // affine, units of 32 k
-                                         {0.91f, 1.12f, 2.0f, 1.12f, 1.32f},   // affine, 64 k
-                                         {0.72f, 0.77f, 1.02f, 1.11f, 1.26f},  // mxfp4, mxfp8
-                                         {0.59f, 0.57f, 0.55f, 0.92f, 1.01f}}; // nvfp4
+  // us per stage of 64 k, at 32, 64 and (f16) 128 rows
+  static constexpr float kStageF16[2][3] = {{1.33f, 1.71f, 3.5f},    // affine, units of 32 k
+                                            {0.91f, 1.12f, 2.0f}};   // affine, 64 k
+  static constexpr float kStageF32[4][2] = {{1.48f, 1.84f}, {1.12f, 1.32f},
+                                            {1.11f, 1.26f},    // mxfp4, mxfp8
+                                            {0.92f, 1.01f}};   // nvfp4
   const Slicing cut = slicing(fmt, K, gs, true);
   const int kind = fmt == kNvfp4 ? 3 : (fmt > kAffine8 ? 2 : (cut.pu == 64 ? 1 : 0));
   const int sms = num_sms();
   const Rounds r = choose_rounds(((N + BN - 1) / BN) * ((M + bm - 1) / bm), cut.blocks, (K + BK - 1) / BK,
                                  [&](int ks) { return sms / ks > 0 ? sms / ks : 1; });
-  return r.rounds * (kStart[i] + kStage[kind][f32 ? 3 + i : i] * r.stages);
+  return r.rounds * (kStart[i] + (f32 ? kStageF32[kind][i] : kStageF16[kind][i]) * r.stages);
 }
 float cuda_core_us(int fmt, bool f32, int M, int N, int K) {
   const bool wide = fmt == kAffine8 || fmt == kMxfp8;   // 8-bit codes take fewer instructions
@@ -804,7 +800,7 @@ float cuda_core_us(int fmt, bool f32, int M, int N, int K) {
 // so do up to three rows, which the estimates do not cover (affine4, f32, 4096 x 8192: 30 us at one row, 62 at four, here
 // 32 for any of them).
 // QMM_FORCE_SPLIT_K=1 brings every call here that the kernel can take (a cross-check; read once per process).
-// fmt: 0 affine 4-bit, 1 affine 8-bit, 2 mxfp4, 3 mxfp8, 4 nvfp4.  K and the group a multiple of 32 (nvfp4: K), weights
+// fmt: 0 affine 4-bit, 1 affine 8-bit, and for f32 activations 2 mxfp4, 3 mxfp8, 4 nvfp4.  K and the group a multiple of 32 (nvfp4: K), weights
 // and activations 16-byte aligned, results aligned for pairs.
 bool opgemm_covers(int64_t M, int64_t N, int64_t K, int fmt, int64_t gs, int f32, const void* x, const void* w, const void* y) {
   using namespace opg;
@@ -833,11 +829,11 @@ int opgemm_launch(int fmt, const void* x, const void* w, const void* scales, con
   a.gs = static_cast<int>(gs);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (fmt) {
-    case kAffine4: return launch_fmt<kAffine4>(a, f32, st);
-    case kAffine8: return launch_fmt<kAffine8>(a, f32, st);
-    case kMxfp4: return launch_fmt<kMxfp4>(a, f32, st);
-    case kMxfp8: return launch_fmt<kMxfp8>(a, f32, st);
-    default: return launch_fmt<kNvfp4>(a, f32, st);
+    case kAffine4: return launch_affine<kAffine4>(a, f32, st);
+    case kAffine8: return launch_affine<kAffine8>(a, f32, st);
+    case kMxfp4: return launch_f32<kMxfp4>(a, st);
+    case kMxfp8: return launch_f32<kMxfp8>(a, st);
+    default: return launch_f32<kNvfp4>(a, st);
   }
 }
 
