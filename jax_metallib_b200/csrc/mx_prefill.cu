@@ -17,8 +17,8 @@
 // Measured (mxfp8, f16, M = 512; before: a scale group of 32 k per accumulator, both operands in shared memory): four linears
 // of 4096 / 14336 wide 857 -> 296 us; 4096 x 28672 462 -> 122 us, 0.60 of the measured bf16 rate; M = 17, 14336 x 4096 36.9 ->
 // 17.8 us.  Bound by the converters where rows are few (a stage of 128 k takes 0.47 us, their instructions half of it); at 192 rows
-// MMAs are 0.40 of a stage's 0.65 us at 1.9 GHz.  Groups below the range, mxfp8, M = 512, 14336 x 4096 (none: 65 us): one in every
-// 128th column 69 us, in every 16th 73, in every column 162; 4096 x 28672 (119 us): 155, 178, 724.
+// MMAs are 0.40 of a stage's 0.65 us at 1.9 GHz.  Groups below the range, mxfp8, M = 512, 14336 x 4096 (none: 63 us): one in every
+// 128th column 68 us, in every 16th 71, in every column 157; 4096 x 28672 (122 us): 156, 178, 764.
 //
 // Persistent CTAs, one per SM.  Warps: TMA of activations, TMA of raw weights, the MMA issuer; two warpgroups of
 // converters that take the 128-k stages in turn; two warpgroups of promoters, a thread of which holds up to 96 rows of a
@@ -592,7 +592,8 @@ mx_prefill_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
         if (++buf == C::kAccBufs) { buf = 0; bpar ^= 1; }
       }
       if (!ok) break;
-      // The last accumulator goes back when it is clear that no column misses groups; else it takes the tile's sums.
+      // The last accumulator goes back when it is clear that no column misses groups; else it takes the tile's sums, behind the
+      // stores (before them: M = 384, 4096 x 28672 7 % slower without such columns).
       [[maybe_unused]] uint32_t marked = 0u;
       [[maybe_unused]] const uint32_t last = buf == 0 ? C::kAccBufs - 1 : buf - 1;
       if constexpr (C::kE8m0) {
